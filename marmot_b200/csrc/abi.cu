@@ -4,6 +4,7 @@
 #include "../../include/marmot_cuda.h"
 
 #include "common.cuh"
+#include "gemm_ts.h"
 #include "kernels.h"
 #include "moe.h"
 
@@ -481,7 +482,7 @@ static int validate_linear(int kind, const void *x, const void *w, const void *o
 
 // Quantize the activations into the context workspace.
 static int pack_activations(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, bool want_half,
-                            int k_order, ActBuffers &ab) {
+                            ActBuffers &ab) {
     const size_t bv = (size_t)block_values(kind);
     const size_t nb = (K + bv - 1) / bv, kp = nb * bv;
     if (int rc = ensure(ctx, ctx->act_qs, T * kp)) return rc;
@@ -498,7 +499,7 @@ static int pack_activations(mcu_context *ctx, int kind, const float *x, size_t l
     MCU_CUDA(launch_quantize_act(kind, x, (int)ldx, (int)T, (int)K, ab, nullptr, ctx->stream));
     count_launches(1);
     if (want_half) {
-        MCU_CUDA(launch_half_acts(kind, ab, (int)T, (int)K, k_order, (__half *)ctx->act_half.ptr,
+        MCU_CUDA(launch_half_acts(kind, ab, (int)T, (int)K, (__half *)ctx->act_half.ptr,
                                   (float *)ctx->act_rowscale.ptr, ctx->stream));
         count_launches(1);
     }
@@ -517,60 +518,41 @@ static void *mapped_host_pointer(const void *host) {
 }
 
 // What the last staging launch of a multi-matmul call left in the context's fp16 activation buffer: a later matmul
-// of the same call that wants the same block format class and K order reuses it.
+// of the same call that wants the same block format class reuses it.
 struct Staged {
     bool valid = false, kq = false;
-    int k_order = -1;
 };
 
-// The tensor-core matmuls (gemm_tc_supported shapes): stage the activations as fp16 (through `src` when the caller
-// folds a gather, GLU or add + RMSNorm into the staging; needs the one-kernel staging), then the GEMM that suits the
-// weights.  ctx->mu is held by the caller.
-static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, const void *w, const void *w2, size_t T, size_t K,
-                       size_t F, const float *bias, float *out, float *out2, size_t ldo, const ActSource *src, Staged *st) {
-    const bool tma = gemm_tma_supported(kind, w, w2, (int)T, (int)K, (int)F);
-    const bool warp_mma = gemm_warp_supported(kind, w, w2, (int)T, (int)K, (int)F);
-    const int k_order = warp_mma ? ACT_ORDER_FRAG16 : tma ? ACT_ORDER_QUAD : ACT_ORDER_NATURAL;
+// The tensor-core matmuls: stage the activations as fp16 (through `src` when the caller folds a gather, GLU or add + RMSNorm
+// into the staging; needs the one-kernel staging), then one launch for all `jobs`, which are of one kind.  ctx->mu is held by
+// the caller.
+static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, const GemvJobSpec *jobs, int n_jobs,
+                       const ActSource *src, Staged *st) {
     const bool kq = kind != MCU_KIND_Q8_0;
     const size_t bv = (size_t)block_values(kind);
     const size_t kp = (K + bv - 1) / bv * bv;
-    if (st != nullptr && st->valid && st->kq == kq && st->k_order == k_order) {
+    if (st != nullptr && st->valid && st->kq == kq) {
         // staged by an earlier matmul of this call
     } else if (act_half_fused_smem(kind, (int)K) <= 48 * 1024) {
         if (int rc = ensure(ctx, ctx->act_half, T * kp * sizeof(__half))) return rc;
         if (int rc = ensure(ctx, ctx->act_rowscale, T * sizeof(float))) return rc;
-        MCU_CUDA(launch_act_half_fused_from(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K, k_order,
+        MCU_CUDA(launch_act_half_fused_from(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K,
                                             (__half *)ctx->act_half.ptr, (float *)ctx->act_rowscale.ptr, ctx->stream));
         count_launches(1);
         if (st != nullptr) {
             st->valid = true;
             st->kq = kq;
-            st->k_order = k_order;
         }
     } else {
         if (src != nullptr) return fail(MCU_ERROR_NOT_IMPLEMENTED, "rows too long for the one-kernel activation staging");
         ActBuffers ab;
-        if (int rc = pack_activations(ctx, kind, x, ldx, T, K, true, k_order, ab)) return rc;
+        if (int rc = pack_activations(ctx, kind, x, ldx, T, K, true, ab)) return rc;
         if (st != nullptr) st->valid = false;
     }
-    int launches = 0;
-    if (warp_mma) {
-        if (int rc = ensure(ctx, ctx->gemm_partial, gemm_warp_workspace_bytes(kind, (int)T, (int)K, (int)F, w2 != nullptr)))
-            return rc;
-        MCU_CUDA(launch_gemm_warp(kind, w, w2, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr,
-                                  (int)kp, (int)T, (int)K, (int)F, bias, out, out2, (int)ldo, (float *)ctx->gemm_partial.ptr,
-                                  ctx->gemm_counters, ctx->dev_err, ctx->stream));
-        launches = 1;
-    } else if (tma) {
-        if (int rc = ensure(ctx, ctx->gemm_partial, gemm_tma_workspace_bytes(kind, (int)T, (int)K, (int)F))) return rc;
-        MCU_CUDA(launch_gemm_tma(kind, w, w2, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr,
-                                 (int)kp, (int)T, (int)K, (int)F, bias, out, out2, (int)ldo, (float *)ctx->gemm_partial.ptr,
-                                 ctx->gemm_counters, ctx->dev_err, ctx->stream, &launches));
-    } else {
-        MCU_CUDA(launch_gemm_tc(kind, w, w2, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr, (int)kp,
-                                (int)T, (int)K, (int)F, bias, out, out2, (int)ldo, ctx->dev_err, ctx->stream, &launches));
-    }
-    count_launches(launches);
+    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+    MCU_CUDA(launch_gemm_ts(kind, jobs, n_jobs, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr, (int)kp,
+                            (int)T, (int)K, (float *)ctx->gemm_partial.ptr, ctx->gemm_counters, ctx->dev_err, ctx->stream));
+    count_launches(1);
     return MCU_SUCCESS;
 }
 
@@ -609,8 +591,10 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
         return MCU_SUCCESS;
     }
     if (gemm) {
-        if (gemm_tc_supported(kind, (int)T, (int)K, (int)F))
-            return gemm_locked(ctx, kind, x, ldx, w, w2, T, K, F, bias, out, out2, ldo, nullptr, nullptr);
+        if (gemm_ts_supported(kind, w, (int)T, (int)K, (int)F) && (w2 == nullptr || gemm_ts_supported(kind, w2, (int)T, (int)K, (int)F))) {
+            const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};
+            return gemm_locked(ctx, kind, x, ldx, T, K, jobs, w2 != nullptr ? 2 : 1, nullptr, nullptr);
+        }
         if (ctx->regime == MCU_REGIME_GEMM)
             return fail(MCU_ERROR_NOT_IMPLEMENTED, "tensor-core GEMM does not cover kind %d T=%zu K=%zu F=%zu", kind, T, K, F);
     }
@@ -621,7 +605,7 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
         count_launches(1);
         return MCU_SUCCESS;
     }
-    if (int rc = pack_activations(ctx, kind, x, ldx, T, K, false, ACT_ORDER_NATURAL, ab)) return rc;
+    if (int rc = pack_activations(ctx, kind, x, ldx, T, K, false, ab)) return rc;
     const size_t bv = (size_t)block_values(kind);
     const size_t nb = (K + bv - 1) / bv, kp = nb * bv;
     for (size_t t0 = 0; t0 < T; t0 += GEMV_MAX_T) {
@@ -652,7 +636,7 @@ int linear_fused_allreduce(mcu_context *ctx, int kind, const float *x, size_t ld
     if (int rc = ensure(ctx, ctx->act_half, T * kp * sizeof(__half))) return rc;
     if (int rc = ensure(ctx, ctx->act_rowscale, T * sizeof(float))) return rc;
     if (int rc = ensure(ctx, ctx->gemm_partial, gemm_tma_workspace_bytes(kind, (int)T, (int)K, (int)F))) return rc;
-    MCU_CUDA(launch_act_half_fused(kind, x, (int)ldx, (int)T, (int)K, ACT_ORDER_QUAD, (__half *)ctx->act_half.ptr,
+    MCU_CUDA(launch_act_half_fused_from(kind, x, (int)ldx, ActSource{}, (int)T, (int)K, (__half *)ctx->act_half.ptr,
                                    (float *)ctx->act_rowscale.ptr, ctx->stream));
     int launches = 0;
     MCU_CUDA(launch_gemm_tma(kind, w, nullptr, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr,
@@ -861,7 +845,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
         bool tensor = (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > 16 &&
             (pr.op == MCU_PROLOGUE_NONE || contiguous);
         for (size_t j = 0; j < n_jobs && tensor; ++j)
-            tensor = gemm_tc_supported(jobs[j].kind, (int)T, (int)K, (int)jobs[j].F) &&
+            tensor = gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) &&
                 act_half_fused_smem(jobs[j].kind, (int)K) <= 48 * 1024;
         if (tensor) {
             ActSource src;
@@ -877,23 +861,25 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
                 src.glu = 1;
             }
             Staged st;
-            for (size_t j = 0; j < n_jobs;) {
-                const mcu_linear_job_t &a = jobs[j];
-                const bool pair = j + 1 < n_jobs && jobs[j + 1].kind == a.kind && jobs[j + 1].F == a.F && jobs[j + 1].ldo == a.ldo &&
-                    a.bias_dev == nullptr && jobs[j + 1].bias_dev == nullptr;
+            // one launch per kind, whatever the order of the jobs
+            bool done[GEMV_MAX_JOBS] = {};
+            for (size_t j = 0; j < n_jobs; ++j) {
+                if (done[j]) continue;
+                GemvJobSpec same[GEMV_MAX_JOBS];
+                int n = 0;
+                for (size_t i = j; i < n_jobs; ++i)
+                    if (specs[i].kind == specs[j].kind) {
+                        same[n++] = specs[i];
+                        done[i] = true;
+                    }
                 // x_out is written by the first staging launch only (a second one would add aux twice if x_out is x)
                 ActSource use = src;
-                if (st.valid || j > 0) {
-                    if (use.norm && use.x_out != nullptr) {
-                        use.add = nullptr;  // the sum is already in x_out
-                        use.x_out = nullptr;
-                    }
+                const bool again = j > 0 && src.norm && src.x_out != nullptr;
+                if (again) {
+                    use.add = nullptr;  // the sum is already in x_out
+                    use.x_out = nullptr;
                 }
-                const float *from = (j > 0 && src.norm && src.x_out != nullptr) ? src.x_out : x_dev;
-                if (int rc = gemm_locked(ctx, a.kind, from, ldx, a.w_dev, pair ? jobs[j + 1].w_dev : nullptr, T, K, a.F, a.bias_dev,
-                                         a.out_dev, pair ? jobs[j + 1].out_dev : nullptr, a.ldo, &use, &st))
-                    return rc;
-                j += pair ? 2 : 1;
+                if (int rc = gemm_locked(ctx, specs[j].kind, again ? src.x_out : x_dev, ldx, T, K, same, n, &use, &st)) return rc;
             }
             return MCU_SUCCESS;
         }
@@ -1041,9 +1027,9 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     // launches whatever its size.
     const bool grouped = !no_grouped && (routes >= 256 || stream_is_capturing(s) || routed_rows_ext != nullptr) &&
         gate_kind == up_kind &&
-        gemm_tma_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
-        gemm_tma_grouped_supported(up_kind, up_dev, (int)H, (int)FF) &&
-        gemm_tma_grouped_supported(down_kind, down_dev, (int)FF, (int)H) &&
+        gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
+        gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) &&
+        gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H) &&
         act_half_fused_smem(gate_kind, (int)H) <= 48 * 1024 && act_half_fused_smem(down_kind, (int)FF) <= 48 * 1024 &&
         routes < ((size_t)1 << 24);
     if (grouped) {
@@ -1064,16 +1050,17 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
         from_hidden.row_hi = from_glu.row_hi = rb.offsets + e_begin + e_count;
         from_glu.x2 = up_out;
         from_glu.glu = ffn_type == MCU_FFN_GEGLU ? 2 : 1;
-        MCU_CUDA(launch_act_half_fused_from(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, ACT_ORDER_QUAD,
-                                            xh, rowscale, s));
-        MCU_CUDA(launch_gemm_tma_grouped(gate_kind, gate_dev, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H,
-                                         (int)FF, cnt, off, gate_out, (int)FF, ctx->dev_err, s));
-        MCU_CUDA(launch_gemm_tma_grouped(up_kind, up_dev, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, (int)FF,
-                                         cnt, off, up_out, (int)FF, ctx->dev_err, s));
-        MCU_CUDA(launch_act_half_fused_from(down_kind, gate_out, (int)FF, from_glu, (int)routes, (int)FF, ACT_ORDER_QUAD, xh,
-                                            rowscale, s));
-        MCU_CUDA(launch_gemm_tma_grouped(down_kind, down_dev, (int)e_count, xh, rowscale, (int)kp_f, (int)routes, (int)FF,
-                                         (int)H, cnt, off, route_down, (int)H, ctx->dev_err, s));
+        if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+        float *part = (float *)ctx->gemm_partial.ptr;
+        int *tick = ctx->gemm_counters;
+        MCU_CUDA(launch_act_half_fused_from(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xh, rowscale, s));
+        MCU_CUDA(launch_gemm_ts_grouped(gate_kind, gate_dev, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, (int)FF,
+                                        cnt, off, gate_out, (int)FF, part, tick, ctx->dev_err, s));
+        MCU_CUDA(launch_gemm_ts_grouped(up_kind, up_dev, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, (int)FF, cnt,
+                                        off, up_out, (int)FF, part, tick, ctx->dev_err, s));
+        MCU_CUDA(launch_act_half_fused_from(down_kind, gate_out, (int)FF, from_glu, (int)routes, (int)FF, xh, rowscale, s));
+        MCU_CUDA(launch_gemm_ts_grouped(down_kind, down_dev, (int)e_count, xh, rowscale, (int)kp_f, (int)routes, (int)FF, (int)H,
+                                        cnt, off, route_down, (int)H, part, tick, ctx->dev_err, s));
         if (routed_rows_ext == nullptr) {
             MCU_CUDA(launch_moe_combine_dev(route_down, rb.sorted_w, rb.route_pos, (int)T, (int)k, (int)H, rb.offsets,
                                             (int)e_begin, (int)(e_begin + e_count), rb.counts + E, ctx->dev_err, out_dev, H, s));

@@ -111,22 +111,15 @@ quantize_q8_0_kernel(const float *__restrict__ x, int ldx, int T, int K, int nb,
     }
 }
 
-// Which value of a row goes to position k (see ACT_ORDER_* in kernels.h).
-__device__ __forceinline__ int act_order_source(int k, int order) {
-    if (order == ACT_ORDER_QUAD) return (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1);
-    if (order == ACT_ORDER_FRAG16) {
-        const int p = k & 15;
-        return (k & ~15) | (((p & 7) >> 1) << 2) | (p >> 3) | ((p & 1) << 1);
-    }
-    return k;
-}
+// Which value of a row goes to position k: every four consecutive values are stored as (0, 2, 1, 3) (see kernels.h).
+__device__ __forceinline__ constexpr int act_order_source(int k) { return (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1); }
 
 // fp16 operands for the tensor-core path: xh[t][k] = (d*q) * 2^-e_t, with one exponent per token chosen so
 // that the largest magnitude of the row is about 2^14.  The power-of-two scale is exact, keeps large
 // activations inside the fp16 range (and tiny ones out of the subnormals); the matmul epilogue multiplies
 // the row back by rowscale[t] = 2^e_t.  One CTA per token.
 __global__ void __launch_bounds__(256)
-half_acts_kernel(int kq, int perm, const int8_t *__restrict__ qs, const float *__restrict__ dq, int nb, int kp,
+half_acts_kernel(int kq, const int8_t *__restrict__ qs, const float *__restrict__ dq, int nb, int kp,
                  __half *__restrict__ xh, float *__restrict__ rowscale) {
     __shared__ float red[8];
     __shared__ float inv_s;
@@ -157,7 +150,7 @@ half_acts_kernel(int kq, int perm, const int8_t *__restrict__ qs, const float *_
     __half *hrow = xh + (size_t)t * kp;
     const int bv = kq ? QK_K : Q8_0_VALUES;
     for (int k = threadIdx.x; k < kp; k += blockDim.x) {
-        const int src = act_order_source(k, perm);
+        const int src = act_order_source(k);
         const int blk = src / bv;
         const int pos = kq ? blk * QK_K + q8k_split_pos(src - blk * QK_K) : src;
         hrow[k] = __float2half_rn(__fmul_rn(__fmul_rn(drow[blk], inv), (float)qrow[pos]));
@@ -168,9 +161,7 @@ half_acts_kernel(int kq, int perm, const int8_t *__restrict__ qs, const float *_
 // sums in global memory: one CTA per token quantises the row block by block exactly as the kernels above (values
 // and scales kept in shared memory), then writes xh and rowscale exactly as half_acts_kernel.  Launched with
 // programmatic stream serialization: everything before griddepcontrol.wait is independent of earlier kernels.
-// Sixteen staged values from sixteen quantised ones: position p of the group takes source act_order_source(p, ORDER)
-// (every order permutes inside aligned groups of sixteen), so the indices resolve at compile time.
-template <int ORDER>
+// Sixteen staged values from sixteen quantised ones.
 __device__ __forceinline__ void stage_group16(const int8_t *q16, float sc, __half *dst) {
     const uint4 raw = *(const uint4 *)q16;
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -180,7 +171,7 @@ __device__ __forceinline__ void stage_group16(const int8_t *q16, float sc, __hal
     uint32_t o[8];
 #pragma unroll
     for (int p2 = 0; p2 < 8; ++p2) {
-        const __half2 h = __floats2half2_rn(f[act_order_source(2 * p2, ORDER)], f[act_order_source(2 * p2 + 1, ORDER)]);
+        const __half2 h = __floats2half2_rn(f[act_order_source(2 * p2)], f[act_order_source(2 * p2 + 1)]);
         o[p2] = *(const uint32_t *)&h;
     }
     uint4 *d = (uint4 *)dst;
@@ -190,18 +181,20 @@ __device__ __forceinline__ void stage_group16(const int8_t *q16, float sc, __hal
 
 // GLU: 0 = the row as it is; 1 = silu(x) * x2; 2 = gelu(x) * x2.  The SiLU uses the fast exponential and division
 // (relative error about 1e-6): its result is quantised to eight bits right here, three orders of magnitude coarser.
+// Few rows: up to a thousand threads per row, so that a row is one or two trips to L2 (latency bounds the launch: 64 rows of
+// 4096 values 3.3 us with 256 threads); many rows: 256 threads, and as many rows at a time.
 template <bool KQ, int GLU>
-__global__ void __launch_bounds__(256)
-act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, int perm,
+__global__ void __launch_bounds__(1024)
+act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb,
                       __half *__restrict__ xh, float *__restrict__ rowscale) {
     extern __shared__ __align__(16) uint8_t act_sm[];
     constexpr int BV = KQ ? QK_K : Q8_0_VALUES;
     const int kp = nb * BV;
     int8_t *q_s = (int8_t *)act_sm;
     float *d_s = (float *)(act_sm + ((kp + 15) & ~15));
-    __shared__ float red[8];
+    __shared__ float red[32];
     __shared__ float inv_s;
-    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (src.row_lo != nullptr && (t < *src.row_lo || t >= *src.row_hi)) return;  // not this rank's row
@@ -214,14 +207,15 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
         arow = src.add != nullptr ? src.add + row_off : nullptr;
         float *orow = src.x_out != nullptr ? src.x_out + row_off : nullptr;
         float sum = 0.0f;
-        for (int i = threadIdx.x; i < K; i += blockDim.x) {
+        // (256 threads whatever the block: the order of the sum is that of the stand-alone kernel)
+        for (int i = threadIdx.x; i < K && threadIdx.x < 256; i += 256) {
             const float v = arow != nullptr ? __fadd_rn(xrow[i], arow[i]) : xrow[i];
             if (orow != nullptr) orow[i] = v;
             sum += v * v;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) red[warp] = sum;
+        if (lane == 0 && warp < 8) red[warp] = sum;
         __syncthreads();
         if (threadIdx.x == 0) {
             float s = 0.0f;
@@ -251,7 +245,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
         return __fmul_rn(a, urow[k]);
     };
     if (KQ) {
-        for (int blk = warp; blk < nb; blk += 8) {
+        for (int blk = warp; blk < nb; blk += n_warps) {
             const int len = min(QK_K, K - blk * QK_K);
             float v[8];
             float best_abs = 0.0f, best_val = 0.0f;
@@ -291,7 +285,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
             if (lane == 0) d_s[blk] = d;
         }
     } else {
-        for (int blk = warp; blk < nb; blk += 8) {
+        for (int blk = warp; blk < nb; blk += n_warps) {
             const int k = blk * Q8_0_VALUES + lane;
             const float v = k < K ? value(k) : 0.0f;
             float amax = fabsf(v);
@@ -315,7 +309,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
     __syncthreads();
     if (threadIdx.x == 0) {
         float mm = 0.0f;
-        for (int i = 0; i < 8; ++i) mm = fmaxf(mm, red[i]);
+        for (int i = 0; i < n_warps; ++i) mm = fmaxf(mm, red[i]);
         mm *= 127.0f;
         int e = 0;
         if (mm > 0.0f && mm < 3.0e38f) {
@@ -331,9 +325,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
     __half *hrow = xh + (size_t)t * kp;
     for (int g = threadIdx.x; g < kp / 16; g += blockDim.x) {
         const float sc = __fmul_rn(d_s[(16 * g) / BV], inv);
-        if (perm == ACT_ORDER_QUAD) stage_group16<ACT_ORDER_QUAD>(q_s + 16 * g, sc, hrow + 16 * g);
-        else if (perm == ACT_ORDER_FRAG16) stage_group16<ACT_ORDER_FRAG16>(q_s + 16 * g, sc, hrow + 16 * g);
-        else stage_group16<ACT_ORDER_NATURAL>(q_s + 16 * g, sc, hrow + 16 * g);
+        stage_group16(q_s + 16 * g, sc, hrow + 16 * g);
     }
 }
 
@@ -342,13 +334,18 @@ size_t act_half_fused_smem(int kind, int K) {
     return (size_t)((nb * bv + 15) & ~15) + (size_t)nb * sizeof(float);
 }
 
-cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const ActSource &src, int T, int K, int k_order,
+cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const ActSource &src, int T, int K,
                                        __half *xh, float *rowscale, cudaStream_t s) {
     if (T <= 0) return cudaSuccess;
     const int bv = block_values(kind), nb = (K + bv - 1) / bv;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)T, 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
+    int warps = 8;
+    if (T < 512) {
+        const int want = kind != KIND_Q8_0 ? nb : nb / 4;  // a 256-value block, or four 32-value ones in turn, per warp
+        warps = want < 8 ? 8 : want > 32 ? 32 : want;
+    }
+    cfg.blockDim = dim3((unsigned)(32 * warps), 1, 1);
     cfg.dynamicSmemBytes = act_half_fused_smem(kind, K);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -358,23 +355,17 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
     cfg.numAttrs = 1;
     const bool kq = kind != KIND_Q8_0;
     const int glu = src.x2 != nullptr ? (src.glu == 2 ? 2 : 1) : 0;
-#define MCU_STAGE(KQ, GLU) cudaLaunchKernelEx(&cfg, act_half_fused_kernel<KQ, GLU>, x, ldx, src, K, nb, k_order, xh, rowscale)
+#define MCU_STAGE(KQ, GLU) cudaLaunchKernelEx(&cfg, act_half_fused_kernel<KQ, GLU>, x, ldx, src, K, nb, xh, rowscale)
     if (glu == 0) return kq ? MCU_STAGE(true, 0) : MCU_STAGE(false, 0);
     if (glu == 1) return kq ? MCU_STAGE(true, 1) : MCU_STAGE(false, 1);
     return kq ? MCU_STAGE(true, 2) : MCU_STAGE(false, 2);
 #undef MCU_STAGE
 }
 
-cudaError_t launch_act_half_fused(int kind, const float *x, int ldx, int T, int K, int k_order, __half *xh,
-                                  float *rowscale, cudaStream_t s) {
-    return launch_act_half_fused_from(kind, x, ldx, ActSource{}, T, K, k_order, xh, rowscale, s);
-}
-
-cudaError_t launch_half_acts(int kind, const ActBuffers &a, int T, int K, int k_order, __half *xh, float *rowscale,
-                             cudaStream_t s) {
+cudaError_t launch_half_acts(int kind, const ActBuffers &a, int T, int K, __half *xh, float *rowscale, cudaStream_t s) {
     if (T <= 0) return cudaSuccess;
     const int bv = block_values(kind), nb = (K + bv - 1) / bv;
-    half_acts_kernel<<<T, 256, 0, s>>>(kind != KIND_Q8_0, k_order, a.qs, a.d, nb, nb * bv, xh, rowscale);
+    half_acts_kernel<<<T, 256, 0, s>>>(kind != KIND_Q8_0, a.qs, a.d, nb, nb * bv, xh, rowscale);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,52 @@
+// Parameters and launchers of the tcgen05 matmul with weights in tensor memory (gemm_ts.cu).
+#pragma once
+
+#include "kernels.h"
+
+#include <cuda.h>
+
+namespace mcu {
+
+constexpr int TS_MAX_JOBS = 4;
+constexpr int TS_MAX_GROUPS = 256;
+constexpr int TS_MAX_SPLIT = 8;
+
+struct TsMaps {
+    CUtensorMap x;               // fp16 activations [rows][kp]
+    CUtensorMap w[TS_MAX_JOBS];  // packed weights, Q4_K only
+};
+struct TsJob {
+    const uint8_t *w;
+    float *out;
+    const float *bias;
+    int F, ldo;
+    int row_tile0;  // first row tile of the job
+};
+struct TsParams {
+    TsJob jobs[TS_MAX_JOBS];
+    const float *rowscale;  // per-token power-of-two factor undone in the epilogue
+    float *partial;         // two slots of 128 x bn floats per CTA
+    int *counters;          // one ticket per CTA, zero between launches
+    int *err;
+    const int *group_counts, *group_offsets;  // grouped launches (MoE experts), device memory
+    long row_bytes;
+    int n_jobs, T, bn, nb, slabs, raw_shift;  // raw_shift: log2 of the slab ring's depth
+    int loose;              // weight rows that are not 16-byte multiples, or do not start on one
+    int split;              // > 1: clusters of `split` CTAs (pairs) share a tile along K; otherwise ranges of units
+    int tiles, t_tiles;     // output tiles in all; token tiles per row tile
+    int groups, row_tiles;  // grouped launches: number of groups, row tiles per group
+};
+
+// Shares of cut tiles (gemm_ts_workspace_bytes(), 0 tickets in `counters` between launches, one int per SM).
+size_t gemm_ts_workspace_bytes();
+bool gemm_ts_supported(int kind, const void *W, int T, int K, int F);
+// up to TS_MAX_JOBS matrices of one kind that read the same activations (fp16 from launch_act_half_fused_from), in one launch
+cudaError_t launch_gemm_ts(int kind, const GemvJobSpec *jobs, int n_jobs, const __half *xh, const float *rowscale, int ldxh,
+                           int T, int K, float *partial, int *counters, int *err_flag, cudaStream_t s);
+// stacked matrices: rows that are not 16-byte multiples need a multiple of eight rows per group
+bool gemm_ts_grouped_supported(int kind, const void *W, int K, int F);
+cudaError_t launch_gemm_ts_grouped(int kind, const void *W, int n_groups, const __half *xh, const float *rowscale, int ldxh,
+                                   int total_rows, int K, int F, const int *group_counts, const int *group_offsets, float *out,
+                                   int ldo, float *partial, int *counters, int *err_flag, cudaStream_t s);
+
+}  // namespace mcu

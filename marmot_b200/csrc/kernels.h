@@ -21,19 +21,13 @@ cudaError_t launch_quantize_act(int kind, const float *x, int ldx, int T, int K,
                                 cudaStream_t s);
 
 // fp16 operands of the tensor-core matmul from the quantized activations: xh[t][k] = d*q*2^-e_t (row stride kp),
-// rowscale[t] = 2^e_t.  k_order: the order of the K values inside a row, matching how the matmul that reads it
-// extracts packed weights: ACT_ORDER_NATURAL; ACT_ORDER_QUAD stores every four consecutive values as (0, 2, 1, 3)
-// (gemm_tma); ACT_ORDER_FRAG16 stores every sixteen values v = 4t + j at position 8(j & 1) + 2t + (j >> 1), the k
-// labelling of the mma.sync fragments of gemm_warp.
-constexpr int ACT_ORDER_NATURAL = 0, ACT_ORDER_QUAD = 1, ACT_ORDER_FRAG16 = 2;
-cudaError_t launch_half_acts(int kind, const ActBuffers &a, int T, int K, int k_order, __half *xh, float *rowscale,
-                             cudaStream_t s);
+// rowscale[t] = 2^e_t.  Every four consecutive values of a row are stored as (0, 2, 1, 3): the pairs that mask-and-or
+// extraction takes out of a packed word of weights.
+cudaError_t launch_half_acts(int kind, const ActBuffers &a, int T, int K, __half *xh, float *rowscale, cudaStream_t s);
 
 // The two steps above in one kernel (one CTA per token, the quantized row kept in shared memory) when the int8
 // values are not needed in global memory; usable while act_half_fused_smem() fits the default 48 KB.
 size_t act_half_fused_smem(int kind, int K);
-cudaError_t launch_act_half_fused(int kind, const float *x, int ldx, int T, int K, int k_order, __half *xh,
-                                  float *rowscale, cudaStream_t s);
 // Where the staging kernel takes its rows from, for callers that would otherwise run a gather or a GLU pass first:
 // row t comes from x + row_index[t] * ldx when row_index is set; with x2 set the value is act(x) * x2 (glu 1 = SiLU,
 // 2 = GELU, rounded like the MoE GLU kernel); rows outside [*row_lo, *row_hi) (device-resident) are skipped.
@@ -50,7 +44,7 @@ struct ActSource {
     float eps = 0.0f, w_off = 0.0f;
     float *x_out = nullptr;
 };
-cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const ActSource &src, int T, int K, int k_order,
+cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const ActSource &src, int T, int K,
                                        __half *xh, float *rowscale, cudaStream_t s);
 
 // blocks -> f32 (bit-exact with the reference dequantizers)
@@ -117,14 +111,6 @@ cudaError_t launch_gemm_i8(int kind, const void *W, const void *W2, const float 
                            const float *bias, float *out, float *out2, int ldo, int8_t *qs, float *dT, float *partial,
                            int *tickets, int *err_flag, cudaStream_t s);
 
-// Prefill / batched regime on the tcgen05 tensor cores: weights dequantised to fp16 tiles in shared
-// memory, activations given as fp16 (d*q of the quantized activations, row stride ldxh), f32
-// accumulation in tensor memory.
-bool gemm_tc_supported(int kind, int T, int K, int F);
-cudaError_t launch_gemm_tc(int kind, const void *W, const void *W2, const __half *xh, const float *rowscale, int ldxh,
-                           int T, int K, int F, const float *bias, float *out, float *out2, int ldo, int *err_flag,
-                           cudaStream_t s, int *launches);
-
 // Row-parallel matmul fused with its all-reduce over peer memory (gemm_tma, T <= 64, full 128-row tiles): every CTA
 // that holds a finished output tile stores it into this rank's peer-visible staging buffer, releases one flag per
 // rank and tile, waits (bounded) for the same tile of all ranks, pulls their tiles with plain peer loads and adds
@@ -151,19 +137,6 @@ cudaError_t launch_gemm_tma(int kind, const void *W, const void *W2, const __hal
                             int T, int K, int F, const float *bias, float *out, float *out2, int ldo, float *partial,
                             int *counters, int *err_flag, cudaStream_t s, int *launches,
                             const PeerFuse *fuse = nullptr);
-// Register-operand variant for 8 < T <= 64 tokens on Q4_K / Q6_K (mma.sync fragments built straight from the packed
-// words, nothing dequantised to shared memory); activations in ACT_ORDER_FRAG16; same workspace contract.
-bool gemm_warp_supported(int kind, const void *W, const void *W2, int T, int K, int F);
-size_t gemm_warp_workspace_bytes(int kind, int T, int K, int F, bool dual);
-cudaError_t launch_gemm_warp(int kind, const void *W, const void *W2, const __half *xh, const float *rowscale, int ldxh,
-                             int T, int K, int F, const float *bias, float *out, float *out2, int ldo, float *partial,
-                             int *counters, int *err_flag, cudaStream_t s);
-// Grouped form (MoE experts): one launch for n_groups matmuls over a stacked weight matrix [n_groups * F, K]; group g
-// owns group_counts[g] rows of xh / rowscale / out starting at row group_offsets[g] (device arrays: no host read-back).
-bool gemm_tma_grouped_supported(int kind, const void *W, int K, int F);
-cudaError_t launch_gemm_tma_grouped(int kind, const void *W, int n_groups, const __half *xh, const float *rowscale,
-                                    int ldxh, int total_rows, int K, int F, const int *group_counts,
-                                    const int *group_offsets, float *out, int ldo, int *err_flag, cudaStream_t s);
 // Can launch_gemm_tma fuse the all-reduce for this shape (same answer on every rank: it depends on T and F only)?
 bool gemm_tma_can_fuse(int kind, int T, int F);
 
