@@ -81,18 +81,18 @@ struct mcu_context {
     // workspace (grows on demand, never shrinks)
     Buffer act_qs, act_d, act_bsums, act_half, act_rowscale, x_stage, out_stage, bias_stage;
     Buffer moe_meta, moe_hidden, moe_gate, moe_up, moe_down;
-    Buffer gemm_partial;         // split-K partial tiles
+    Buffer gemm_partial;         // shares of cut tiles
     Buffer rope_table;              // {cos, sin} per token and pair when a decode attention call brings none
     Buffer attn_tickets;            // fused decode attention: one counter per (token, KV head)
     Buffer pro_h;                   // activations after a stand-alone prologue kernel (mcu_linear_multi's general form)
-    Buffer i8_partial, i8_tickets;  // integer-MMA matmul: shares of row groups split between CTAs, and their tickets
     Buffer attn_partial;         // split-KV partial attention states
     int *gemm_counters = nullptr;  // split-K tile tickets (zero between launches)
     std::vector<int> host_counts;
     size_t moe_last_routes = 0, moe_last_experts = 0;  // shape of the last MoE call (mcu_moe_last_buffers)
     int moe_last_grouped = 0;
     int *dev_err = nullptr;  // set by kernels whose bounded device-side waits ran out
-    int *err_host = nullptr; // page-locked word the flag is copied into on a synchronize
+    int *err_host = nullptr; // page-locked words: the flag's copy on a synchronize, the bad-id count of a small MoE call
+    cudaEvent_t moe_event = nullptr;
     // Small host <-> device copies go through page-locked slots owned by the context: an upload is a host memcpy into a
     // slot plus an asynchronous copy (the caller's buffer is free on return and nothing waits for the copy engine), a
     // download lands in a slot and is copied out after the one synchronize it needs anyway.
@@ -241,7 +241,7 @@ int mcu_context_create(int device, mcu_context_t **out) {
     ctx->stream = ctx->own_stream;
     e = cudaMalloc(&ctx->dev_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->dev_err, 0, sizeof(int));
-    if (e == cudaSuccess && cudaHostAlloc((void **)&ctx->err_host, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+    if (e == cudaSuccess && cudaHostAlloc((void **)&ctx->err_host, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
         (void)cudaGetLastError();
         ctx->err_host = nullptr;  // the flag is then fetched with a blocking copy
     }
@@ -266,11 +266,12 @@ void mcu_context_destroy(mcu_context_t *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     Buffer *bufs[] = {&ctx->act_qs,   &ctx->act_d,      &ctx->act_bsums, &ctx->act_half, &ctx->act_rowscale, &ctx->x_stage, &ctx->out_stage,
-                      &ctx->bias_stage, &ctx->moe_meta, &ctx->moe_hidden, &ctx->moe_gate, &ctx->moe_up, &ctx->moe_down, &ctx->gemm_partial, &ctx->attn_partial, &ctx->i8_partial, &ctx->i8_tickets, &ctx->pro_h, &ctx->attn_tickets, &ctx->rope_table};
+                      &ctx->bias_stage, &ctx->moe_meta, &ctx->moe_hidden, &ctx->moe_gate, &ctx->moe_up, &ctx->moe_down, &ctx->gemm_partial, &ctx->attn_partial, &ctx->pro_h, &ctx->attn_tickets, &ctx->rope_table};
     for (Buffer *b : bufs)
         if (b->ptr != nullptr) cudaFree(b->ptr);
     if (ctx->dev_err != nullptr) cudaFree(ctx->dev_err);
     if (ctx->err_host != nullptr) cudaFreeHost(ctx->err_host);
+    if (ctx->moe_event != nullptr) cudaEventDestroy(ctx->moe_event);
     if (ctx->pin_ring != nullptr) {
         for (int i = 0; i < PIN_SLOTS; ++i)
             if (ctx->pin_event[i] != nullptr) cudaEventDestroy(ctx->pin_event[i]);
@@ -556,6 +557,45 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
     return MCU_SUCCESS;
 }
 
+// The integer tensor-core matmul for few tokens (Q4_K, Q6_K): the same two steps.
+// Its time hardly depends on the token count, the dp4a kernel's (one launch, no staging) grows with it, so up to eight tokens
+// the line is one of tokens x values; times in us at K x F, dp4a then tensor cores:
+//   Q4_K  3 tokens  4096 x 4096 8.5, 9.0; x 14336 18.8, 13.6     4 tokens  2048 x 2048 4.9, 7.3; 4096 x 4096 10.3, 9.0
+//         5 tokens  1024 x 1024 4.7, 6.8; 2048 x 2048 7.3, 7.3; 4096 x 1024 8.2, 7.4; 4096 x 4096 11.9, 9.0
+//   Q6_K  4 tokens  4096 x 4096 11.0, 11.7; 14336 x 4096 33.3, 23.6; 4096 x 28672 39.7, 44.7
+//         5 tokens  1024 x 1024 4.2, 7.0; 2048 x 2048 7.9, 8.0; 4096 x 1024 8.8, 8.6; 4096 x 4096 13.5, 11.7
+// From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
+static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t values) {
+    static const bool off = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch
+    if (off || ctx->regime != MCU_REGIME_AUTO || T > (size_t)TI_COLS) return false;
+    if (T > (size_t)GEMV_MAX_T) return true;
+    if (T >= 5) return values >= (size_t)4 << 20;
+    return kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20;
+}
+static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K) {
+    for (int j = 0; j < n_jobs; ++j)
+        if (!gemm_ti_supported(jobs[j].kind, jobs[j].W, (int)K, jobs[j].F) || act_half_fused_smem(jobs[j].kind, (int)K) > 48 * 1024) return false;
+    return true;
+}
+static int integer_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, const GemvJobSpec *jobs, int n_jobs,
+                          const ActSource *src, int *staged_kind) {
+    const size_t nb = (K + QK_K - 1) / QK_K;
+    if (int rc = ensure(ctx, ctx->act_qs, gemm_ti_xq_bytes(kind, (int)T, (int)K))) return rc;
+    if (int rc = ensure(ctx, ctx->act_d, T * nb * sizeof(float))) return rc;
+    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+    uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
+    float *dT = (float *)ctx->act_d.ptr;
+    if (staged_kind == nullptr || *staged_kind != kind) {
+        MCU_CUDA(launch_act_int_fused(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K, xq, dT, ctx->stream));
+        count_launches(1);
+        if (staged_kind != nullptr) *staged_kind = kind;
+    }
+    MCU_CUDA(launch_gemm_ti(kind, jobs, n_jobs, xq, dT, (int)T, (int)K, (float *)ctx->gemm_partial.ptr, ctx->gemm_counters, ctx->dev_err,
+                            ctx->stream));
+    count_launches(1);
+    return MCU_SUCCESS;
+}
+
 // Core of mcu_linear / mcu_linear_dual on device pointers; ctx->mu is held by the caller.
 static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, const void *w, const void *w2, size_t T,
                          size_t K, size_t F, const float *bias, float *out, float *out2, size_t ldo) {
@@ -563,32 +603,13 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     const bool gemm = ctx->regime == MCU_REGIME_GEMM ||
         ((ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_I8MMA) && T > (size_t)GEMV_MAX_T);
     ActBuffers ab;
-    // A handful of tokens: exact integer dots on mma.sync s8 (Q4_K, Q6_K).  Measured against the neighbours on
-    // K = 4096 (F = 4096 / 14336, microseconds per call): 8 tokens 12.1 / 19.4 here, 15.3 / 33.6 on the dp4a kernel
-    // (which re-reads the activations from shared memory per token); 16 tokens 13.4 / 22.5 here, 12.4 / 25.8 on the
-    // tcgen05 kernel; below five tokens the dp4a kernel's single launch wins, beyond sixteen the integer MMA rate of
-    // this part (about 30 cycles per m16n8k32 and SM sub-partition) does not keep up with the fp16 paths.
-    static const bool no_i8 = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch
-    const size_t w_total = F * mcu_row_bytes(kind, K) * (w2 != nullptr ? 2 : 1);
-    const bool i8_pays = ctx->regime == MCU_REGIME_I8MMA
-        ? (T >= 2 && T <= 64)
-        : (!no_i8 && ctx->regime == MCU_REGIME_AUTO && T >= 5 && T <= 16 && (T <= 12 || w_total >= ((size_t)24 << 20)));
-    if (i8_pays &&
-        gemm_i8_supported(kind, w, w2, (int)T, (int)K, (int)F) && (w2 == nullptr || bias == nullptr)) {
-        size_t qs_b, dT_b, part_b, tick_b;
-        gemm_i8_workspace_bytes((int)T, (int)K, (int)F, w2 != nullptr, &qs_b, &dT_b, &part_b, &tick_b);
-        if (int rc = ensure(ctx, ctx->act_qs, qs_b)) return rc;
-        if (int rc = ensure(ctx, ctx->act_d, dT_b)) return rc;
-        if (int rc = ensure(ctx, ctx->i8_partial, part_b)) return rc;
-        if (tick_b > ctx->i8_tickets.cap) {  // a fresh ticket area starts at zero; the kernel keeps it so
-            if (int rc = ensure(ctx, ctx->i8_tickets, tick_b)) return rc;
-            MCU_CUDA(cudaMemsetAsync(ctx->i8_tickets.ptr, 0, ctx->i8_tickets.cap, ctx->stream));
-        }
-        MCU_CUDA(launch_gemm_i8(kind, w, w2, x, (int)ldx, (int)T, (int)K, (int)F, bias, out, out2, (int)ldo,
-                                (int8_t *)ctx->act_qs.ptr, (float *)ctx->act_d.ptr, (float *)ctx->i8_partial.ptr,
-                                (int *)ctx->i8_tickets.ptr, ctx->dev_err, ctx->stream));
-        count_launches(2);
-        return MCU_SUCCESS;
+    // a handful of tokens: exact integer dots on the tensor core
+    const size_t values = K * F * (w2 != nullptr ? 2 : 1);
+    const bool i8_pays = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, values);
+    if (i8_pays && (w2 == nullptr || bias == nullptr)) {
+        const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};
+        if (integer_jobs_supported(jobs, w2 != nullptr ? 2 : 1, K))
+            return integer_locked(ctx, kind, x, ldx, T, K, jobs, w2 != nullptr ? 2 : 1, nullptr, nullptr);
     }
     if (gemm) {
         if (gemm_ts_supported(kind, w, (int)T, (int)K, (int)F) && (w2 == nullptr || gemm_ts_supported(kind, w2, (int)T, (int)K, (int)F))) {
@@ -822,32 +843,28 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
     {
         std::lock_guard<std::mutex> lock(ctx->mu);
         const bool contiguous = ldx == K && (pr.aux_dev == nullptr || pr.ld_aux == K) && (gp.x_out == nullptr || pr.ld_x_out == K);
-        // Five to eight tokens over large K-quant matrices: the dp4a kernel is bound by its integer dots there (8 tokens,
-        // 2 x 14336 x 4096 Q4_K: 73 us with the prologue folded in, 29 us on the integer-MMA kernel), so the prologue runs
-        // as a kernel of its own and the matmuls take mcu_linear's regimes.  Small matrices keep the one-launch form.
-        size_t w_total = 0;
-        bool k_quants = true;
-        for (size_t j = 0; j < n_jobs; ++j) {
-            w_total += jobs[j].F * mcu_row_bytes(jobs[j].kind, K);
-            k_quants = k_quants && (jobs[j].kind == KIND_Q4_K || jobs[j].kind == KIND_Q6_K);
+        // A handful of tokens on K-quant matrices: the integer tensor-core kernel, one launch per kind, with the prologue in
+        // its activation staging (8 tokens, 2 x 14336 x 4096 Q4_K, add + RMSNorm: 43 us, 36 here).
+        bool integer = integer_jobs_supported(specs, (int)n_jobs, K) && (pr.op == MCU_PROLOGUE_NONE || contiguous);
+        for (size_t j = 0; j < n_jobs && integer; ++j) {
+            size_t values = 0;
+            for (size_t i = 0; i < n_jobs; ++i) values += specs[i].kind == specs[j].kind ? K * (size_t)specs[i].F : 0;
+            integer = integer_pays(ctx, specs[j].kind, T, values);
         }
-        static const bool no_i8 = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch, as in linear_locked
-        const bool integer_mma_pays = ctx->regime == MCU_REGIME_AUTO && !no_i8 && T >= 5 && k_quants &&
-            w_total >= ((size_t)24 << 20) && (pr.op == MCU_PROLOGUE_NONE || contiguous);
-        if (!integer_mma_pays && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
+        if (!integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
             gemv_stream_jobs_supported(specs, (int)n_jobs, (int)T, (int)K, gp)) {
             MCU_CUDA(launch_gemv_stream_jobs(specs, (int)n_jobs, x_dev, (int)ldx, (int)T, (int)K, gp, ctx->dev_err, ctx->stream));
             count_launches(1);
             return MCU_SUCCESS;
         }
-        // More than eight tokens on the tensor cores: one staging launch (the prologue folded into it) feeds every
+        // More tokens on the tensor cores: one staging launch (the prologue folded into it) feeds every
         // matmul that wants the same staging; weights of the other block format class get a second one.
-        bool tensor = (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > 16 &&
+        bool tensor = !integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > 16 &&
             (pr.op == MCU_PROLOGUE_NONE || contiguous);
         for (size_t j = 0; j < n_jobs && tensor; ++j)
             tensor = gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) &&
                 act_half_fused_smem(jobs[j].kind, (int)K) <= 48 * 1024;
-        if (tensor) {
+        if (tensor || integer) {
             ActSource src;
             if (pr.op == MCU_PROLOGUE_ADD_RMSNORM) {
                 src.norm = 1;
@@ -861,6 +878,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
                 src.glu = 1;
             }
             Staged st;
+            int staged_kind = -1;
             // one launch per kind, whatever the order of the jobs
             bool done[GEMV_MAX_JOBS] = {};
             for (size_t j = 0; j < n_jobs; ++j) {
@@ -879,7 +897,9 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
                     use.add = nullptr;  // the sum is already in x_out
                     use.x_out = nullptr;
                 }
-                if (int rc = gemm_locked(ctx, specs[j].kind, again ? src.x_out : x_dev, ldx, T, K, same, n, &use, &st)) return rc;
+                if (integer) {
+                    if (int rc = integer_locked(ctx, specs[j].kind, again ? src.x_out : x_dev, ldx, T, K, same, n, &use, &staged_kind)) return rc;
+                } else if (int rc = gemm_locked(ctx, specs[j].kind, again ? src.x_out : x_dev, ldx, T, K, same, n, &use, &st)) return rc;
             }
             return MCU_SUCCESS;
         }
@@ -1015,16 +1035,79 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     ctx->moe_last_grouped = 0;
     const int renorm = router_weight_policy == MCU_ROUTER_RENORMALIZE_SELECTED;
     MCU_CUDA(launch_moe_route(topk_ids_dev, topk_weights_dev, (int)T, (int)k, (int)E, weights_scale, renorm, rb, s));
-    count_launches(3);
+    count_launches(routes < (size_t)MOE_ROUTE_SMALL && E <= (size_t)MOE_ROUTE_SMALL_E ? 1 : 3);
     float *route_hidden = (float *)ctx->moe_hidden.ptr, *gate_out = (float *)ctx->moe_gate.ptr;
     float *up_out = (float *)ctx->moe_up.ptr;
     float *route_down = routed_rows_ext != nullptr ? routed_rows_ext : (float *)ctx->moe_down.ptr;
-    // Large batches: one grouped launch per projection over all local experts, sized from the device-resident counts.
-    // Nothing is read back, so the call neither waits for the device nor breaks a stream capture.
+    const ActSource from_hidden = [&] {
+        ActSource src;
+        src.row_index = rb.sorted_tok;
+        src.row_lo = rb.offsets + e_begin;
+        src.row_hi = rb.offsets + e_begin + e_count;
+        return src;
+    }();
+    const ActSource from_glu = [&] {
+        ActSource src;
+        src.row_lo = rb.offsets + e_begin;
+        src.row_hi = rb.offsets + e_begin + e_count;
+        src.x2 = up_out;
+        src.glu = ffn_type == MCU_FFN_GEGLU ? 2 : 1;
+        return src;
+    }();
+    const GemvJobSpec gate_up[2] = {{gate_kind, gate_dev, (int)FF, nullptr, gate_out, (int)FF}, {up_kind, up_dev, (int)FF, nullptr, up_out, (int)FF}};
+    const GemvJobSpec down_job = {down_kind, down_dev, (int)H, nullptr, route_down, (int)H};
+    const int *cnt = rb.counts + e_begin, *off = rb.offsets + e_begin;
     static const bool no_grouped = getenv("MARMOT_CUDA_MOE_NO_GROUPED") != nullptr;  // diagnostic switch
-    // Fewer routes normally take per-expert launches sized from counts read back on the host (small groups then get the
-    // GEMV kernels); a call that is being recorded into a CUDA graph cannot read anything back, so it takes the grouped
-    // launches whatever its size.
+    // Few routes (a decode batch): the integer tensor-core kernel over all local experts, one launch for gate and up, one for
+    // down, tiles of sixteen tokens sized from the device-resident counts; exact sub-block dots, as the per-expert launches
+    // below (16 tokens, top 2 of 8 experts of 3 x 14336 x 4096: 480 us with those, which wait for the counts on the host, 244 here).
+    const bool few = !no_grouped && routes < 256 && routed_rows_ext == nullptr && gate_kind == up_kind && e_count <= (size_t)TS_MAX_GROUPS &&
+        integer_jobs_supported(gate_up, 2, H) && integer_jobs_supported(&down_job, 1, FF) && gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
+        gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) && gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H);
+    if (few) {
+        const bool capturing = stream_is_capturing(s);
+        // A bad expert id is reported by the call itself, as ever for few routes: the flag is fetched behind the routing and
+        // waited for once everything is enqueued, so that the device does not wait for the host.
+        int *flag_host = ctx->err_host != nullptr ? ctx->err_host + 1 : nullptr;
+        if (!capturing && flag_host != nullptr) {
+            if (ctx->moe_event == nullptr) MCU_CUDA(cudaEventCreateWithFlags(&ctx->moe_event, cudaEventDisableTiming));
+            MCU_CUDA(cudaMemcpyAsync(flag_host, rb.counts + E, sizeof(int), cudaMemcpyDeviceToHost, s));
+            MCU_CUDA(cudaEventRecord(ctx->moe_event, s));
+        }
+        const size_t xq_h = gemm_ti_xq_bytes(gate_kind, (int)routes, (int)H), xq_f = gemm_ti_xq_bytes(down_kind, (int)routes, (int)FF);
+        const size_t nb_max = ((H > FF ? H : FF) + QK_K - 1) / QK_K;
+        if (int rc = ensure(ctx, ctx->act_qs, xq_h > xq_f ? xq_h : xq_f)) return rc;
+        if (int rc = ensure(ctx, ctx->act_d, routes * nb_max * sizeof(float))) return rc;
+        if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+        uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
+        float *dT = (float *)ctx->act_d.ptr, *part = (float *)ctx->gemm_partial.ptr;
+        MCU_CUDA(launch_act_int_fused(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xq, dT, s));
+        MCU_CUDA(launch_gemm_ti_grouped(gate_kind, gate_up, 2, (int)e_count, xq, dT, (int)routes, (int)H, cnt, off, INT_MAX, part,
+                                        ctx->gemm_counters, ctx->dev_err, s));
+        ActSource down_src = from_glu;
+        down_src.x_out = gate_out;  // (gate_out holds act(gate) * up afterwards, as with the per-expert launches)
+        MCU_CUDA(launch_act_int_fused(down_kind, gate_out, (int)FF, down_src, (int)routes, (int)FF, xq, dT, s));
+        MCU_CUDA(launch_gemm_ti_grouped(down_kind, &down_job, 1, (int)e_count, xq, dT, (int)routes, (int)FF, cnt, off, INT_MAX, part,
+                                        ctx->gemm_counters, ctx->dev_err, s));
+        MCU_CUDA(launch_moe_combine_dev(route_down, rb.sorted_w, rb.route_pos, (int)T, (int)k, (int)H, rb.offsets, (int)e_begin,
+                                        (int)(e_begin + e_count), rb.counts + E, capturing ? ctx->dev_err : nullptr, out_dev, H, s));
+        count_launches(5);
+        if (capturing) return MCU_SUCCESS;
+        int bad = 0;
+        if (flag_host != nullptr) {
+            MCU_CUDA(cudaEventSynchronize(ctx->moe_event));
+            bad = *(volatile int *)flag_host;
+        } else {
+            MCU_CUDA(cudaStreamSynchronize(s));
+            MCU_CUDA(cudaMemcpy(&bad, rb.counts + E, sizeof(int), cudaMemcpyDeviceToHost));
+        }
+        return bad != 0 ? fail(MCU_ERROR_INVALID_ARGUMENT, "MoE expert id is out of range") : MCU_SUCCESS;
+    }
+    // Large batches: grouped launches over all local experts, sized from the device-resident counts.
+    // Nothing is read back, so the call neither waits for the device nor breaks a stream capture.
+    // Fewer routes that the integer kernel does not take have per-expert launches sized from counts read back on the host
+    // (small groups then get the GEMV kernels); a call that is being recorded into a CUDA graph cannot read anything back, so it
+    // takes the grouped launches whatever its size.
     const bool grouped = !no_grouped && (routes >= 256 || stream_is_capturing(s) || routed_rows_ext != nullptr) &&
         gate_kind == up_kind &&
         gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
@@ -1040,27 +1123,19 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
         if (int rc = ensure(ctx, ctx->act_rowscale, routes * sizeof(float))) return rc;
         __half *xh = (__half *)ctx->act_half.ptr;
         float *rowscale = (float *)ctx->act_rowscale.ptr;
-        const int *cnt = rb.counts + e_begin, *off = rb.offsets + e_begin;
         // The staging kernels fetch their rows themselves: the routed token's hidden row for gate/up, act(gate) * up
         // for down.  Routes of other ranks' experts (outside [offsets[e_begin], offsets[e_end])) are skipped there,
         // never multiplied and never combined.
-        ActSource from_hidden, from_glu;
-        from_hidden.row_index = rb.sorted_tok;
-        from_hidden.row_lo = from_glu.row_lo = rb.offsets + e_begin;
-        from_hidden.row_hi = from_glu.row_hi = rb.offsets + e_begin + e_count;
-        from_glu.x2 = up_out;
-        from_glu.glu = ffn_type == MCU_FFN_GEGLU ? 2 : 1;
         if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
         float *part = (float *)ctx->gemm_partial.ptr;
         int *tick = ctx->gemm_counters;
         MCU_CUDA(launch_act_half_fused_from(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xh, rowscale, s));
-        MCU_CUDA(launch_gemm_ts_grouped(gate_kind, gate_dev, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, (int)FF,
-                                        cnt, off, gate_out, (int)FF, part, tick, ctx->dev_err, s));
-        MCU_CUDA(launch_gemm_ts_grouped(up_kind, up_dev, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, (int)FF, cnt,
-                                        off, up_out, (int)FF, part, tick, ctx->dev_err, s));
+        for (int j = 0; j < 2; ++j)
+            MCU_CUDA(launch_gemm_ts_grouped(gate_kind, &gate_up[j], 1, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, cnt,
+                                            off, 1, part, tick, ctx->dev_err, s));
         MCU_CUDA(launch_act_half_fused_from(down_kind, gate_out, (int)FF, from_glu, (int)routes, (int)FF, xh, rowscale, s));
-        MCU_CUDA(launch_gemm_ts_grouped(down_kind, down_dev, (int)e_count, xh, rowscale, (int)kp_f, (int)routes, (int)FF, (int)H,
-                                        cnt, off, route_down, (int)H, part, tick, ctx->dev_err, s));
+        MCU_CUDA(launch_gemm_ts_grouped(down_kind, &down_job, 1, (int)e_count, xh, rowscale, (int)kp_f, (int)routes, (int)FF, cnt, off, 1,
+                                        part, tick, ctx->dev_err, s));
         if (routed_rows_ext == nullptr) {
             MCU_CUDA(launch_moe_combine_dev(route_down, rb.sorted_w, rb.route_pos, (int)T, (int)k, (int)H, rb.offsets,
                                             (int)e_begin, (int)(e_begin + e_count), rb.counts + E, ctx->dev_err, out_dev, H, s));

@@ -179,25 +179,16 @@ __device__ __forceinline__ void stage_group16(const int8_t *q16, float sc, __hal
     d[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
+// Quantise row t (of the staged matrix) block by block, exactly as the kernels above: values to q_s, scales to d_s (shared
+// memory).  False when the row is not this rank's.
 // GLU: 0 = the row as it is; 1 = silu(x) * x2; 2 = gelu(x) * x2.  The SiLU uses the fast exponential and division
 // (relative error about 1e-6): its result is quantised to eight bits right here, three orders of magnitude coarser.
-// Few rows: up to a thousand threads per row, so that a row is one or two trips to L2 (latency bounds the launch: 64 rows of
-// 4096 values 3.3 us with 256 threads); many rows: 256 threads, and as many rows at a time.
+// 3 = SiLU with the separately rounded exponential and division of the stand-alone kernels.
 template <bool KQ, int GLU>
-__global__ void __launch_bounds__(1024)
-act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb,
-                      __half *__restrict__ xh, float *__restrict__ rowscale) {
-    extern __shared__ __align__(16) uint8_t act_sm[];
-    constexpr int BV = KQ ? QK_K : Q8_0_VALUES;
-    const int kp = nb * BV;
-    int8_t *q_s = (int8_t *)act_sm;
-    float *d_s = (float *)(act_sm + ((kp + 15) & ~15));
-    __shared__ float red[32];
-    __shared__ float inv_s;
-    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (src.row_lo != nullptr && (t < *src.row_lo || t >= *src.row_hi)) return;  // not this rank's row
+__device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ldx, const ActSource &src, int K, int nb, int t,
+                                             int8_t *q_s, float *d_s, float *red, float &inv_s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    if (src.row_lo != nullptr && (t < *src.row_lo || t >= *src.row_hi)) return false;  // not this rank's row
     const size_t row_off = (size_t)(src.row_index != nullptr ? src.row_index[t] : t) * ldx;
     const float *xrow = x + row_off;
     const float *urow = GLU != 0 ? src.x2 + row_off : nullptr;
@@ -241,6 +232,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
         if constexpr (GLU == 0) return g;
         float a;
         if constexpr (GLU == 2) a = __fmul_rn(__fmul_rn(0.5f, g), __fadd_rn(1.0f, erff(__fmul_rn(g, 0.7071067811865475f))));
+        else if constexpr (GLU == 3) a = __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)));
         else a = __fdividef(g, __fadd_rn(1.0f, __expf(-g)));
         return __fmul_rn(a, urow[k]);
     };
@@ -254,6 +246,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
             for (int i = 0; i < 8; ++i) {
                 const int idx = lane + 32 * i;
                 v[i] = idx < len ? value(blk * QK_K + idx) : 0.0f;
+                if (GLU != 0 && src.x_out != nullptr && idx < len) src.x_out[row_off + blk * QK_K + idx] = v[i];
                 const float a = fabsf(v[i]);
                 if (a > best_abs) {
                     best_abs = a;
@@ -300,6 +293,26 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
             if (lane == 0) d_s[blk] = __half2float(__float2half_rn(scale));
         }
     }
+    return true;
+}
+
+// Few rows: up to a thousand threads per row, so that a row is one or two trips to L2 (latency bounds the launch: 64 rows of
+// 4096 values 3.3 us with 256 threads); many rows: 256 threads, and as many rows at a time.
+template <bool KQ, int GLU>
+__global__ void __launch_bounds__(1024)
+act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, __half *__restrict__ xh,
+                      float *__restrict__ rowscale) {
+    extern __shared__ __align__(16) uint8_t act_sm[];
+    constexpr int BV = KQ ? QK_K : Q8_0_VALUES;
+    const int kp = nb * BV;
+    int8_t *q_s = (int8_t *)act_sm;
+    float *d_s = (float *)(act_sm + ((kp + 15) & ~15));
+    __shared__ float red[32];
+    __shared__ float inv_s;
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!quantize_row<KQ, GLU>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
     __syncthreads();
     float m = 0.0f;
     for (int b = threadIdx.x; b < nb; b += blockDim.x) m = fmaxf(m, fabsf(d_s[b]));
@@ -326,6 +339,53 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
     for (int g = threadIdx.x; g < kp / 16; g += blockDim.x) {
         const float sc = __fmul_rn(d_s[(16 * g) / BV], inv);
         stage_group16(q_s + 16 * g, sc, hrow + 16 * g);
+    }
+}
+
+// The operands of the integer tensor-core matmul (gemm_ti.cu) for K-quants: per row and 256-value block 384 bytes, the 256
+// quants, then the sums of its sub-blocks split as 64 * hi + lo into 8-bit values (lo from byte 256, hi from byte 288 on).
+// SUB = 32 (Q4_K: eight sums) or 16 (Q6_K: sixteen sums, and two planes of quants, in which the even / the odd sub-blocks are
+// zero: the matmul multiplies 32 values at a time and needs the sums of 16).  dT[block][row]: the block scales.
+template <int SUB, int GLU>
+__global__ void __launch_bounds__(1024)
+act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, uint8_t *__restrict__ xq, size_t plane,
+                     float *__restrict__ dT, int ld_dT) {
+    extern __shared__ __align__(16) uint8_t act_sm[];
+    int8_t *q_s = (int8_t *)act_sm;
+    float *d_s = (float *)(act_sm + nb * QK_K);
+    __shared__ float red[32];
+    __shared__ float inv_s;
+    const int t = blockIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!quantize_row<true, GLU>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
+    __syncthreads();
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) dT[(size_t)b * ld_dT + t] = d_s[b];
+    uint8_t *row = xq + (size_t)t * nb * 384;
+    for (int g = threadIdx.x; g < nb * 16; g += blockDim.x) {  // sixteen values
+        const int blk = g >> 4, i = g & 15;
+        const uint4 v = *(const uint4 *)(q_s + 16 * g);
+        int sum = __dp4a((int)v.x, 0x01010101, __dp4a((int)v.y, 0x01010101, __dp4a((int)v.z, 0x01010101, __dp4a((int)v.w, 0x01010101, 0))));
+        uint8_t *o = row + blk * 384;
+        if (SUB == 16) {
+            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+            *(uint4 *)(o + 16 * i) = i & 1 ? zero : v;
+            *(uint4 *)(o + plane + 16 * i) = i & 1 ? v : zero;
+        } else {
+            *(uint4 *)(o + 16 * i) = v;
+            sum += __shfl_xor_sync(__activemask(), sum, 1);  // (the lanes of a pair are always here together)
+        }
+        const int at = SUB == 16 ? i : i >> 1, lo = sum & 63;
+        if (SUB == 16 || (i & 1) == 0) {
+            o[256 + at] = (uint8_t)lo;
+            o[288 + at] = (uint8_t)((sum - lo) >> 6);
+        }
+        // the rest of the two 32-byte groups is zero
+        if (SUB == 16 || (i & 1) != 0) {
+            const int z = SUB == 16 ? 16 + i : 8 + 3 * at;
+#pragma unroll
+            for (int n = 0; n < (SUB == 16 ? 1 : 3); ++n) o[256 + z + n] = o[288 + z + n] = 0;
+        }
     }
 }
 
@@ -359,6 +419,28 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
     if (glu == 0) return kq ? MCU_STAGE(true, 0) : MCU_STAGE(false, 0);
     if (glu == 1) return kq ? MCU_STAGE(true, 1) : MCU_STAGE(false, 1);
     return kq ? MCU_STAGE(true, 2) : MCU_STAGE(false, 2);
+#undef MCU_STAGE
+}
+
+cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSource &src, int rows, int K, uint8_t *xq, float *dT,
+                                 cudaStream_t s) {
+    if (rows <= 0) return cudaSuccess;
+    const int nb = (K + QK_K - 1) / QK_K;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)rows, 1, 1);
+    cfg.blockDim = dim3((unsigned)(32 * (nb < 8 ? 8 : nb > 32 ? 32 : nb)), 1, 1);
+    cfg.dynamicSmemBytes = act_half_fused_smem(kind, K);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const size_t plane = (size_t)rows * nb * 384;
+    const int glu = src.x2 != nullptr ? (src.glu == 2 ? 2 : 1) : 0;
+#define MCU_STAGE(SUB, GLU) cudaLaunchKernelEx(&cfg, act_int_fused_kernel<SUB, GLU>, x, ldx, src, K, nb, xq, plane, dT, rows)
+    if (kind == KIND_Q6_K) return glu == 0 ? MCU_STAGE(16, 0) : glu == 1 ? MCU_STAGE(16, 3) : MCU_STAGE(16, 2);
+    return glu == 0 ? MCU_STAGE(32, 0) : glu == 1 ? MCU_STAGE(32, 3) : MCU_STAGE(32, 2);
 #undef MCU_STAGE
 }
 

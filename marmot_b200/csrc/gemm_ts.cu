@@ -26,20 +26,20 @@
 // draws the last ticket, in a fixed order; nobody waits for another CTA (kernels on several streams may share the device).
 // Every mbarrier wait is bounded; no TMA multicast.
 #include "common.cuh"
-#include "gemm_ts.h"
+#include "gemm_ts_dev.cuh"
 #include "kernels.h"
 #include "tma_utils.cuh"
 
 #include <cuda.h>
 
 #include <atomic>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
 
 namespace mcu {
 
-constexpr int TS_ROWS = 128;    // weight rows per CTA (TMEM lanes)
 constexpr int TS_BK = 128;      // values of K per stage, half a slab: eight MMAs per barrier wait and commit (see the issuer)
 constexpr int TS_STAGES = 4;    // = converter groups: group g owns stage slot g, so every barrier phase is seen in order
 constexpr int TS_SLAB_STAGES = 256 / TS_BK;
@@ -47,78 +47,13 @@ constexpr int TS_CONV = 16;     // converter warps
 constexpr int TS_MMA_WARP = TS_CONV, TS_B_WARP = TS_CONV + 1, TS_W_WARP = TS_CONV + 2;
 constexpr int TS_THREADS = (TS_W_WARP + 1) * 32;
 constexpr int TS_D_COLS = 256;  // accumulator columns; the A ring (4 x 64 columns) follows
-constexpr int TS_SLAB_K = 256;
 
-// A slab in shared memory: BYTES of every row, BOX bytes fetched (a 16-byte aligned window that covers them) and the pitch.  The
-// pitch is an odd number of 16-byte units, so that 16-byte loads of a warp's 32 rows are conflict free.
-template <int KIND>
-struct TsSlab;
-template <>
-struct TsSlab<KIND_Q4_K> {
-    static constexpr int BYTES = 144, PITCH = 144, LOOSE_PITCH = 144;
-};
-template <>
-struct TsSlab<KIND_Q6_K> {
-    static constexpr int BYTES = 210, PITCH = 240, LOOSE_PITCH = 240;
-};
-template <>
-struct TsSlab<KIND_Q8_0> {
-    static constexpr int BYTES = 272, PITCH = 272, LOOSE_PITCH = 304;  // loose: rows that start anywhere
-};
-template <int KIND>
-constexpr int ts_slab_bytes(bool loose) {  // loose slabs keep the up to seven last rows of the matrix behind the 128
-    return ((loose ? (TS_ROWS + 8) * TsSlab<KIND>::LOOSE_PITCH : TS_ROWS * TsSlab<KIND>::PITCH) + 16 + 127) / 128 * 128;
-}
-
-// ---- PTX wrappers ----
-__device__ __forceinline__ void ts_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t ts_mapa(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-// Bounded wait.
-__device__ __forceinline__ bool ts_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < 1u << 17; ++i) {  // a try suspends the thread for up to 20 us
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
 // D += A * B, A in tensor memory (two fp16 per 32-bit column), B in shared memory.
 __device__ __forceinline__ void ts_mma(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
-__device__ __forceinline__ void ts_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
-        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]),
-        "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-__device__ __forceinline__ void ts_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-
 // ---- converters: 128 values of one weight row (half `n` of a 256-value slab) as 64 packed-half columns, K order (0, 2, 1, 3)
 //      inside every group of four.  Everything is read from the slab first and the slab released (`done`),
 //      so that its refill overlaps the arithmetic; `emit` gets the columns in two halves. ----
@@ -282,13 +217,6 @@ __device__ __forceinline__ void ts_store16(float *outp, int ldo, int col0, int c
     }
 }
 
-// One output tile: which weights, which tokens, where the result goes.
-struct TsTile {
-    int job, f0, rows;       // rows that exist
-    int w_row0;              // first weight row in the (stacked) matrix
-    int t_row0, t_count;     // first activation / output row, and how many of the BN columns are tokens
-};
-
 template <int KIND>
 __global__ void __launch_bounds__(TS_THREADS, 1)
 gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsParams p) {
@@ -338,21 +266,7 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (grouped && warp == TS_W_WARP) {
-        // The counts were written by kernels that finished before the kernel ahead of this one started (they do not trigger
-        // their dependents early), so they may be read before griddepcontrol.wait.
-        int base = 0;
-        for (int g0 = 0; g0 < p.groups; g0 += 32) {
-            const int g = g0 + lane;
-            int n = g < p.groups ? (p.group_counts[g] + bn - 1) / bn * p.row_tiles : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, n, o);
-                if (lane >= o) n += up;
-            }
-            if (g < p.groups) group_tile0[g + 1] = base + n;
-            base += __shfl_sync(0xffffffffu, n, 31);
-        }
-        if (lane == 0) group_tile0[0] = 0;
+        ts_group_table(p, bn, group_tile0, lane);
     }
     if (warp == TS_MMA_WARP)  // (all columns are taken: the permit to allocate need not be given back)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(tm_smem_u32(&tmem_slot)) : "memory");
@@ -362,49 +276,10 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     const uint32_t tmem = tmem_slot;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // ---- this CTA's share of the units ----
-    const int KS = p.slabs;
-    const int tiles = grouped ? group_tile0[p.groups] : p.tiles;
-    const long long U = (long long)tiles * KS;
-    const int n_use = (int)min((long long)n_cta, U);  // (a grouped launch may find fewer units than CTAs)
-    int u0 = cta < n_use ? (int)(U * cta / n_use) : 0, u1 = cta < n_use ? (int)(U * (cta + 1) / n_use) : 0;
-    if (split > 1) {
-        const int t = cta / split, part = cta - t * split;
-        u0 = t * KS + KS * part / split;
-        u1 = t * KS + KS * (part + 1) / split;
-    }
-
-    auto tile_of = [&](int tile) -> TsTile {
-        TsTile t;
-        int rt, tt, T_here, row_off, cols = bn;
-        t.job = 0;
-        if (grouped) {
-            int g = 0;
-            while (tile >= group_tile0[g + 1]) ++g;
-            const int in = tile - group_tile0[g], t_tiles = (group_tile0[g + 1] - group_tile0[g]) / p.row_tiles;
-            rt = in / t_tiles;
-            tt = in - rt * t_tiles;
-            T_here = p.group_counts[g];
-            row_off = p.group_offsets[g];
-            cols = ((T_here + t_tiles - 1) / t_tiles + 15) & ~15;  // the group's tokens dealt evenly to its tiles
-            t.w_row0 = g * p.jobs[0].F;
-        } else {
-            rt = tile / p.t_tiles;
-            tt = tile - rt * p.t_tiles;
-            while (t.job + 1 < p.n_jobs && rt >= p.jobs[t.job + 1].row_tile0) ++t.job;
-            rt -= p.jobs[t.job].row_tile0;
-            T_here = p.T;
-            row_off = 0;
-            t.w_row0 = 0;
-        }
-        t.f0 = rt * TS_ROWS;
-        t.w_row0 += t.f0;
-        t.rows = min(TS_ROWS, p.jobs[t.job].F - t.f0);
-        t.t_row0 = row_off + tt * cols;
-        t.t_count = min(cols, T_here - tt * cols);
-        return t;
-    };
-
+    const TsWork work = ts_work(p, grouped, group_tile0, bn, cta, n_cta);
+    const int KS = p.slabs, u0 = work.u0, u1 = work.u1, n_use = work.n_use;
+    const long long U = work.units;
+    auto tile_of = [&](int tile) { return work.tile(p, tile); };
 
     bool ok = true;
     int err_code = 0;
@@ -435,44 +310,7 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
         __syncwarp();
     } else if (warp == TS_W_WARP) {
         // ------------------------------ packed weight slabs ------------------------------
-        uint32_t j = 0;
-        for (int u = u0; u < u1 && ok;) {
-            const int tile = u / KS, k_lo = u - tile * KS, k_hi = min(KS, k_lo + (u1 - u));
-            const TsTile t = tile_of(tile);
-            const TsJob &jb = p.jobs[t.job];
-            const int rest0 = jb.F & ~7;  // loose rows: the last ones, not a whole group of eight, are fetched with plain loads
-            const int rest_lo = max(t.f0, rest0), rest_hi = loose ? min(jb.F, t.f0 + TS_ROWS) : rest_lo;
-            for (int k = k_lo; k < k_hi; ++k, ++j) {
-                const uint32_t rs = j & (R - 1u), use = j >> p.raw_shift;
-                if (use >= 1) ok = ts_wait(raw_empty + 8u * rs, (use - 1) & 1u);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                const uint32_t dst = ring_addr + rs * SLAB, bar = raw_full + 8u * rs;
-                for (int f = rest_lo; f < rest_hi; ++f) {
-                    const uintptr_t row = (uintptr_t)jb.w + (size_t)f * p.row_bytes + (size_t)k * SL::BYTES;
-                    const int bytes = min(SL::BYTES, (int)(p.row_bytes - (long)k * SL::BYTES)) + (int)(row & 3u);
-                    uint8_t *to = ring + (size_t)rs * SLAB + (size_t)(TS_ROWS + f - rest0) * SL::LOOSE_PITCH;
-                    for (int w = lane; 4 * w < bytes; w += 32) *(uint32_t *)(to + 4 * w) = *(const uint32_t *)((row & ~(uintptr_t)3) + 4 * w);
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    if (!loose) {
-                        tm_mbar_expect_tx(bar, (uint32_t)(TS_ROWS * SL::PITCH));
-                        const int x = KIND == KIND_Q8_0 ? k * (SL::BYTES / 4) : (k * SL::BYTES) & ~15;
-                        tm_tma_load_2d(dst, &maps.w[t.job], x, t.w_row0, bar);
-                    } else {
-                        tm_mbar_expect_tx(bar, (uint32_t)(TS_ROWS * SL::LOOSE_PITCH));
-                        const uint32_t shift = (uint32_t)((uintptr_t)jb.w & 15u);
-                        for (int e = 0; e < 8; ++e) {
-                            const long at = (long)shift + (long)e * p.row_bytes + (long)k * SL::BYTES;
-                            const int x = (int)(at & ~15l) / (KIND == KIND_Q8_0 ? 4 : 1);
-                            tm_tma_load_2d(dst + (uint32_t)(e * (TS_ROWS / 8) * SL::LOOSE_PITCH), &maps.w[t.job], x, t.w_row0 >> 3, bar);
-                        }
-                    }
-                }
-            }
-            u += k_hi - k_lo;
-        }
+        ok = ts_stream_slabs<KIND>(maps, p, work, loose, ring_addr, ring, SLAB, raw_full, raw_empty, lane);
         err_code = 10;
         __syncwarp();
     } else if (warp == TS_MMA_WARP) {
@@ -793,8 +631,9 @@ static TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles) {
     };
     if (tiles <= room) consider(1, tiles, KS * unit + tile_end);
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2) {
-        // clusters are placed inside a GPC (16 to 20 SMs): a few SMs stay out
-        const int usable = sp >= 8 ? room * 7 / 8 : room;
+        // A cluster is placed inside a GPC (16 to 20 SMs): sixteen clusters of eight did not run at once (2048 x 2048: 12.6 us,
+        // 64 CTAs in clusters of four 7.5).
+        const int usable = sp >= 8 ? room / 2 : room;
         if ((long)tiles * sp <= usable) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + tile_end + 1000.0);
     }
     const long n = U < room ? U : room;
@@ -833,10 +672,7 @@ bool gemm_ts_supported(int kind, const void *W, int T, int K, int F) {
     return kind != KIND_Q4_K || (((uintptr_t)W & 15) == 0 && rb % 16 == 0);
 }
 
-// Tensor map of a weight matrix: [rows][row bytes], or, for rows that are not 16-byte multiples, [rows / 8][eight rows].
-static cudaError_t ts_encode_weights(int kind, CUtensorMap *m, const void *W, long row_bytes, size_t rows, bool loose);
-
-static bool ts_loose(int kind, const void *W, long row_bytes) {
+bool ts_loose(int kind, const void *W, long row_bytes) {
     return kind != KIND_Q4_K && (((uintptr_t)W & 15) != 0 || row_bytes % 16 != 0);
 }
 
@@ -879,7 +715,7 @@ static cudaError_t ts_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_
     }
 }
 
-static cudaError_t ts_encode(CUtensorMap *m, CUtensorMapDataType type, const void *base, cuuint64_t d0, cuuint64_t d1,
+cudaError_t ts_encode(CUtensorMap *m, CUtensorMapDataType type, const void *base, cuuint64_t d0, cuuint64_t d1,
                              cuuint64_t stride, cuuint32_t b0, cuuint32_t b1, CUtensorMapSwizzle sw) {
     const cuuint64_t dims[2] = {d0, d1}, strides[1] = {stride};
     const cuuint32_t box[2] = {b0, b1}, es[2] = {1, 1};
@@ -889,7 +725,8 @@ static cudaError_t ts_encode(CUtensorMap *m, CUtensorMapDataType type, const voi
         : cudaErrorInvalidValue;
 }
 
-static cudaError_t ts_encode_weights(int kind, CUtensorMap *m, const void *W, long row_bytes, size_t rows, bool loose) {
+// Tensor map of a weight matrix: [rows][row bytes], or, for rows that are not 16-byte multiples, [rows / 8][eight rows].
+cudaError_t ts_encode_weights(int kind, CUtensorMap *m, const void *W, long row_bytes, size_t rows, bool loose) {
     const int unit = kind == KIND_Q8_0 ? 4 : 1;  // a box is at most 256 elements wide
     const CUtensorMapDataType type = kind == KIND_Q8_0 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
     if (!loose) {
@@ -945,29 +782,63 @@ bool gemm_ts_grouped_supported(int kind, const void *W, int K, int F) {
     return F % 8 == 0 || !ts_loose(kind, W, (long)((K + block_values(kind) - 1) / block_values(kind)) * block_bytes(kind));
 }
 
-// n_groups matmuls over a stacked weight matrix (MoE experts): group g multiplies its group_counts[g] rows of xh (from row
-// group_offsets[g], both device data) with the weight rows [g * F, (g + 1) * F).
-cudaError_t launch_gemm_ts_grouped(int kind, const void *W, int n_groups, const __half *xh, const float *rowscale, int ldxh,
-                                   int total_rows, int K, int F, const int *group_counts, const int *group_offsets, float *out,
-                                   int ldo, float *partial, int *counters, int *err_flag, cudaStream_t s) {
+// What grouped launches share: the weights and the tiles (activations and their map are the caller's).
+cudaError_t ts_grouped_params(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, int total_rows, int K,
+                              const int *group_counts, const int *group_offsets, int count_lo, int count_hi, TsParams &p, TsMaps &maps) {
+    memset(&p, 0, sizeof(p));
+    p.nb = (K + block_values(kind) - 1) / block_values(kind);
+    p.row_bytes = (long)p.nb * block_bytes(kind);
+    p.slabs = (p.nb * block_values(kind) + TS_SLAB_K - 1) / TS_SLAB_K;
+    p.n_jobs = n_jobs;
+    p.split = 1;
+    p.T = total_rows;
+    p.groups = n_groups;
+    p.count_lo = count_lo;
+    p.count_hi = count_hi;
+    p.group_counts = group_counts;
+    p.group_offsets = group_offsets;
+    for (int j = 0; j < n_jobs; ++j) {
+        p.loose |= ts_loose(kind, jobs[j].W, p.row_bytes);
+        if (!gemm_ts_grouped_supported(kind, jobs[j].W, K, jobs[j].F)) return cudaErrorNotSupported;
+    }
+    if (p.loose)
+        for (int j = 0; j < n_jobs; ++j)
+            if (jobs[j].F % 8 != 0) return cudaErrorNotSupported;
+    for (int j = 0; j < n_jobs; ++j) {
+        p.jobs[j] = TsJob{(const uint8_t *)jobs[j].W, jobs[j].out, jobs[j].bias, jobs[j].F, jobs[j].ldo, p.row_tiles};
+        p.row_tiles += (jobs[j].F + TS_ROWS - 1) / TS_ROWS;
+        if (cudaError_t e = ts_encode_weights(kind, &maps.w[j], jobs[j].W, p.row_bytes, (size_t)jobs[j].F * n_groups, p.loose != 0))
+            return e;
+    }
+    return cudaSuccess;
+}
+
+// n_groups matmuls over stacked weight matrices (MoE experts): group g multiplies its group_counts[g] rows of xh (from row
+// group_offsets[g], both device data) with the weight rows [g * F, (g + 1) * F) of every job.
+cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const __half *xh, const float *rowscale,
+                                   int ldxh, int total_rows, int K, const int *group_counts, const int *group_offsets, int count_lo,
+                                   float *partial, int *counters, int *err_flag, cudaStream_t s) {
     if (n_groups <= 0 || total_rows <= 0) return cudaSuccess;
+    if (n_jobs < 1 || n_jobs > TS_MAX_JOBS) return cudaErrorInvalidValue;
     if (n_groups > TS_MAX_GROUPS) {  // the kernel keeps a table of the groups' tiles
-        const size_t part = (size_t)TS_MAX_GROUPS * F * ((K + block_values(kind) - 1) / block_values(kind)) * block_bytes(kind);
         for (int g = 0; g < n_groups; g += TS_MAX_GROUPS) {
             const int n = n_groups - g < TS_MAX_GROUPS ? n_groups - g : TS_MAX_GROUPS;
-            if (cudaError_t e = launch_gemm_ts_grouped(kind, (const uint8_t *)W + g / TS_MAX_GROUPS * part, n, xh, rowscale, ldxh,
-                                                       total_rows, K, F, group_counts + g, group_offsets + g, out, ldo, partial,
-                                                       counters, err_flag, s))
+            GemvJobSpec part[TS_MAX_JOBS];
+            for (int j = 0; j < n_jobs; ++j) {
+                part[j] = jobs[j];
+                part[j].W = (const uint8_t *)jobs[j].W +
+                    (size_t)g * jobs[j].F * ((K + block_values(kind) - 1) / block_values(kind)) * block_bytes(kind);
+            }
+            if (cudaError_t e = launch_gemm_ts_grouped(kind, part, n_jobs, n, xh, rowscale, ldxh, total_rows, K, group_counts + g,
+                                                       group_offsets + g, count_lo, partial, counters, err_flag, s))
                 return e;
         }
         return cudaSuccess;
     }
     TsParams p;
     TsMaps maps;
-    memset(&p, 0, sizeof(p));
-    p.nb = (K + block_values(kind) - 1) / block_values(kind);
-    p.row_bytes = (long)p.nb * block_bytes(kind);
-    p.slabs = (p.nb * block_values(kind) + TS_SLAB_K - 1) / TS_SLAB_K;
+    if (cudaError_t e = ts_grouped_params(kind, jobs, n_jobs, n_groups, total_rows, K, group_counts, group_offsets, count_lo, INT_MAX, p, maps))
+        return e;
     // The counts are not known here: tiles for an even spread, up to 256 tokens.
     const int even = (total_rows + n_groups - 1) / n_groups;
     p.bn = even > 96 ? 256 : even > 48 ? 128 : 64;
@@ -975,17 +846,6 @@ cudaError_t launch_gemm_ts_grouped(int kind, const void *W, int n_groups, const 
     p.partial = partial;
     p.counters = counters;
     p.err = err_flag;
-    p.n_jobs = 1;
-    p.split = 1;
-    p.T = total_rows;
-    p.groups = n_groups;
-    p.group_counts = group_counts;
-    p.group_offsets = group_offsets;
-    p.row_tiles = (F + TS_ROWS - 1) / TS_ROWS;
-    p.jobs[0] = TsJob{(const uint8_t *)W, out, nullptr, F, ldo, 0};
-    p.loose = ts_loose(kind, W, p.row_bytes);
-    if (p.loose && F % 8 != 0) return cudaErrorNotSupported;
-    if (cudaError_t e = ts_encode_weights(kind, &maps.w[0], W, p.row_bytes, (size_t)F * n_groups, p.loose != 0)) return e;
     if (cudaError_t e = ts_encode(&maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, ldxh, total_rows, (cuuint64_t)ldxh * 2, 64,
                                   p.bn, CU_TENSOR_MAP_SWIZZLE_128B))
         return e;

@@ -24,7 +24,7 @@ struct TsJob {
 };
 struct TsParams {
     TsJob jobs[TS_MAX_JOBS];
-    const float *rowscale;  // per-token power-of-two factor undone in the epilogue
+    const float *rowscale;  // fp16: per-token power-of-two factor undone in the epilogue; integers: block scales [block][row]
     float *partial;         // two slots of 128 x bn floats per CTA
     int *counters;          // one ticket per CTA, zero between launches
     int *err;
@@ -35,6 +35,7 @@ struct TsParams {
     int split;              // > 1: clusters of `split` CTAs (pairs) share a tile along K; otherwise ranges of units
     int tiles, t_tiles;     // output tiles in all; token tiles per row tile
     int groups, row_tiles;  // grouped launches: number of groups, row tiles per group
+    int count_lo, count_hi; // grouped launches: groups with a count in this range
 };
 
 // Shares of cut tiles (gemm_ts_workspace_bytes(), 0 tickets in `counters` between launches, one int per SM).
@@ -45,8 +46,28 @@ cudaError_t launch_gemm_ts(int kind, const GemvJobSpec *jobs, int n_jobs, const 
                            int T, int K, float *partial, int *counters, int *err_flag, cudaStream_t s);
 // stacked matrices: rows that are not 16-byte multiples need a multiple of eight rows per group
 bool gemm_ts_grouped_supported(int kind, const void *W, int K, int F);
-cudaError_t launch_gemm_ts_grouped(int kind, const void *W, int n_groups, const __half *xh, const float *rowscale, int ldxh,
-                                   int total_rows, int K, int F, const int *group_counts, const int *group_offsets, float *out,
-                                   int ldo, float *partial, int *counters, int *err_flag, cudaStream_t s);
+cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const __half *xh, const float *rowscale,
+                                   int ldxh, int total_rows, int K, const int *group_counts, const int *group_offsets, int count_lo,
+                                   float *partial, int *counters, int *err_flag, cudaStream_t s);
+
+// The same on integers for a handful of tokens (gemm_ti.cu: Q4_K, Q6_K): exact sub-block dots.  xq / dT from
+// launch_act_int_fused.  The grouped form takes the groups with a count up to count_hi.
+constexpr int TI_COLS = 16;
+constexpr int TI_MAX_K = 65536;
+size_t gemm_ti_xq_bytes(int kind, int rows, int K);
+bool gemm_ti_supported(int kind, const void *W, int K, int F);
+cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const uint8_t *xq, const float *dT, int T, int K,
+                           float *partial, int *counters, int *err_flag, cudaStream_t s);
+cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq, const float *dT,
+                                   int total_rows, int K, const int *group_counts, const int *group_offsets, int count_hi,
+                                   float *partial, int *counters, int *err_flag, cudaStream_t s);
+
+// host helpers of the two
+bool ts_loose(int kind, const void *W, long row_bytes);
+cudaError_t ts_encode(CUtensorMap *m, CUtensorMapDataType type, const void *base, cuuint64_t d0, cuuint64_t d1, cuuint64_t stride,
+                      cuuint32_t b0, cuuint32_t b1, CUtensorMapSwizzle sw);
+cudaError_t ts_encode_weights(int kind, CUtensorMap *m, const void *W, long row_bytes, size_t rows, bool loose);
+cudaError_t ts_grouped_params(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, int total_rows, int K,
+                              const int *group_counts, const int *group_offsets, int count_lo, int count_hi, TsParams &p, TsMaps &maps);
 
 }  // namespace mcu

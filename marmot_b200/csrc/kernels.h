@@ -30,7 +30,7 @@ cudaError_t launch_half_acts(int kind, const ActBuffers &a, int T, int K, __half
 size_t act_half_fused_smem(int kind, int K);
 // Where the staging kernel takes its rows from, for callers that would otherwise run a gather or a GLU pass first:
 // row t comes from x + row_index[t] * ldx when row_index is set; with x2 set the value is act(x) * x2 (glu 1 = SiLU,
-// 2 = GELU, rounded like the MoE GLU kernel); rows outside [*row_lo, *row_hi) (device-resident) are skipped.
+// 2 = GELU, rounded like the MoE GLU kernel), and with K-quants goes to x_out (which may be x) when that is set; rows outside [*row_lo, *row_hi) (device-resident) are skipped.
 // With norm set the row is first x + add (add may be null; the sum goes to x_out when that is set, which may be x
 // itself: a CTA owns its row) and the values are rms_norm(row) * (norm_w + w_off), the operations and their order
 // those of the stand-alone add + RMSNorm kernel.
@@ -46,6 +46,11 @@ struct ActSource {
 };
 cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const ActSource &src, int T, int K,
                                        __half *xh, float *rowscale, cudaStream_t s);
+
+// The same rows as operands of the integer tensor-core matmul (K-quants; layout at the kernel, act_quant.cu): xq
+// [planes][rows][blocks][384] bytes, dT [blocks][rows].
+cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSource &src, int rows, int K, uint8_t *xq, float *dT,
+                                 cudaStream_t s);
 
 // blocks -> f32 (bit-exact with the reference dequantizers)
 cudaError_t launch_dequantize(int kind, const void *blocks, size_t n_values, float *out, cudaStream_t s);
@@ -99,17 +104,6 @@ cudaError_t launch_gemv_stream(int kind, const void *W, const void *W2, const fl
 // (exactly one of out32 / out16 set).  See linear_f16.cu for the Q6_K reading.
 cudaError_t launch_linear_f16(int kind, const void *W, const __half *x, size_t ldx, int T, int K, int F, const float *bias,
                               float *out32, __half *out16, size_t ldo, cudaStream_t s);
-
-// Few-token regime (2 <= T <= 64) on integer tensor-core instructions: activations packed to Q8_K by a first launch,
-// exact int32 sub-block dots (mma.sync s8), f32 scaling per block; Q4_K and Q6_K, rows a multiple of 16 bytes.
-// The caller provides the workspace (sizes from gemm_i8_workspace_bytes); `tickets` must be zero before the first
-// launch and is left zero.
-bool gemm_i8_supported(int kind, const void *W, const void *W2, int T, int K, int F);
-void gemm_i8_workspace_bytes(int T, int K, int F, bool dual, size_t *qs_bytes, size_t *dT_bytes, size_t *partial_bytes,
-                             size_t *ticket_bytes);
-cudaError_t launch_gemm_i8(int kind, const void *W, const void *W2, const float *x, int ldx, int T, int K, int F,
-                           const float *bias, float *out, float *out2, int ldo, int8_t *qs, float *dT, float *partial,
-                           int *tickets, int *err_flag, cudaStream_t s);
 
 // Row-parallel matmul fused with its all-reduce over peer memory (gemm_tma, T <= 64, full 128-row tiles): every CTA
 // that holds a finished output tile stores it into this rank's peer-visible staging buffer, releases one flag per

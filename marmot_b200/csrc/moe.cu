@@ -183,7 +183,7 @@ __global__ void moe_combine_dev_kernel(const float *__restrict__ route_down, con
                                        const int *__restrict__ bad_id_count, int *err, float *__restrict__ out, size_t ldo) {
     const int t = blockIdx.x;
     const int pos_lo = offsets[e_begin], pos_hi = offsets[e_end];
-    if (t == 0 && threadIdx.x == 0 && *bad_id_count != 0) atomicExch(err, 40);
+    if (t == 0 && threadIdx.x == 0 && *bad_id_count != 0 && err != nullptr) atomicExch(err, 40);
     int pos[MAXK];
     float w[MAXK];
     for (int j = 0; j < k; ++j) pos[j] = route_pos[(size_t)t * k + j];
@@ -225,9 +225,82 @@ cudaError_t launch_topk(const float *x, int rows, int cols, size_t ldx, int k, f
     return cudaGetLastError();
 }
 
+// All of the routing in one launch for few routes: counts, offsets, and every route's stable position (the routes ahead of it
+// with the same expert, counted one by one).  The same results as the three kernels above, which cost three launches and a
+// memset: 9 us against 3 at 32 routes.  Does not trigger its dependents early: the grouped matmuls read the counts ahead of
+// griddepcontrol.wait.
+__global__ void __launch_bounds__(MOE_ROUTE_SMALL)
+moe_route_small_kernel(const int32_t *__restrict__ ids, const float *__restrict__ weights, int routes, int k, int E, float weights_scale,
+                       int renormalize, MoeRouteBuffers b) {
+    __shared__ int id_s[MOE_ROUTE_SMALL], count_s[MOE_ROUTE_SMALL_E + 1];
+    const int i = threadIdx.x, lane = i & 31;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int e = i; e <= E; e += blockDim.x) count_s[e] = 0;
+    __syncthreads();
+    int e = -1;
+    if (i < routes) {
+        e = ids[i];
+        if (e < 0 || e >= E) {
+            atomicExch(&count_s[E], 1);
+            b.route_pos[i] = -1;
+            e = -1;
+        } else {
+            atomicAdd(&count_s[e], 1);
+        }
+    }
+    id_s[i] = e;
+    __syncthreads();
+    for (int c = i; c <= E; c += blockDim.x) b.counts[c] = count_s[c];
+    __syncthreads();
+    if (i < 32) {  // exclusive prefix, in place
+        int base = 0;
+        for (int c0 = 0; c0 < E; c0 += 32) {
+            const int c = c0 + lane, mine = c < E ? count_s[c] : 0;
+            int incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (c < E) {
+                count_s[c] = base + incl - mine;
+                b.offsets[c] = base + incl - mine;
+            }
+            base += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) b.offsets[E] = base;
+    }
+    __syncthreads();
+    if (e < 0) return;
+    int pos = count_s[e];
+    for (int j = 0; j < i; ++j) pos += id_s[j] == e ? 1 : 0;
+    const int t = i / k;
+    float norm = weights_scale;
+    if (renormalize) {
+        float s = 0.0f;
+        for (int j = 0; j < k; ++j) s = __fadd_rn(s, weights[(size_t)t * k + j]);
+        norm = s > FLT_MIN ? __fdiv_rn(weights_scale, s) : 0.0f;
+    }
+    b.sorted_tok[pos] = t;
+    b.sorted_w[pos] = __fmul_rn(weights[i], norm);
+    b.route_pos[i] = pos;
+}
+
 cudaError_t launch_moe_route(const int32_t *ids, const float *weights, int T, int k, int E, float weights_scale,
                              int renormalize, const MoeRouteBuffers &b, cudaStream_t s) {
     const int routes = T * k;
+    if (routes < MOE_ROUTE_SMALL && E <= MOE_ROUTE_SMALL_E) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, 1);
+        cfg.blockDim = dim3((unsigned)((routes + 31) / 32 * 32), 1, 1);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, moe_route_small_kernel, ids, weights, routes, k, E, weights_scale, renormalize, b);
+    }
     cudaError_t err = cudaMemsetAsync(b.counts, 0, (size_t)(E + 1) * sizeof(int), s);
     if (err != cudaSuccess) return err;
     moe_count_kernel<<<(routes + 255) / 256, 256, 0, s>>>(ids, routes, E, b.counts, b.counts + E, b.route_pos);

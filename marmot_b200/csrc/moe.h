@@ -8,6 +8,7 @@
 namespace mcu {
 
 constexpr int MOE_MAX_TOPK = 16;
+constexpr int MOE_ROUTE_SMALL = 256, MOE_ROUTE_SMALL_E = 1024;  // fewer routes, and at most so many experts: one launch
 
 struct MoeRouteBuffers {
     int *counts;           // [E] + one "bad id" flag at [E]

@@ -1,0 +1,102 @@
+"""The integer tensor-core matmul for a handful of tokens, at the edges of its tiles (16 tokens, 128 rows, one slab of K up to
+several split over a cluster or over ranges, Q6_K rows of any alignment), and the few-route MoE that is built on it."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from tests.util import KIND_Q4_K, KIND_Q6_K, TOL_FP32, TOL_MOE, max_rel_err, random_blocks
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from marmot_b200 import Context
+
+    c = Context(0)
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("kind", [KIND_Q4_K, KIND_Q6_K])
+@pytest.mark.parametrize("T,K,F", [(2, 256, 1), (7, 512, 129), (8, 2048, 130), (9, 4096, 1000), (15, 2304, 257), (16, 768, 20000),
+                                   (17, 1280, 135), (33, 256, 128), (64, 2816, 96)])
+def test_tile_edges(ctx, oracle, kind, T, K, F):
+    import torch
+    from marmot_b200.runtime import REGIME_AUTO, REGIME_I8MMA
+
+    rng = np.random.default_rng(T * 7 + K * 3 + F)
+    W = random_blocks(kind, F, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    bias = rng.normal(0, 1, F).astype(np.float32)
+    ctx.set_regime(REGIME_I8MMA)
+    got = ctx.linear(kind, torch.from_numpy(x).cuda(), ctx.upload(W), F, bias=torch.from_numpy(bias).cuda()).cpu().numpy()
+    ctx.set_regime(REGIME_AUTO)
+    ctx.synchronize()
+    assert max_rel_err(got, oracle.linear(kind, x, W, F) + bias) <= TOL_FP32
+
+
+@pytest.mark.parametrize("T,K,F", [(3, 4096, 5632), (4, 4096, 4096), (5, 2048, 2056), (8, 4096, 1030), (16, 512, 40)])
+def test_two_matrices_of_each_kind_with_prologues(ctx, oracle, T, K, F):
+    """The sizes at which linear_multi leaves the dp4a kernel: every result equals the one of the plain regime, and x' is exact."""
+    import torch
+    from marmot_b200.runtime import REGIME_AUTO, REGIME_GEMV_PLAIN
+
+    rng = np.random.default_rng(T + K + F)
+    dev = lambda a: torch.from_numpy(a.astype(np.float32)).cuda()
+    x, aux, w = dev(rng.normal(0, 1, (T, K))), dev(rng.normal(0, 1, (T, K))), dev(rng.normal(1, 0.2, K))
+    kinds = (KIND_Q4_K, KIND_Q4_K) if T < 5 else (KIND_Q4_K, KIND_Q6_K, KIND_Q4_K, KIND_Q6_K)
+    ws = [ctx.upload(random_blocks(k, F, K, rng)) for k in kinds]
+
+    def run(prologue, x_out=None):
+        outs = [torch.zeros((T, F), device="cuda") for _ in kinds]
+        ctx.linear_multi(x, [(k, m, F, o) for k, m, o in zip(kinds, ws, outs)], prologue(x_out) if prologue else None)
+        ctx.synchronize()
+        return outs
+
+    for prologue in (None, lambda xo: ("swiglu", aux), lambda xo: ("add_rmsnorm", aux, w, 1e-5, 0.0, xo)):
+        x_out = torch.zeros((T, K), device="cuda")
+        got = run(prologue, x_out)
+        if prologue is not None and x_out.abs().max() > 0:
+            assert torch.equal(x_out, x + aux)
+        ctx.set_regime(REGIME_GEMV_PLAIN)
+        ref = run(prologue, torch.zeros((T, K), device="cuda"))
+        ctx.set_regime(REGIME_AUTO)
+        for a, b in zip(got, ref):  # a last bit of the prologue may move an int8 quant by one
+            assert max_rel_err(a.cpu().numpy(), b.cpu().numpy()) <= 2e-3
+
+
+@pytest.mark.parametrize("kinds", [(KIND_Q4_K, KIND_Q4_K, KIND_Q6_K), (KIND_Q6_K, KIND_Q6_K, KIND_Q4_K)])
+@pytest.mark.parametrize("T,E,k", [(1, 4, 1), (17, 6, 2), (40, 3, 3), (127, 300, 2)])
+def test_few_route_moe(ctx, oracle, kinds, T, E, k):
+    import torch
+    from marmot_b200 import MarmotCudaError
+
+    H, FF = 512, 256
+    rng = np.random.default_rng(T + E + k)
+    hid = rng.normal(0, 1, (T, H)).astype(np.float32)
+    rows = ((E * FF, H), (E * FF, H), (E * H, FF))
+    gate, up, down = (random_blocks(kd, F, K, rng, d_sigma=0.0005) for kd, (F, K) in zip(kinds, rows))
+    p = rng.random((T, E)).astype(np.float32)
+    p[:, E - 1] = 0.0  # the last expert is hardly chosen
+    vals, ids = oracle.topk(p, k)
+    ref = oracle.moe_experts(kinds, hid, gate, up, down, ids, vals, FF, E)
+    hd, vd = torch.from_numpy(hid).cuda(), torch.from_numpy(np.ascontiguousarray(vals)).cuda()
+    idd = torch.from_numpy(np.ascontiguousarray(ids)).cuda()
+    gd, ud, dd = ctx.upload(gate), ctx.upload(up), ctx.upload(down)
+    got = ctx.moe_experts(kinds, hd, gd, ud, dd, idd, vd, FF, E)
+    ctx.synchronize()
+    assert max_rel_err(got.cpu().numpy(), ref) <= TOL_MOE
+    bad = ids.copy()
+    bad[T - 1, k - 1] = E
+    with pytest.raises(MarmotCudaError):
+        ctx.moe_experts(kinds, hd, gd, ud, dd, torch.from_numpy(np.ascontiguousarray(bad)).cuda(), vd, FF, E)
+        ctx.synchronize()
+    again = ctx.moe_experts(kinds, hd, gd, ud, dd, idd, vd, FF, E)
+    ctx.synchronize()
+    assert torch.equal(again, got)
