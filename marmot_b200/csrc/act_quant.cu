@@ -181,28 +181,49 @@ __device__ __forceinline__ void stage_group16(const int8_t *q16, float sc, __hal
 
 // Quantise row t (of the staged matrix) block by block, exactly as the kernels above: values to q_s, scales to d_s (shared
 // memory).  False when the row is not this rank's.
-// GLU: 0 = the row as it is; 1 = silu(x) * x2; 2 = gelu(x) * x2.  The SiLU uses the fast exponential and division
-// (relative error about 1e-6): its result is quantised to eight bits right here, three orders of magnitude coarser.
-// 3 = SiLU with the separately rounded exponential and division of the stand-alone kernels.
-template <bool KQ, int GLU>
+// OP: STAGE_PLAIN = the row as it is; STAGE_NORM = rms_norm(x + add) * w; STAGE_SILU = silu(x) * x2 with the fast exponential and
+// division (relative error about 1e-6: the result is quantised to eight bits right here, three orders of magnitude coarser);
+// STAGE_SILU_RN = the same with the separately rounded exponential and division of the stand-alone kernels; STAGE_GELU.
+// What bounds these launches is the latency of their loads, so every loop issues all loads of its turn before the first
+// operation on them: a division's slow path, or the test for a pointer, between two loads made each one a trip of its own
+// (rows of 14336 values: SiLU of 32 21 -> 9 us, of 4096 208 -> 124, 4.7 TB/s; add + RMSNorm of 64 rows of 4096 14.6 -> 5.9).
+enum { STAGE_PLAIN = 0, STAGE_SILU = 1, STAGE_GELU = 2, STAGE_SILU_RN = 3, STAGE_NORM = 4 };
+constexpr int NORM_BATCH = 16;
+
+template <bool KQ, int OP>
 __device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ldx, const ActSource &src, int K, int nb, int t,
                                              int8_t *q_s, float *d_s, float *red, float &inv_s) {
+    constexpr bool GLU = OP == STAGE_SILU || OP == STAGE_GELU || OP == STAGE_SILU_RN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     if (src.row_lo != nullptr && (t < *src.row_lo || t >= *src.row_hi)) return false;  // not this rank's row
     const size_t row_off = (size_t)(src.row_index != nullptr ? src.row_index[t] : t) * ldx;
-    const float *xrow = x + row_off;
-    const float *urow = GLU != 0 ? src.x2 + row_off : nullptr;
-    const float *arow = nullptr, *nrow = xrow;  // norm: what is added, and where the sum is read back from
+    // what is read: the row itself (norm: the sum, once it is stored), the other half of the GLU or what is added
+    const float *row = x + row_off;
+    const float *other = GLU ? src.x2 + row_off : nullptr;
+    float *x_out = src.x_out != nullptr ? src.x_out + row_off : nullptr;
     float norm_inv = 1.0f;
-    if (GLU == 0 && src.norm) {
-        arow = src.add != nullptr ? src.add + row_off : nullptr;
-        float *orow = src.x_out != nullptr ? src.x_out + row_off : nullptr;
+    if constexpr (OP == STAGE_NORM) {
+        other = src.add != nullptr ? src.add + row_off : nullptr;
         float sum = 0.0f;
         // (256 threads whatever the block: the order of the sum is that of the stand-alone kernel)
-        for (int i = threadIdx.x; i < K && threadIdx.x < 256; i += 256) {
-            const float v = arow != nullptr ? __fadd_rn(xrow[i], arow[i]) : xrow[i];
-            if (orow != nullptr) orow[i] = v;
-            sum += v * v;
+        for (int i0 = threadIdx.x; i0 < K && threadIdx.x < 256; i0 += 256 * NORM_BATCH) {
+            float v[NORM_BATCH];
+#pragma unroll
+            for (int j = 0; j < NORM_BATCH; ++j) v[j] = i0 + 256 * j < K ? row[i0 + 256 * j] : 0.0f;
+            if (other != nullptr) {
+                float a[NORM_BATCH];
+#pragma unroll
+                for (int j = 0; j < NORM_BATCH; ++j) a[j] = i0 + 256 * j < K ? other[i0 + 256 * j] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < NORM_BATCH; ++j) v[j] = __fadd_rn(v[j], a[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < NORM_BATCH; ++j) sum += v[j] * v[j];
+            if (x_out != nullptr) {
+#pragma unroll
+                for (int j = 0; j < NORM_BATCH; ++j)
+                    if (i0 + 256 * j < K) x_out[i0 + 256 * j] = v[j];
+            }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -216,42 +237,71 @@ __device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ld
         __syncthreads();
         norm_inv = inv_s;
         __syncthreads();  // red and inv_s are used again below
-        if (orow != nullptr) {  // the packer reads the sums back (other threads' elements too: all written before
-            nrow = orow;        // the barriers above) instead of adding again
-            arow = nullptr;
+        if (x_out != nullptr) {  // the packer reads the sums back (other threads' elements too: all written before
+            row = x_out;         // the barriers above) instead of adding again
+            other = nullptr;
         }
     }
-    auto value = [&](int k) -> float {
-        if (GLU == 0 && src.norm) {
-            const float v = arow != nullptr ? __fadd_rn(nrow[k], arow[k]) : nrow[k];
-            float y = __fmul_rn(v, norm_inv);
-            if (src.norm_w != nullptr) y = __fmul_rn(y, __fadd_rn(src.norm_w[k], src.w_off));
-            return y;
+    // N values of a block, 32 apart: all loads, then the operations
+    auto values = [&](int k0, auto &v) {
+        constexpr int N = sizeof(v) / sizeof(v[0]);
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = k0 + 32 * i < K ? row[k0 + 32 * i] : 0.0f;
+        if constexpr (OP == STAGE_PLAIN) return;
+        float o[N];
+        if (other != nullptr) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) o[i] = k0 + 32 * i < K ? other[k0 + 32 * i] : 0.0f;
         }
-        const float g = xrow[k];
-        if constexpr (GLU == 0) return g;
-        float a;
-        if constexpr (GLU == 2) a = __fmul_rn(__fmul_rn(0.5f, g), __fadd_rn(1.0f, erff(__fmul_rn(g, 0.7071067811865475f))));
-        else if constexpr (GLU == 3) a = __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)));
-        else a = __fdividef(g, __fadd_rn(1.0f, __expf(-g)));
-        return __fmul_rn(a, urow[k]);
+        if constexpr (OP == STAGE_NORM) {
+            float w[N];
+            if (src.norm_w != nullptr) {
+#pragma unroll
+                for (int i = 0; i < N; ++i) w[i] = k0 + 32 * i < K ? src.norm_w[k0 + 32 * i] : 0.0f;
+            }
+            if (other != nullptr) {
+#pragma unroll
+                for (int i = 0; i < N; ++i) v[i] = __fadd_rn(v[i], o[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < N; ++i) v[i] = __fmul_rn(v[i], norm_inv);
+            if (src.norm_w != nullptr) {
+#pragma unroll
+                for (int i = 0; i < N; ++i) v[i] = __fmul_rn(v[i], __fadd_rn(w[i], src.w_off));
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const float g = v[i];
+                float a;
+                if constexpr (OP == STAGE_GELU) a = __fmul_rn(__fmul_rn(0.5f, g), __fadd_rn(1.0f, erff(__fmul_rn(g, 0.7071067811865475f))));
+                else if constexpr (OP == STAGE_SILU_RN) a = __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)));
+                else a = __fdividef(g, __fadd_rn(1.0f, __expf(-g)));
+                v[i] = __fmul_rn(a, o[i]);
+            }
+            if (KQ && x_out != nullptr) {
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                    if (k0 + 32 * i < K) x_out[k0 + 32 * i] = v[i];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (k0 + 32 * i >= K) v[i] = 0.0f;
     };
     if (KQ) {
         for (int blk = warp; blk < nb; blk += n_warps) {
-            const int len = min(QK_K, K - blk * QK_K);
             float v[8];
+            values(blk * QK_K + lane, v);
             float best_abs = 0.0f, best_val = 0.0f;
             int best_idx = 0x7fffffff;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int idx = lane + 32 * i;
-                v[i] = idx < len ? value(blk * QK_K + idx) : 0.0f;
-                if (GLU != 0 && src.x_out != nullptr && idx < len) src.x_out[row_off + blk * QK_K + idx] = v[i];
                 const float a = fabsf(v[i]);
                 if (a > best_abs) {
                     best_abs = a;
                     best_val = v[i];
-                    best_idx = idx;
+                    best_idx = lane + 32 * i;
                 }
             }
 #pragma unroll
@@ -278,19 +328,25 @@ __device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ld
             if (lane == 0) d_s[blk] = d;
         }
     } else {
-        for (int blk = warp; blk < nb; blk += n_warps) {
-            const int k = blk * Q8_0_VALUES + lane;
-            const float v = k < K ? value(k) : 0.0f;
-            float amax = fabsf(v);
+        // four blocks in turn per warp, their loads together
+        for (int blk0 = 4 * warp; blk0 < nb; blk0 += 4 * n_warps) {
+            float v[4];
+            values(blk0 * Q8_0_VALUES + lane, v);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-            float scale = __fdiv_rn(amax, 127.0f);
-            if (scale < FLT_MIN) scale = 1.0f;
-            const float inv = __fdiv_rn(1.0f, scale);
-            int q = (int)roundf(__fmul_rn(v, inv));
-            q = max(-127, min(127, q));
-            q_s[k] = (int8_t)q;
-            if (lane == 0) d_s[blk] = __half2float(__float2half_rn(scale));
+            for (int i = 0; i < 4; ++i) {
+                const int blk = blk0 + i;
+                if (blk >= nb) break;
+                float amax = fabsf(v[i]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+                float scale = __fdiv_rn(amax, 127.0f);
+                if (scale < FLT_MIN) scale = 1.0f;
+                const float inv = __fdiv_rn(1.0f, scale);
+                int q = (int)roundf(__fmul_rn(v[i], inv));
+                q = max(-127, min(127, q));
+                q_s[blk * Q8_0_VALUES + lane] = (int8_t)q;
+                if (lane == 0) d_s[blk] = __half2float(__float2half_rn(scale));
+            }
         }
     }
     return true;
@@ -298,7 +354,7 @@ __device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ld
 
 // Few rows: up to a thousand threads per row, so that a row is one or two trips to L2 (latency bounds the launch: 64 rows of
 // 4096 values 3.3 us with 256 threads); many rows: 256 threads, and as many rows at a time.
-template <bool KQ, int GLU>
+template <bool KQ, int OP>
 __global__ void __launch_bounds__(1024)
 act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, __half *__restrict__ xh,
                       float *__restrict__ rowscale) {
@@ -312,7 +368,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!quantize_row<KQ, GLU>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
+    if (!quantize_row<KQ, OP>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
     __syncthreads();
     float m = 0.0f;
     for (int b = threadIdx.x; b < nb; b += blockDim.x) m = fmaxf(m, fabsf(d_s[b]));
@@ -346,7 +402,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
 // quants, then the sums of its sub-blocks split as 64 * hi + lo into 8-bit values (lo from byte 256, hi from byte 288 on).
 // SUB = 32 (Q4_K: eight sums) or 16 (Q6_K: sixteen sums, and two planes of quants, in which the even / the odd sub-blocks are
 // zero: the matmul multiplies 32 values at a time and needs the sums of 16).  dT[block][row]: the block scales.
-template <int SUB, int GLU>
+template <int SUB, int OP>
 __global__ void __launch_bounds__(1024)
 act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, uint8_t *__restrict__ xq, size_t plane,
                      float *__restrict__ dT, int ld_dT) {
@@ -358,7 +414,7 @@ act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K,
     const int t = blockIdx.x;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!quantize_row<true, GLU>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
+    if (!quantize_row<true, OP>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
     __syncthreads();
     for (int b = threadIdx.x; b < nb; b += blockDim.x) dT[(size_t)b * ld_dT + t] = d_s[b];
     uint8_t *row = xq + (size_t)t * nb * 384;
@@ -389,6 +445,11 @@ act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K,
     }
 }
 
+static int stage_op(const ActSource &src) {
+    if (src.x2 != nullptr) return src.glu == 2 ? STAGE_GELU : src.glu == 3 ? STAGE_SILU_RN : STAGE_SILU;
+    return src.norm ? STAGE_NORM : STAGE_PLAIN;
+}
+
 size_t act_half_fused_smem(int kind, int K) {
     const int bv = block_values(kind), nb = (K + bv - 1) / bv;
     return (size_t)((nb * bv + 15) & ~15) + (size_t)nb * sizeof(float);
@@ -414,11 +475,16 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const bool kq = kind != KIND_Q8_0;
-    const int glu = src.x2 != nullptr ? (src.glu == 2 ? 2 : 1) : 0;
-#define MCU_STAGE(KQ, GLU) cudaLaunchKernelEx(&cfg, act_half_fused_kernel<KQ, GLU>, x, ldx, src, K, nb, xh, rowscale)
-    if (glu == 0) return kq ? MCU_STAGE(true, 0) : MCU_STAGE(false, 0);
-    if (glu == 1) return kq ? MCU_STAGE(true, 1) : MCU_STAGE(false, 1);
-    return kq ? MCU_STAGE(true, 2) : MCU_STAGE(false, 2);
+#define MCU_STAGE(OP) \
+    (kq ? cudaLaunchKernelEx(&cfg, act_half_fused_kernel<true, OP>, x, ldx, src, K, nb, xh, rowscale) \
+        : cudaLaunchKernelEx(&cfg, act_half_fused_kernel<false, OP>, x, ldx, src, K, nb, xh, rowscale))
+    switch (stage_op(src)) {
+    case STAGE_SILU: return MCU_STAGE(STAGE_SILU);
+    case STAGE_SILU_RN: return MCU_STAGE(STAGE_SILU_RN);
+    case STAGE_GELU: return MCU_STAGE(STAGE_GELU);
+    case STAGE_NORM: return MCU_STAGE(STAGE_NORM);
+    default: return MCU_STAGE(STAGE_PLAIN);
+    }
 #undef MCU_STAGE
 }
 
@@ -437,10 +503,16 @@ cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSou
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const size_t plane = (size_t)rows * nb * 384;
-    const int glu = src.x2 != nullptr ? (src.glu == 2 ? 2 : 1) : 0;
-#define MCU_STAGE(SUB, GLU) cudaLaunchKernelEx(&cfg, act_int_fused_kernel<SUB, GLU>, x, ldx, src, K, nb, xq, plane, dT, rows)
-    if (kind == KIND_Q6_K) return glu == 0 ? MCU_STAGE(16, 0) : glu == 1 ? MCU_STAGE(16, 3) : MCU_STAGE(16, 2);
-    return glu == 0 ? MCU_STAGE(32, 0) : glu == 1 ? MCU_STAGE(32, 3) : MCU_STAGE(32, 2);
+#define MCU_STAGE(OP) \
+    (kind == KIND_Q6_K ? cudaLaunchKernelEx(&cfg, act_int_fused_kernel<16, OP>, x, ldx, src, K, nb, xq, plane, dT, rows) \
+                       : cudaLaunchKernelEx(&cfg, act_int_fused_kernel<32, OP>, x, ldx, src, K, nb, xq, plane, dT, rows))
+    switch (stage_op(src)) {
+    case STAGE_SILU:
+    case STAGE_SILU_RN: return MCU_STAGE(STAGE_SILU_RN);
+    case STAGE_GELU: return MCU_STAGE(STAGE_GELU);
+    case STAGE_NORM: return MCU_STAGE(STAGE_NORM);
+    default: return MCU_STAGE(STAGE_PLAIN);
+    }
 #undef MCU_STAGE
 }
 

@@ -30,7 +30,7 @@ cudaError_t launch_half_acts(int kind, const ActBuffers &a, int T, int K, __half
 size_t act_half_fused_smem(int kind, int K);
 // Where the staging kernel takes its rows from, for callers that would otherwise run a gather or a GLU pass first:
 // row t comes from x + row_index[t] * ldx when row_index is set; with x2 set the value is act(x) * x2 (glu 1 = SiLU,
-// 2 = GELU, rounded like the MoE GLU kernel), and with K-quants goes to x_out (which may be x) when that is set; rows outside [*row_lo, *row_hi) (device-resident) are skipped.
+// 2 = GELU, rounded like the MoE GLU kernel, 3 = SiLU, rounded like it), and with K-quants goes to x_out (which may be x) when that is set; rows outside [*row_lo, *row_hi) (device-resident) are skipped.
 // With norm set the row is first x + add (add may be null; the sum goes to x_out when that is set, which may be x
 // itself: a CTA owns its row) and the values are rms_norm(row) * (norm_w + w_off), the operations and their order
 // those of the stand-alone add + RMSNorm kernel.

@@ -145,77 +145,93 @@ __global__ void moe_glu_kernel(float *__restrict__ gate, const float *__restrict
 }
 
 // out[t][c] = sum over the token's routes, in ascending sorted position (= the reference's route
-// order, moe_ops.c:1034-1042), of w * down[pos][c]; products and sums rounded separately.
-template <int MAXK>
-__global__ void moe_combine_kernel(const float *__restrict__ route_down, const float *__restrict__ sorted_w,
-                                   const int32_t *__restrict__ route_pos, int k, int H, int pos_lo, int pos_hi,
-                                   float *__restrict__ out, size_t ldo) {
+// order, moe_ops.c:1034-1042), of w * down[pos][c]; products and sums rounded separately.  Positions outside [pos_lo, pos_hi) are
+// another rank's experts or rejected ids.  With offsets the range comes from the device (experts [e_begin, e_end)): no host
+// read-back; block 0 then also reports an out-of-range expert id through the error flag.
+// grid (tokens, slices of 1024 columns): loads of several routes and slices are in flight together (one column and route at a time
+// per thread: 21 us for 16 tokens of 4096, 43 for 2048; 4 and 18 so).
+struct CombineRange {
+    int pos_lo, pos_hi;
+    const int *offsets, *bad_id_count;
+    int e_begin, e_end;
+    int *err;
+};
+constexpr int COMBINE_COLS = 1024;
+
+template <typename V>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(const float *__restrict__ route_down, const float *__restrict__ sorted_w, const int32_t *__restrict__ route_pos, int k,
+                   int H, CombineRange range, float *__restrict__ out, size_t ldo) {
+    constexpr int N = sizeof(V) / sizeof(float), BATCH = 4;
+    __shared__ int pos_s[MOE_MAX_TOPK];
+    __shared__ float w_s[MOE_MAX_TOPK];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.x;
-    int pos[MAXK];
-    float w[MAXK];
-    for (int j = 0; j < k; ++j) pos[j] = route_pos[(size_t)t * k + j];
-    for (int i = 1; i < k; ++i) {  // insertion sort, k is tiny
-        const int p = pos[i];
-        int j = i;
-        while (j > 0 && pos[j - 1] > p) {
-            pos[j] = pos[j - 1];
-            --j;
+    if (threadIdx.x < (unsigned)k) {
+        int lo = range.pos_lo, hi = range.pos_hi;
+        bool bad = false;
+        if (range.offsets != nullptr) {
+            lo = range.offsets[range.e_begin], hi = range.offsets[range.e_end];
+            bad = *range.bad_id_count != 0;  // the call is rejected as a whole: zeros out
+            if (bad && t == 0 && blockIdx.y == 0 && threadIdx.x == 0 && range.err != nullptr) atomicExch(range.err, 40);
         }
-        pos[j] = p;
+        const int32_t *mine = route_pos + (size_t)t * k;
+        const int p = mine[threadIdx.x];
+        int rank = 0;
+        for (int j = 0; j < k; ++j) rank += mine[j] < p || (mine[j] == p && j < (int)threadIdx.x);
+        const bool use = !bad && p >= lo && p < hi;
+        pos_s[rank] = use ? p : -1;
+        w_s[rank] = use ? sorted_w[p] : 0.0f;
     }
-    for (int j = 0; j < k; ++j) w[j] = (pos[j] >= pos_lo && pos[j] < pos_hi) ? sorted_w[pos[j]] : 0.0f;
-    for (int c = threadIdx.x; c < H; c += blockDim.x) {
-        float acc = 0.0f;
-        for (int j = 0; j < k; ++j) {
-            if (pos[j] < pos_lo || pos[j] >= pos_hi) continue;  // another rank's expert, or a rejected id
-            acc = __fadd_rn(acc, __fmul_rn(w[j], route_down[(size_t)pos[j] * H + c]));
+    __syncthreads();
+    const int c1 = min(H, ((int)blockIdx.y + 1) * COMBINE_COLS);
+    for (int c = (int)blockIdx.y * COMBINE_COLS + N * (int)threadIdx.x; c < c1; c += N * 256) {
+        float acc[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) acc[i] = 0.0f;
+        for (int j0 = 0; j0 < k; j0 += BATCH) {
+            V v[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) {
+                const int p = j0 + j < k ? pos_s[j0 + j] : -1;
+                if (p >= 0) v[j] = *(const V *)(route_down + (size_t)p * H + c);
+            }
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) {
+                if (j0 + j >= k || pos_s[j0 + j] < 0) continue;
+#pragma unroll
+                for (int i = 0; i < N; ++i) acc[i] = __fadd_rn(acc[i], __fmul_rn(w_s[j0 + j], ((const float *)&v[j])[i]));
+            }
         }
-        out[(size_t)t * ldo + c] = acc;
+        V y;
+#pragma unroll
+        for (int i = 0; i < N; ++i) ((float *)&y)[i] = acc[i];
+        *(V *)(out + (size_t)t * ldo + c) = y;
     }
 }
 
-// The same with the local range of sorted positions taken from the device-resident offsets (experts
-// [e_begin, e_end)): no host read-back.  Block 0 also reports an out-of-range expert id through the error flag.
-template <int MAXK>
-__global__ void moe_combine_dev_kernel(const float *__restrict__ route_down, const float *__restrict__ sorted_w,
-                                       const int32_t *__restrict__ route_pos, int k, int H,
-                                       const int *__restrict__ offsets, int e_begin, int e_end,
-                                       const int *__restrict__ bad_id_count, int *err, float *__restrict__ out, size_t ldo) {
-    const int t = blockIdx.x;
-    const int pos_lo = offsets[e_begin], pos_hi = offsets[e_end];
-    if (t == 0 && threadIdx.x == 0 && *bad_id_count != 0 && err != nullptr) atomicExch(err, 40);
-    int pos[MAXK];
-    float w[MAXK];
-    for (int j = 0; j < k; ++j) pos[j] = route_pos[(size_t)t * k + j];
-    for (int i = 1; i < k; ++i) {
-        const int p = pos[i];
-        int j = i;
-        while (j > 0 && pos[j - 1] > p) {
-            pos[j] = pos[j - 1];
-            --j;
-        }
-        pos[j] = p;
-    }
-    const bool bad = *bad_id_count != 0;  // the call is rejected as a whole: zeros out, error at synchronize
-    for (int j = 0; j < k; ++j) w[j] = (!bad && pos[j] >= pos_lo && pos[j] < pos_hi) ? sorted_w[pos[j]] : 0.0f;
-    for (int c = threadIdx.x; c < H; c += blockDim.x) {
-        float acc = 0.0f;
-        for (int j = 0; j < k; ++j) {
-            if (bad || pos[j] < pos_lo || pos[j] >= pos_hi) continue;
-            acc = __fadd_rn(acc, __fmul_rn(w[j], route_down[(size_t)pos[j] * H + c]));
-        }
-        out[(size_t)t * ldo + c] = acc;
-    }
+static cudaError_t combine(const float *route_down, const float *sorted_w, const int32_t *route_pos, int T, int k, int H,
+                           const CombineRange &range, float *out, size_t ldo, cudaStream_t s) {
+    if (T <= 0) return cudaSuccess;
+    if (k > MOE_MAX_TOPK) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)T, (unsigned)((H + COMBINE_COLS - 1) / COMBINE_COLS), 1);
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (H % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)out | (uintptr_t)route_down) & 15u) == 0)
+        return cudaLaunchKernelEx(&cfg, moe_combine_kernel<float4>, route_down, sorted_w, route_pos, k, H, range, out, ldo);
+    return cudaLaunchKernelEx(&cfg, moe_combine_kernel<float>, route_down, sorted_w, route_pos, k, H, range, out, ldo);
 }
 
 cudaError_t launch_moe_combine_dev(const float *route_down, const float *sorted_w, const int32_t *route_pos, int T, int k,
                                    int H, const int *offsets, int e_begin, int e_end, const int *bad_id_count, int *err,
                                    float *out, size_t ldo, cudaStream_t s) {
-    if (T <= 0) return cudaSuccess;
-    if (k > MOE_MAX_TOPK) return cudaErrorInvalidValue;
-    moe_combine_dev_kernel<MOE_MAX_TOPK><<<T, 256, 0, s>>>(route_down, sorted_w, route_pos, k, H, offsets, e_begin, e_end,
-                                                            bad_id_count, err, out, ldo);
-    return cudaGetLastError();
+    return combine(route_down, sorted_w, route_pos, T, k, H, CombineRange{0, 0, offsets, bad_id_count, e_begin, e_end, err}, out, ldo, s);
 }
 
 cudaError_t launch_topk(const float *x, int rows, int cols, size_t ldx, int k, float *values, int32_t *indices,
@@ -325,10 +341,7 @@ cudaError_t launch_moe_glu(float *gate, const float *up, size_t n, int geglu, cu
 
 cudaError_t launch_moe_combine(const float *route_down, const float *sorted_w, const int32_t *route_pos, int T, int k,
                                int H, int pos_lo, int pos_hi, float *out, size_t ldo, cudaStream_t s) {
-    if (T <= 0) return cudaSuccess;
-    if (k > MOE_MAX_TOPK) return cudaErrorInvalidValue;
-    moe_combine_kernel<MOE_MAX_TOPK><<<T, 256, 0, s>>>(route_down, sorted_w, route_pos, k, H, pos_lo, pos_hi, out, ldo);
-    return cudaGetLastError();
+    return combine(route_down, sorted_w, route_pos, T, k, H, CombineRange{pos_lo, pos_hi, nullptr, nullptr, 0, 0, nullptr}, out, ldo, s);
 }
 
 }  // namespace mcu
