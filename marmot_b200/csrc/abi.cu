@@ -859,7 +859,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
         }
         // More tokens on the tensor cores: one staging launch (the prologue folded into it) feeds every
         // matmul that wants the same staging; weights of the other block format class get a second one.
-        bool tensor = !integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > 16 &&
+        bool tensor = !integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > (size_t)GEMV_MAX_T &&
             (pr.op == MCU_PROLOGUE_NONE || contiguous);
         for (size_t j = 0; j < n_jobs && tensor; ++j)
             tensor = gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) &&
@@ -875,7 +875,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
                 src.x_out = gp.x_out;
             } else if (pr.op == MCU_PROLOGUE_SWIGLU) {
                 src.x2 = pr.aux_dev;
-                src.glu = 1;
+                src.glu = 3;  // (rounded like mcu_swiglu)
             }
             Staged st;
             int staged_kind = -1;

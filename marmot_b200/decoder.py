@@ -173,32 +173,6 @@ class Decoder:
             self.block_table = torch.from_numpy(table).to(dev)
         self._bufs = {}
         self._plans = {}  # one-token step plans (persistent kernel), per set of caller tensors
-        self._side = None
-
-    def _side_contexts(self):
-        """Two more contexts on streams of their own (each with its own workspace), for the key and value projections,
-        which read the same normalised activations as the query projection and are small enough at decode batch sizes
-        that their duration is mostly fixed latency: the three run side by side and rejoin before RoPE.  The fork and
-        the join are stream-to-stream waits, so a CUDA-graph capture of the step records them as graph edges."""
-        if self._side is None:
-            import os
-
-            torch = self.torch
-            if os.environ.get("MARMOT_DECODER_SERIAL_QKV"):  # diagnostic switch: one stream, three calls in turn
-                self._side = ()
-            else:
-                streams = [torch.cuda.Stream(self.dev) for _ in range(2)]
-                ctxs = [Context(self.ctx.device, use_torch_stream=False) for _ in streams]
-                for c, st in zip(ctxs, streams):
-                    c.set_stream(st.cuda_stream)
-                self._side = (ctxs, streams)
-        return self._side
-
-    def _main_stream(self):
-        handle = self.ctx.lib.mcu_context_get_stream(self.ctx.handle) or 0
-        if handle in (0, 1):  # the legacy default stream
-            return self.torch.cuda.default_stream(self.dev)
-        return self.torch.cuda.ExternalStream(handle, device=self.dev)
 
     def _buf(self, name, shape, dtype=None):
         key = (name, tuple(shape))
@@ -257,11 +231,11 @@ class Decoder:
         Returns logits [T, vocab] (tensor parallel: this rank's vocabulary slice [T, local_vocab]).
 
         decode=True promises at most one token per sequence in the call (a decode step): RoPE, the KV append, the
-        attention and the merge of its context chunks then run as one kernel, and on one GPU every elementwise step
-        (residual add + RMSNorm, SwiGLU) rides in the prologue of the matmul that consumes it -- five launches per layer
-        for up to eight tokens."""
-        if decode and self.group.world == 1 and ids.shape[0] <= 8:
-            return self._step_fused(ids, meta, positions, logits_out)
+        attention and the merge of its context chunks then run as one kernel.  Every elementwise step (residual add + RMSNorm,
+        SwiGLU) rides in the matmul that consumes it: in the prologue of the decode kernels, in the activation staging of the
+        tensor-core ones."""
+        if self.group.world == 1:
+            return self._step_single(ids, meta, positions, logits_out, decode)
         ctx, s = self.ctx, self.local
         T = ids.shape[0]
         hq, hkv, hd = s.n_heads, s.n_kv_heads, s.head_dim
@@ -271,58 +245,47 @@ class Decoder:
         q, k, v = self._buf("q", (T, hq * hd)), self._buf("k", (T, hkv * hd)), self._buf("v", (T, hkv * hd))
         att, proj = self._buf("att", (T, hq * hd)), self._buf("proj", (T, s.d))
         gate, up = self._buf("gate", (T, max(s.ffn, 1))), self._buf("up", (T, max(s.ffn, 1)))
-        scale = float(hd) ** -0.5
         # the residual add that ends a block and the rms_norm that opens the next one run as one kernel
         ctx.rmsnorm(x, self.layers[0]["attn_norm"], s.rms_eps, out=h)
-        # up to eight tokens q / k / v are one launch; beyond, three matmuls that run side by side on streams of their own
-        side = self._side_contexts() if T > 8 else ()
-        fuse_ffn = T > 16 and s.ffn > 0 and not os.environ.get("MARMOT_DECODER_UNFUSED_FFN")  # (diagnostic switch)
-        main = self._main_stream() if side else None
         for i, lw in enumerate(self.layers):
-            if side:
-                (ctx_k, ctx_v), (st_k, st_v) = side
-                st_k.wait_stream(main)
-                st_v.wait_stream(main)
-                ctx_k.linear(kd[f"l{i}.wk"], h, lw["wk"], hkv * hd, out=k)
-                ctx_v.linear(kd[f"l{i}.wv"], h, lw["wv"], hkv * hd, out=v)
-                ctx.linear(kd[f"l{i}.wq"], h, lw["wq"], hq * hd, out=q)
-                main.wait_stream(st_k)
-                main.wait_stream(st_v)
-            else:
-                ctx.linear_multi(h, [(kd[f"l{i}.wq"], lw["wq"], hq * hd, q), (kd[f"l{i}.wk"], lw["wk"], hkv * hd, k),
-                                     (kd[f"l{i}.wv"], lw["wv"], hkv * hd, v)])
-            if decode:
-                if i == 0:
-                    rope = ctx.rope_table(positions, hd, s.rope_theta, out=self._buf("rope", (T, hd // 2, 2)))
-                ctx.paged_attention_decode(meta, q, k, v, self.kv_k, self.kv_v, self.block_table, i, hq, hkv, hd,
-                                           self.block_size, scale, positions, s.rope_theta, rope_table=rope, out=att)
-            else:
-                ctx.rope_qk(q, k, positions, hq, hkv, hd, s.rope_theta)
-                ctx.paged_attention(meta, q, k, v, self.kv_k, self.kv_v, self.block_table, i, hq, hkv, hd, self.block_size,
-                                    scale, out=att)
+            ctx.linear_multi(h, [(kd[f"l{i}.wq"], lw["wq"], hq * hd, q), (kd[f"l{i}.wk"], lw["wk"], hkv * hd, k),
+                                 (kd[f"l{i}.wv"], lw["wv"], hkv * hd, v)])
+            self._attention(i, meta, positions, q, k, v, att, decode)
             self._row_parallel(kd[f"l{i}.wo"], att, lw["wo"], s.d, proj, hq * hd)
-            if fuse_ffn:
+            ffn = [(kd[f"l{i}.gate"], lw["gate"], s.ffn, gate), (kd[f"l{i}.up"], lw["up"], s.ffn, up)]
+            if s.ffn > 0 and T > 16:
                 # the residual add + RMSNorm ride in the staging of gate / up; the sum goes to the other residual buffer
-                # (the prologue's output may not be its input)
                 x_next = self._buf("x2" if x is self._buf("x", (T, s.d)) else "x", (T, s.d))
-                ctx.linear_multi(x, [(kd[f"l{i}.gate"], lw["gate"], s.ffn, gate), (kd[f"l{i}.up"], lw["up"], s.ffn, up)],
-                                 ("add_rmsnorm", proj, lw["ffn_norm"], s.rms_eps, 0.0, x_next))
+                ctx.linear_multi(x, ffn, ("add_rmsnorm", proj, lw["ffn_norm"], s.rms_eps, 0.0, x_next))
                 x = x_next
-                # SwiGLU stays a kernel of its own here: inside the staging kernel (one CTA per token) it ran over
-                # 14336 values per CTA on 64 CTAs and cost 29 us against 7 + 6 us for the two kernels, measured
-                ctx.swiglu(gate, up, out=gate)
-                self._row_parallel(kd[f"l{i}.down"], gate, lw["down"], s.d, proj, s.ffn)
             else:
                 ctx.add_rmsnorm(x, proj, lw["ffn_norm"], s.rms_eps, x, h)
                 if s.ffn > 0:
-                    ctx.linear_multi(h, [(kd[f"l{i}.gate"], lw["gate"], s.ffn, gate), (kd[f"l{i}.up"], lw["up"], s.ffn, up)])
-                    ctx.swiglu(gate, up, out=gate)
-                self._row_parallel(kd[f"l{i}.down"], gate, lw["down"], s.d, proj, s.ffn)
+                    ctx.linear_multi(h, ffn)
+            if s.ffn > 0:
+                ctx.swiglu(gate, up, out=gate)
+            self._row_parallel(kd[f"l{i}.down"], gate, lw["down"], s.d, proj, s.ffn)
             nxt = self.layers[i + 1]["attn_norm"] if i + 1 < len(self.layers) else self.out_norm
             ctx.add_rmsnorm(x, proj, nxt, s.rms_eps, x, h)
         logits = logits_out if logits_out is not None else self._buf("logits", (T, self.local_vocab))
         ctx.linear(kd["output"], h, self.output, self.local_vocab, out=logits)
         return logits
+
+    def _attention(self, i, meta, positions, q, k, v, att, decode):
+        """RoPE, KV append and attention of layer i into att; a decode step's angles are computed once, at layer 0."""
+        ctx, s = self.ctx, self.local
+        T, hq, hkv, hd = q.shape[0], s.n_heads, s.n_kv_heads, s.head_dim
+        scale = float(hd) ** -0.5
+        if decode:
+            rope = self._buf("rope", (T, hd // 2, 2))
+            if i == 0:
+                ctx.rope_table(positions, hd, s.rope_theta, out=rope)
+            ctx.paged_attention_decode(meta, q, k, v, self.kv_k, self.kv_v, self.block_table, i, hq, hkv, hd,
+                                       self.block_size, scale, positions, s.rope_theta, rope_table=rope, out=att)
+        else:
+            ctx.rope_qk(q, k, positions, hq, hkv, hd, s.rope_theta)
+            ctx.paged_attention(meta, q, k, v, self.kv_k, self.kv_v, self.block_table, i, hq, hkv, hd, self.block_size,
+                                scale, out=att)
 
     def _one_token_plan(self, meta, positions, logits):
         """The persistent-kernel plan for a one-token step on these very tensors (mcu_decode_plan), or None when the
@@ -374,15 +337,14 @@ class Decoder:
         self._plans[key] = plan
         return plan
 
-    def _step_fused(self, ids, meta, positions, logits_out):
-        """The decode step with every elementwise operator folded into its consumer (see step).  One token: a single
-        persistent kernel walks all layers (mcu_decode_plan; embedding gather and RoPE table before it).  Otherwise five
-        launches per layer; the residual stream alternates between two buffers: a prologue reads x and the pending
-        projection and stores their sum to the other buffer (the CTAs of one launch all read x, so the sum cannot go
-        back in place)."""
+    def _step_single(self, ids, meta, positions, logits_out, decode):
+        """The step on one GPU with every elementwise operator folded into its consumer (see step).  One token of a decode
+        step: a single persistent kernel walks all layers (mcu_decode_plan; embedding gather and RoPE table before it).
+        Otherwise the residual stream alternates between two buffers: a prologue reads x and the pending projection and stores
+        their sum to the other buffer (the CTAs of one launch all read x, so the sum cannot go back in place)."""
         ctx, s = self.ctx, self.local
         T = ids.shape[0]
-        if T == 1:
+        if decode and T == 1:
             logits = logits_out if logits_out is not None else self._buf("logits", (1, self.local_vocab))
             plan = self._one_token_plan(meta, positions, logits)
             if plan is not None:
@@ -398,17 +360,14 @@ class Decoder:
         q, k, v = self._buf("q", (T, hq * hd)), self._buf("k", (T, hkv * hd)), self._buf("v", (T, hkv * hd))
         att, proj = self._buf("att", (T, hq * hd)), self._buf("proj", (T, s.d))
         gate, up = self._buf("gate", (T, max(s.ffn, 1))), self._buf("up", (T, max(s.ffn, 1)))
-        scale = float(hd) ** -0.5
         pending = None  # the projection not yet added to the residual stream
-        rope = ctx.rope_table(positions, hd, s.rope_theta, out=self._buf("rope", (T, hd // 2, 2)))
         for i, lw in enumerate(self.layers):
             ctx.linear_multi(xs[cur], [(kd[f"l{i}.wq"], lw["wq"], hq * hd, q), (kd[f"l{i}.wk"], lw["wk"], hkv * hd, k),
                                        (kd[f"l{i}.wv"], lw["wv"], hkv * hd, v)],
                              ("add_rmsnorm", pending, lw["attn_norm"], s.rms_eps, 0.0, xs[1 - cur] if pending is not None else None))
             if pending is not None:
                 cur = 1 - cur
-            ctx.paged_attention_decode(meta, q, k, v, self.kv_k, self.kv_v, self.block_table, i, hq, hkv, hd,
-                                       self.block_size, scale, positions, s.rope_theta, rope_table=rope, out=att)
+            self._attention(i, meta, positions, q, k, v, att, decode)
             ctx.linear(kd[f"l{i}.wo"], att, lw["wo"], s.d, out=proj)
             pending = proj
             if s.ffn > 0:
