@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "paged_attention.cuh"
 
 #include <climits>
 #include <cmath>
@@ -300,16 +301,6 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ x
 }
 
 // ---------------------------------------------------------------- paged attention
-struct PagedParams {
-    const uint32_t *meta;   // [T][4]: seq_slot, pos, kv_slot, flags
-    const uint32_t *table;  // [seqs][max_blocks]
-    const float *q, *k_new, *v_new;
-    void *kv_k, *kv_v;      // [blocks][layers][kv_heads][block_size][head_dim]
-    float *out;
-    int n_q_heads, n_kv_heads, max_blocks, n_layers, layer, block_shift;
-    float scale;
-};
-
 __device__ __forceinline__ float kv_load(const float *p) { return *p; }
 __device__ __forceinline__ float kv_load(const __half *p) { return __half2float(*p); }
 __device__ __forceinline__ void kv_store(float *p, float v) { *p = v; }
@@ -493,54 +484,17 @@ __global__ void __launch_bounds__(32 * PA_MAX_GROUP) paged_attention_kernel(Page
 // so the products carry about 22 significant bits and the result stays within 1e-6 of f32 arithmetic.
 // A warp sees exactly one tile, so its softmax needs no running rescale; the four warps' states are merged through
 // shared memory in warp order and written as one partial state per (token, query head, chunk).
-constexpr int PM_WARPS = 4;
-constexpr int PM_TILE = 32;
-constexpr int PM_CHUNK = PM_WARPS * PM_TILE;
-
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"(addr));
-}
-// D += A B, all sixteen rows of A: rows 0..7 carry the f16 heads of the eight query heads' values, rows 8..15 their
-// f16 tails, so one instruction yields both partial products (c[0..1] = head row g, c[2..3] = tail row g).
-__device__ __forceinline__ void mma_hi_lo(float (&c)[4], uint32_t a_hi0, uint32_t a_lo0, uint32_t a_hi1, uint32_t a_lo1, uint32_t b0,
-                                          uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a_hi0), "r"(a_lo0), "r"(a_hi1), "r"(a_lo1), "r"(b0), "r"(b1));
-}
-// (x, y) as an f16 pair plus the f16 pair of what that rounding lost.
-__device__ __forceinline__ void split_half2(float x, float y, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(x, y);
-    const float2 f = __half22float2(h);
-    const __half2 t = __floats2half2_rn(x - f.x, y - f.y);
-    hi = *(const uint32_t *)&h;
-    lo = *(const uint32_t *)&t;
-}
-
-// FUSED (decode steps: at most one token per sequence in the call) folds the neighbours of the attention into the
+// Decode steps (at most one token per sequence in the call) only: the neighbours of the attention are folded into the
 // same launch.  RoPE: the query heads are rotated on their way into the A fragments, and the warp whose tile holds the
 // token's own position rotates the new K row, converts K and V to f16 and puts them into its tile AND into the pool
 // (no other CTA of the launch reads that pool row: every other position belongs to an earlier step).  Merge: a CTA
 // that is alone on its token writes the output itself; otherwise each CTA writes its chunk state, takes a ticket, and
 // the CTA that draws the last ticket of a (token, KV head) merges the chunk states in chunk order -- the arithmetic of
 // paged_attention_merge_kernel, so both forms give the same bits.
-struct FusedDecode {
-    const float2 *rope;  // [T][HD / 2] {cos, sin} of position * frequency, from rope_table_kernel
-    int *tickets;        // [T][kv_heads], zero between launches; null: the chunk states are merged by a kernel of its own
-    int neox;
-};
-
-template <int HD, bool FUSED>
+template <int HD>
 __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(PagedParams p, float *partial, FusedDecode fd) {
     constexpr int ROWB = HD * 2;            // bytes of a K or V row
     constexpr int PIECES = ROWB / 16;       // 16-byte pieces per row
@@ -567,9 +521,9 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
     const uint32_t sV = sK + TILEB;
     const uint32_t k0 = p0 + (uint32_t)(warp * PM_TILE);  // this warp's positions [k0, k0 + 32)
     const bool has_tile = k0 < p1;                        // uniform over the warp
-    // FUSED: the token's own row (position kv_len - 1) comes from k_new / v_new, not from the pool
+    // the token's own row (position kv_len - 1) comes from k_new / v_new, not from the pool
     const uint32_t new_pos = kv_len - 1u;
-    const int new_row = FUSED && new_pos >= k0 && new_pos < k0 + PM_TILE ? (int)(new_pos - k0) : -1;
+    const int new_row = new_pos >= k0 && new_pos < k0 + PM_TILE ? (int)(new_pos - k0) : -1;
     // stage the tile: lane r looks up the pool block of position k0 + r, the warp copies two rows per step
     uint32_t live = 0;
     if (has_tile) {
@@ -593,7 +547,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (FUSED && new_row >= 0) {
+        if (new_row >= 0) {
             // the new K row rotated, the new V row, both as f16: into this warp's tile and into the pool slot
             const int half = HD / 2, r = new_row;
             const float2 *rope = fd.rope + (size_t)t * half;
@@ -623,7 +577,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
     }
 
     // A fragments of Q (row g = query head g of the group): a0 = dims 16s + 2tq, +1; a2 = dims 16s + 8 + 2tq, +1.
-    // FUSED: the values are rotated on the way (the partner of a dimension is its neighbour, or lies half a head
+    // The values are rotated on the way (the partner of a dimension is its neighbour, or lies half a head
     // away with the NeoX pairing; either way this lane reads it itself).
     uint32_t qhi[KS][2], qlo[KS][2];
     {
@@ -637,7 +591,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
 #pragma unroll
             for (int hk = 0; hk < 2; ++hk)
                 qv[s][hk] = head_ok ? *(const float2 *)(qrow + 16 * s + 8 * hk + 2 * tq) : make_float2(0.0f, 0.0f);
-        if (FUSED) {
+        {
             const float2 *rope = fd.rope + (size_t)t * (HD / 2);
             if (!fd.neox) {  // the pair (d, d + 1) is one float2
                 float2 cs[KS][2];
@@ -794,7 +748,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
             L += s_l[w * 8 + hh] * e;
             O += s_o[((size_t)w * 8 + hh) * HD + d] * e;
         }
-        if (FUSED && fd.tickets != nullptr && (kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1)) {  // the only chunk of its token: this is the result
+        if (fd.tickets != nullptr && (kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1)) {  // the only chunk of its token: this is the result
             p.out[((size_t)t * p.n_q_heads + (size_t)h * gsize + hh) * HD + d] = L > 0.0f ? O / L : 0.0f;
             continue;
         }
@@ -808,7 +762,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
         }
         pr[2 + d] = O;
     }
-    if (!FUSED || kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1 || fd.tickets == nullptr) return;
+    if (kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1 || fd.tickets == nullptr) return;
     // the last CTA of this (token, KV head) to finish merges the chunk states
     const int live_chunks = min(n_chunks, (int)((kv_len + (uint32_t)PM_CHUNK - 1u) / (uint32_t)PM_CHUNK));
     __threadfence();
@@ -826,8 +780,8 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
     // every (head, dimension) adds up its column with the loads of eight chunks in flight.  Same operations in the same
     // order as paged_attention_merge_kernel.
     float *s_cm = (float *)pm_smem;                 // [head][chunk] m, later the chunk's weight exp(m - M)
-    float *s_cl = s_cm + 8 * live_chunks;           // [head][chunk] l
-    float *s_M = s_cl + 8 * live_chunks;            // [head]
+    float *s_cl = s_cm + gsize * live_chunks;       // [head][chunk] l
+    float *s_M = s_cl + gsize * live_chunks;        // [head]
     __syncthreads();
     for (int idx = threadIdx.x; idx < gsize * live_chunks; idx += blockDim.x) {
         const int hh = idx / live_chunks, cc = idx - hh * live_chunks;
@@ -875,51 +829,77 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
     }
 }
 
-// out[t][qh][:] from the chunk states; grid (query heads, tokens), HD threads.  The chunks' maxima and sums go to shared
-// memory first (one load per thread, all in flight together), then every thread adds up its column eight chunks at a
-// time; chunk order throughout, so the result does not depend on how the work was cut.
+// out[t][qh][:] from the chunk states, one warp per (token, query head), eight to a CTA: lane c reads the maximum and the sum of
+// chunk c, the warp agrees on the maximum and every lane adds up its HD / 32 columns eight chunks at a time; chunk order
+// throughout, so the result does not depend on how the work was cut.  A token with a single chunk has its result already when
+// `direct` is set.  (A CTA of HD threads per pair: 21 us for 500 tokens of 32 heads.)
+constexpr int MERGE_WARPS = 8;
 template <int HD>
-__global__ void paged_attention_merge_kernel(PagedParams p, int chunk, int n_chunks, const float *partial) {
-    extern __shared__ float mg_s[];  // m [live], then weight exp(m - M) in place; l [live]
+__global__ void __launch_bounds__(32 * MERGE_WARPS)
+paged_attention_merge_kernel(PagedParams p, int chunk, int n_chunks, int direct, const float *partial) {
     MCU_PDL_PROLOGUE();
-    const int qh = blockIdx.x, t = blockIdx.y, d = threadIdx.x;
+    constexpr int N = HD / 64;  // float2 columns of a lane
+    const int lane = threadIdx.x & 31;
+    const long pair = (long)blockIdx.x * MERGE_WARPS + (threadIdx.x >> 5);
+    const int t = (int)(pair / p.n_q_heads);
+    if (t >= p.n_tokens) return;
     const uint32_t kv_len = p.meta[t * 4 + 1] + 1u;
     const int live = min(n_chunks, (int)((kv_len + (uint32_t)chunk - 1u) / (uint32_t)chunk));
-    const float *pr = partial + ((size_t)t * p.n_q_heads + qh) * n_chunks * (HD + 2);
-    float *s_e = mg_s, *s_l = mg_s + n_chunks;
-    for (int c = d; c < live; c += HD) {
-        s_e[c] = pr[(size_t)c * (HD + 2)];
-        s_l[c] = pr[(size_t)c * (HD + 2) + 1];
+    if (direct && live == 1) return;
+    const float *pr = partial + (size_t)pair * n_chunks * (HD + 2);
+    float M = -INFINITY, m0 = -INFINITY, l0 = 0.0f;  // of chunk `lane`
+    for (int c = lane; c < live; c += 32) {
+        const float2 ml = *(const float2 *)(pr + (size_t)c * (HD + 2));
+        if (c < 32) m0 = ml.x, l0 = ml.y;
+        M = fmaxf(M, ml.x);
     }
-    __syncthreads();
-    float M = -INFINITY;
-    for (int c = 0; c < live; ++c) M = fmaxf(M, s_e[c]);
-    __syncthreads();
-    for (int c = d; c < live; c += HD) {
-        const float mc = s_e[c];
-        s_e[c] = (M == -INFINITY || mc == -INFINITY) ? 0.0f : expf(mc - M);  // 0: the chunk adds nothing
-    }
-    __syncthreads();
-    float L = 0.0f, o = 0.0f;
-    const float *col = pr + 2 + d;
-    int c = 0;
-    for (; c + 8 <= live; c += 8) {
-        float v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = col[(size_t)(c + u) * (HD + 2)];
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    float L = 0.0f;
+    float2 acc[N];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (s_e[c + u] != 0.0f) {
-                L += s_l[c + u] * s_e[c + u];
-                o += v[u] * s_e[c + u];
-            }
-    }
-    for (; c < live; ++c)
-        if (s_e[c] != 0.0f) {
-            L += s_l[c] * s_e[c];
-            o += col[(size_t)c * (HD + 2)] * s_e[c];
+    for (int i = 0; i < N; ++i) acc[i] = make_float2(0.0f, 0.0f);
+    for (int base = 0; base < live; base += 32) {
+        if (base > 0) {
+            const float2 ml = base + lane < live ? *(const float2 *)(pr + (size_t)(base + lane) * (HD + 2)) : make_float2(-INFINITY, 0.0f);
+            m0 = ml.x, l0 = ml.y;
         }
-    p.out[((size_t)t * p.n_q_heads + qh) * HD + d] = L > 0.0f ? o / L : 0.0f;
+        const float e = (M == -INFINITY || m0 == -INFINITY) ? 0.0f : expf(m0 - M);  // 0: the chunk adds nothing
+        const int n = min(32, live - base);
+        for (int c = 0; c < n; c += 8) {
+            float2 v[8][N];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                    if (c + u < n) v[u][i] = *(const float2 *)(pr + (size_t)(base + c + u) * (HD + 2) + 2 + 2 * (lane + 32 * i));
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float eu = __shfl_sync(0xffffffffu, e, (c + u) & 31), lu = __shfl_sync(0xffffffffu, l0, (c + u) & 31);
+                if (c + u < n && eu != 0.0f) {
+                    L += lu * eu;
+#pragma unroll
+                    for (int i = 0; i < N; ++i) {
+                        acc[i].x += v[u][i].x * eu;
+                        acc[i].y += v[u][i].y * eu;
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        float *to = p.out + (size_t)pair * HD + 2 * (lane + 32 * i);
+        to[0] = L > 0.0f ? acc[i].x / L : 0.0f;
+        to[1] = L > 0.0f ? acc[i].y / L : 0.0f;
+    }
+}
+
+static cudaError_t launch_merge(const PagedParams &p, size_t head_dim, size_t chunk, size_t n_chunks, bool direct, const float *partial,
+                                cudaStream_t s) {
+    const dim3 grid((unsigned)(((size_t)p.n_tokens * p.n_q_heads + MERGE_WARPS - 1) / MERGE_WARPS));
+    return launch_pdl(head_dim == 64 ? paged_attention_merge_kernel<64> : paged_attention_merge_kernel<128>, grid, dim3(32 * MERGE_WARPS), s, p,
+                      (int)chunk, (int)n_chunks, direct ? 1 : 0, partial);
 }
 
 }  // namespace mcu
@@ -1119,6 +1099,7 @@ int mcu_paged_attention(mcu_context_t *ctx, const uint32_t *token_meta_dev, size
     p.block_shift = 0;
     while (((size_t)1 << p.block_shift) < block_size) ++p.block_shift;
     p.scale = scale;
+    p.n_tokens = (int)T;
     if (n_q_heads / n_kv_heads > (size_t)PA_MAX_GROUP)
         return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention supports up to 8 query heads per KV head");
     // chunk of positions per CTA: long enough to amortise the set-up, short enough that every SM gets several CTAs
@@ -1131,35 +1112,22 @@ int mcu_paged_attention(mcu_context_t *ctx, const uint32_t *token_meta_dev, size
            n_kv_heads * T * ((max_positions + chunk - 1) / chunk) < 2 * (size_t)device_sm_count())
         chunk /= 2;
     const size_t n_chunks = (max_positions + chunk - 1) / chunk;
-    if (n_chunks > 6000) return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention context bound too long");  // (the merge keeps two floats per chunk in shared memory)
+    if (n_chunks > 6000) return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention context bound too long");
     void *scratch = nullptr;
     if (int rc = context_attention_scratch(ctx, T * n_q_heads * n_chunks * (head_dim + 2) * sizeof(float), &scratch))
         return rc;
     float *partial = (float *)scratch;
-    const dim3 ag((unsigned)T, (unsigned)n_kv_heads), qg((unsigned)n_kv_heads, (unsigned)T, (unsigned)n_chunks);
-    const dim3 mg((unsigned)n_q_heads, (unsigned)T);
-    const unsigned threads = 32u * (unsigned)(n_q_heads / n_kv_heads);
-    const dim3 tb(threads);
+    const dim3 ag((unsigned)T, (unsigned)n_kv_heads);
     if (mma_path) {
-        const size_t smem = (size_t)PM_WARPS * 2 * PM_TILE * head_dim * 2;  // >= the warps' merge states (8 heads each)
-        if (head_dim == 64)
-            DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        else
-            DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         DEC_CUDA(launch_pdl(kv_append_kernel<__half>, ag, dim3(128), s, p, (int)head_dim));
-        if (head_dim == 64)
-            DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<64, false>, qg, dim3(32 * PM_WARPS), smem, s, p, partial, FusedDecode{}));
-        else
-            DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<128, false>, qg, dim3(32 * PM_WARPS), smem, s, p, partial, FusedDecode{}));
+        DEC_CUDA(launch_attention_prompt(p, (int)head_dim, (int)n_chunks, partial, context_err_flag(ctx), s));
     } else {
+        const dim3 qg((unsigned)n_kv_heads, (unsigned)T, (unsigned)n_chunks), tb(32u * (unsigned)(n_q_heads / n_kv_heads));
         DEC_CUDA(launch_pdl(kv_append_kernel<float>, ag, dim3(128), s, p, (int)head_dim));
         if (head_dim == 64) DEC_CUDA(launch_pdl(paged_attention_kernel<float, 64>, qg, tb, s, p, (int)chunk, partial));
         else DEC_CUDA(launch_pdl(paged_attention_kernel<float, 128>, qg, tb, s, p, (int)chunk, partial));
     }
-    if (head_dim == 64)
-        DEC_CUDA(launch_pdl_smem(paged_attention_merge_kernel<64>, mg, dim3(64), 2 * n_chunks * sizeof(float), s, p, (int)chunk, (int)n_chunks, (const float *)partial));
-    else
-        DEC_CUDA(launch_pdl_smem(paged_attention_merge_kernel<128>, mg, dim3(128), 2 * n_chunks * sizeof(float), s, p, (int)chunk, (int)n_chunks, (const float *)partial));
+    DEC_CUDA(launch_merge(p, head_dim, chunk, n_chunks, mma_path, partial, s));
     count_launches(3);
     return MCU_SUCCESS;
 }
@@ -1230,13 +1198,15 @@ int mcu_paged_attention_decode(mcu_context_t *ctx, const uint32_t *token_meta_de
     p.block_shift = 0;
     while (((size_t)1 << p.block_shift) < block_size) ++p.block_shift;
     p.scale = scale;
+    p.n_tokens = (int)T;
     const size_t max_positions = max_blocks_per_seq * block_size;
     const size_t n_chunks = (max_positions + PM_CHUNK - 1) / PM_CHUNK;
-    if (n_chunks > 6000) return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention context bound too long");  // (the merge keeps two floats per chunk in shared memory)
+    if (n_chunks > 6000) return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention context bound too long");
     // Few CTAs: the step is a chain of latencies, and the last CTA of a token merging in place saves a launch.  Many
     // CTAs: the fence and the ticket keep every CTA (and its shared memory) alive for a round trip to L2 longer, which
     // at 64 sequences x 8 KV heads x ~17 chunks cost 25 % of the kernel (measured); a merge kernel is cheaper there.
     const bool ticket_merge = n_kv_heads * T * n_chunks <= 4 * (size_t)device_sm_count();
+    const bool by_warp = !ticket_merge && attention_decode_supported((int)T);
     void *scratch = nullptr, *tickets = nullptr;
     if (int rc = context_attention_scratch(ctx, T * n_q_heads * n_chunks * (head_dim + 2) * sizeof(float), &scratch)) return rc;
     if (ticket_merge)
@@ -1253,20 +1223,18 @@ int mcu_paged_attention_decode(mcu_context_t *ctx, const uint32_t *token_meta_de
     fd.neox = rope_type == MCU_ROPE_NEOX ? 1 : 0;
     const dim3 qg((unsigned)n_kv_heads, (unsigned)T, (unsigned)n_chunks);
     const size_t smem = (size_t)PM_WARPS * 2 * PM_TILE * head_dim * 2;
-    if (head_dim == 64) {
-        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<64, true>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
+    if (by_warp) {
+        DEC_CUDA(launch_attention_decode(p, (int)head_dim, (int)n_chunks, (float *)scratch, fd, context_err_flag(ctx), s));
+    } else if (head_dim == 64) {
+        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<64>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
     } else {
-        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<128, true>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
+        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<128>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
     }
     count_launches(1);
     if (!ticket_merge) {
-        const dim3 mg((unsigned)n_q_heads, (unsigned)T);
-        if (head_dim == 64)
-            DEC_CUDA(launch_pdl_smem(paged_attention_merge_kernel<64>, mg, dim3(64), 2 * n_chunks * sizeof(float), s, p, (int)PM_CHUNK, (int)n_chunks, (const float *)scratch));
-        else
-            DEC_CUDA(launch_pdl_smem(paged_attention_merge_kernel<128>, mg, dim3(128), 2 * n_chunks * sizeof(float), s, p, (int)PM_CHUNK, (int)n_chunks, (const float *)scratch));
+        DEC_CUDA(launch_merge(p, head_dim, PM_CHUNK, n_chunks, by_warp, (const float *)scratch, s));
         count_launches(1);
     }
     return MCU_SUCCESS;
