@@ -1,4 +1,5 @@
-"""Build libmarmot_cuda.so in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
+"""Build libmarmot_cuda.so in-tree with nvcc for sm_100a (cross-compiles without a GPU), and the Python binding of its smallest
+operator with g++."""
 from __future__ import annotations
 
 import os
@@ -11,6 +12,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT = PKG / "libmarmot_cuda.so"
 OBJ_DIR = PKG / "build"
+BINDING = PKG / "_binding.so"
 
 SOURCES = ["abi.cu", "act_quant.cu", "dequant.cu", "gemv.cu", "gemv_stream.cu", "gemv_stream_addnorm.cu", "gemv_stream_swiglu.cu", "gemm_tma.cu", "gemm_ts.cu", "gemm_ti.cu", "linear_f16.cu", "moe.cu", "static_scratch.cu", "peer.cu", "decoder.cu", "attention.cu", "decode_step.cu", "kv_pool.cu", "gguf.cu"]
 NVCC_FLAGS = [
@@ -28,6 +30,25 @@ def _newest_input() -> float:
     files = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
     files.append(PKG.parent / "include" / "marmot_cuda.h")
     return max(f.stat().st_mtime for f in files)
+
+
+def build_binding(force: bool = False) -> Path:
+    """The extension module of csrc/binding.cpp, against the torch that is installed here."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    src = CSRC / "binding.cpp"
+    if not force and BINDING.exists() and BINDING.stat().st_mtime >= src.stat().st_mtime:
+        return BINDING
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    cmd += [f"-I{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], str(Path(_nvcc()).resolve().parent.parent / "include"))]
+    cmd += [str(src), "-o", str(BINDING), *(f"-L{p}" for p in library_paths()), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {src}\n{r.stderr}")
+    return BINDING
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -57,3 +78,4 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 if __name__ == "__main__":
     print(build(force=True, verbose="-v" in sys.argv))
+    print(build_binding())

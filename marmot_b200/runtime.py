@@ -194,6 +194,29 @@ def load_library() -> C.CDLL:
     return L
 
 
+_binding = None
+
+
+def load_binding():
+    """The native form of Context.linear (csrc/binding.cpp), or False where it has not been built: the same call through ctypes."""
+    global _binding
+    if _binding is None:
+        path = LIB_PATH.with_name("_binding.so")
+        _binding = False
+        if path.exists():
+            import importlib.machinery
+            import importlib.util
+
+            import torch  # noqa: F401  (the module links against its libraries)
+
+            loader = importlib.machinery.ExtensionFileLoader("_binding", str(path))
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_binding", loader))
+            loader.exec_module(module)
+            module.set_entry_points(C.cast(load_library().mcu_linear, C.c_void_p).value)
+            _binding = module
+    return _binding
+
+
 def _ptr(t) -> int:
     return 0 if t is None else int(t.data_ptr())
 
@@ -210,6 +233,9 @@ class Context:
         h = C.c_void_p()
         self._check(self.lib.mcu_context_create(device, C.byref(h)))
         self.handle = h
+        self._address = h.value  # of the native calls
+        binding = load_binding()
+        self._linear = binding.linear if binding else None
         if use_torch_stream:
             with torch.cuda.device(device):
                 # torch reports the legacy default stream as handle 0, which this ABI reads as
@@ -220,7 +246,7 @@ class Context:
     def close(self):
         if getattr(self, "handle", None):
             self.lib.mcu_context_destroy(self.handle)
-            self.handle = None
+            self.handle, self._address = None, 0
 
     def __del__(self):
         try:
@@ -270,6 +296,12 @@ class Context:
         return qs, d, bs
 
     def linear(self, kind: int, x, w, F: int, bias=None, out=None):
+        if self._linear is not None and kind in BLOCK_BYTES:
+            r = self._linear(self._address, kind, BLOCK_VALUES[kind], BLOCK_BYTES[kind], x, w, F, bias, out)
+            if r.__class__ is not int:
+                return r
+            if r < 0:
+                self._check(r)
         T, K = x.shape
         assert x.stride(1) == 1 and w.numel() * w.element_size() >= F * row_bytes(kind, K)
         if out is None:
