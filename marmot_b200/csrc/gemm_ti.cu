@@ -136,7 +136,8 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     const uint32_t tile_base = (bar_base + 512u + 1023u) & ~1023u;
     float *sums = (float *)(smem_raw + (tile_base + TI_B_SLOTS * B_BYTES - raw_addr));  // [16][128]: group 1's part of a tile
     const uint32_t share_addr = tile_base + TI_B_SLOTS * B_BYTES + TI_COLS * TS_ROWS * 4u;
-    const uint32_t ring_addr = share_addr + (TI_COLS + TS_MAX_SPLIT) * TS_ROWS * 4u;  // (share_addr: the shares of a split tile)
+    float *shared_share = (float *)(smem_raw + (share_addr - raw_addr));  // [16][128]: this CTA's share of a split tile
+    const uint32_t ring_addr = share_addr + TI_COLS * TS_ROWS * 4u;
     uint8_t *ring = smem_raw + (ring_addr - raw_addr);
     const uint32_t R = 1u << p.raw_shift;
     const uint32_t a_full = bar_base, b_full = bar_base + 16u, ab_empty = bar_base + 48u, d_full = bar_base + 80u, d_empty = bar_base + 96u,
@@ -179,13 +180,12 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (split > 1) ts_cluster_arrive();
 
     const TsWork work = ts_work(p, grouped, group_tile0, TI_COLS, cta, n_cta);
     const int KS = p.slabs, u0 = work.u0, u1 = work.u1, n_use = work.n_use, n_slabs = u1 - u0;
     const long long U = work.units;
 
-    bool ok = true, joined = split == 1;  // joined: through the first cluster barrier
+    bool ok = true;
     int err_code = 0;
     if (warp == TI_B_WARP) {
         // ------------------------------ activation tiles ------------------------------
@@ -442,10 +442,8 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                 const int u_lo = u;
                 u = u_hi;
                 if (split > 1) {
-                    ts_cluster_wait();
-                    joined = true;
-                    ts_push_share<16>(share_addr, cta - cta / split * split, ts_split_cols(t.t_count, split), 0, t.t_count, r,
-                                      [&](int c) { return acc[c >> 3][c & 7]; });
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) shared_share[c * TS_ROWS + r] = acc[c >> 3][c & 7];
                     continue;
                 }
                 if (u_hi - u_lo != KS) {
@@ -498,10 +496,6 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
             err_code = 50;
         }
     }
-    if (!joined) {
-        __syncwarp();
-        ts_cluster_wait();
-    }
     if (!ok) {
         if (lane == 0) atomicExch(p.err, err_code);
         abort_flag = 1;
@@ -514,22 +508,31 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     }
     if (split > 1) {
         __syncwarp();
-        ts_cluster_sync();  // the shares have arrived
+        ts_cluster_sync();  // the shares of the split tile are complete
         const TsTile t = work.tile(p, cta / split);
         const TsJob &jb = p.jobs[t.job];
-        const int part = cta - cta / split * split, cw = ts_split_cols(t.t_count, split), mine = min(cw, t.t_count - part * cw);
+        const int part = cta - cta / split * split, c_lo = t.t_count * part / split, c_hi = t.t_count * (part + 1) / split;
         const int r = threadIdx.x & (TS_ROWS - 1), fr = loose ? (r >> 4) + 8 * (r & 15) : r, f = t.f0 + fr;
         if (threadIdx.x >= 256 && threadIdx.x < 512 && fr < t.rows) {  // (the scalers: they have waited for the kernel ahead)
-            const float *got = (const float *)(smem_raw + (share_addr - raw_addr)) + r;
             const float bias = jb.bias != nullptr ? jb.bias[f] : 0.0f;
-            for (int c = (int)((threadIdx.x - 256) >> 7); c < mine; c += 2) {
-                float sum = got[c * TS_ROWS];
+            for (int c = c_lo + (int)((threadIdx.x - 256) >> 7); c < c_hi; c += 2) {
+                float v[TS_MAX_SPLIT];
 #pragma unroll
-                for (int k = 1; k < TS_MAX_SPLIT; ++k)
-                    if (k < split) sum += got[(k * cw + c) * TS_ROWS];
-                jb.out[(size_t)(t.t_row0 + part * cw + c) * jb.ldo + f] = sum + bias;
+                for (int i = 0; i < TS_MAX_SPLIT; ++i) {
+                    v[i] = 0.0f;
+                    if (i < split)
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                                     : "=f"(v[i]) : "r"(ts_mapa(share_addr + 4u * (uint32_t)(c * TS_ROWS + r), (uint32_t)i)) : "memory");
+                }
+                float sum = v[0];
+#pragma unroll
+                for (int i = 1; i < TS_MAX_SPLIT; ++i)
+                    if (i < split) sum += v[i];
+                jb.out[(size_t)(t.t_row0 + c) * jb.ldo + f] = sum + bias;
             }
         }
+        __syncwarp();
+        ts_cluster_sync();  // nobody leaves while its share is being read
     }
     if (warp == TI_MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -548,7 +551,7 @@ bool gemm_ti_supported(int kind, const void *W, int K, int F) {
 
 template <int KIND>
 static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
-    const int fixed = 16 + 512 + 1024 + TI_B_SLOTS * (int)ti_b_bytes<KIND>() + (2 * TI_COLS + TS_MAX_SPLIT) * TS_ROWS * 4;
+    const int fixed = 16 + 512 + 1024 + TI_B_SLOTS * (int)ti_b_bytes<KIND>() + 2 * TI_COLS * TS_ROWS * 4;
     const int slab = ts_slab_bytes<KIND>(p.loose != 0);
     constexpr int MOST = 224 * 1024;
     p.raw_shift = fixed + 8 * slab <= MOST ? 3 : 2;

@@ -36,9 +36,6 @@ constexpr int ts_slab_bytes(bool loose) {  // loose slabs keep the up to seven l
 __device__ __forceinline__ void ts_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The two halves of a cluster barrier, once per warp each.
-__device__ __forceinline__ void ts_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void ts_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t ts_mapa(uint32_t addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
@@ -162,24 +159,6 @@ __device__ __forceinline__ TsWork ts_work(const TsParams &p, bool grouped, const
         w.u1 = t * KS + KS * (part + 1) / p.split;
     }
     return w;
-}
-
-// A tile split over a cluster: every CTA has the sums of its part of K and finishes `cw` of the tile's columns.  The shares are pushed
-// into the shared memory of the CTA that needs them, [CTA they come from][column][128 rows], while the sums are read out of tensor
-// memory; one cluster barrier later everybody adds up what it has got.  (Pulled out of the other CTAs' shared memory they cost a
-// trip per column and a second barrier before anybody may leave: 16 x 2048 x 2048 Q4_K 7.8 -> 7.2 us.  The fp16 kernel pulls: pushed
-// it was no faster at 32 and 64 tokens, whose larger tiles have no place of their own to be pushed to.)
-__device__ __forceinline__ int ts_split_cols(int t_count, int split) { return (t_count + split - 1) / split; }
-template <int N, class Value>
-__device__ __forceinline__ void ts_push_share(uint32_t recv, int part, int cw, int c0, int count, int r, Value value) {
-    int owner = c0 / cw, local = c0 - owner * cw;
-    uint32_t to = ts_mapa(recv, (uint32_t)owner);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        if (c0 + i < count)
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4u * (uint32_t)((part * cw + local) * TS_ROWS + r)), "f"(value(i)) : "memory");
-        if (++local == cw && c0 + i + 1 < count) local = 0, to = ts_mapa(recv, (uint32_t)++owner);
-    }
 }
 
 // The slab producer (one warp): every slab of the CTA's range, in order, into the ring.
