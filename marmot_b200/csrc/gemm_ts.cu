@@ -584,7 +584,29 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
             for (int i = 0; i < TS_MAX_SPLIT; ++i)
                 from[i] = i < split ? ts_mapa(tile_base + 4u * (uint32_t)r, (uint32_t)i) : 0u;
             const float bias = jb.bias != nullptr ? jb.bias[f] : 0.0f;
-            for (int c = c_lo + (int)(threadIdx.x >> 7); c < c_hi; c += 4) {
+            int c = c_lo + (int)(threadIdx.x >> 7);
+            if (split == 2) {
+                // Pairs share wide tiles: eight columns at a time, so that sixteen loads are under way (500 x 4096 x 4096 Q4_K, 125
+                // columns for each CTA: 31.1 -> 27.6 us; with four and eight CTAs to a tile it was slower, 13.4 -> 13.7 at 64 tokens).
+                constexpr int BATCH = 8;
+                for (; c < c_hi; c += 4 * BATCH) {
+                    float v[2][BATCH];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int j = 0; j < BATCH; ++j) {
+                            v[i][j] = 0.0f;
+                            if (c + 4 * j < c_hi)
+                                asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                                             : "=f"(v[i][j]) : "r"(from[i] + (uint32_t)(c + 4 * j) * (TS_ROWS * 4u)) : "memory");
+                        }
+#pragma unroll
+                    for (int j = 0; j < BATCH; ++j)
+                        if (c + 4 * j < c_hi)
+                            jb.out[(size_t)(t.t_row0 + c + 4 * j) * jb.ldo + f] = (v[0][j] + v[1][j]) * p.rowscale[t.t_row0 + c + 4 * j] + bias;
+                }
+            }
+            for (; c < c_hi; c += 4) {
                 float v[TS_MAX_SPLIT];
 #pragma unroll
                 for (int i = 0; i < TS_MAX_SPLIT; ++i) {
