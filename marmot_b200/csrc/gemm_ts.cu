@@ -638,31 +638,36 @@ struct TsPlan {
     double cost;
 };
 
-// How to spread `tiles` output tiles of KS slabs over the SMs, and what it costs in cycles.  A slab takes the longer of its
-// conversion and its MMAs (8 bn; 10 bn for wide tiles, whose activation traffic fills shared memory's bandwidth); a tile shared
-// by a cluster costs two cluster barriers and the exchange, a tile cut between ranges a trip of every share through L2 and a
-// ticket (5000 measured).
+// How to spread `tiles` output tiles of KS slabs over the SMs, and what it costs in cycles, by measurements of all the forms at 70 to 512
+// tokens and 2048 x 2048 to 4096 x 28672 weights.  A slab takes the longer of its conversion (less in tiles of up to 64 columns, whose
+// stages hold 128 values of K) and its MMAs; a tile ends with its epilogue.
+// - One tile per CTA, in as many waves as it takes: 2000 for a CTA's start.
+// - A tile over a cluster: the exchange of the shares through the CTAs' shared memories.
+// - Equal ranges of slabs: cut tiles have their shares written to memory, and read again by the CTA that comes last; a tile of 256
+//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).
 static TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles) {
     const int room = device_sm_count();
     const long U = (long)tiles * KS;
-    const double conv = kind == KIND_Q4_K ? 1500 : kind == KIND_Q6_K ? 2200 : 2000, mma = (bn > 128 ? 10.0 : 8.0) * bn;
-    const double unit = mma > conv ? mma : conv, tile_end = 1000.0 + 8.0 * bn;
+    const bool wide = bn > 64;
+    const double conv = kind == KIND_Q4_K ? (wide ? 1500 : 1120) : kind == KIND_Q6_K ? (wide ? 2100 : 1700) : (wide ? 1750 : 1500);
+    const double mma = 8.5 * bn, unit = mma > conv ? mma : conv, tile_end = 1000.0 + 8.0 * bn;
     TsPlan best{bn, t_tiles, 1, 0, 1e30};
     auto consider = [&](int split, long n, double cost) {
         if (cost < best.cost) best = TsPlan{bn, t_tiles, split, (int)n, cost};
     };
-    if (tiles <= room) consider(1, tiles, KS * unit + tile_end);
+    consider(1, tiles, (double)((tiles + room - 1) / room) * (KS * unit + tile_end + 2000.0));
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2) {
         // A cluster is placed inside a GPC (16 to 20 SMs): sixteen clusters of eight did not run at once (2048 x 2048: 12.6 us,
         // 64 CTAs in clusters of four 7.5).
         const int usable = sp >= 8 ? room / 2 : room;
-        if ((long)tiles * sp <= usable) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + tile_end + 1000.0);
+        const double exchange = sp == 2 ? 3500.0 + 30.0 * bn : 5000.0 + 20.0 * bn;
+        if ((long)tiles * sp <= usable) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + tile_end + 2000.0 + exchange);
     }
     const long n = U < room ? U : room;
     const long upc = (U + n - 1) / n;
     const bool cut = U % n != 0 || upc % KS != 0;
     const double shares = cut ? (double)KS / upc + 1.0 : 0.0;
-    consider(1, n, upc * unit + ((double)upc / KS + 1.0) * tile_end + (cut ? 5000.0 + shares * 10.0 * bn : 0.0));
+    consider(1, n, upc * unit + ((double)upc / KS + 1.0) * tile_end + 2000.0 + shares * 65.0 * bn);
     return best;
 }
 
@@ -673,12 +678,14 @@ static TsPlan ts_plan(int kind, int T, int K, const int *F, int n_jobs) {
     for (int j = 0; j < n_jobs; ++j) rows += (F[j] + TS_ROWS - 1) / TS_ROWS;
     TsPlan best{};
     best.cost = 1e30;
-    for (int most = 256; most >= 128; most -= 128) {
-        const int t_tiles = (T + most - 1) / most;
+    // as few token tiles as there can be, or a few more: narrower tiles fill the SMs better, but the weights are converted more often
+    // (6 % for each: with all SMs at work the chip runs into its power limit)
+    const int fewest = (T + 255) / 256, most = (T + 63) / 64;
+    for (int t_tiles = fewest; t_tiles <= most && t_tiles <= fewest + 3; ++t_tiles) {
         const int bn = ((T + t_tiles - 1) / t_tiles + 15) / 16 * 16;
-        const TsPlan pl = ts_spread(kind, rows * t_tiles, KS, bn, t_tiles);
+        TsPlan pl = ts_spread(kind, rows * t_tiles, KS, bn, t_tiles);
+        pl.cost *= 1.0 + 0.06 * (t_tiles - fewest);
         if (pl.cost < best.cost) best = pl;
-        if (t_tiles == 1 && bn <= 128) break;
     }
     return best;
 }
