@@ -649,7 +649,7 @@ int linear_fused_allreduce(mcu_context *ctx, int kind, const float *x, size_t ld
     if (int rc = check_ctx(ctx)) return rc;
     if (int rc = validate_linear(kind, x, w, out, T, K, F, ldx, F)) return rc;
     if (ctx->regime == MCU_REGIME_GEMV || ctx->regime == MCU_REGIME_GEMV_PLAIN || !gemm_tma_can_fuse(kind, (int)T, (int)F) ||
-        !gemm_tma_supported(kind, w, nullptr, (int)T, (int)K, (int)F) || act_half_fused_smem(kind, (int)K) > 48 * 1024)
+        !gemm_tma_supported(kind, w, (int)T, (int)K, (int)F) || act_half_fused_smem(kind, (int)K) > 48 * 1024)
         return fail(MCU_ERROR_NOT_IMPLEMENTED, "shape or weights do not suit the fused matmul + all-reduce");
     std::lock_guard<std::mutex> lock(ctx->mu);
     const size_t bv = (size_t)block_values(kind);
@@ -659,11 +659,9 @@ int linear_fused_allreduce(mcu_context *ctx, int kind, const float *x, size_t ld
     if (int rc = ensure(ctx, ctx->gemm_partial, gemm_tma_workspace_bytes(kind, (int)T, (int)K, (int)F))) return rc;
     MCU_CUDA(launch_act_half_fused_from(kind, x, (int)ldx, ActSource{}, (int)T, (int)K, (__half *)ctx->act_half.ptr,
                                    (float *)ctx->act_rowscale.ptr, ctx->stream));
-    int launches = 0;
-    MCU_CUDA(launch_gemm_tma(kind, w, nullptr, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr,
-                             (int)kp, (int)T, (int)K, (int)F, nullptr, out, nullptr, (int)F, (float *)ctx->gemm_partial.ptr,
-                             ctx->gemm_counters, ctx->dev_err, ctx->stream, &launches, &fuse));
-    count_launches(1 + launches);
+    MCU_CUDA(launch_gemm_tma(kind, w, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr, (int)kp, (int)T, (int)K,
+                             (int)F, out, (float *)ctx->gemm_partial.ptr, ctx->gemm_counters, ctx->dev_err, ctx->stream, fuse));
+    count_launches(2);
     return MCU_SUCCESS;
 }
 }  // namespace mcu

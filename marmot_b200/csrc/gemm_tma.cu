@@ -1,21 +1,20 @@
-// TMA-fed variant of the tensor-core quantized matmul (tcgen05 + TMEM), used when the weight rows are
-// 16-byte multiples (K % 2048 == 0 for Q6_K, K % 256 == 0 for Q8_0, always for Q4_K).
+// Row-parallel matmul fused with its all-reduce over peer memory, 8 < T <= 64 (tcgen05 + TMEM, rows of 16-byte multiples: K % 2048 == 0
+// for Q6_K, K % 256 == 0 for Q8_0, always for Q4_K).  The plain matmul is gemm_ts.cu, whose weights go to tensor memory; this kernel
+// keeps them in shared memory, and was built around the exchange of finished tiles.
 //
 //   warp 21     one thread streams slabs of RAW packed weight blocks (rows_box rows x one super-block
 //               column, no swizzle) from HBM into a ring with cp.async.bulk.tensor.
-//   warp 20     one thread loads the BN x 64 fp16 activation tile of every K step (SWIZZLE_128B) straight
+//   warp 20     one thread loads the 64 x 64 fp16 activation tile of every K step (SWIZZLE_128B) straight
 //               into the MMA stage, also with cp.async.bulk.tensor.
 //   warps 0..15 converters, four groups of four warps, group g taking the K steps with ks % 4 == g: every
 //               thread dequantises the 64 values of one weight row from the packed blocks in shared memory
 //               with packed-half arithmetic (nibble -> 1024+q by mask-and-or, -1024, one HFMA2 per two
 //               values) and stores them into the fp16 A tile in the canonical K-major SWIZZLE_128B layout;
 //               warps 0..7 later run the epilogue (tcgen05.ld, + bias, coalesced stores).
-//   warps 16..19 one thread each issues tcgen05.mma (M = 128, N = BN, K = 16) and tcgen05.commit for the K
+//   warps 16..19 one thread each issues tcgen05.mma (M = 128, N = 64, K = 16) and tcgen05.commit for the K
 //               steps ks % issuers == i into its own TMEM accumulator (narrow tiles are issue bound).
 //
-// For few tokens (T <= 64) the matmul is bound by the weight stream, so the CTAs take fewer than 128
-// weight rows each (F split evenly over the SMs, rounded up to 8) instead of full 128-row tiles that
-// would leave SMs idle; the unused accumulator lanes are simply not read back.
+// K is split over blockIdx.z when there are few row tiles; full 128-row tiles, the same on every rank.
 // No TMA multicast anywhere; every mbarrier wait is bounded.
 #include "common.cuh"
 #include "kernels.h"
@@ -31,11 +30,10 @@
 namespace mcu {
 
 constexpr int TM_BK = 64;
-constexpr int TM_ALL_CONV = 16;  // converter warps, split into G groups (template parameter of the kernel):
-                                 // G = 4: one weight row (64 values) per thread, group g takes the K steps ks % 4 == g;
-                                 // G = 2: half a row (32 values) per thread, the groups alternate K steps.
-                                 // A group must never be two uses of a stage ahead of the MMA (a parity wait cannot
-                                 // tell them apart), which holds when the stage ring is at least G deep.
+constexpr int TM_BN = 64;        // tokens of a tile
+constexpr int TM_ALL_CONV = 16;  // converter warps in TM_GROUPS groups: one weight row (64 values) per thread, group g takes the K steps
+constexpr int TM_GROUPS = 4;     // ks % 4 == g.  A group must never be two uses of a stage ahead of the MMA (a parity wait cannot
+                                 // tell them apart), which holds when the stage ring is at least four deep.
 constexpr int TM_MAX_ISSUERS = 4;  // MMA-issuing warps, each with its own TMEM accumulator (see NACC in the kernel)
 constexpr int TM_B_PRODUCER = TM_ALL_CONV + TM_MAX_ISSUERS;
 constexpr int TM_W_PRODUCER = TM_B_PRODUCER + 1;
@@ -71,7 +69,7 @@ struct GemmTmaParams {
     int *err;
     int ldo, T, F, nb;
     int ksteps;
-    int rows_per_cta;  // weight rows per CTA (= tensor-map box rows): <= 128, or 256 for two row tiles
+    int rows_per_cta;  // weight rows per CTA (= tensor-map box rows)
     int stages;        // MMA stage ring depth
     int raw_stages;    // raw slab ring depth
     int raw_stage_bytes;  // bytes of one slab slot (a multiple of 128)
@@ -83,10 +81,6 @@ struct GemmTmaParams {
     float *partial;
     int *counters;
     PeerFuse fuse;  // world > 0: finished tiles go to all ranks' slots and are summed there (see kernels.h)
-    // Grouped launch (MoE experts): blockIdx.z is the group; it owns group_counts[z] activation rows starting at row
-    // group_offsets[z] of xh / rowscale / out, and the weight rows [z * F, (z + 1) * F) of the stacked matrix.  The
-    // counts live in device memory (no host read-back); token tiles beyond a group's count exit at once.
-    const int *group_counts, *group_offsets;
 #ifdef MCU_TRACE
     long long *trace;  // development aid: clock64 samples of CTA 0, [agent][step][point]
 #endif
@@ -140,34 +134,6 @@ __device__ __forceinline__ void conv_q4k(const uint8_t *rowp, int kq, uint4 (&ou
     }
 }
 
-// The same for half a row: h = 0 takes the low nibbles (sub-block 2*kq), h = 1 the high nibbles (2*kq+1) of the
-// step's 32 bytes; out[0..3] are the 16-byte chunks 4h .. 4h+3 of the tile row.
-__device__ __forceinline__ void conv_q4k_half(const uint8_t *rowp, int kq, int h, uint4 (&outv)[4]) {
-    const uint4 hdr = *(const uint4 *)rowp;
-    const uint4 q0 = *(const uint4 *)(rowp + 16 + 32 * kq), q1 = *(const uint4 *)(rowp + 32 + 32 * kq);
-    uint32_t sc2, mn2;
-    q4k_scale_bytes(hdr, kq, sc2, mn2);
-    const __half2 k1024 = as_half2(0x64006400u);
-    const __half2 sc_h = __hsub2(as_half2(__byte_perm(sc2, 0x64646464u, 0x4140)), k1024);
-    const __half2 mn_h = __hsub2(as_half2(__byte_perm(mn2, 0x64646464u, 0x4140)), k1024);
-    const __half2 dd = as_half2(__byte_perm(hdr.x, 0u, 0x1010));
-    const __half2 nd = as_half2(__byte_perm(hdr.x, 0u, 0x3232) ^ 0x80008000u);
-    const __half2 s2 = __hmul2(sc_h, dd), m2 = __hmul2(mn_h, nd);
-    const __half2 sv = h ? bcast_hi(s2) : bcast_lo(s2), mv = h ? bcast_hi(m2) : bcast_lo(m2);
-    const uint32_t mask = h ? 0x00F000F0u : 0x000F000Fu, magic = h ? 0x54005400u : 0x64006400u;
-    const __half2 off = as_half2(magic);
-    const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    uint32_t o[16];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const __half2 v0 = as_half2((w[i] & mask) | magic), v1 = as_half2(((w[i] >> 8) & mask) | magic);
-        o[2 * i] = as_u32(__hfma2(__hsub2(v0, off), sv, mv));
-        o[2 * i + 1] = as_u32(__hfma2(__hsub2(v1, off), sv, mv));
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) outv[c] = make_uint4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-}
-
 // Q6_K: 32 values (half h of K step kq) of one block.
 __device__ __forceinline__ void conv_q6k(const uint8_t *blk, int kq, int h, uint4 *outv) {
     const int n = kq >> 1, c = 2 * (kq & 1) + h;  // values 128n + 32c + l
@@ -212,26 +178,22 @@ __device__ __forceinline__ void conv_q8_0(const uint8_t *blk, uint4 *outv) {
     for (int cc = 0; cc < 4; ++cc) outv[cc] = make_uint4(o[4 * cc], o[4 * cc + 1], o[4 * cc + 2], o[4 * cc + 3]);
 }
 
-// RT = 2 (with BN = 256, G = 1): the CTA owns two 128-row weight tiles and multiplies both with the same activation
-// tile of a K step into two accumulators (all 512 TMEM columns).  With one row tile the 256-token activation tile
-// (32 KB from L2 per K step) bounds the step at about half the tensor rate; two row tiles halve the activation bytes
-// per MMA.  All sixteen converter warps then work on the same K step (half a row per thread, 256 rows).
-template <int KIND, int BN, int G, int RT = 1>
+template <int KIND>
 __global__ void __launch_bounds__(TM_THREADS, 1)
 gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                 const GemmTmaParams p) {
     extern __shared__ uint8_t smem_raw[];
     using RC = RawCfg<KIND>;
+    constexpr int BN = TM_BN, G = TM_GROUPS;
     constexpr int B_BYTES = BN * TM_BK * 2;
-    static_assert(RT == 1 || (RT == 2 && BN == 256 && G == 1), "two row tiles need the 256-token tile");
-    constexpr int A_BYTES = RT * TM_A_BYTES;
+    constexpr int A_BYTES = TM_A_BYTES;
     constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     const int RAW_STAGE_BYTES = p.raw_stage_bytes;  // rows_per_cta * BOX_W rounded to 128, + slack for the one-word over-read
     // One thread can issue tcgen05.mma only so fast (a few hundred cycles per K step including its barrier
     // wait and commit), which is far slower than the tensor core for narrow tiles.  NACC threads therefore issue
     // interleaved K steps (step ks -> issuer ks % NACC), each into its own accumulator; the epilogue adds them.
-    constexpr int NACC = BN == 64 ? 4 : (BN == 128 ? 2 : 1);
-    constexpr uint32_t TMEM_COLS = RT * NACC * BN;  // 256 for every BN with one row tile, 512 with two
+    constexpr int NACC = TM_MAX_ISSUERS;
+    constexpr uint32_t TMEM_COLS = NACC * BN;
     constexpr int GW = TM_ALL_CONV / G;        // warps per converter group
 
     const uint32_t raw_addr = tm_smem_u32(smem_raw);
@@ -256,15 +218,10 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     if (threadIdx.x == 0) MCU_TRACE_POINT(3, 32, 0);
     const int f0 = blockIdx.x * p.rows_per_cta, t0 = blockIdx.y * BN;
     const int rows_here = min(p.rows_per_cta, p.F - f0);
-    const bool grouped = p.group_counts != nullptr;
-    // The group tables were written by kernels that finished before the kernel ahead of this one started (they do
-    // not trigger their dependents early), so they may be read before griddepcontrol.wait.
-    const int T_here = grouped ? p.group_counts[blockIdx.z] : p.T;
-    const int row_off = grouped ? p.group_offsets[blockIdx.z] : 0;  // first activation / output row of the group
-    const int w_row0 = (grouped ? (int)blockIdx.z * p.F : 0) + f0;  // first weight row in the (stacked) matrix
+    const int T_here = p.T;
     if (t0 >= T_here) return;  // uniform over the CTA, before any barrier or tensor memory exists
     // this CTA's share of K: slabs [j0, j1), K steps [ks0, ks0 + nsteps)
-    const int j0 = grouped ? 0 : (int)blockIdx.z * p.slabs_per_split;
+    const int j0 = (int)blockIdx.z * p.slabs_per_split;
     const int j1 = min((p.ksteps + RC::KR - 1) / RC::KR, j0 + p.slabs_per_split);
     const int ks0 = j0 * RC::KR;
     const int nsteps = min(p.ksteps, j1 * RC::KR) - ks0;
@@ -316,7 +273,7 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     ok = tm_mbar_wait_relaxed((((use - 1) & 1u) ? st_empty_odd : st_empty) + 8u * st, ((use - 1) >> 1) & 1u);
                 if (!ok) break;
                 tm_mbar_expect_tx(a_full + 8u * st, (uint32_t)B_BYTES);
-                tm_tma_load_2d(tile_base + (uint32_t)st * STAGE_BYTES + A_BYTES, &map_x, (ks0 + ks) * TM_BK, row_off + t0, a_full + 8u * st);
+                tm_tma_load_2d(tile_base + (uint32_t)st * STAGE_BYTES + A_BYTES, &map_x, (ks0 + ks) * TM_BK, t0, a_full + 8u * st);
                 MCU_TRACE_POINT(2, ks, 1);
                 if (++st == S) {
                     st = 0;
@@ -342,7 +299,7 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (j - j0 >= R) ok = tm_mbar_wait_relaxed(raw_empty + 8u * rs, phase);
                 if (!ok) break;
                 tm_mbar_expect_tx(raw_full + 8u * rs, raw_bytes);
-                tm_tma_load_2d(raw_ring_addr + (uint32_t)rs * RAW_STAGE_BYTES, &map_w, (j * RC::UNIT) & ~15, w_row0,
+                tm_tma_load_2d(raw_ring_addr + (uint32_t)rs * RAW_STAGE_BYTES, &map_w, (j * RC::UNIT) & ~15, f0,
                                raw_full + 8u * rs);
                 MCU_TRACE_POINT(3, j - j0, 1);
                 if (++rs == R) {
@@ -383,13 +340,6 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     tm_mma(tmem_acc, a_desc + 2, b_desc + 2, idesc, 1u);  // +32 bytes along K inside the swizzle row
                     tm_mma(tmem_acc, a_desc + 4, b_desc + 4, idesc, 1u);
                     tm_mma(tmem_acc, a_desc + 6, b_desc + 6, idesc, 1u);
-                    if constexpr (RT == 2) {  // the second row tile: next 16 KB of the stage, next BN columns of TMEM
-                        constexpr uint64_t a2 = (uint64_t)(TM_A_BYTES >> 4);
-                        tm_mma(tmem_acc + BN, a_desc + a2, b_desc, idesc, acc);
-                        tm_mma(tmem_acc + BN, a_desc + a2 + 2, b_desc + 2, idesc, 1u);
-                        tm_mma(tmem_acc + BN, a_desc + a2 + 4, b_desc + 4, idesc, 1u);
-                        tm_mma(tmem_acc + BN, a_desc + a2 + 6, b_desc + 6, idesc, 1u);
-                    }
                     MCU_TRACE_POINT(0, ks, 2);
                     tm_commit(((use & 1u) ? st_empty_odd : st_empty) + 8u * st);
                     MCU_TRACE_POINT(0, ks, 3);
@@ -415,8 +365,7 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         // G groups of GW warps; group g converts the K steps with ks % G == g.
         const int group = warp / GW;
         const int gtid = threadIdx.x - group * (GW * 32);
-        const int r = G == 4 ? gtid : gtid >> 1;  // weight row of this thread
-        const int hc = gtid & 1;                  // G == 2: which half of the row's step
+        const int r = gtid;  // weight row of this thread
         const bool row_live = r < rows_here;
         bool ok = true;
         // Every warp visits every slab in order (wait for it, release it), and converts the K steps of its group
@@ -443,53 +392,30 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 const uint32_t rel_parity = ((use - 1) >> 1) & 1u;
                 const bool stage_free = use >= 1 ? tm_mbar_test(rel_bar, rel_parity) : true;
                 uint8_t *a_row = tiles + (size_t)st * STAGE_BYTES + r * 128;
-                if constexpr (G == 4) {
-                    uint4 wv[8];
-                    if (row_live) {
-                        if constexpr (KIND == KIND_Q4_K) {
-                            conv_q4k(rowp, kq, wv);
-                        } else if constexpr (KIND == KIND_Q6_K) {
-                            conv_q6k(rowp, kq, 0, wv);
-                            conv_q6k(rowp, kq, 1, wv + 4);
-                        } else {
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const int blk = 4 * j + 2 * kq + h;
-                                if (blk < p.nb) conv_q8_0(rowp + (2 * kq + h) * Q8_0_BYTES, wv + 4 * h);
-                                else wv[4 * h] = wv[4 * h + 1] = wv[4 * h + 2] = wv[4 * h + 3] = make_uint4(0, 0, 0, 0);
-                            }
-                        }
+                uint4 wv[8];
+                if (row_live) {
+                    if constexpr (KIND == KIND_Q4_K) {
+                        conv_q4k(rowp, kq, wv);
+                    } else if constexpr (KIND == KIND_Q6_K) {
+                        conv_q6k(rowp, kq, 0, wv);
+                        conv_q6k(rowp, kq, 1, wv + 4);
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) wv[c] = make_uint4(0, 0, 0, 0);
-                    }
-                    if (!stage_free) ok = tm_mbar_wait_relaxed(rel_bar, rel_parity);
-                    if (gtid == 0) MCU_TRACE_POINT(1, ks - ks0, 1);
-                    if (ok) {
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) *(uint4 *)(a_row + ((c ^ (r & 7)) << 4)) = wv[c];
+                        for (int h = 0; h < 2; ++h) {
+                            const int blk = 4 * j + 2 * kq + h;
+                            if (blk < p.nb) conv_q8_0(rowp + (2 * kq + h) * Q8_0_BYTES, wv + 4 * h);
+                            else wv[4 * h] = wv[4 * h + 1] = wv[4 * h + 2] = wv[4 * h + 3] = make_uint4(0, 0, 0, 0);
+                        }
                     }
                 } else {
-                    uint4 wv[4];
-                    if (row_live) {
-                        if constexpr (KIND == KIND_Q4_K) {
-                            conv_q4k_half(rowp, kq, hc, wv);
-                        } else if constexpr (KIND == KIND_Q6_K) {
-                            conv_q6k(rowp, kq, hc, wv);
-                        } else {
-                            const int blk = 4 * j + 2 * kq + hc;
-                            if (blk < p.nb) conv_q8_0(rowp + (2 * kq + hc) * Q8_0_BYTES, wv);
-                            else wv[0] = wv[1] = wv[2] = wv[3] = make_uint4(0, 0, 0, 0);
-                        }
-                    } else {
-                        wv[0] = wv[1] = wv[2] = wv[3] = make_uint4(0, 0, 0, 0);
-                    }
-                    if (!stage_free) ok = tm_mbar_wait_relaxed(rel_bar, rel_parity);
-                    if (gtid == 0) MCU_TRACE_POINT(1, ks - ks0, 1);
-                    if (ok) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) *(uint4 *)(a_row + (((4 * hc + c) ^ (r & 7)) << 4)) = wv[c];
-                    }
+                    for (int c = 0; c < 8; ++c) wv[c] = make_uint4(0, 0, 0, 0);
+                }
+                if (!stage_free) ok = tm_mbar_wait_relaxed(rel_bar, rel_parity);
+                if (gtid == 0) MCU_TRACE_POINT(1, ks - ks0, 1);
+                if (ok) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) *(uint4 *)(a_row + ((c ^ (r & 7)) << 4)) = wv[c];
                 }
                 if (!__all_sync(0xffffffffu, ok)) {  // a wait ran out: the stage was not written, nothing is signalled
                     ok = false;
@@ -530,9 +456,7 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         if (ok && warp < 8 && !*abort_flag) {
             const int q = warp & 3;
             const int col0 = (warp >> 2) * (BN / 2);
-#pragma unroll 1
-            for (int rt = 0; rt < RT; ++rt) {
-            const int fr = TM_BM * rt + 32 * q + lane;
+            const int fr = 32 * q + lane;
             const int f = f0 + fr;
             const bool f_ok = fr < rows_here;
             const float bias = (p.bias != nullptr && f_ok) ? p.bias[f] : 0.0f;
@@ -546,7 +470,7 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int a = 0; a < NACC; ++a) {
                     if (a >= n_used) break;  // warp-uniform
                     uint32_t v[32];
-                    const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)((rt * NACC + a) * BN + col0 + cb);
+                    const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(a * BN + col0 + cb);
                     asm volatile(
                         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -576,7 +500,7 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         for (int jj = 0; jj < 32; ++jj) {
                             const int t = t0 + col0 + cb + jj;
                             if (t < T_here)
-                                p.out[(size_t)(row_off + t) * p.ldo + f] = sum[jj] * p.rowscale[row_off + t] + bias;
+                                p.out[(size_t)t * p.ldo + f] = sum[jj] * p.rowscale[t] + bias;
                         }
                     } else {
                         float *part = p.partial + (size_t)blockIdx.z * p.T * p.F;
@@ -588,7 +512,6 @@ gemm_tma_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                 }
             }
-            }  // row tiles
         }
     }
     if (threadIdx.x == 0) MCU_TRACE_POINT(3, 36, 0);
@@ -747,51 +670,25 @@ static bool force_v1() {
     return v;
 }
 
-// Tiling for few tokens (T <= 64), where the matmul is bound by the weight stream and by the latency of the K loop:
-// full 128-row tiles when K can be split so that tiles x splits still fills the SMs (the serial K loop gets
-// shorter), otherwise the rows spread evenly over the SMs.
+// Full 128-row tiles, K split so that tiles x splits fills the SMs (the serial K loop gets shorter).
 struct TmaPlan {
-    int rows_per_cta, splits, slabs_per_split;
+    int splits, slabs_per_split;
 };
-static TmaPlan plan_tma(int kind, int T, int K, int F) {
+static TmaPlan plan_tma(int kind, int K, int F) {
     const int bv = block_values(kind), nb = (K + bv - 1) / bv;
     const int ksteps = (nb * bv + TM_BK - 1) / TM_BK;
     const int kr = kind == KIND_Q8_0 ? 2 : 4;
     const int n_slabs = (ksteps + kr - 1) / kr;
-    TmaPlan pl{TM_BM, 1, n_slabs};
-    const int sms = device_sm_count();
-    // T > 64: full tiles (shorter tiles that would fill the last wave better finish no sooner: the MMA computes
-    // M = 128 rows whatever the tile holds, and a converter warp takes as long for a half-empty tile).  With 256-token
-    // tiles and enough work to fill most SMs a CTA takes two row tiles (see the kernel's RT parameter); Q6_K slabs are
-    // too large for that.
-    if (T > 64) {
-        static const bool one_tile = getenv("MARMOT_CUDA_GEMM_ONE_ROW_TILE") != nullptr;  // diagnostic switch
-        // Measured K-step times: about 1290 cycles with one row tile, 2250 with two (F = 14336, T = 512: 99 -> 90 us for
-        // Q8_0, 83 -> 76 us for Q4_K); two tiles win when they save a wave (224 units on 148 SMs -> 112).
-        const long t_tiles = (T + 255) / 256;
-        const long waves2 = ((long)((F + 2 * TM_BM - 1) / (2 * TM_BM)) * t_tiles + sms - 1) / sms;
-        const long waves1 = ((long)((F + TM_BM - 1) / TM_BM) * t_tiles + sms - 1) / sms;
-        if (T > 128 && kind != KIND_Q6_K && !one_tile && waves2 * 175 < waves1 * 97) pl.rows_per_cta = 2 * TM_BM;
-        return pl;
-    }
+    TmaPlan pl{1, n_slabs};
     static const bool no_split = getenv("MARMOT_CUDA_GEMM_NO_SPLITK") != nullptr;  // diagnostic switch
     const int tiles = (F + TM_BM - 1) / TM_BM;
-    int splits = no_split ? 1 : sms / tiles;
+    int splits = no_split ? 1 : device_sm_count() / tiles;
     if (splits > 16) splits = 16;
-    if (splits >= 2 && n_slabs >= 2) {
-        if (splits > n_slabs) splits = n_slabs;
+    if (splits > n_slabs) splits = n_slabs;
+    if (splits >= 2) {
         pl.slabs_per_split = (n_slabs + splits - 1) / splits;
         pl.splits = (n_slabs + pl.slabs_per_split - 1) / pl.slabs_per_split;
-        if (pl.splits >= 2) return pl;
-        pl.splits = 1;
-        pl.slabs_per_split = n_slabs;
     }
-    const int waves = (F + TM_BM * sms - 1) / (TM_BM * sms);  // passes over the SMs with full tiles
-    int rows = (F + sms * waves - 1) / (sms * waves);
-    rows = (rows + 7) / 8 * 8;
-    if (rows > TM_BM) rows = TM_BM;
-    if (rows < 8) rows = 8;
-    pl.rows_per_cta = rows;
     return pl;
 }
 
@@ -800,28 +697,28 @@ bool gemm_tma_can_fuse(int kind, int T, int F) {
 }
 
 size_t gemm_tma_workspace_bytes(int kind, int T, int K, int F) {
-    const TmaPlan pl = plan_tma(kind, T, K, F);
+    const TmaPlan pl = plan_tma(kind, K, F);
     return pl.splits > 1 ? (size_t)pl.splits * T * F * sizeof(float) : 0;
 }
 
-bool gemm_tma_supported(int kind, const void *W, const void *W2, int T, int K, int F) {
+bool gemm_tma_supported(int kind, const void *W, int T, int K, int F) {
     if (force_v1() || !kind_supported(kind) || T < 1 || F < 1 || K < 1) return false;
-    if (((uintptr_t)W & 15) || ((uintptr_t)W2 & 15)) return false;
+    if ((uintptr_t)W & 15) return false;
     const int bv = block_values(kind), nb = (K + bv - 1) / bv;
     const long row_bytes = (long)nb * block_bytes(kind);
     if (row_bytes % 16) return false;  // tensor-map row stride
     return encode_tiled_fn() != nullptr;
 }
 
-template <int KIND, int BN, int G, int RT = 1>
-static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, GemmTmaParams p, long row_bytes,
-                                 cudaStream_t s, int groups = 0, int total_rows = 0) {
+template <int KIND>
+static cudaError_t launch_tma_kind(const void *W, const __half *xh, int ldxh, GemmTmaParams p, long row_bytes, cudaStream_t s) {
     using RC = RawCfg<KIND>;
+    constexpr int BN = TM_BN, G = TM_GROUPS, NACC = TM_MAX_ISSUERS;
     EncodeTiledFn enc = encode_tiled_fn();
     if (enc == nullptr) return cudaErrorNotSupported;
     alignas(64) CUtensorMap map_w, map_x;
     {
-        const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)p.F * (cuuint64_t)(groups > 0 ? groups : 1)};
+        const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)p.F};
         const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
         const cuuint32_t box[2] = {(cuuint32_t)RC::BOX_W, (cuuint32_t)p.rows_per_cta};
         const cuuint32_t es[2] = {1, 1};
@@ -831,7 +728,7 @@ static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, Gemm
             return cudaErrorInvalidValue;
     }
     {
-        const cuuint64_t dims[2] = {(cuuint64_t)ldxh, (cuuint64_t)(groups > 0 ? total_rows : p.T)};
+        const cuuint64_t dims[2] = {(cuuint64_t)ldxh, (cuuint64_t)p.T};
         const cuuint64_t strides[1] = {(cuuint64_t)ldxh * 2};
         const cuuint32_t box[2] = {(cuuint32_t)TM_BK, (cuuint32_t)BN};
         const cuuint32_t es[2] = {1, 1};
@@ -840,7 +737,7 @@ static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, Gemm
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    constexpr int stage_bytes = RT * TM_A_BYTES + BN * TM_BK * 2;
+    constexpr int stage_bytes = TM_A_BYTES + BN * TM_BK * 2;
     const int raw_stage_bytes = (p.rows_per_cta * RC::BOX_W + 127) / 128 * 128 + 128;
     const int budget = 210 * 1024 - 2048;
     const int raw_slabs = p.slabs_per_split;
@@ -850,7 +747,7 @@ static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, Gemm
     // full-barrier are waited on by one thread in order.  (A parity wait cannot tell "this phase" from "two
     // phases ago"; an issuer that got ahead of the thread owning the previous use of the stage would fall
     // through its wait.)
-    int R = RT == 2 ? 2 : (BN <= 128 ? 4 : 3);  // two row tiles: two 64 KB stages and two 256-row slabs fill the SM
+    int R = 4;
     if (R > raw_slabs) R = raw_slabs;
     int S = (budget - R * raw_stage_bytes) / stage_bytes;
     if (S < G + 2 && R > 3) {  // a ring deeper than G lets a group convert while its previous step is still in the MMA
@@ -863,7 +760,6 @@ static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, Gemm
     }
     if (S < G) return cudaErrorInvalidConfiguration;
     if (S > TM_MAX_RING) S = TM_MAX_RING;
-    constexpr int NACC = BN == 64 ? 4 : (BN == 128 ? 2 : 1);
     static const int issuer_cap = getenv("MARMOT_CUDA_GEMM_ISSUERS") ? atoi(getenv("MARMOT_CUDA_GEMM_ISSUERS")) : NACC;
     int max_issuers = NACC;
     if (issuer_cap >= 1 && max_issuers > issuer_cap) max_issuers = issuer_cap;
@@ -878,12 +774,11 @@ static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, Gemm
     const int smem = 2048 + S * stage_bytes + R * raw_stage_bytes;
     static int configured = 0;
     if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tma_kernel<KIND, BN, G, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tma_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         configured = smem;
     }
-    dim3 grid((unsigned)((p.F + p.rows_per_cta - 1) / p.rows_per_cta), (unsigned)((p.T + BN - 1) / BN), (unsigned)p.splits);
-    if (groups > 0) grid = dim3(grid.x, (unsigned)((total_rows + BN - 1) / BN), (unsigned)groups);
+    const dim3 grid((unsigned)((p.F + p.rows_per_cta - 1) / p.rows_per_cta), (unsigned)((p.T + BN - 1) / BN), (unsigned)p.splits);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(TM_THREADS, 1, 1);
@@ -895,17 +790,7 @@ static cudaError_t launch_tma_bn(const void *W, const __half *xh, int ldxh, Gemm
     cfg.attrs = attr;
     static const bool no_pdl = getenv("MARMOT_CUDA_NO_PDL") != nullptr;  // diagnostic switch
     cfg.numAttrs = no_pdl ? 0 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tma_kernel<KIND, BN, G, RT>, map_w, map_x, p);
-}
-
-template <int KIND>
-static cudaError_t launch_tma_kind(const void *W, const __half *xh, int ldxh, const GemmTmaParams &p, long row_bytes,
-                                   cudaStream_t s) {
-    if (p.T <= 64) return launch_tma_bn<KIND, 64, 4>(W, xh, ldxh, p, row_bytes, s);
-    if (p.T <= 128) return launch_tma_bn<KIND, 128, 4>(W, xh, ldxh, p, row_bytes, s);
-    if constexpr (KIND != KIND_Q6_K)
-        if (p.rows_per_cta == 2 * TM_BM) return launch_tma_bn<KIND, 256, 1, 2>(W, xh, ldxh, p, row_bytes, s);
-    return launch_tma_bn<KIND, 256, 2>(W, xh, ldxh, p, row_bytes, s);
+    return cudaLaunchKernelEx(&cfg, gemm_tma_kernel<KIND>, map_w, map_x, p);
 }
 
 #ifdef MCU_TRACE
@@ -913,30 +798,24 @@ long long *g_trace_buf = nullptr;
 extern "C" long long *mcu_debug_trace_buffer() { return g_trace_buf; }
 #endif
 
-cudaError_t launch_gemm_tma(int kind, const void *W, const void *W2, const __half *xh, const float *rowscale, int ldxh,
-                            int T, int K, int F, const float *bias, float *out, float *out2, int ldo, float *partial,
-                            int *counters, int *err_flag, cudaStream_t s, int *launches, const PeerFuse *fuse) {
+cudaError_t launch_gemm_tma(int kind, const void *W, const __half *xh, const float *rowscale, int ldxh, int T, int K, int F, float *out,
+                            float *partial, int *counters, int *err_flag, cudaStream_t s, const PeerFuse &fuse) {
+    if (fuse.world <= 0 || !gemm_tma_can_fuse(kind, T, F) || (size_t)T * F > fuse.slot_floats) return cudaErrorInvalidValue;
     GemmTmaParams p;
-    p.bias = bias;
+    p.bias = nullptr;
     p.rowscale = rowscale;
     p.err = err_flag;
-    p.ldo = ldo;
+    p.out = out;
+    p.ldo = F;
     p.T = T;
     p.F = F;
     const int bv = block_values(kind);
     p.nb = (K + bv - 1) / bv;
     p.ksteps = (p.nb * bv + TM_BK - 1) / TM_BK;
     const long row_bytes = (long)p.nb * block_bytes(kind);
-    TmaPlan pl = plan_tma(kind, T, K, F);
-    memset(&p.fuse, 0, sizeof(p.fuse));
-    p.group_counts = p.group_offsets = nullptr;
-    if (fuse != nullptr && fuse->world > 0) {
-        if (!gemm_tma_can_fuse(kind, T, F) || W2 != nullptr || ldo != F || (size_t)T * F > fuse->slot_floats)
-            return cudaErrorInvalidValue;
-        pl.rows_per_cta = TM_BM;  // tiles must be the same on every rank, whatever its share of K
-        p.fuse = *fuse;
-    }
-    p.rows_per_cta = pl.rows_per_cta;
+    const TmaPlan pl = plan_tma(kind, K, F);
+    p.rows_per_cta = TM_BM;  // tiles must be the same on every rank, whatever its share of K
+    p.fuse = fuse;
     p.splits = pl.splits;
     p.slabs_per_split = pl.slabs_per_split;
     p.partial = partial;
@@ -953,58 +832,9 @@ cudaError_t launch_gemm_tma(int kind, const void *W, const void *W2, const __hal
         g_trace_buf = trace_buf;
     }
 #endif
-    int n = 0;
-    for (int pass = 0; pass < (W2 != nullptr ? 2 : 1); ++pass) {
-        const void *w = pass == 0 ? W : W2;
-        p.out = pass == 0 ? out : out2;
-        cudaError_t e = kind == KIND_Q4_K ? launch_tma_kind<KIND_Q4_K>(w, xh, ldxh, p, row_bytes, s)
-            : kind == KIND_Q6_K           ? launch_tma_kind<KIND_Q6_K>(w, xh, ldxh, p, row_bytes, s)
-                                          : launch_tma_kind<KIND_Q8_0>(w, xh, ldxh, p, row_bytes, s);
-        if (e != cudaSuccess) return e;
-        ++n;
-    }
-    if (launches != nullptr) *launches = n;
-    return cudaSuccess;
-}
-
-bool gemm_tma_grouped_supported(int kind, const void *W, int K, int F) {
-    return gemm_tma_supported(kind, W, nullptr, 256, K, F);
-}
-
-// n_groups matmuls in one launch: group g multiplies its group_counts[g] rows of xh (from row group_offsets[g]) with the
-// weight rows [g * F, (g + 1) * F) of the stacked matrix W.  The 256-token tile configuration is used whatever the
-// counts turn out to be (they are device data): meant for batches with many rows per group.
-cudaError_t launch_gemm_tma_grouped(int kind, const void *W, int n_groups, const __half *xh, const float *rowscale,
-                                    int ldxh, int total_rows, int K, int F, const int *group_counts,
-                                    const int *group_offsets, float *out, int ldo, int *err_flag, cudaStream_t s) {
-    if (n_groups <= 0 || total_rows <= 0) return cudaSuccess;
-    if (n_groups > 65535 || (total_rows + 255) / 256 > 65535) return cudaErrorInvalidValue;
-    GemmTmaParams p;
-    memset(&p, 0, sizeof(p));
-    p.rowscale = rowscale;
-    p.out = out;
-    p.err = err_flag;
-    p.ldo = ldo;
-    p.T = total_rows;
-    p.F = F;
-    const int bv = block_values(kind);
-    p.nb = (K + bv - 1) / bv;
-    p.ksteps = (p.nb * bv + TM_BK - 1) / TM_BK;
-    const long row_bytes = (long)p.nb * block_bytes(kind);
-    p.splits = 1;
-    p.slabs_per_split = (p.ksteps + (kind == KIND_Q8_0 ? 2 : 4) - 1) / (kind == KIND_Q8_0 ? 2 : 4);
-    p.group_counts = group_counts;
-    p.group_offsets = group_offsets;
-    static const bool one_tile = getenv("MARMOT_CUDA_GEMM_ONE_ROW_TILE") != nullptr;  // diagnostic switch
-    const bool two = kind != KIND_Q6_K && !one_tile && F % (2 * TM_BM) == 0;
-    p.rows_per_cta = two ? 2 * TM_BM : TM_BM;
-    if (kind == KIND_Q4_K)
-        return two ? launch_tma_bn<KIND_Q4_K, 256, 1, 2>(W, xh, ldxh, p, row_bytes, s, n_groups, total_rows)
-                   : launch_tma_bn<KIND_Q4_K, 256, 2>(W, xh, ldxh, p, row_bytes, s, n_groups, total_rows);
-    if (kind == KIND_Q8_0)
-        return two ? launch_tma_bn<KIND_Q8_0, 256, 1, 2>(W, xh, ldxh, p, row_bytes, s, n_groups, total_rows)
-                   : launch_tma_bn<KIND_Q8_0, 256, 2>(W, xh, ldxh, p, row_bytes, s, n_groups, total_rows);
-    return launch_tma_bn<KIND_Q6_K, 256, 2>(W, xh, ldxh, p, row_bytes, s, n_groups, total_rows);
+    return kind == KIND_Q4_K ? launch_tma_kind<KIND_Q4_K>(W, xh, ldxh, p, row_bytes, s)
+        : kind == KIND_Q6_K  ? launch_tma_kind<KIND_Q6_K>(W, xh, ldxh, p, row_bytes, s)
+                             : launch_tma_kind<KIND_Q8_0>(W, xh, ldxh, p, row_bytes, s);
 }
 
 }  // namespace mcu

@@ -120,17 +120,15 @@ struct PeerFuse {
     uint32_t parity_of_next;               // parity the host expects for the next epoch (consistency check)
 };
 
-// TMA-fed variant of the tensor-core matmul (packed weight slabs and activation tiles arrive by
-// cp.async.bulk.tensor); needs 16-byte aligned weights whose rows are 16-byte multiples.
-bool gemm_tma_supported(int kind, const void *W, const void *W2, int T, int K, int F);
+// The matmul that is fused with it (packed weight slabs and activation tiles arrive by cp.async.bulk.tensor); needs 16-byte aligned
+// weights whose rows are 16-byte multiples.
+bool gemm_tma_supported(int kind, const void *W, int T, int K, int F);
 // Split-K workspace: `partial` needs gemm_tma_workspace_bytes() bytes (0: no split for this shape), `counters`
 // GEMM_TMA_MAX_TILE_COUNTERS zero-initialised ints that the kernel leaves zero again.
 constexpr int GEMM_TMA_MAX_TILE_COUNTERS = 4096;
 size_t gemm_tma_workspace_bytes(int kind, int T, int K, int F);
-cudaError_t launch_gemm_tma(int kind, const void *W, const void *W2, const __half *xh, const float *rowscale, int ldxh,
-                            int T, int K, int F, const float *bias, float *out, float *out2, int ldo, float *partial,
-                            int *counters, int *err_flag, cudaStream_t s, int *launches,
-                            const PeerFuse *fuse = nullptr);
+cudaError_t launch_gemm_tma(int kind, const void *W, const __half *xh, const float *rowscale, int ldxh, int T, int K, int F, float *out,
+                            float *partial, int *counters, int *err_flag, cudaStream_t s, const PeerFuse &fuse);
 // Can launch_gemm_tma fuse the all-reduce for this shape (same answer on every rank: it depends on T and F only)?
 bool gemm_tma_can_fuse(int kind, int T, int F);
 
