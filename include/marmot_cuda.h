@@ -181,11 +181,10 @@ int mcu_linear_dual(
  *                                  rms_norm(x') * (norm_weight + weight_offset); x' is stored to x_out when that is
  *                                  set.  x_out must not overlap x or aux.
  *        MCU_PROLOGUE_SWIGLU       the weights multiply silu(x) * aux (x = gate, aux = up projection)
- *      Up to 8 tokens with every weight on the streaming path this is ONE launch -- except for 5 to 8 tokens over 24 MB
- *      or more of Q4_K / Q6_K weights, where the integer-MMA kernel behind a stand-alone prologue kernel is faster than
- *      the one launch; more than 16 tokens: the prologue rides in the tensor-core path's activation staging; otherwise the
- *      prologue runs as its stand-alone kernel (which needs contiguous rows: ldx = ld_aux = ld_x_out = K) followed by
- *      the matmuls. ---- */
+ *      Up to 8 tokens with every weight on the streaming path this is ONE launch, unless the weights are large enough for
+ *      the integer tensor-core kernel (Q4_K / Q6_K, see integer_pays in abi.cu).  On the tensor cores the prologue rides in
+ *      the activation staging: one launch, then one per block format.  Otherwise the prologue runs as its stand-alone kernel
+ *      followed by the matmuls.  Beyond one launch the rows must be contiguous (ldx = ld_aux = ld_x_out = K). ---- */
 enum { MCU_PROLOGUE_NONE = 0, MCU_PROLOGUE_ADD_RMSNORM = 1, MCU_PROLOGUE_SWIGLU = 2 };
 #define MCU_LINEAR_MAX_JOBS 4
 typedef struct mcu_linear_job {
@@ -254,10 +253,10 @@ int mcu_topk(
  *      (src/backends/cpu/ops/moe/moe_ops.c:1069-1178, 891-1049, 622-787).
  *      hidden [T][H] f32; gate/up: E contiguous [FF][H] quantized matrices; down: E contiguous [H][FF];
  *      topk_ids [T][k] int32, topk_weights [T][k] f32; out [T][H] f32.
- *      With T * k >= 256 (gate and up of one kind, weight rows a multiple of 16 bytes) the call reads nothing back: it is
- *      asynchronous, may be recorded by mcu_graph_capture_begin/end, and an expert id outside [0, E) is reported by the
- *      next mcu_synchronize as MCU_ERROR_INVALID_ARGUMENT.  Smaller batches read the group sizes back (one stream
- *      synchronisation), report a bad id from the call itself and refuse to be captured. ---- */
+ *      With T * k >= 256 (gate and up of one kind) the call reads nothing back: it is asynchronous, may be recorded by
+ *      mcu_graph_capture_begin/end, and an expert id outside [0, E) is reported by the next mcu_synchronize as
+ *      MCU_ERROR_INVALID_ARGUMENT.  Smaller batches report a bad id from the call itself, which waits for the routing (a recorded
+ *      call reports it as above); those with weights other than Q4_K / Q6_K, or of two kinds, read the group sizes back too. ---- */
 int mcu_moe_experts(
     mcu_context_t *ctx, int gate_kind, int up_kind, int down_kind, const float *hidden_dev, size_t T, size_t H,
     size_t FF, size_t E, const void *gate_dev, const void *up_dev, const void *down_dev, const int32_t *topk_ids_dev,

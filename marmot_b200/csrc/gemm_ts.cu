@@ -19,11 +19,12 @@
 // 17 x 4096 x 4096 12.8 -> 10.4, 64 x 4096 x 1024 18.5 -> 9.8, 2048 x 4096 x 14336 274 -> 214 (1120 TFLOP/s: 0.82 of the
 // sustained cuBLAS rate, the clock is at the power limit); Q6_K 37 x 14336 x 4096 39.6 -> 29.4, 512 x 5632 x 2048 142 -> 43.
 // Up to 128 tokens the converters bound a slab (about 1500 cycles for 32768 weights, instruction issue); from 256 on the MMAs
-// run at their peak rate (2075 cycles per slab) and what is left is the epilogue (4000 cycles of a tile's 37000).
+// run at their peak rate (2075 cycles per slab) and what is left is the epilogue (4000 cycles of a tile's 37000).  Beside the
+// kernel a call has its staging launch: of the 17 us at 64 x 4096 x 14336 it and the releases around it take 6.5.
 //
-// The work is cut into units of one slab of one output tile; CTA i of G takes the units [i U / G, (i + 1) U / G), whatever
-// tile they fall into, so no SM idles in a last wave.  A tile cut between CTAs is summed from partial tiles by the one that
-// draws the last ticket, in a fixed order; nobody waits for another CTA (kernels on several streams may share the device).
+// A CTA has one output tile, or a cluster shares one along K and adds its shares up through distributed shared memory, or the slabs of
+// all tiles are cut into equal ranges: a tile cut between CTAs is then summed from partial tiles by the one that draws the last
+// ticket, in a fixed order; nobody waits for another CTA (kernels on several streams may share the device).  ts_spread chooses.
 // Every mbarrier wait is bounded; no TMA multicast.
 #include "common.cuh"
 #include "gemm_ts_dev.cuh"
@@ -42,7 +43,6 @@ namespace mcu {
 
 constexpr int TS_BK = 128;      // values of K per stage, half a slab: eight MMAs per barrier wait and commit (see the issuer)
 constexpr int TS_STAGES = 4;    // = converter groups: group g owns stage slot g, so every barrier phase is seen in order
-constexpr int TS_SLAB_STAGES = 256 / TS_BK;
 constexpr int TS_CONV = 16;     // converter warps
 constexpr int TS_MMA_WARP = TS_CONV, TS_B_WARP = TS_CONV + 1, TS_W_WARP = TS_CONV + 2;
 constexpr int TS_THREADS = (TS_W_WARP + 1) * 32;
