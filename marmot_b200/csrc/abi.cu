@@ -565,10 +565,12 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
 //   Q6_K  4 tokens  4096 x 4096 11.0, 11.7; 14336 x 4096 33.3, 23.6; 4096 x 28672 39.7, 44.7
 //         5 tokens  1024 x 1024 4.2, 7.0; 2048 x 2048 7.9, 8.0; 4096 x 1024 8.8, 8.6; 4096 x 4096 13.5, 11.7
 // From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
-static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t values) {
+// And from three tokens on where the rows cannot be streamed (Q6_K of ragged sizes), against the plain-load kernel: 3072 x 125 3, 4,
+// 8 tokens 13.5, 16.6, 21.2 us, 7.5, 7.7, 7.8 here; 1280 x 300 7.5, 9.1, 12.5, then 7.6 to 7.7.
+static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t values, bool streams) {
     static const bool off = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch
     if (off || ctx->regime != MCU_REGIME_AUTO || T > (size_t)TI_COLS) return false;
-    if (T > (size_t)GEMV_MAX_T) return true;
+    if (T > (size_t)GEMV_MAX_T || (T >= 3 && !streams)) return true;
     if (T >= 5) return values >= (size_t)4 << 20;
     return kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20;
 }
@@ -605,7 +607,8 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     ActBuffers ab;
     // a handful of tokens: exact integer dots on the tensor core
     const size_t values = K * F * (w2 != nullptr ? 2 : 1);
-    const bool i8_pays = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, values);
+    const bool streams = T < 3 || T > (size_t)GEMV_MAX_T || gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F);
+    const bool i8_pays = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, values, streams);
     if (i8_pays && (w2 == nullptr || bias == nullptr)) {
         const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};
         if (integer_jobs_supported(jobs, w2 != nullptr ? 2 : 1, K))
@@ -847,7 +850,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
         for (size_t j = 0; j < n_jobs && integer; ++j) {
             size_t values = 0;
             for (size_t i = 0; i < n_jobs; ++i) values += specs[i].kind == specs[j].kind ? K * (size_t)specs[i].F : 0;
-            integer = integer_pays(ctx, specs[j].kind, T, values);
+            integer = integer_pays(ctx, specs[j].kind, T, values, true);
         }
         if (!integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
             gemv_stream_jobs_supported(specs, (int)n_jobs, (int)T, (int)K, gp)) {

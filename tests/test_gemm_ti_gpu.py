@@ -41,6 +41,18 @@ def test_tile_edges(ctx, oracle, kind, T, K, F):
     assert max_rel_err(got, oracle.linear(kind, x, W, F) + bias) <= TOL_FP32
 
 
+@pytest.mark.parametrize("T,K,F", [(3, 3072, 125), (8, 1280, 61), (4, 768, 1)])
+def test_rows_that_cannot_be_streamed(ctx, oracle, T, K, F):
+    import torch
+
+    rng = np.random.default_rng(T + K)
+    W = random_blocks(KIND_Q6_K, F, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    got = ctx.linear(KIND_Q6_K, torch.from_numpy(x).cuda(), ctx.upload(W), F).cpu().numpy()
+    ctx.synchronize()
+    assert max_rel_err(got, oracle.linear(KIND_Q6_K, x, W, F)) <= TOL_FP32
+
+
 @pytest.mark.parametrize("T,K,F", [(3, 4096, 5632), (4, 4096, 4096), (5, 2048, 2056), (8, 4096, 1030), (16, 512, 40)])
 def test_two_matrices_of_each_kind_with_prologues(ctx, oracle, T, K, F):
     """The sizes at which linear_multi leaves the dp4a kernel: every result equals the one of the plain regime, and x' is exact."""
