@@ -610,10 +610,13 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     }
     p.tiles = row_tiles * p.t_tiles;
     if (cudaError_t e = ti_encode_x(kind, &maps.x, xq, T, p.nb)) return e;
-    // One tile per CTA, a tile over a cluster, or equal ranges, whichever ends first: a slab takes about 800 cycles (its share of
-    // the HBM stream with all SMs at work), a cluster's exchange 1000, the ticket of a cut tile 4000.
+    // One tile per CTA, in waves if need be, a tile over a cluster, or equal ranges, whichever ends first, by a sweep of all three at
+    // nine tokens: a slab takes about 900 cycles (Q6_K 2100), the start of a CTA 3500, a cluster's exchange 1500; a tile cut between
+    // ranges costs 9000 and 700 for every share that the last CTA reads (13056 x 1792 Q4_K: 22 us in ranges of five slabs, 13 in
+    // clusters of eight).  Clusters of eight: as in ts_spread.
     const int sms = device_sm_count(), KS = p.slabs;
-    const long U = (long)p.tiles * KS, n_most = U < sms ? U : sms;
+    const long U = (long)p.tiles * KS, n_most = U < sms ? U : sms, upc = (U + n_most - 1) / n_most;
+    const double unit = kind == KIND_Q4_K ? 900.0 : 2100.0;
     double best = 1e30;
     int n_cta = (int)n_most;
     p.split = 1;
@@ -624,11 +627,11 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
             n_cta = (int)n;
         }
     };
-    if (p.tiles <= sms) consider(1, p.tiles, KS * 800.0);
+    consider(1, p.tiles, (double)((p.tiles + sms - 1) / sms) * (KS * unit + 3500.0));
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2)
-        if ((long)p.tiles * sp <= (sp >= 8 ? sms / 2 : sms)) consider(sp, (long)p.tiles * sp, (KS + sp - 1) / sp * 800.0 + 1000.0);
-    const bool cut = U % n_most != 0 || U / n_most % KS != 0;
-    consider(1, n_most, (double)((U + n_most - 1) / n_most) * 800.0 + (cut ? 4000.0 : 0.0));
+        if ((long)p.tiles * sp <= (sp >= 8 ? sms * 7 / 9 : sms)) consider(sp, (long)p.tiles * sp, (KS + sp - 1) / sp * unit + 5000.0);
+    const bool cut = U % n_most != 0 || upc % KS != 0;
+    consider(1, n_most, (double)upc * unit + 2000.0 + (cut ? 9000.0 + 700.0 * ((double)KS / upc + 1.0) : 0.0));
     return ti_dispatch(kind, maps, p, n_cta, s);
 }
 

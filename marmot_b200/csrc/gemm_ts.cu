@@ -658,8 +658,8 @@ static TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles) {
     consider(1, tiles, (double)((tiles + room - 1) / room) * (KS * unit + tile_end + 2000.0));
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2) {
         // A cluster is placed inside a GPC (16 to 20 SMs): sixteen clusters of eight did not run at once (2048 x 2048: 12.6 us,
-        // 64 CTAs in clusters of four 7.5).
-        const int usable = sp >= 8 ? room / 2 : room;
+        // 64 CTAs in clusters of four 7.5), fourteen do.
+        const int usable = sp >= 8 ? room * 7 / 9 : room;
         const double exchange = sp == 2 ? 3500.0 + 30.0 * bn : 5000.0 + 20.0 * bn;
         if ((long)tiles * sp <= usable) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + tile_end + 2000.0 + exchange);
     }
