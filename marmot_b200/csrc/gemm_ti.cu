@@ -122,7 +122,10 @@ __device__ __forceinline__ void ti_conv_q6k(const uint8_t *blk, Done done, Emit 
     emit.corrections(c);
 }
 
-template <int KIND>
+// EARLY: the scalers give the sums' place back as soon as they have read them, ahead of the last operations on them.  Worth 4 % where tiles
+// hold one to eight tokens (MoE of 16 tokens 231 -> 222 us) and with Q6_K; with Q4_K it costs registers that larger tiles miss (16 x 4096 x
+// 14336 15.6 -> 15.9), so single matrices do without.
+template <int KIND, bool EARLY>
 __global__ void __launch_bounds__(TI_THREADS, 1)
 gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -373,6 +376,11 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t from = lanes + (uint32_t)group * TI_D_COLS;
+                    auto release = [&] {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) tm_mbar_arrive(d_empty + 8u * group);
+                    };
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {  // eight tokens at a time
                         if (8 * hh >= t.t_count) break;
@@ -400,6 +408,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                         ti_ld8(from + 128u + 8u * hh, lo);
                         ti_ld8(from + 144u + 8u * hh, hi);
                         ti_wait_ld();
+                        if (EARLY && (hh == 1 || t.t_count <= 8)) release();
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             const int corr = lo[i] + 64 * hi[i];
@@ -409,9 +418,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                                 acc[hh][i] = fmaf(dxv[i], __fmul_rn(d, (float)(sum[i] - 32 * corr)), acc[hh][i]);
                         }
                     }
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) tm_mbar_arrive(d_empty + 8u * group);
+                    if (!EARLY) release();
                 }
                 if (!ok) break;
                 // ---- the tile's part is complete: group 1's sums go to group 0 ----
@@ -549,7 +556,7 @@ bool gemm_ti_supported(int kind, const void *W, int K, int F) {
     return (kind == KIND_Q4_K || kind == KIND_Q6_K) && K <= TI_MAX_K && gemm_ts_supported(kind, W, 1, K, F);
 }
 
-template <int KIND>
+template <int KIND, bool EARLY>
 static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
     const int fixed = 16 + 512 + 1024 + TI_B_SLOTS * (int)ti_b_bytes<KIND>() + 2 * TI_COLS * TS_ROWS * 4;
     const int slab = ts_slab_bytes<KIND>(p.loose != 0);
@@ -560,7 +567,7 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     if (dev >= 64 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
-        if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
+        if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
         if (dev < 64) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
@@ -576,10 +583,11 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.split > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND>, maps, p);
+    return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND, EARLY>, maps, p);
 }
 static cudaError_t ti_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
-    return kind == KIND_Q4_K ? ti_launch<KIND_Q4_K>(maps, p, n_cta, s) : ti_launch<KIND_Q6_K>(maps, p, n_cta, s);
+    if (kind == KIND_Q6_K) return ti_launch<KIND_Q6_K, true>(maps, p, n_cta, s);
+    return p.group_counts != nullptr ? ti_launch<KIND_Q4_K, true>(maps, p, n_cta, s) : ti_launch<KIND_Q4_K, false>(maps, p, n_cta, s);
 }
 static cudaError_t ti_encode_x(int kind, CUtensorMap *m, const uint8_t *xq, int rows, int nb) {
     return ts_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, xq, (cuuint64_t)nb * 384, (cuuint64_t)rows * ti_planes(kind), (cuuint64_t)nb * 384, 128,
