@@ -6,27 +6,13 @@
 // so the compiler cannot contract a multiply and an add into one FMA.
 #pragma once
 
+#include "block_formats.h"
+
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace mcu {
-
-constexpr int QK_K = 256;
-constexpr int Q8_0_VALUES = 32;
-constexpr int Q4_K_BYTES = 144;
-constexpr int Q6_K_BYTES = 210;
-constexpr int Q8_0_BYTES = 34;
-
-enum Kind : int { KIND_Q8_0 = 5, KIND_Q4_K = 9, KIND_Q6_K = 11 };
-
-__host__ __device__ inline int block_values(int kind) { return kind == KIND_Q8_0 ? Q8_0_VALUES : QK_K; }
-__host__ __device__ inline int block_bytes(int kind) {
-    return kind == KIND_Q4_K ? Q4_K_BYTES : kind == KIND_Q6_K ? Q6_K_BYTES : Q8_0_BYTES;
-}
-__host__ __device__ inline bool kind_supported(int kind) {
-    return kind == KIND_Q8_0 || kind == KIND_Q4_K || kind == KIND_Q6_K;
-}
 
 // Quantized activations, structure-of-arrays (values identical to the reference's Q8_K / Q8_0
 // activation blocks, matmul_quant_pack.c:23-62,106-169; only the memory layout differs).

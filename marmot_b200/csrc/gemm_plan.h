@@ -1,0 +1,198 @@
+// How the tcgen05 matmuls with weights in tensor memory (gemm_ts.cu, gemm_ti.cu) divide a call: the plan that the host makes, and what
+// a CTA's share of it is.  Plain C++ apart from the qualifiers (block_formats.h), so that the CPU tests run this very code.
+#pragma once
+
+#include "block_formats.h"
+
+#include <stddef.h>
+#include <stdint.h>
+
+namespace mcu {
+
+constexpr int TS_ROWS = 128;     // weight rows per tile (TMEM lanes)
+constexpr int TS_SLAB_K = 256;   // values of K per slab
+constexpr int TS_MAX_JOBS = 4;
+constexpr int TS_MAX_GROUPS = 256;
+constexpr int TS_MAX_SPLIT = 8;
+constexpr int TI_COLS = 16;      // tokens of a tile of the integer kernel
+
+MCU_HD int ts_min(int a, int b) { return a < b ? a : b; }
+
+struct TsJob {
+    const uint8_t *w;
+    float *out;
+    const float *bias;
+    int F, ldo;
+    int row_tile0;  // first row tile of the job
+};
+struct TsParams {
+    TsJob jobs[TS_MAX_JOBS];
+    const float *rowscale;  // fp16: per-token power-of-two factor undone in the epilogue; integers: block scales [block][row]
+    float *partial;         // two slots of 128 x bn floats per CTA
+    int *counters;          // one ticket per CTA, zero between launches
+    int *err;
+    const int *group_counts, *group_offsets;  // grouped launches (MoE experts), device memory
+    long row_bytes;
+    int n_jobs, T, bn, nb, slabs, raw_shift;  // raw_shift: log2 of the slab ring's depth
+    int loose;              // weight rows that are not 16-byte multiples, or do not start on one
+    int split;              // > 1: clusters of `split` CTAs (pairs) share a tile along K; otherwise ranges of units
+    int tiles, t_tiles;     // output tiles in all; token tiles per row tile
+    int groups, row_tiles;  // grouped launches: number of groups, row tiles per group
+    int count_lo, count_hi; // grouped launches: groups with a count in this range
+};
+
+// One output tile: which weights, which tokens, where the result goes.
+struct TsTile {
+    int job, f0, rows;       // rows that exist
+    int w_row0;              // first weight row in the (stacked) matrix
+    int t_row0, t_count;     // first activation / output row, and how many of the BN columns are tokens
+};
+
+// The units [u0, u1) of this CTA (one slab of one tile each), and what a tile is.
+struct TsWork {
+    const int *group_tile0;
+    bool grouped;
+    int bn, u0, u1, n_use;
+    long long units;
+
+    MCU_HD TsTile tile(const TsParams &p, int tile) const {
+        TsTile t;
+        int rt, tt, T_here, row_off, cols = bn;
+        t.job = 0;
+        if (grouped) {
+            int g = 0;
+            while (tile >= group_tile0[g + 1]) ++g;
+            int in = tile - group_tile0[g];
+            const int t_tiles = (group_tile0[g + 1] - group_tile0[g]) / p.row_tiles;
+            rt = in / t_tiles;
+            tt = in - rt * t_tiles;
+            while (t.job + 1 < p.n_jobs && rt >= p.jobs[t.job + 1].row_tile0) ++t.job;
+            rt -= p.jobs[t.job].row_tile0;
+            T_here = p.group_counts[g];
+            row_off = p.group_offsets[g];
+            cols = ((T_here + t_tiles - 1) / t_tiles + 15) & ~15;  // the group's tokens dealt evenly to its tiles
+            t.w_row0 = g * p.jobs[t.job].F;
+        } else {
+            rt = tile / p.t_tiles;
+            tt = tile - rt * p.t_tiles;
+            while (t.job + 1 < p.n_jobs && rt >= p.jobs[t.job + 1].row_tile0) ++t.job;
+            rt -= p.jobs[t.job].row_tile0;
+            T_here = p.T;
+            row_off = 0;
+            t.w_row0 = 0;
+        }
+        t.f0 = rt * TS_ROWS;
+        t.w_row0 += t.f0;
+        t.rows = ts_min(TS_ROWS, p.jobs[t.job].F - t.f0);
+        t.t_row0 = row_off + tt * cols;
+        t.t_count = ts_min(cols, T_here - tt * cols);
+        return t;
+    }
+};
+MCU_HD TsWork ts_work(const TsParams &p, bool grouped, const int *group_tile0, int bn, int cta, int n_cta) {
+    TsWork w;
+    const int KS = p.slabs;
+    w.group_tile0 = group_tile0;
+    w.grouped = grouped;
+    w.bn = bn;
+    w.units = (long long)(grouped ? group_tile0[p.groups] : p.tiles) * KS;
+    w.n_use = (int)(w.units < n_cta ? w.units : n_cta);  // (a grouped launch may find fewer units than CTAs)
+    w.u0 = cta < w.n_use ? (int)(w.units * cta / w.n_use) : 0;
+    w.u1 = cta < w.n_use ? (int)(w.units * (cta + 1) / w.n_use) : 0;
+    if (p.split > 1) {
+        const int t = cta / p.split, part = cta - t * p.split;
+        w.u0 = t * KS + KS * part / p.split;
+        w.u1 = t * KS + KS * (part + 1) / p.split;
+    }
+    return w;
+}
+
+// A tile cut between CTAs (ranges of units): the CTAs that hold a share of it, and the slot of each (0: its range starts inside the
+// tile or at its start, 1: before it).
+struct TsOwners {
+    int first, last;
+};
+MCU_HD TsOwners ts_owners(const TsWork &w, int tile, int KS) {
+    const long long lo = (long long)tile * KS, hi = lo + KS;
+    return {(int)(((lo + 1) * w.n_use - 1) / w.units), (int)((hi * w.n_use - 1) / w.units)};
+}
+MCU_HD int ts_share_slot(const TsWork &w, int tile, int KS, int cta) { return w.units * cta / w.n_use >= (long long)tile * KS ? 0 : 1; }
+
+// ---- host ----
+struct TsPlan {
+    int bn, t_tiles, split, n_cta;
+    double cost;
+};
+
+// How to spread `tiles` output tiles of KS slabs over `room` SMs, and what it costs in cycles, by measurements of all the forms at 70 to 512
+// tokens and 2048 x 2048 to 4096 x 28672 weights.  A slab takes the longer of its conversion (less in tiles of up to 64 columns, whose
+// stages hold 128 values of K) and its MMAs; a tile ends with its epilogue.
+// - One tile per CTA, in as many waves as it takes: 2000 for a CTA's start.
+// - A tile over a cluster: the exchange of the shares through the CTAs' shared memories.
+// - Equal ranges of slabs: cut tiles have their shares written to memory, and read again by the CTA that comes last; a tile of 256
+//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).
+inline TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles, int room) {
+    const long U = (long)tiles * KS;
+    const bool wide = bn > 64;
+    const double conv = kind == KIND_Q4_K ? (wide ? 1500 : 1120) : kind == KIND_Q6_K ? (wide ? 2100 : 1700) : (wide ? 1750 : 1500);
+    const double mma = 8.5 * bn, unit = mma > conv ? mma : conv, tile_end = 1000.0 + 8.0 * bn;
+    TsPlan best{bn, t_tiles, 1, 0, 1e30};
+    auto consider = [&](int split, long n, double cost) {
+        if (cost < best.cost) best = TsPlan{bn, t_tiles, split, (int)n, cost};
+    };
+    consider(1, tiles, (double)((tiles + room - 1) / room) * (KS * unit + tile_end + 2000.0));
+    for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2) {
+        // A cluster is placed inside a GPC (16 to 20 SMs): sixteen clusters of eight did not run at once (2048 x 2048: 12.6 us,
+        // 64 CTAs in clusters of four 7.5), fourteen do.
+        const int usable = sp >= 8 ? room * 7 / 9 : room;
+        const double exchange = sp == 2 ? 3500.0 + 30.0 * bn : 5000.0 + 20.0 * bn;
+        if ((long)tiles * sp <= usable) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + tile_end + 2000.0 + exchange);
+    }
+    const long n = U < room ? U : room;
+    const long upc = (U + n - 1) / n;
+    const bool cut = U % n != 0 || upc % KS != 0;
+    const double shares = cut ? (double)KS / upc + 1.0 : 0.0;
+    consider(1, n, upc * unit + ((double)upc / KS + 1.0) * tile_end + 2000.0 + shares * 65.0 * bn);
+    return best;
+}
+
+inline TsPlan ts_plan(int kind, int T, int K, const int *F, int n_jobs, int sms) {
+    const int nb = (K + block_values(kind) - 1) / block_values(kind);
+    const int KS = (nb * block_values(kind) + TS_SLAB_K - 1) / TS_SLAB_K;
+    int rows = 0;
+    for (int j = 0; j < n_jobs; ++j) rows += (F[j] + TS_ROWS - 1) / TS_ROWS;
+    TsPlan best{};
+    best.cost = 1e30;
+    // as few token tiles as there can be, or a few more: narrower tiles fill the SMs better, but the weights are converted more often
+    // (6 % for each: with all SMs at work the chip runs into its power limit)
+    const int fewest = (T + 255) / 256, most = (T + 63) / 64;
+    for (int tried = fewest; tried <= most && tried <= fewest + 3; ++tried) {
+        const int bn = ((T + tried - 1) / tried + 15) / 16 * 16;
+        const int t_tiles = (T + bn - 1) / bn;  // (not `tried`: widened to 16 columns, fewer tiles may hold all tokens, and the last would be empty)
+        TsPlan pl = ts_spread(kind, rows * t_tiles, KS, bn, t_tiles, sms);
+        pl.cost *= 1.0 + 0.06 * (t_tiles - fewest);
+        if (pl.cost < best.cost) best = pl;
+    }
+    return best;
+}
+
+// The same for the integer kernel: one tile per CTA, in waves if need be, a tile over a cluster, or equal ranges, whichever ends
+// first, by a sweep of all three at nine tokens: a slab takes about 900 cycles (Q6_K 2100), the start of a CTA 3500, a cluster's exchange 1500; a tile cut between
+// ranges costs 9000 and 700 for every share that the last CTA reads (13056 x 1792 Q4_K: 22 us in ranges of five slabs, 13 in
+// clusters of eight).  Clusters of eight: as in ts_spread.
+inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
+    const long U = (long)tiles * KS, n_most = U < sms ? U : sms, upc = (U + n_most - 1) / n_most;
+    const double unit = kind == KIND_Q4_K ? 900.0 : 2100.0;
+    TsPlan best{TI_COLS, 0, 1, (int)n_most, 1e30};
+    auto consider = [&](int split, long n, double cost) {
+        if (cost < best.cost) best = TsPlan{TI_COLS, 0, split, (int)n, cost};
+    };
+    consider(1, tiles, (double)((tiles + sms - 1) / sms) * (KS * unit + 3500.0));
+    for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2)
+        if ((long)tiles * sp <= (sp >= 8 ? sms * 7 / 9 : sms)) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + 5000.0);
+    const bool cut = U % n_most != 0 || upc % KS != 0;
+    consider(1, n_most, (double)upc * unit + 2000.0 + (cut ? 9000.0 + 700.0 * ((double)KS / upc + 1.0) : 0.0));
+    return best;
+}
+
+}  // namespace mcu

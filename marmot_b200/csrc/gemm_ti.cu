@@ -185,8 +185,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const TsWork work = ts_work(p, grouped, group_tile0, TI_COLS, cta, n_cta);
-    const int KS = p.slabs, u0 = work.u0, u1 = work.u1, n_use = work.n_use, n_slabs = u1 - u0;
-    const long long U = work.units;
+    const int KS = p.slabs, u0 = work.u0, u1 = work.u1, n_slabs = u1 - u0;
 
     bool ok = true;
     int err_code = 0;
@@ -462,15 +461,14 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     __threadfence();
                     __syncwarp();
                     if (lane == 0) tm_mbar_arrive(share_bar);
-                    const long long first = (long long)tile * KS, past = first + KS;
-                    const int c0 = (int)(((first + 1) * n_use - 1) / U), c1 = (int)((past * n_use - 1) / U);
+                    const TsOwners own = ts_owners(work, tile, KS);
                     if (warp == TI_CONV) {
                         ok = ts_wait(share_bar, shares & 1u);
                         ok = __all_sync(0xffffffffu, ok);
                         if (lane == 0 && ok) {
-                            int *ctr = p.counters + c0;
+                            int *ctr = p.counters + own.first;
                             const int ticket = atomicAdd(ctr, 1);
-                            last_s = ticket == c1 - c0;
+                            last_s = ticket == own.last - own.first;
                             if (last_s) *ctr = 0;  // ready for the next launch
                             tm_mbar_arrive(ticket_bar);
                         }
@@ -485,8 +483,8 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
 #pragma unroll
                     for (int c = 0; c < 16; ++c) acc[c >> 3][c & 7] = 0.0f;
 #pragma unroll 1
-                    for (int k = c0; k <= c1; ++k) {
-                        const float *from = slot(k, U * k / n_use >= first ? 0 : 1);
+                    for (int k = own.first; k <= own.last; ++k) {
+                        const float *from = slot(k, ts_share_slot(work, tile, KS, k));
                         float v[16];
 #pragma unroll
                         for (int c = 0; c < 16; ++c) v[c] = __ldcg(from + c * TS_ROWS);
@@ -618,29 +616,9 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     }
     p.tiles = row_tiles * p.t_tiles;
     if (cudaError_t e = ti_encode_x(kind, &maps.x, xq, T, p.nb)) return e;
-    // One tile per CTA, in waves if need be, a tile over a cluster, or equal ranges, whichever ends first, by a sweep of all three at
-    // nine tokens: a slab takes about 900 cycles (Q6_K 2100), the start of a CTA 3500, a cluster's exchange 1500; a tile cut between
-    // ranges costs 9000 and 700 for every share that the last CTA reads (13056 x 1792 Q4_K: 22 us in ranges of five slabs, 13 in
-    // clusters of eight).  Clusters of eight: as in ts_spread.
-    const int sms = device_sm_count(), KS = p.slabs;
-    const long U = (long)p.tiles * KS, n_most = U < sms ? U : sms, upc = (U + n_most - 1) / n_most;
-    const double unit = kind == KIND_Q4_K ? 900.0 : 2100.0;
-    double best = 1e30;
-    int n_cta = (int)n_most;
-    p.split = 1;
-    auto consider = [&](int split, long n, double cost) {
-        if (cost < best) {
-            best = cost;
-            p.split = split;
-            n_cta = (int)n;
-        }
-    };
-    consider(1, p.tiles, (double)((p.tiles + sms - 1) / sms) * (KS * unit + 3500.0));
-    for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2)
-        if ((long)p.tiles * sp <= (sp >= 8 ? sms * 7 / 9 : sms)) consider(sp, (long)p.tiles * sp, (KS + sp - 1) / sp * unit + 5000.0);
-    const bool cut = U % n_most != 0 || upc % KS != 0;
-    consider(1, n_most, (double)upc * unit + 2000.0 + (cut ? 9000.0 + 700.0 * ((double)KS / upc + 1.0) : 0.0));
-    return ti_dispatch(kind, maps, p, n_cta, s);
+    const TsPlan pl = ti_plan(kind, p.tiles, p.slabs, device_sm_count());
+    p.split = pl.split;
+    return ti_dispatch(kind, maps, p, pl.n_cta, s);
 }
 
 cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq, const float *dT,

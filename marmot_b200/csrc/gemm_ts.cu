@@ -277,8 +277,7 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const TsWork work = ts_work(p, grouped, group_tile0, bn, cta, n_cta);
-    const int KS = p.slabs, u0 = work.u0, u1 = work.u1, n_use = work.n_use;
-    const long long U = work.units;
+    const int KS = p.slabs, u0 = work.u0, u1 = work.u1;
     auto tile_of = [&](int tile) { return work.tile(p, tile); };
 
     bool ok = true;
@@ -443,16 +442,15 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
             __threadfence();
             __syncwarp();
             if (lane == 0) tm_mbar_arrive(share_bar);
-            const long long first = (long long)tile * KS, past = first + KS;
-            const int c0 = (int)(((first + 1) * n_use - 1) / U), c1 = (int)((past * n_use - 1) / U);
+            const TsOwners own = ts_owners(work, tile, KS);
             if (warp == 0) {
                 ok = ts_wait(share_bar, shares & 1u);
                 ok = __all_sync(0xffffffffu, ok);
             }
             if (threadIdx.x == 0 && ok) {
-                int *ctr = p.counters + c0;
+                int *ctr = p.counters + own.first;
                 const int ticket = atomicAdd(ctr, 1);
-                last_s = ticket == c1 - c0;
+                last_s = ticket == own.last - own.first;
                 if (last_s) *ctr = 0;  // ready for the next launch
                 tm_mbar_arrive(ticket_bar);
             }
@@ -468,9 +466,9 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
 #pragma unroll
                 for (int jj = 0; jj < 16; ++jj) acc[jj] = 0.0f;
 #pragma unroll 2
-                for (int k = c0; k <= c1; ++k) {
+                for (int k = own.first; k <= own.last; ++k) {
                     // a CTA whose range starts inside the tile, or exactly at its start, holds the share in slot 0
-                    const float *from = slot(k, U * k / n_use >= first ? 0 : 1) + (16 * c) * TS_ROWS + r;
+                    const float *from = slot(k, ts_share_slot(work, tile, KS, k)) + (16 * c) * TS_ROWS + r;
                     float w[16];
 #pragma unroll
                     for (int jj = 0; jj < 16; ++jj) w[jj] = __ldcg(from + jj * TS_ROWS);
@@ -633,63 +631,6 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
-struct TsPlan {
-    int bn, t_tiles, split, n_cta;
-    double cost;
-};
-
-// How to spread `tiles` output tiles of KS slabs over the SMs, and what it costs in cycles, by measurements of all the forms at 70 to 512
-// tokens and 2048 x 2048 to 4096 x 28672 weights.  A slab takes the longer of its conversion (less in tiles of up to 64 columns, whose
-// stages hold 128 values of K) and its MMAs; a tile ends with its epilogue.
-// - One tile per CTA, in as many waves as it takes: 2000 for a CTA's start.
-// - A tile over a cluster: the exchange of the shares through the CTAs' shared memories.
-// - Equal ranges of slabs: cut tiles have their shares written to memory, and read again by the CTA that comes last; a tile of 256
-//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).
-static TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles) {
-    const int room = device_sm_count();
-    const long U = (long)tiles * KS;
-    const bool wide = bn > 64;
-    const double conv = kind == KIND_Q4_K ? (wide ? 1500 : 1120) : kind == KIND_Q6_K ? (wide ? 2100 : 1700) : (wide ? 1750 : 1500);
-    const double mma = 8.5 * bn, unit = mma > conv ? mma : conv, tile_end = 1000.0 + 8.0 * bn;
-    TsPlan best{bn, t_tiles, 1, 0, 1e30};
-    auto consider = [&](int split, long n, double cost) {
-        if (cost < best.cost) best = TsPlan{bn, t_tiles, split, (int)n, cost};
-    };
-    consider(1, tiles, (double)((tiles + room - 1) / room) * (KS * unit + tile_end + 2000.0));
-    for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2) {
-        // A cluster is placed inside a GPC (16 to 20 SMs): sixteen clusters of eight did not run at once (2048 x 2048: 12.6 us,
-        // 64 CTAs in clusters of four 7.5), fourteen do.
-        const int usable = sp >= 8 ? room * 7 / 9 : room;
-        const double exchange = sp == 2 ? 3500.0 + 30.0 * bn : 5000.0 + 20.0 * bn;
-        if ((long)tiles * sp <= usable) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + tile_end + 2000.0 + exchange);
-    }
-    const long n = U < room ? U : room;
-    const long upc = (U + n - 1) / n;
-    const bool cut = U % n != 0 || upc % KS != 0;
-    const double shares = cut ? (double)KS / upc + 1.0 : 0.0;
-    consider(1, n, upc * unit + ((double)upc / KS + 1.0) * tile_end + 2000.0 + shares * 65.0 * bn);
-    return best;
-}
-
-static TsPlan ts_plan(int kind, int T, int K, const int *F, int n_jobs) {
-    const int nb = (K + block_values(kind) - 1) / block_values(kind);
-    const int KS = (nb * block_values(kind) + TS_SLAB_K - 1) / TS_SLAB_K;
-    int rows = 0;
-    for (int j = 0; j < n_jobs; ++j) rows += (F[j] + TS_ROWS - 1) / TS_ROWS;
-    TsPlan best{};
-    best.cost = 1e30;
-    // as few token tiles as there can be, or a few more: narrower tiles fill the SMs better, but the weights are converted more often
-    // (6 % for each: with all SMs at work the chip runs into its power limit)
-    const int fewest = (T + 255) / 256, most = (T + 63) / 64;
-    for (int t_tiles = fewest; t_tiles <= most && t_tiles <= fewest + 3; ++t_tiles) {
-        const int bn = ((T + t_tiles - 1) / t_tiles + 15) / 16 * 16;
-        TsPlan pl = ts_spread(kind, rows * t_tiles, KS, bn, t_tiles);
-        pl.cost *= 1.0 + 0.06 * (t_tiles - fewest);
-        if (pl.cost < best.cost) best = pl;
-    }
-    return best;
-}
-
 size_t gemm_ts_workspace_bytes() {
     // two shares of 128 x 256 floats per CTA, and a ticket each
     return (size_t)device_sm_count() * 2 * TS_ROWS * 256 * sizeof(float);
@@ -779,7 +720,8 @@ cudaError_t launch_gemm_ts(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     memset(&p, 0, sizeof(p));
     int F[TS_MAX_JOBS];
     for (int j = 0; j < n_jobs; ++j) F[j] = jobs[j].F;
-    const TsPlan pl = ts_plan(kind, T, K, F, n_jobs);
+    const TsPlan pl = ts_plan(kind, T, K, F, n_jobs, device_sm_count());
+    if ((long)(pl.t_tiles - 1) * pl.bn >= T) return cudaErrorInvalidValue;  // a tile without tokens is no MMA
     p.nb = (K + block_values(kind) - 1) / block_values(kind);
     p.row_bytes = (long)p.nb * block_bytes(kind);
     p.slabs = (p.nb * block_values(kind) + TS_SLAB_K - 1) / TS_SLAB_K;

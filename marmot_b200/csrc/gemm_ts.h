@@ -1,43 +1,17 @@
 // Parameters and launchers of the tcgen05 matmul with weights in tensor memory (gemm_ts.cu).
 #pragma once
 
+#include "gemm_plan.h"
 #include "kernels.h"
 
 #include <cuda.h>
 
 namespace mcu {
 
-constexpr int TS_MAX_JOBS = 4;
-constexpr int TS_MAX_GROUPS = 256;
-constexpr int TS_MAX_SPLIT = 8;
-
 struct TsMaps {
     CUtensorMap x;               // fp16 activations [rows][kp]
     CUtensorMap w[TS_MAX_JOBS];  // packed weights, Q4_K only
 };
-struct TsJob {
-    const uint8_t *w;
-    float *out;
-    const float *bias;
-    int F, ldo;
-    int row_tile0;  // first row tile of the job
-};
-struct TsParams {
-    TsJob jobs[TS_MAX_JOBS];
-    const float *rowscale;  // fp16: per-token power-of-two factor undone in the epilogue; integers: block scales [block][row]
-    float *partial;         // two slots of 128 x bn floats per CTA
-    int *counters;          // one ticket per CTA, zero between launches
-    int *err;
-    const int *group_counts, *group_offsets;  // grouped launches (MoE experts), device memory
-    long row_bytes;
-    int n_jobs, T, bn, nb, slabs, raw_shift;  // raw_shift: log2 of the slab ring's depth
-    int loose;              // weight rows that are not 16-byte multiples, or do not start on one
-    int split;              // > 1: clusters of `split` CTAs (pairs) share a tile along K; otherwise ranges of units
-    int tiles, t_tiles;     // output tiles in all; token tiles per row tile
-    int groups, row_tiles;  // grouped launches: number of groups, row tiles per group
-    int count_lo, count_hi; // grouped launches: groups with a count in this range
-};
-
 // Shares of cut tiles (gemm_ts_workspace_bytes(), 0 tickets in `counters` between launches, one int per SM).
 size_t gemm_ts_workspace_bytes();
 bool gemm_ts_supported(int kind, const void *W, int T, int K, int F);
@@ -52,7 +26,6 @@ cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
 
 // The same on integers for a handful of tokens (gemm_ti.cu: Q4_K, Q6_K): exact sub-block dots.  xq / dT from
 // launch_act_int_fused.  The grouped form takes the groups with a count up to count_hi.
-constexpr int TI_COLS = 16;
 constexpr int TI_MAX_K = 65536;
 size_t gemm_ti_xq_bytes(int kind, int rows, int K);
 bool gemm_ti_supported(int kind, const void *W, int K, int F);

@@ -8,9 +8,6 @@
 
 namespace mcu {
 
-constexpr int TS_ROWS = 128;     // weight rows per tile (TMEM lanes)
-constexpr int TS_SLAB_K = 256;   // values of K per slab
-
 // A slab in shared memory: BYTES of every row, BOX bytes fetched (a 16-byte aligned window that covers them) and the pitch.  The
 // pitch is an odd number of 16-byte units, so that 16-byte loads of a warp's 32 rows are conflict free.
 template <int KIND>
@@ -93,72 +90,6 @@ __device__ __forceinline__ void ts_group_table(const TsParams &p, int bn, int *g
         base += __shfl_sync(0xffffffffu, n, 31);
     }
     if (lane == 0) group_tile0[0] = 0;
-}
-
-// One output tile: which weights, which tokens, where the result goes.
-struct TsTile {
-    int job, f0, rows;       // rows that exist
-    int w_row0;              // first weight row in the (stacked) matrix
-    int t_row0, t_count;     // first activation / output row, and how many of the BN columns are tokens
-};
-
-// The units [u0, u1) of this CTA (one slab of one tile each), and what a tile is.
-struct TsWork {
-    const int *group_tile0;
-    bool grouped;
-    int bn, u0, u1, n_use;
-    long long units;
-
-    __device__ __forceinline__ TsTile tile(const TsParams &p, int tile) const {
-        TsTile t;
-        int rt, tt, T_here, row_off, cols = bn;
-        t.job = 0;
-        if (grouped) {
-            int g = 0;
-            while (tile >= group_tile0[g + 1]) ++g;
-            int in = tile - group_tile0[g];
-            const int t_tiles = (group_tile0[g + 1] - group_tile0[g]) / p.row_tiles;
-            rt = in / t_tiles;
-            tt = in - rt * t_tiles;
-            while (t.job + 1 < p.n_jobs && rt >= p.jobs[t.job + 1].row_tile0) ++t.job;
-            rt -= p.jobs[t.job].row_tile0;
-            T_here = p.group_counts[g];
-            row_off = p.group_offsets[g];
-            cols = ((T_here + t_tiles - 1) / t_tiles + 15) & ~15;  // the group's tokens dealt evenly to its tiles
-            t.w_row0 = g * p.jobs[t.job].F;
-        } else {
-            rt = tile / p.t_tiles;
-            tt = tile - rt * p.t_tiles;
-            while (t.job + 1 < p.n_jobs && rt >= p.jobs[t.job + 1].row_tile0) ++t.job;
-            rt -= p.jobs[t.job].row_tile0;
-            T_here = p.T;
-            row_off = 0;
-            t.w_row0 = 0;
-        }
-        t.f0 = rt * TS_ROWS;
-        t.w_row0 += t.f0;
-        t.rows = min(TS_ROWS, p.jobs[t.job].F - t.f0);
-        t.t_row0 = row_off + tt * cols;
-        t.t_count = min(cols, T_here - tt * cols);
-        return t;
-    }
-};
-__device__ __forceinline__ TsWork ts_work(const TsParams &p, bool grouped, const int *group_tile0, int bn, int cta, int n_cta) {
-    TsWork w;
-    const int KS = p.slabs;
-    w.group_tile0 = group_tile0;
-    w.grouped = grouped;
-    w.bn = bn;
-    w.units = (long long)(grouped ? group_tile0[p.groups] : p.tiles) * KS;
-    w.n_use = (int)min((long long)n_cta, w.units);  // (a grouped launch may find fewer units than CTAs)
-    w.u0 = cta < w.n_use ? (int)(w.units * cta / w.n_use) : 0;
-    w.u1 = cta < w.n_use ? (int)(w.units * (cta + 1) / w.n_use) : 0;
-    if (p.split > 1) {
-        const int t = cta / p.split, part = cta - t * p.split;
-        w.u0 = t * KS + KS * part / p.split;
-        w.u1 = t * KS + KS * (part + 1) / p.split;
-    }
-    return w;
 }
 
 // The slab producer (one warp): every slab of the CTA's range, in order, into the ring.

@@ -69,3 +69,18 @@ def test_jobs_of_two_kinds_equal_single_calls(ctx, T):
     for (k, F), w, o in zip(sizes, ws, outs):
         assert max_rel_err(o.cpu().numpy(), ctx.linear(k, x, w, F).cpu().numpy()) <= 1e-5
     ctx.synchronize()
+
+
+@pytest.mark.parametrize("name,T", [("q4_k", 3073), ("q8_0", 3120), ("q6_k", 4161)])
+def test_many_tokens_equal_calls_on_slices(ctx, name, T):
+    """Token counts at which tiles widened to 16 columns are fewer than the plan asked for.  The sums' order differs: 32-bit rounding."""
+    import torch
+
+    K, F, kind = 1536, 4700, KINDS[name]
+    rng = np.random.default_rng(T)
+    w = ctx.upload(random_blocks(kind, F, K, rng))
+    x = torch.from_numpy(rng.normal(0, 1, (T, K)).astype(np.float32)).cuda()
+    got = ctx.linear(kind, x, w, F)
+    ref = torch.cat([ctx.linear(kind, part, w, F) for part in x.split(500)])
+    ctx.synchronize()
+    assert max_rel_err(got.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
