@@ -129,29 +129,29 @@ static int ensure(mcu_context *ctx, Buffer &b, size_t bytes) {
     return MCU_SUCCESS;
 }
 
-// After a synchronize: did a kernel give up on a bounded wait?
+// A kernel reported `flag` and the stream `s` is idle.  A matmul that gave up on a bounded wait leaves the tickets that it has drawn: the
+// next one would take a share for the last of its tile too early, so they start from zero again.
+static int report_flag(mcu_context *ctx, cudaStream_t s, int flag) {
+    MCU_CUDA(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), s));
+    MCU_CUDA(cudaMemsetAsync(ctx->gemm_counters, 0, GEMM_TMA_MAX_TILE_COUNTERS * sizeof(int), s));  // (whatever the flag: the last report wins)
+    if (flag == 40) return fail(MCU_ERROR_INVALID_ARGUMENT, "MoE expert id is out of range (found by an earlier call)");
+    return fail(MCU_ERROR_INVALID_OPERATION, "a device-side wait timed out (code %d)", flag);
+}
+
 // Wait for the stream `s` of the context and report a device-side error flag, if one was set.  The flag travels with
 // the wait (an asynchronous copy into a page-locked word enqueued ahead of the synchronize): a separate blocking copy
 // of four bytes cost ten microseconds on every synchronising call.
 static int sync_and_check(mcu_context *ctx, cudaStream_t s) {
+    int flag = 0;
     if (ctx->err_host == nullptr) {
         MCU_CUDA(cudaStreamSynchronize(s));
-        int flag = 0;
         MCU_CUDA(cudaMemcpy(&flag, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost));
-        if (flag == 0) return MCU_SUCCESS;
-        cudaMemset(ctx->dev_err, 0, sizeof(int));
-        if (flag == 40) return fail(MCU_ERROR_INVALID_ARGUMENT, "MoE expert id is out of range (found by an earlier call)");
-        return fail(MCU_ERROR_INVALID_OPERATION, "a device-side wait timed out (code %d)", flag);
+    } else {
+        MCU_CUDA(cudaMemcpyAsync(ctx->err_host, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        MCU_CUDA(cudaStreamSynchronize(s));
+        flag = *(volatile int *)ctx->err_host;
     }
-    MCU_CUDA(cudaMemcpyAsync(ctx->err_host, ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MCU_CUDA(cudaStreamSynchronize(s));
-    const int flag = *(volatile int *)ctx->err_host;
-    if (flag != 0) {
-        cudaMemset(ctx->dev_err, 0, sizeof(int));
-        if (flag == 40) return fail(MCU_ERROR_INVALID_ARGUMENT, "MoE expert id is out of range (found by an earlier call)");
-        return fail(MCU_ERROR_INVALID_OPERATION, "a device-side wait timed out (code %d)", flag);
-    }
-    return MCU_SUCCESS;
+    return flag == 0 ? MCU_SUCCESS : report_flag(ctx, s, flag);
 }
 
 namespace mcu {
@@ -280,6 +280,18 @@ void mcu_context_destroy(mcu_context_t *ctx) {
     if (ctx->gemm_counters != nullptr) cudaFree(ctx->gemm_counters);
     if (ctx->own_stream != nullptr) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
+}
+
+// Test hook (not in the header): the state that a matmul leaves behind when a bounded wait runs out, some tickets drawn and the
+// flag set, without such a wait.
+int mcu_test_matmul_gave_up(mcu_context_t *ctx) {
+    if (int rc = check_ctx(ctx)) return rc;
+    const std::vector<int> ones(GEMM_TMA_MAX_TILE_COUNTERS, 1);
+    const int code = 8;
+    MCU_CUDA(cudaMemcpyAsync(ctx->gemm_counters, ones.data(), ones.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    MCU_CUDA(cudaMemcpyAsync(ctx->dev_err, &code, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    MCU_CUDA(cudaStreamSynchronize(ctx->stream));
+    return MCU_SUCCESS;
 }
 
 int mcu_context_set_stream(mcu_context_t *ctx, void *cuda_stream) {

@@ -112,3 +112,23 @@ def test_few_route_moe(ctx, oracle, kinds, T, E, k):
     again = ctx.moe_experts(kinds, hd, gd, ud, dd, idd, vd, FF, E)
     ctx.synchronize()
     assert torch.equal(again, got)
+
+
+@pytest.mark.parametrize("T", [9, 64])  # the integer and the fp16 kernel, both with tiles cut between CTAs
+def test_calls_after_a_wait_that_ran_out(ctx, T):
+    """The tickets of cut tiles that a kernel left drawn do not reach the next call (a host-side hook sets the state; nothing times out)."""
+    import torch
+    from marmot_b200 import MarmotCudaError
+
+    K, F = 2048, 20000
+    rng = np.random.default_rng(T)
+    w = ctx.upload(random_blocks(KIND_Q4_K, F, K, rng))
+    x, before = (torch.from_numpy(rng.normal(0, 1, (T, K)).astype(np.float32)).cuda() for _ in range(2))
+    want = ctx.linear(KIND_Q4_K, x, w, F)
+    ctx.linear(KIND_Q4_K, before, w, F)  # its shares are what a ticket drawn too early would add up
+    ctx.synchronize()
+    assert ctx.lib.mcu_test_matmul_gave_up(ctx.handle) == 0
+    with pytest.raises(MarmotCudaError, match="timed out"):
+        ctx.synchronize()
+    assert torch.equal(ctx.linear(KIND_Q4_K, x, w, F), want)
+    ctx.synchronize()
