@@ -352,6 +352,14 @@ __device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ld
     return true;
 }
 
+// Lets the matmul behind start, and waits for the kernel ahead.  A grouped matmul reads the groups' counts before its own wait, so it may
+// start only when the routing kernels are complete: this kernel's wait first.
+__device__ __forceinline__ void stage_begin(const ActSource &src) {
+    if (src.row_lo == nullptr) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (src.row_lo != nullptr) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Few rows: up to a thousand threads per row, so that a row is one or two trips to L2 (latency bounds the launch: 64 rows of
 // 4096 values 3.3 us with 256 threads); many rows: 256 threads, and as many rows at a time.
 template <bool KQ, int OP>
@@ -366,8 +374,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
     __shared__ float red[32];
     __shared__ float inv_s;
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    stage_begin(src);
     if (!quantize_row<KQ, OP>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
     __syncthreads();
     float m = 0.0f;
@@ -412,8 +419,7 @@ act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K,
     __shared__ float red[32];
     __shared__ float inv_s;
     const int t = blockIdx.x;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    stage_begin(src);
     if (!quantize_row<true, OP>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
     __syncthreads();
     for (int b = threadIdx.x; b < nb; b += blockDim.x) dT[(size_t)b * ld_dT + t] = d_s[b];

@@ -284,7 +284,8 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     int err_code = 0;
     if (warp == TS_B_WARP) {
         // ------------------------------ activation tiles ------------------------------
-        if (lane == 0 && u0 < u1) {
+        if (lane == 0) {
+            // (without work too: the kernel behind relies on this grid's end to order it behind the staging kernel)
             asm volatile("griddepcontrol.wait;" ::: "memory");
             uint32_t s = 0;
             for (int u = u0; u < u1 && ok;) {

@@ -73,8 +73,8 @@ __device__ __forceinline__ void ts_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 
 // The first tile of every group of a grouped launch (one warp).  Groups with a count outside [count_lo, count_hi] are another
-// launch's.  The counts were written by kernels that finished before the kernel ahead of this one started (they do not trigger
-// their dependents early), so they may be read before griddepcontrol.wait.
+// launch's.  May be called before griddepcontrol.wait: the staging kernel ahead lets this one start only after its own wait, when the
+// kernels that wrote the counts are complete (stage_begin in act_quant.cu).
 __device__ __forceinline__ void ts_group_table(const TsParams &p, int bn, int *group_tile0, int lane) {
     int base = 0;
     for (int g0 = 0; g0 < p.groups; g0 += 32) {

@@ -243,8 +243,7 @@ cudaError_t launch_topk(const float *x, int rows, int cols, size_t ldx, int k, f
 
 // All of the routing in one launch for few routes: counts, offsets, and every route's stable position (the routes ahead of it
 // with the same expert, counted one by one).  The same results as the three kernels above, which cost three launches and a
-// memset: 9 us against 3 at 32 routes.  Does not trigger its dependents early: the grouped matmuls read the counts ahead of
-// griddepcontrol.wait.
+// memset: 9 us against 3 at 32 routes.  Does not trigger its dependents early.
 __global__ void __launch_bounds__(MOE_ROUTE_SMALL)
 moe_route_small_kernel(const int32_t *__restrict__ ids, const float *__restrict__ weights, int routes, int k, int E, float weights_scale,
                        int renormalize, MoeRouteBuffers b) {

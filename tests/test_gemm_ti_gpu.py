@@ -132,3 +132,59 @@ def test_calls_after_a_wait_that_ran_out(ctx, T):
         ctx.synchronize()
     assert torch.equal(ctx.linear(KIND_Q4_K, x, w, F), want)
     ctx.synchronize()
+
+
+@pytest.mark.parametrize("T", [17, 130])  # few routes on the integer kernel, 260 on the fp16 one
+def test_recorded_moe_follows_its_routes(ctx, T):
+    """Replays whose routes were written just ahead of them equal eager calls: the matmuls read the groups' sizes of this replay."""
+    import torch
+
+    H, FF, E, k = 512, 256, 8, 2
+    rng = np.random.default_rng(T)
+    kinds = (KIND_Q4_K,) * 3
+    gate, up, down = (ctx.upload(random_blocks(KIND_Q4_K, F, K, rng, d_sigma=0.0005)) for F, K in ((E * FF, H), (E * FF, H), (E * H, FF)))
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    try:
+        with torch.cuda.stream(stream):
+            hid = torch.randn((T, H), device="cuda")
+            weights = torch.full((T, k), 0.5, device="cuda")
+            routes = [torch.from_numpy(np.stack([rng.permutation(e)[:k] for _ in range(T)]).astype(np.int32)).cuda() for e in (2, 8, 3, 5) * 4]
+            ids = routes[0].clone()
+            call = lambda i: ctx.moe_experts(kinds, hid, gate, up, down, i, weights, FF, E)
+            want = [call(r) for r in routes]
+            ctx.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                out = call(ids)
+            got = []
+            for r in routes:
+                ids.copy_(r)
+                g.replay()
+                got.append(out.clone())
+            ctx.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+            del g
+    finally:
+        ctx.synchronize()
+        ctx.set_stream(0)
+
+
+def test_a_rank_without_routes_between_others(ctx):
+    """Grouped launches that find no work do not let the kernels behind them run ahead: calls for empty expert ranges in between."""
+    import torch
+
+    T, H, FF, E, k = 200, 512, 256, 8, 2
+    rng = np.random.default_rng(5)
+    kinds = (KIND_Q4_K,) * 3
+    blocks = lambda F, K: ctx.upload(random_blocks(KIND_Q4_K, F, K, rng, d_sigma=0.0005))
+    gate, up, down = blocks(4 * FF, H), blocks(4 * FF, H), blocks(4 * H, FF)
+    hid, weights = torch.randn((T, H), device="cuda"), torch.full((T, k), 0.5, device="cuda")
+    ids = torch.from_numpy(np.stack([rng.permutation(4)[:k] for _ in range(T)]).astype(np.int32)).cuda()
+    local = lambda lo: ctx.moe_experts_local(kinds, hid, gate, up, down, ids, weights, FF, E, lo, 4)
+    want = local(0)
+    ctx.synchronize()
+    for _ in range(5):
+        none, some = local(4), local(0)
+        ctx.synchronize()
+        assert not none.any() and torch.equal(some, want)
