@@ -424,30 +424,30 @@ act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K,
     __syncthreads();
     for (int b = threadIdx.x; b < nb; b += blockDim.x) dT[(size_t)b * ld_dT + t] = d_s[b];
     uint8_t *row = xq + (size_t)t * nb * 384;
-    for (int g = threadIdx.x; g < nb * 16; g += blockDim.x) {  // sixteen values
-        const int blk = g >> 4, i = g & 15;
-        const uint4 v = *(const uint4 *)(q_s + 16 * g);
-        int sum = __dp4a((int)v.x, 0x01010101, __dp4a((int)v.y, 0x01010101, __dp4a((int)v.z, 0x01010101, __dp4a((int)v.w, 0x01010101, 0))));
+    constexpr int PER = SUB / 16;  // a sub-block per thread: one or two 16-byte words
+    for (int g = threadIdx.x; g < nb * (QK_K / SUB); g += blockDim.x) {
+        const int blk = g / (QK_K / SUB), at = g % (QK_K / SUB);
         uint8_t *o = row + blk * 384;
-        if (SUB == 16) {
-            const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-            *(uint4 *)(o + 16 * i) = i & 1 ? zero : v;
-            *(uint4 *)(o + plane + 16 * i) = i & 1 ? v : zero;
-        } else {
-            *(uint4 *)(o + 16 * i) = v;
-            sum += __shfl_xor_sync(__activemask(), sum, 1);  // (the lanes of a pair are always here together)
-        }
-        const int at = SUB == 16 ? i : i >> 1, lo = sum & 63;
-        if (SUB == 16 || (i & 1) == 0) {
-            o[256 + at] = (uint8_t)lo;
-            o[288 + at] = (uint8_t)((sum - lo) >> 6);
-        }
-        // the rest of the two 32-byte groups is zero
-        if (SUB == 16 || (i & 1) != 0) {
-            const int z = SUB == 16 ? 16 + i : 8 + 3 * at;
+        int sum = 0;
 #pragma unroll
-            for (int n = 0; n < (SUB == 16 ? 1 : 3); ++n) o[256 + z + n] = o[288 + z + n] = 0;
+        for (int n = 0; n < PER; ++n) {
+            const uint4 v = *(const uint4 *)(q_s + SUB * g + 16 * n);
+            sum = __dp4a((int)v.x, 0x01010101, __dp4a((int)v.y, 0x01010101, __dp4a((int)v.z, 0x01010101, __dp4a((int)v.w, 0x01010101, sum))));
+            if (SUB == 16) {
+                const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+                *(uint4 *)(o + 16 * at) = at & 1 ? zero : v;
+                *(uint4 *)(o + plane + 16 * at) = at & 1 ? v : zero;
+            } else {
+                *(uint4 *)(o + SUB * at + 16 * n) = v;
+            }
         }
+        const int lo = sum & 63;
+        o[256 + at] = (uint8_t)lo;
+        o[288 + at] = (uint8_t)((sum - lo) >> 6);
+        // the rest of the two 32-byte groups is zero
+        constexpr int REST = 32 * SUB / QK_K - 1;  // per thread
+#pragma unroll
+        for (int n = 0; n < REST; ++n) o[256 + QK_K / SUB + REST * at + n] = o[288 + QK_K / SUB + REST * at + n] = 0;
     }
 }
 

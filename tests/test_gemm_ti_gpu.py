@@ -188,3 +188,18 @@ def test_a_rank_without_routes_between_others(ctx):
         none, some = local(4), local(0)
         ctx.synchronize()
         assert not none.any() and torch.equal(some, want)
+
+
+@pytest.mark.parametrize("kind", [KIND_Q4_K, KIND_Q6_K])
+@pytest.mark.parametrize("K", [256 * 33, 256 * 65, 256 * 130])
+def test_staging_of_long_rows(ctx, oracle, kind, K):
+    """Rows whose sub-blocks take less than a turn of the staging's threads, or a turn and a little."""
+    import torch
+
+    T, F = 9, 130
+    rng = np.random.default_rng(K)
+    W = random_blocks(kind, F, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    got = ctx.linear(kind, torch.from_numpy(x).cuda(), ctx.upload(W), F).cpu().numpy()
+    ctx.synchronize()
+    assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= TOL_FP32
