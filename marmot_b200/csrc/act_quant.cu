@@ -180,7 +180,7 @@ __device__ __forceinline__ void stage_group16(const int8_t *q16, float sc, __hal
 }
 
 // Quantise row t (of the staged matrix) block by block, exactly as the kernels above: values to q_s, scales to d_s (shared
-// memory).  False when the row is not this rank's.
+// memory).  False when the row is not this rank's.  (src.x_out may be x: neither is __restrict__.)
 // OP: STAGE_PLAIN = the row as it is; STAGE_NORM = rms_norm(x + add) * w; STAGE_SILU = silu(x) * x2 with the fast exponential and
 // division (relative error about 1e-6: the result is quantised to eight bits right here, three orders of magnitude coarser);
 // STAGE_SILU_RN = the same with the separately rounded exponential and division of the stand-alone kernels; STAGE_GELU.
@@ -191,7 +191,7 @@ enum { STAGE_PLAIN = 0, STAGE_SILU = 1, STAGE_GELU = 2, STAGE_SILU_RN = 3, STAGE
 constexpr int NORM_BATCH = 16;
 
 template <bool KQ, int OP>
-__device__ __forceinline__ bool quantize_row(const float *__restrict__ x, int ldx, const ActSource &src, int K, int nb, int t,
+__device__ __forceinline__ bool quantize_row(const float *x, int ldx, const ActSource &src, int K, int nb, int t,
                                              int8_t *q_s, float *d_s, float *red, float &inv_s) {
     constexpr bool GLU = OP == STAGE_SILU || OP == STAGE_GELU || OP == STAGE_SILU_RN;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
@@ -364,7 +364,7 @@ __device__ __forceinline__ void stage_begin(const ActSource &src) {
 // 4096 values 3.3 us with 256 threads); many rows: 256 threads, and as many rows at a time.
 template <bool KQ, int OP>
 __global__ void __launch_bounds__(1024)
-act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, __half *__restrict__ xh,
+act_half_fused_kernel(const float *x, int ldx, ActSource src, int K, int nb, __half *__restrict__ xh,
                       float *__restrict__ rowscale) {
     extern __shared__ __align__(16) uint8_t act_sm[];
     constexpr int BV = KQ ? QK_K : Q8_0_VALUES;
@@ -411,7 +411,7 @@ act_half_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K
 // zero: the matmul multiplies 32 values at a time and needs the sums of 16).  dT[block][row]: the block scales.
 template <int SUB, int OP>
 __global__ void __launch_bounds__(1024)
-act_int_fused_kernel(const float *__restrict__ x, int ldx, ActSource src, int K, int nb, uint8_t *__restrict__ xq, size_t plane,
+act_int_fused_kernel(const float *x, int ldx, ActSource src, int K, int nb, uint8_t *__restrict__ xq, size_t plane,
                      float *__restrict__ dT, int ld_dT) {
     extern __shared__ __align__(16) uint8_t act_sm[];
     int8_t *q_s = (int8_t *)act_sm;

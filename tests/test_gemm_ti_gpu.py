@@ -203,3 +203,25 @@ def test_staging_of_long_rows(ctx, oracle, kind, K):
     got = ctx.linear(kind, torch.from_numpy(x).cuda(), ctx.upload(W), F).cpu().numpy()
     ctx.synchronize()
     assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= TOL_FP32
+
+
+def test_few_route_moe_leaves_the_glu_in_its_buffer(ctx):
+    """The down staging writes act(gate) * up over the gate rows that it reads: rows of more blocks than a CTA has warps."""
+    T, k, E, H, FF = 20, 2, 2, 256, 256 * 40
+    rng = np.random.default_rng(9)
+    import torch
+
+    kinds = (KIND_Q4_K,) * 3
+    gate, up, down = (ctx.upload(random_blocks(KIND_Q4_K, F, K, rng, d_sigma=0.0005)) for F, K in ((E * FF, H), (E * FF, H), (E * H, FF)))
+    hid = torch.from_numpy(rng.normal(0, 1, (T, H)).astype(np.float32)).cuda()
+    ids = torch.from_numpy(np.tile(np.arange(E, dtype=np.int32), (T, 1))).cuda()  # every token to both experts
+    ctx.moe_experts(kinds, hid, gate, up, down, ids, torch.full((T, k), 0.5, device="cuda"), FF, E)
+    b = ctx.moe_last_buffers(T, k, H, FF)
+    assert not b["grouped"]
+    half = gate.numel() // 2
+    for e in range(E):  # sorted routes: expert by expert, tokens in order
+        # (the calls below do not use the MoE buffers; slices of sixteen tokens take the same kernel)
+        g, u = (torch.cat([ctx.linear(KIND_Q4_K, p, w[e * half:(e + 1) * half], FF) for p in (hid[:10], hid[10:])]) for w in (gate, up))
+        want = g / (1 + torch.exp(-g)) * u
+        assert max_rel_err(b["gate_out"][e * T:(e + 1) * T].cpu().numpy(), want.cpu().numpy()) <= 1e-4
+    ctx.synchronize()
