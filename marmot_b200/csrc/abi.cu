@@ -856,28 +856,31 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
     {
         std::lock_guard<std::mutex> lock(ctx->mu);
         const bool contiguous = ldx == K && (pr.aux_dev == nullptr || pr.ld_aux == K) && (gp.x_out == nullptr || pr.ld_x_out == K);
-        // A handful of tokens on K-quant matrices: the integer tensor-core kernel, one launch per kind, with the prologue in
-        // its activation staging (8 tokens, 2 x 14336 x 4096 Q4_K, add + RMSNorm: 43 us, 36 here).
-        bool integer = integer_jobs_supported(specs, (int)n_jobs, K) && (pr.op == MCU_PROLOGUE_NONE || contiguous);
-        for (size_t j = 0; j < n_jobs && integer; ++j) {
+        // Every kind of the call has its kernel, as mcu_linear would choose it.  A handful of tokens on K-quant matrices: the integer
+        // tensor-core kernel, one launch per kind, with the prologue in its activation staging (8 tokens, 2 x 14336 x 4096 Q4_K, add +
+        // RMSNorm: 43 us, 28.5 here).  More than eight tokens otherwise: the fp16 one; its staging launch (the prologue folded into it)
+        // feeds every matmul that wants the same staging, weights of the other block format class get a second one.
+        const bool folds = pr.op == MCU_PROLOGUE_NONE || contiguous;
+        bool integer[GEMV_MAX_JOBS], all_integer = folds, tensor = folds;  // integer: by job
+        for (size_t j = 0; j < n_jobs && tensor; ++j) {
             size_t values = 0;
             for (size_t i = 0; i < n_jobs; ++i) values += specs[i].kind == specs[j].kind ? K * (size_t)specs[i].F : 0;
-            integer = integer_pays(ctx, specs[j].kind, T, values, true);
+            bool supported = true;  // for all matrices of the kind
+            for (size_t i = 0; i < n_jobs; ++i) supported = supported && (specs[i].kind != specs[j].kind || integer_jobs_supported(&specs[i], 1, K));
+            integer[j] = supported && integer_pays(ctx, specs[j].kind, T, values, true);
+            all_integer = all_integer && integer[j];
+            tensor = integer[j] ||
+                ((ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > (size_t)GEMV_MAX_T &&
+                 gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) && act_half_fused_smem(jobs[j].kind, (int)K) <= 48 * 1024);
         }
-        if (!integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
+        tensor = tensor && (all_integer || T > (size_t)GEMV_MAX_T);
+        if (!tensor && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
             gemv_stream_jobs_supported(specs, (int)n_jobs, (int)T, (int)K, gp)) {
             MCU_CUDA(launch_gemv_stream_jobs(specs, (int)n_jobs, x_dev, (int)ldx, (int)T, (int)K, gp, ctx->dev_err, ctx->stream));
             count_launches(1);
             return MCU_SUCCESS;
         }
-        // More tokens on the tensor cores: one staging launch (the prologue folded into it) feeds every
-        // matmul that wants the same staging; weights of the other block format class get a second one.
-        bool tensor = !integer && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > (size_t)GEMV_MAX_T &&
-            (pr.op == MCU_PROLOGUE_NONE || contiguous);
-        for (size_t j = 0; j < n_jobs && tensor; ++j)
-            tensor = gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) &&
-                act_half_fused_smem(jobs[j].kind, (int)K) <= 48 * 1024;
-        if (tensor || integer) {
+        if (tensor) {
             ActSource src;
             if (pr.op == MCU_PROLOGUE_ADD_RMSNORM) {
                 src.norm = 1;
@@ -910,7 +913,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
                     use.add = nullptr;  // the sum is already in x_out
                     use.x_out = nullptr;
                 }
-                if (integer) {
+                if (integer[j]) {
                     if (int rc = integer_locked(ctx, specs[j].kind, again ? src.x_out : x_dev, ldx, T, K, same, n, &use, &staged_kind)) return rc;
                 } else if (int rc = gemm_locked(ctx, specs[j].kind, again ? src.x_out : x_dev, ldx, T, K, same, n, &use, &st)) return rc;
             }

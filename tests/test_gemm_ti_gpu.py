@@ -225,3 +225,29 @@ def test_few_route_moe_leaves_the_glu_in_its_buffer(ctx):
         want = g / (1 + torch.exp(-g)) * u
         assert max_rel_err(b["gate_out"][e * T:(e + 1) * T].cpu().numpy(), want.cpu().numpy()) <= 1e-4
     ctx.synchronize()
+
+
+@pytest.mark.parametrize("T", [9, 16])
+@pytest.mark.parametrize("prologue", [False, True])
+def test_q8_0_among_k_quants_leaves_them_exact(ctx, oracle, T, prologue):
+    """Nine to sixteen tokens: the K-quant matrices of a call keep their integer dots (32-bit rounding) beside a Q8_0 matrix."""
+    import torch
+    from tests.util import KIND_Q8_0, TOL_MMA
+
+    K, F = 2048, 300
+    rng = np.random.default_rng(T)
+    kinds = (KIND_Q8_0, KIND_Q4_K, KIND_Q6_K, KIND_Q4_K)
+    ws = [random_blocks(k, F, K, rng) for k in kinds]
+    x, aux, w = (rng.normal(0, 1, s).astype(np.float32) for s in ((T, K), (T, K), (K,)))
+    xd, ad, wd = (torch.from_numpy(a).cuda() for a in (x, aux, w))
+    outs, x_out = [torch.zeros((T, F), device="cuda") for _ in kinds], torch.zeros((T, K), device="cuda")
+    ctx.linear_multi(xd, [(k, ctx.upload(m), F, o) for k, m, o in zip(kinds, ws, outs)],
+                     ("add_rmsnorm", ad, wd, 1e-5, 0.0, x_out) if prologue else None)
+    ctx.synchronize()
+    if prologue:
+        assert torch.equal(x_out, xd + ad)
+        h = torch.empty_like(xd)
+        ctx.add_rmsnorm(xd, ad, wd, 1e-5, torch.empty_like(xd), h)  # the same operations in the same order
+        x = h.cpu().numpy()
+    for k, m, o in zip(kinds, ws, outs):
+        assert max_rel_err(o.cpu().numpy(), oracle.linear(k, x, m, F)) <= (TOL_MMA if k == KIND_Q8_0 else 2e-5)
