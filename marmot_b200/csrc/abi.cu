@@ -588,7 +588,7 @@ static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t valu
 }
 static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K) {
     for (int j = 0; j < n_jobs; ++j)
-        if (!gemm_ti_supported(jobs[j].kind, jobs[j].W, (int)K, jobs[j].F) || act_half_fused_smem(jobs[j].kind, (int)K) > 48 * 1024) return false;
+        if (!gemm_ti_supported(jobs[j].kind, jobs[j].W, (int)K, jobs[j].F) || act_half_fused_smem(jobs[j].kind, (int)K) > ACT_INT_MAX_SMEM) return false;
     return true;
 }
 static int integer_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, const GemvJobSpec *jobs, int n_jobs,

@@ -509,9 +509,12 @@ cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSou
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const size_t plane = (size_t)rows * nb * 384;
-#define MCU_STAGE(OP) \
-    (kind == KIND_Q6_K ? cudaLaunchKernelEx(&cfg, act_int_fused_kernel<16, OP>, x, ldx, src, K, nb, xq, plane, dT, rows) \
-                       : cudaLaunchKernelEx(&cfg, act_int_fused_kernel<32, OP>, x, ldx, src, K, nb, xq, plane, dT, rows))
+    auto launch = [&](auto kernel) {
+        if (cfg.dynamicSmemBytes > 48 * 1024)  // (rows of more than 48,000 values)
+            if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ACT_INT_MAX_SMEM)) return e;
+        return cudaLaunchKernelEx(&cfg, kernel, x, ldx, src, K, nb, xq, plane, dT, rows);
+    };
+#define MCU_STAGE(OP) (kind == KIND_Q6_K ? launch(act_int_fused_kernel<16, OP>) : launch(act_int_fused_kernel<32, OP>))
     switch (stage_op(src)) {
     case STAGE_SILU:
     case STAGE_SILU_RN: return MCU_STAGE(STAGE_SILU_RN);

@@ -551,7 +551,7 @@ static int ti_planes(int kind) { return kind == KIND_Q6_K ? 2 : 1; }
 size_t gemm_ti_xq_bytes(int kind, int rows, int K) { return (size_t)ti_planes(kind) * rows * ((K + QK_K - 1) / QK_K) * 384; }
 
 bool gemm_ti_supported(int kind, const void *W, int K, int F) {
-    return (kind == KIND_Q4_K || kind == KIND_Q6_K) && K <= TI_MAX_K && gemm_ts_supported(kind, W, 1, K, F);
+    return (kind == KIND_Q4_K || kind == KIND_Q6_K) && gemm_ts_supported(kind, W, 1, K, F);
 }
 
 template <int KIND, bool EARLY>

@@ -26,7 +26,6 @@ cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
 
 // The same on integers for a handful of tokens (gemm_ti.cu: Q4_K, Q6_K): exact sub-block dots.  xq / dT from
 // launch_act_int_fused.  The grouped form takes the groups with a count up to count_hi.
-constexpr int TI_MAX_K = 65536;
 size_t gemm_ti_xq_bytes(int kind, int rows, int K);
 bool gemm_ti_supported(int kind, const void *W, int K, int F);
 cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const uint8_t *xq, const float *dT, int T, int K,

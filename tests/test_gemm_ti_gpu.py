@@ -251,3 +251,17 @@ def test_q8_0_among_k_quants_leaves_them_exact(ctx, oracle, T, prologue):
         x = h.cpu().numpy()
     for k, m, o in zip(kinds, ws, outs):
         assert max_rel_err(o.cpu().numpy(), oracle.linear(k, x, m, F)) <= (TOL_MMA if k == KIND_Q8_0 else 2e-5)
+
+
+@pytest.mark.parametrize("kind,T,K", [(KIND_Q4_K, 9, 53248), (KIND_Q6_K, 12, 50176), (KIND_Q4_K, 10, 131072)])
+def test_rows_longer_than_the_static_shared_memory(ctx, oracle, kind, T, K):
+    """More than 48,000 values to a row: still integer dots, so 32-bit rounding."""
+    import torch
+
+    F = 40
+    rng = np.random.default_rng(K)
+    W = random_blocks(kind, F, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    got = ctx.linear(kind, torch.from_numpy(x).cuda(), ctx.upload(W), F).cpu().numpy()
+    ctx.synchronize()
+    assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= 5e-5
