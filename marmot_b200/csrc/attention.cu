@@ -101,6 +101,20 @@ __device__ __forceinline__ void at_zero_rows(const AtRows<HD> &rows, uint32_t ti
     }
 }
 
+// Does a V tile hold an infinity or a NaN?  (Rows without data are zero by now.)
+template <int HD>
+__device__ __forceinline__ bool at_not_finite(uint32_t tile, int lane) {
+    uint32_t bad = 0;
+#pragma unroll 4
+    for (int i = lane; i < At<HD>::TILE / 16; i += 32) {
+        uint32_t w[4];
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(tile + 16u * (uint32_t)i) : "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bad |= __vcmpeq2(w[j] & 0x7C007C00u, 0x7C007C00u);  // all bits of the exponent
+    }
+    return __any_sync(0xffffffffu, bad != 0);
+}
+
 // A fragments of Q into this lane's part of `qf`: row g of A (of this lane) is `qrow` (null: zeros), rotated when there is a table.
 // a0 = dimensions 16 s + 2 tq, + 1; a2 = dimensions 16 s + 8 + 2 tq, + 1.
 template <int HD>
@@ -491,7 +505,7 @@ attention_prompt_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, in
     using A = At<HD>;
     extern __shared__ uint8_t at_smem[];
     __shared__ __align__(8) uint64_t bars[AT_WARPS];
-    __shared__ uint32_t tile_live[AT_WARPS], s_seq[AT_BLOCK], s_pos[AT_BLOCK];
+    __shared__ uint32_t tile_live[AT_WARPS], tile_odd[AT_WARPS], s_seq[AT_BLOCK], s_pos[AT_BLOCK];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
     const uint32_t raw = tm_smem_u32(at_smem), base = (raw + 1023u) & ~1023u;  // K tiles 0..3, V tiles 0..3
     uint4 *qf = (uint4 *)(at_smem + (base - raw) + 8 * A::TILE + warp * A::Q_BYTES);
@@ -531,37 +545,56 @@ attention_prompt_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, in
             if (warp >= 4 && live != 0xffffffffu) {
                 at_zero_rows<HD>(rows, tile, live, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
             }
+            const bool odd = warp >= 4 && live != 0u && ok && at_not_finite<HD>(tile, lane);
+            if (lane == 0) tile_odd[warp] = odd;
         }
         if (__syncthreads_or(!ok)) break;
-        for (int sub = warp * per_pass; sub < n; sub += AT_WARPS * per_pass) {
-            // row g of A: query head g % gsize of token g / gsize of the pass
-            const int tok = g / gsize, last = min(sub + per_pass, n);  // of the pass
-            const bool row_ok = tok < per_pass && sub + tok < n;
-            const int t = t_lo + first + sub + (row_ok ? tok : 0);
-            const uint32_t row_len = s_pos[t - t_lo] + 1u, most = pos + (uint32_t)last;  // context of the row's token; the longest
-            if (most <= p0) continue;
-            const size_t row = (size_t)t * p.n_q_heads + (size_t)h * gsize + (row_ok ? g - tok * gsize : 0);
-            at_load_q<HD>(row_ok ? p.q + row * HD : nullptr, nullptr, 0, p.scale, qf, lane);
-            AtTiles tiles;
-            float M, L;
+        // A token's probabilities are zero beyond its own context, but the V rows there, of later tokens, are in the tiles: where one
+        // is not finite, zero times it would be NaN.  Then the tokens are taken one by one, the last first, and a token's V row is
+        // cleared behind it.
+        const bool one_by_one = (tile_odd[4] | tile_odd[5] | tile_odd[6] | tile_odd[7]) && n > 1 && pos < p0 + PM_CHUNK;
+        for (int hi = n, lo; hi > 0; hi = lo) {
+            lo = one_by_one ? hi - 1 : 0;
+            for (int sub = lo + warp * per_pass; sub < hi; sub += AT_WARPS * per_pass) {
+                // row g of A: query head g % gsize of token g / gsize of the pass
+                const int tok = g / gsize, last = min(sub + per_pass, hi);  // of the pass
+                const bool row_ok = tok < per_pass && sub + tok < hi;
+                const int t = t_lo + first + sub + (row_ok ? tok : 0);
+                const uint32_t row_len = s_pos[t - t_lo] + 1u, most = pos + (uint32_t)last;  // context of the row's token; the longest
+                if (most <= p0) continue;
+                const size_t row = (size_t)t * p.n_q_heads + (size_t)h * gsize + (row_ok ? g - tok * gsize : 0);
+                at_load_q<HD>(row_ok ? p.q + row * HD : nullptr, nullptr, 0, p.scale, qf, lane);
+                AtTiles tiles;
+                float M, L;
 #pragma unroll 1
-            for (int w = 0; w < 4; ++w) {
-                const uint32_t k0 = p0 + (uint32_t)w * PM_TILE;
-                tiles.push();
-                if (k0 >= most) continue;
-                const uint32_t row_live = row_len <= k0 ? 0u : tile_live[w] & (row_len - k0 >= 32u ? 0xffffffffu : (1u << (row_len - k0)) - 1u);
-                at_scores<HD>(rows, base + (uint32_t)(w * A::TILE), qf, row_live, lane, tiles.phi[0], tiles.plo[0], tiles.m[0], tiles.l[0]);
-            }
-            tiles.weigh(M, L);
-            float acc[A::NT][2];
+                for (int w = 0; w < 4; ++w) {
+                    const uint32_t k0 = p0 + (uint32_t)w * PM_TILE;
+                    tiles.push();
+                    if (k0 >= most) continue;
+                    const uint32_t row_live = row_len <= k0 ? 0u : tile_live[w] & (row_len - k0 >= 32u ? 0xffffffffu : (1u << (row_len - k0)) - 1u);
+                    at_scores<HD>(rows, base + (uint32_t)(w * A::TILE), qf, row_live, lane, tiles.phi[0], tiles.plo[0], tiles.m[0], tiles.l[0]);
+                }
+                tiles.weigh(M, L);
+                float acc[A::NT][2];
 #pragma unroll
-            for (int k = 0; k < A::NT; ++k) acc[k][0] = acc[k][1] = 0.0f;
+                for (int k = 0; k < A::NT; ++k) acc[k][0] = acc[k][1] = 0.0f;
 #pragma unroll 1
-            for (int w = 0; w < 4 && p0 + (uint32_t)w * PM_TILE < most; ++w, tiles.shift())
-                at_pv<HD>(rows, base + (uint32_t)((4 + w) * A::TILE), tiles.phi[3], tiles.plo[3], tiles.l[3], lane, acc);
-            if (row_ok && row_len > p0)
-                at_store<HD>(p, partial, n_chunks, row, c, row_len <= (uint32_t)PM_CHUNK || n_chunks == 1, M, L, tq, acc);
+                for (int w = 0; w < 4 && p0 + (uint32_t)w * PM_TILE < most; ++w, tiles.shift())
+                    at_pv<HD>(rows, base + (uint32_t)((4 + w) * A::TILE), tiles.phi[3], tiles.plo[3], tiles.l[3], lane, acc);
+                if (row_ok && row_len > p0)
+                    at_store<HD>(p, partial, n_chunks, row, c, row_len <= (uint32_t)PM_CHUNK || n_chunks == 1, M, L, tq, acc);
+            }
+            if (one_by_one && lo > 0) {
+                __syncthreads();
+                const uint32_t own = pos + (uint32_t)lo - p0;  // position of token lo, in the chunk
+                if (pos + (uint32_t)lo >= p0 && own < PM_CHUNK && warp == 4 + (int)(own / PM_TILE)) {
+                    at_zero_rows<HD>(rows, base + (uint32_t)(warp * A::TILE), ~(1u << (own % PM_TILE)), lane);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                __syncthreads();
+            }
         }
     }
     if (!ok) {

@@ -82,3 +82,42 @@ def test_decode_blocks_equal_three_steps(n_seq, hd, bs):
     ctx.synchronize()
     assert torch.equal(k1, k2) and torch.equal(v1, v2) and torch.equal(got, want)
     ctx.close()
+
+
+@pytest.mark.parametrize("hq,hkv,hd,bs", [(8, 2, 128, 16), (8, 8, 64, 16), (16, 2, 64, 32)])
+@pytest.mark.parametrize("lengths", [(1,), (20,), (1, 7, 33, 2)])
+def test_values_that_are_not_finite_stay_with_the_tokens_that_see_them(hq, hkv, hd, bs, lengths):
+    """Many sequences, runs of the given lengths whose last V rows overflow f16 or are NaN: the tokens ahead of them, which share
+    their CTAs, equal single-token calls bit for bit, as do the last ones."""
+    import torch
+    from marmot_b200 import Context
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ctx = Context(0)
+    rng = np.random.default_rng(hq + len(lengths))
+    n_seq = 400 // sum(lengths) * len(lengths)
+    spans = [(int(rng.integers(0, 300)), lengths[i % len(lengths)]) for i in range(n_seq)]
+    max_blocks = max(a + n for a, n in spans) // bs + 1
+    table = rng.permutation(max_blocks * n_seq).reshape(n_seq, max_blocks).astype(np.uint32)
+    meta = np.array([(s, pos, int(table[s, pos // bs]) * bs + pos % bs, 0) for s, (a, n) in enumerate(spans) for pos in range(a, a + n)],
+                    dtype=np.uint32)
+    T = len(meta)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    randn = lambda *shape: torch.from_numpy(rng.normal(0, 1, shape).astype(np.float32)).cuda()
+    pool_k, pool_v = randn(max_blocks * n_seq, 1, hkv, bs, hd).half(), randn(max_blocks * n_seq, 1, hkv, bs, hd).half()
+    q, k, v = randn(T, hq * hd), randn(T, hkv * hd), randn(T, hkv * hd)
+    last = np.cumsum([n for _, n in spans]) - 1
+    v[last[::2], 5] = 1e6
+    v[last[1::2], hkv * hd - 1] = float("nan")
+    tab, m = dev(table), dev(meta)
+    k1, v1, k2, v2 = pool_k.clone(), pool_v.clone(), pool_k.clone(), pool_v.clone()
+    got = ctx.paged_attention(m, q, k, v, k1, v1, tab, 0, hq, hkv, hd, bs, hd ** -0.5)
+    one = torch.cat([ctx.paged_attention(m[i:i + 1].clone(), q[i:i + 1].clone(), k[i:i + 1].clone(), v[i:i + 1].clone(), k2, v2, tab, 0, hq, hkv, hd,
+                                         bs, hd ** -0.5) for i in range(T)])
+    ctx.synchronize()
+    others = torch.ones(T, dtype=torch.bool)
+    others[last] = False
+    assert torch.isfinite(got[others.cuda()]).all()
+    assert torch.equal(got.nan_to_num(7.0, 8.0, 9.0), one.nan_to_num(7.0, 8.0, 9.0))
+    ctx.close()
