@@ -130,7 +130,10 @@ struct TsPlan {
 // - One tile per CTA, in as many waves as it takes: 2000 for a CTA's start.
 // - A tile over a cluster: the exchange of the shares through the CTAs' shared memories.
 // - Equal ranges of slabs: cut tiles have their shares written to memory, and read again by the CTA that comes last; a tile of 256
-//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).
+//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).  The way
+//   through memory and the tickets costs 6000 besides, 11000 in narrow tiles, by all forms at 9 to 2048 tokens and thirteen sizes
+//   (9 x 2048 x 5632 Q8_0: 19.1 us in ranges, 10.2 in clusters of two; 17 x 2048 x 32000 Q4_K: 25.1, 20.7 in waves; 2048 x 14336 x 4096
+//   Q4_K: 261, 226 in waves; 512 x 4096 x 28672 Q4_K: 119 in ranges, 137 in waves).
 inline TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles, int room) {
     const long U = (long)tiles * KS;
     const bool wide = bn > 64;
@@ -152,7 +155,8 @@ inline TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles, int ro
     const long upc = (U + n - 1) / n;
     const bool cut = U % n != 0 || upc % KS != 0;
     const double shares = cut ? (double)KS / upc + 1.0 : 0.0;
-    consider(1, n, upc * unit + ((double)upc / KS + 1.0) * tile_end + 2000.0 + shares * 65.0 * bn);
+    const double exchange = shares * 65.0 * bn + (!cut ? 0.0 : wide ? 6000.0 : 11000.0);
+    consider(1, n, upc * unit + ((double)upc / KS + 1.0) * tile_end + 2000.0 + exchange);
     return best;
 }
 
