@@ -84,3 +84,21 @@ def test_many_tokens_equal_calls_on_slices(ctx, name, T):
     ref = torch.cat([ctx.linear(kind, part, w, F) for part in x.split(500)])
     ctx.synchronize()
     assert max_rel_err(got.cpu().numpy(), ref.cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("T,K,F", [(20, 1024, 130), (70, 3072, 64), (150, 5632, 200)])
+def test_q6_k_rows_off_16_bytes_round_their_weights_once(ctx, T, K, F):
+    """Integer activations with a largest value of 127 are exact operands, so the result is that of the weights rounded to fp16, up to the
+    order of 32-bit sums.  (Rounded twice, by way of the scale, it is 2e-4 off.)"""
+    import torch
+    from marmot_b200.synthetic import normal_blocks
+
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K)
+    w = normal_blocks(torch, KIND_Q6_K, F, K, torch.device("cuda"), gen).reshape(-1)
+    x = torch.randint(-126, 127, (T, K), device="cuda", generator=gen).float()
+    x[:, ::256] = 127.0
+    got = ctx.linear(KIND_Q6_K, x, w, F)
+    want = x.double() @ ctx.dequantize(KIND_Q6_K, w, F * K).view(F, K).half().double().T
+    ctx.synchronize()
+    assert max_rel_err(got.cpu().numpy(), want.cpu().numpy()) <= 1e-5
