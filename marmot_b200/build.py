@@ -39,8 +39,9 @@ def build_binding(force: bool = False) -> Path:
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
 
-    src = CSRC / "binding.cpp"
-    if not force and BINDING.exists() and BINDING.stat().st_mtime >= src.stat().st_mtime:
+    src, stamp = CSRC / "binding.cpp", OBJ_DIR / "binding.stamp"
+    built_for = f"{torch.__version__} {torch.__file__} {sys.version}"
+    if not force and BINDING.exists() and BINDING.stat().st_mtime >= src.stat().st_mtime and stamp.exists() and stamp.read_text() == built_for:
         return BINDING
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
     cmd += [f"-I{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], str(Path(_nvcc()).resolve().parent.parent / "include"))]
@@ -48,6 +49,8 @@ def build_binding(force: bool = False) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {src}\n{r.stderr}")
+    OBJ_DIR.mkdir(exist_ok=True)
+    stamp.write_text(built_for)
     return BINDING
 
 

@@ -198,7 +198,8 @@ _binding = None
 
 
 def load_binding():
-    """The native form of Context.linear (csrc/binding.cpp), or False where it has not been built: the same call through ctypes."""
+    """The native form of Context.linear (csrc/binding.cpp), or False where it has not been built, or for another torch than this
+    one: the same call through ctypes."""
     global _binding
     if _binding is None:
         path = LIB_PATH.with_name("_binding.so")
@@ -207,13 +208,17 @@ def load_binding():
             import importlib.machinery
             import importlib.util
 
-            import torch  # noqa: F401  (the module links against its libraries)
+            import torch  # (the module links against its libraries)
 
             loader = importlib.machinery.ExtensionFileLoader("_binding", str(path))
-            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_binding", loader))
-            loader.exec_module(module)
-            module.set_entry_points(C.cast(load_library().mcu_linear, C.c_void_p).value)
-            _binding = module
+            try:
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_binding", loader))
+                loader.exec_module(module)
+            except (ImportError, OSError):
+                return _binding
+            if torch.__version__.startswith(module.torch_version):
+                module.set_entry_points(C.cast(load_library().mcu_linear, C.c_void_p).value)
+                _binding = module
     return _binding
 
 

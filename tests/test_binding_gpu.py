@@ -39,3 +39,22 @@ def test_native_call_equals_ctypes(kind, T, K, F):
         c.close()
         with pytest.raises(MarmotCudaError):
             c.linear(kind, x, w, F)
+
+
+def test_errors_are_those_of_the_ctypes_call():
+    """Out of memory and sizes beyond the library's limits come as the same exceptions."""
+    import torch
+    from marmot_b200 import Context
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ctx, plain = Context(0), Context(0)
+    plain._linear = None
+    rows = 1 << 20
+    w, x = torch.zeros(rows * 34, dtype=torch.uint8, device="cuda"), torch.zeros((rows, 32), device="cuda")
+    for c in (ctx, plain):
+        with pytest.raises(torch.OutOfMemoryError):
+            c.linear(KIND_Q8_0, x, w, rows)  # a result of four terabytes
+        with pytest.raises(AssertionError):
+            c.linear(KIND_Q8_0, x[:1], w, 1 << 62, out=torch.zeros((1, 4), device="cuda"))  # rows x bytes overflows 64 bits
+        c.close()
