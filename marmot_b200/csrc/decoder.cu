@@ -50,37 +50,38 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, c
 
 // ---------------------------------------------------------------- RMSNorm
 // One CTA per row.  The latency of its loads bounds it (64 or 500 rows of 4096: 15.5 us with one load at a time, 5 with all
-// loads of a row issued together), so a thread takes sixteen elements, 256 apart, per turn: all loads, then the operations.  Rows
-// of up to 4096 values stay in registers between the two passes.
-constexpr int NORM_BATCH = 16;
+// loads of a row issued together), so a thread takes up to sixteen elements (B), 256 apart, per turn: all loads, then the operations.
+// Rows of up to 4096 values stay in registers between the two passes.  Short rows take as few as they fill: many of them are bound by
+// instructions (2048 rows of 100: 5.5 us with sixteen, 3.0 with one; of 1024: 7.0 and 5.8 with four).
 
 // v = x + add for this thread's elements from i0 on (add may be null)
-__device__ __forceinline__ void norm_load(const float *x, const float *add, int i0, int n, float (&v)[NORM_BATCH]) {
+template <int B>
+__device__ __forceinline__ void norm_load(const float *x, const float *add, int i0, int n, float (&v)[B]) {
 #pragma unroll
-    for (int j = 0; j < NORM_BATCH; ++j) v[j] = i0 + 256 * j < n ? x[i0 + 256 * j] : 0.0f;
+    for (int j = 0; j < B; ++j) v[j] = i0 + 256 * j < n ? x[i0 + 256 * j] : 0.0f;
     if (add != nullptr) {
-        float a[NORM_BATCH];
+        float a[B];
 #pragma unroll
-        for (int j = 0; j < NORM_BATCH; ++j) a[j] = i0 + 256 * j < n ? add[i0 + 256 * j] : 0.0f;
+        for (int j = 0; j < B; ++j) a[j] = i0 + 256 * j < n ? add[i0 + 256 * j] : 0.0f;
 #pragma unroll
-        for (int j = 0; j < NORM_BATCH; ++j) v[j] = __fadd_rn(v[j], a[j]);
+        for (int j = 0; j < B; ++j) v[j] = __fadd_rn(v[j], a[j]);
     }
 }
 // STORE_SUM: x_out = x + add goes to memory too, and the second pass of a longer row reads it back (a thread's own elements)
-template <bool STORE_SUM>
+template <bool STORE_SUM, int B>
 __device__ __forceinline__ void norm_row(const float *x, const float *add, const float *__restrict__ weight, int n, float eps,
                                          float weight_offset, float *x_out, float *__restrict__ h_out) {
     __shared__ float red[8];
     __shared__ float inv_s;
-    float v[NORM_BATCH];
+    float v[B];
     float sum = 0.0f;
-    for (int i0 = threadIdx.x; i0 < n; i0 += 256 * NORM_BATCH) {
-        norm_load(x, add, i0, n, v);
+    for (int i0 = threadIdx.x; i0 < n; i0 += 256 * B) {
+        norm_load<B>(x, add, i0, n, v);
 #pragma unroll
-        for (int j = 0; j < NORM_BATCH; ++j) sum += v[j] * v[j];
+        for (int j = 0; j < B; ++j) sum += v[j] * v[j];
         if (STORE_SUM) {
 #pragma unroll
-            for (int j = 0; j < NORM_BATCH; ++j)
+            for (int j = 0; j < B; ++j)
                 if (i0 + 256 * j < n) x_out[i0 + 256 * j] = v[j];
         }
     }
@@ -95,15 +96,15 @@ __device__ __forceinline__ void norm_row(const float *x, const float *add, const
     }
     __syncthreads();
     const float inv = inv_s;
-    for (int i0 = threadIdx.x; i0 < n; i0 += 256 * NORM_BATCH) {
-        if (n > 256 * NORM_BATCH) norm_load(STORE_SUM ? x_out : x, STORE_SUM ? nullptr : add, i0, n, v);
-        float w[NORM_BATCH];
+    for (int i0 = threadIdx.x; i0 < n; i0 += 256 * B) {
+        if (n > 256 * B) norm_load<B>(STORE_SUM ? x_out : x, STORE_SUM ? nullptr : add, i0, n, v);
+        float w[B];
         if (weight != nullptr) {
 #pragma unroll
-            for (int j = 0; j < NORM_BATCH; ++j) w[j] = i0 + 256 * j < n ? weight[i0 + 256 * j] : 0.0f;
+            for (int j = 0; j < B; ++j) w[j] = i0 + 256 * j < n ? weight[i0 + 256 * j] : 0.0f;
         }
 #pragma unroll
-        for (int j = 0; j < NORM_BATCH; ++j) {
+        for (int j = 0; j < B; ++j) {
             if (i0 + 256 * j >= n) continue;
             float y = __fmul_rn(v[j], inv);
             if (weight != nullptr) y = __fmul_rn(y, __fadd_rn(w[j], weight_offset));
@@ -112,22 +113,24 @@ __device__ __forceinline__ void norm_row(const float *x, const float *add, const
     }
 }
 
+template <int B>
 __global__ void __launch_bounds__(256)
 rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ residual, const float *__restrict__ weight, int n,
                float eps, float weight_offset, float *__restrict__ out) {
     MCU_PDL_PROLOGUE();
     const size_t row = (size_t)blockIdx.x * n;
-    norm_row<false>(x + row, residual != nullptr ? residual + row : nullptr, weight, n, eps, weight_offset, nullptr, out + row);
+    norm_row<false, B>(x + row, residual != nullptr ? residual + row : nullptr, weight, n, eps, weight_offset, nullptr, out + row);
 }
 
 // x_out = x + delta (the residual update), h_out = RMSNorm(x_out) * weight: the add and the rms_norm that follow every
 // row-parallel projection, in one pass over the row.  x_out may alias x.
+template <int B>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_kernel(const float *x, const float *__restrict__ delta, const float *__restrict__ weight, int n, float eps,
                    float weight_offset, float *x_out, float *__restrict__ h_out) {
     MCU_PDL_PROLOGUE();
     const size_t row = (size_t)blockIdx.x * n;
-    norm_row<true>(x + row, delta + row, weight, n, eps, weight_offset, x_out + row, h_out + row);
+    norm_row<true, B>(x + row, delta + row, weight, n, eps, weight_offset, x_out + row, h_out + row);
 }
 
 // ---------------------------------------------------------------- RoPE
@@ -211,7 +214,8 @@ __global__ void rope_table_kernel(const int32_t *__restrict__ positions, int hal
 }
 
 // ---------------------------------------------------------------- elementwise
-// Four values per thread where the rows allow it.
+// Four values per thread where the alignment allows it and there are enough of them to fill the SMs so (57344 values: 1.6 us, 1.35 with one
+// value per thread; 262144: 1.5 and 1.6; 2 million 5.5 and 9).
 __device__ __forceinline__ float swiglu_one(float a, float b) { return __fmul_rn(__fdiv_rn(a, __fadd_rn(1.0f, expf(-a))), b); }
 __global__ void swiglu_kernel(const float *a, const float *b, size_t n, float *out) {
     MCU_PDL_PROLOGUE();
@@ -932,7 +936,8 @@ int mcu_rmsnorm(mcu_context_t *ctx, const float *x_dev, const float *residual_de
     if (rows == 0 || n == 0) return MCU_SUCCESS;
     if (x_dev == nullptr || out_dev == nullptr) return set_error(MCU_ERROR_INVALID_ARGUMENT, "null tensor data");
     if (n > (size_t)1 << 30 || rows > (size_t)1 << 30) return set_error(MCU_ERROR_INVALID_ARGUMENT, "dimension too large");
-    DEC_CUDA(launch_pdl(rmsnorm_kernel, dim3((unsigned)rows), dim3(256), s, x_dev, residual_dev, weight_dev, (int)n, eps,
+    auto kernel = n <= 256 ? rmsnorm_kernel<1> : n <= 1024 ? rmsnorm_kernel<4> : n <= 2048 ? rmsnorm_kernel<8> : rmsnorm_kernel<16>;
+    DEC_CUDA(launch_pdl(kernel, dim3((unsigned)rows), dim3(256), s, x_dev, residual_dev, weight_dev, (int)n, eps,
                         weight_offset, out_dev));
     count_launches(1);
     return MCU_SUCCESS;
@@ -968,7 +973,8 @@ int mcu_add_rmsnorm(mcu_context_t *ctx, const float *x_dev, const float *delta_d
     if (x_dev == nullptr || delta_dev == nullptr || x_out_dev == nullptr || h_out_dev == nullptr)
         return set_error(MCU_ERROR_INVALID_ARGUMENT, "null tensor data");
     if (n > (size_t)1 << 30 || rows > (size_t)1 << 30) return set_error(MCU_ERROR_INVALID_ARGUMENT, "dimension too large");
-    DEC_CUDA(launch_pdl(add_rmsnorm_kernel, dim3((unsigned)rows), dim3(256), s, x_dev, delta_dev, weight_dev, (int)n, eps,
+    auto kernel = n <= 256 ? add_rmsnorm_kernel<1> : n <= 1024 ? add_rmsnorm_kernel<4> : n <= 2048 ? add_rmsnorm_kernel<8> : add_rmsnorm_kernel<16>;
+    DEC_CUDA(launch_pdl(kernel, dim3((unsigned)rows), dim3(256), s, x_dev, delta_dev, weight_dev, (int)n, eps,
                         weight_offset, x_out_dev, h_out_dev));
     count_launches(1);
     return MCU_SUCCESS;
@@ -1001,7 +1007,7 @@ int mcu_swiglu(mcu_context_t *ctx, const float *gate_dev, const float *up_dev, s
     if (n == 0) return MCU_SUCCESS;
     if (gate_dev == nullptr || up_dev == nullptr || out_dev == nullptr)
         return set_error(MCU_ERROR_INVALID_ARGUMENT, "null tensor data");
-    if (n % 4 == 0 && (((uintptr_t)gate_dev | (uintptr_t)up_dev | (uintptr_t)out_dev) & 15u) == 0)
+    if (n >= (size_t)3 << 16 && n % 4 == 0 && (((uintptr_t)gate_dev | (uintptr_t)up_dev | (uintptr_t)out_dev) & 15u) == 0)
         DEC_CUDA(launch_pdl(swiglu4_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), s, (const float4 *)gate_dev,
                             (const float4 *)up_dev, n / 4, (float4 *)out_dev));
     else
