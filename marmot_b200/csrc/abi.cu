@@ -85,6 +85,7 @@ struct mcu_context {
     Buffer rope_table;              // {cos, sin} per token and pair when a decode attention call brings none
     Buffer attn_tickets;            // fused decode attention: one counter per (token, KV head)
     Buffer pro_h;                   // activations after a stand-alone prologue kernel (mcu_linear_multi's general form)
+    Buffer i8_partial, i8_tickets;  // mma.sync integer matmul: shares of row groups split between CTAs, and their tickets
     Buffer attn_partial;         // split-KV partial attention states
     int *gemm_counters = nullptr;  // split-K tile tickets (zero between launches)
     std::vector<int> host_counts;
@@ -134,6 +135,7 @@ static int ensure(mcu_context *ctx, Buffer &b, size_t bytes) {
 static int report_flag(mcu_context *ctx, cudaStream_t s, int flag) {
     MCU_CUDA(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), s));
     MCU_CUDA(cudaMemsetAsync(ctx->gemm_counters, 0, GEMM_TMA_MAX_TILE_COUNTERS * sizeof(int), s));  // (whatever the flag: the last report wins)
+    if (ctx->i8_tickets.ptr != nullptr) MCU_CUDA(cudaMemsetAsync(ctx->i8_tickets.ptr, 0, ctx->i8_tickets.cap, s));
     if (flag == 40) return fail(MCU_ERROR_INVALID_ARGUMENT, "MoE expert id is out of range (found by an earlier call)");
     return fail(MCU_ERROR_INVALID_OPERATION, "a device-side wait timed out (code %d)", flag);
 }
@@ -266,7 +268,7 @@ void mcu_context_destroy(mcu_context_t *ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     Buffer *bufs[] = {&ctx->act_qs,   &ctx->act_d,      &ctx->act_bsums, &ctx->act_half, &ctx->act_rowscale, &ctx->x_stage, &ctx->out_stage,
-                      &ctx->bias_stage, &ctx->moe_meta, &ctx->moe_hidden, &ctx->moe_gate, &ctx->moe_up, &ctx->moe_down, &ctx->gemm_partial, &ctx->attn_partial, &ctx->pro_h, &ctx->attn_tickets, &ctx->rope_table};
+                      &ctx->bias_stage, &ctx->moe_meta, &ctx->moe_hidden, &ctx->moe_gate, &ctx->moe_up, &ctx->moe_down, &ctx->gemm_partial, &ctx->attn_partial, &ctx->i8_partial, &ctx->i8_tickets, &ctx->pro_h, &ctx->attn_tickets, &ctx->rope_table};
     for (Buffer *b : bufs)
         if (b->ptr != nullptr) cudaFree(b->ptr);
     if (ctx->dev_err != nullptr) cudaFree(ctx->dev_err);
@@ -577,16 +579,39 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
 //   Q6_K  4 tokens  4096 x 4096 11.0, 11.7; 14336 x 4096 33.3, 23.6; 4096 x 28672 39.7, 44.7
 //         5 tokens  1024 x 1024 4.2, 7.0; 2048 x 2048 7.9, 8.0; 4096 x 1024 8.8, 8.6; 4096 x 4096 13.5, 11.7
 // From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
+// Small matrices of long rows are a chain for the dp4a kernel's warps, short rows leave little to chain: a line of tokens x K, or of
+// tokens x rows, for those (8 tokens: 3072 x 125 Q4_K 9.5, 7.0; 2048 x 256 7.8, 6.9; 1024 x 1024 5.6, 4.9 with gemm_i8; 1024 x 512 5.0, 4.8).
 // And from three tokens on where the rows cannot be streamed (Q6_K of ragged sizes), against the plain-load kernel: 3072 x 125 3, 4,
 // 8 tokens 13.5, 16.6, 21.2 us, 7.5, 7.7, 7.8 here; 1280 x 300 7.5, 9.1, 12.5, then 7.6 to 7.7.
-static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t values, bool streams) {
+static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, size_t values, bool streams) {
     static const bool off = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch
     if (off || ctx->regime != MCU_REGIME_AUTO || T > (size_t)TI_COLS) return false;
     if (T > (size_t)GEMV_MAX_T || (T >= 3 && !streams)) return true;
-    if (T >= 5) return values >= (size_t)4 << 20;
+    if (T >= 5) return values >= (size_t)4 << 20 || T * K >= 16384 || (kind == KIND_Q4_K && K <= 1024 && T * values >= 8192 * K);
     return kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20;
 }
 static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K) {
+// The integer matmul by mma.sync, for the sizes where it is the faster one.
+static bool i8_takes(const mcu_context *ctx, int kind, const void *w, const void *w2, size_t T, size_t K, size_t F) {
+    return ctx->regime == MCU_REGIME_AUTO && T >= 5 && T <= (size_t)I8_MAX_T && gemm_i8_supported(kind, w, w2, (int)T, (int)K, (int)F) &&
+        i8_pays(kind, (int)T, (int)K, (int)F, w2 != nullptr ? 2 : 1, device_sm_count());
+}
+static int i8_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, const void *w, const void *w2, size_t T, size_t K, size_t F,
+                     const float *bias, float *out, float *out2, size_t ldo) {
+    size_t qs_b, dT_b, part_b, tick_b;
+    gemm_i8_workspace_bytes((int)T, (int)K, (int)F, w2 != nullptr, &qs_b, &dT_b, &part_b, &tick_b);
+    if (int rc = ensure(ctx, ctx->act_qs, qs_b)) return rc;
+    if (int rc = ensure(ctx, ctx->act_d, dT_b)) return rc;
+    if (int rc = ensure(ctx, ctx->i8_partial, part_b)) return rc;
+    if (tick_b > ctx->i8_tickets.cap) {  // a fresh ticket area starts at zero; the kernel keeps it so
+        if (int rc = ensure(ctx, ctx->i8_tickets, tick_b)) return rc;
+        MCU_CUDA(cudaMemsetAsync(ctx->i8_tickets.ptr, 0, ctx->i8_tickets.cap, ctx->stream));
+    }
+    MCU_CUDA(launch_gemm_i8(kind, w, w2, x, (int)ldx, (int)T, (int)K, (int)F, bias, out, out2, (int)ldo, (int8_t *)ctx->act_qs.ptr,
+                            (float *)ctx->act_d.ptr, (float *)ctx->i8_partial.ptr, (int *)ctx->i8_tickets.ptr, ctx->dev_err, ctx->stream));
+    count_launches(2);
+    return MCU_SUCCESS;
+}
     for (int j = 0; j < n_jobs; ++j)
         if (!gemm_ti_supported(jobs[j].kind, jobs[j].W, (int)K, jobs[j].F) || act_half_fused_smem(jobs[j].kind, (int)K) > ACT_INT_MAX_SMEM) return false;
     return true;
@@ -620,8 +645,9 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     // a handful of tokens: exact integer dots on the tensor core
     const size_t values = K * F * (w2 != nullptr ? 2 : 1);
     const bool streams = T < 3 || T > (size_t)GEMV_MAX_T || gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F);
-    const bool i8_pays = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, values, streams);
-    if (i8_pays && (w2 == nullptr || bias == nullptr)) {
+    const bool integer = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, K, values, streams);
+    if (integer && (w2 == nullptr || bias == nullptr)) {
+        if (i8_takes(ctx, kind, w, w2, T, K, F)) return i8_locked(ctx, kind, x, ldx, w, w2, T, K, F, bias, out, out2, ldo);
         const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};
         if (integer_jobs_supported(jobs, w2 != nullptr ? 2 : 1, K))
             return integer_locked(ctx, kind, x, ldx, T, K, jobs, w2 != nullptr ? 2 : 1, nullptr, nullptr);
@@ -815,6 +841,12 @@ int mcu_linear_dual(mcu_context_t *ctx, int kind, const float *x_dev, size_t ldx
 }
 
 int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t T, size_t K, const mcu_prologue_t *prologue,
+// Matrices j and j + 1 as one dual matmul?
+static bool alike(const mcu_linear_job_t *jobs, size_t n_jobs, size_t j) {
+    return j + 1 < n_jobs && jobs[j + 1].kind == jobs[j].kind && jobs[j + 1].F == jobs[j].F && jobs[j + 1].ldo == jobs[j].ldo &&
+        jobs[j].bias_dev == nullptr && jobs[j + 1].bias_dev == nullptr;
+}
+
                      const mcu_linear_job_t *jobs, size_t n_jobs) {
     if (int rc = check_ctx(ctx)) return rc;
     if (jobs == nullptr || n_jobs == 0 || n_jobs > (size_t)MCU_LINEAR_MAX_JOBS)
@@ -861,20 +893,44 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
         // RMSNorm: 43 us, 28.5 here).  More than eight tokens otherwise: the fp16 one; its staging launch (the prologue folded into it)
         // feeds every matmul that wants the same staging, weights of the other block format class get a second one.
         const bool folds = pr.op == MCU_PROLOGUE_NONE || contiguous;
-        bool integer[GEMV_MAX_JOBS], all_integer = folds, tensor = folds;  // integer: by job
+        // Two kinds are two stagings and two launches, against one of the dp4a kernel (Q4_K + Q6_K: 2 x 4096 x 4096 at five, six, eight tokens
+        // 21.4, 23.4, 29.2 us there and 25.2 here; 2 x 2048 x 5632 21.7, 24.8, 32.2 and 23.1; 2 x 4096 x 14336 45.4 at five, 42.9 here).
+        size_t all_values = 0;
+        bool mixed = false;
+        for (size_t i = 0; i < n_jobs; ++i) all_values += K * (size_t)specs[i].F, mixed = mixed || specs[i].kind != specs[0].kind;
+        const bool few = mixed && all_values < (size_t)64 << 20 && T <= (K >= 4096 ? 6u : 5u);
+        bool integer[GEMV_MAX_JOBS] = {}, all_integer = folds, tensor = folds && !few, by_parts = false;  // integer: by job
         for (size_t j = 0; j < n_jobs && tensor; ++j) {
             size_t values = 0;
-            for (size_t i = 0; i < n_jobs; ++i) values += specs[i].kind == specs[j].kind ? K * (size_t)specs[i].F : 0;
-            bool supported = true;  // for all matrices of the kind
-            for (size_t i = 0; i < n_jobs; ++i) supported = supported && (specs[i].kind != specs[j].kind || integer_jobs_supported(&specs[i], 1, K));
-            integer[j] = supported && integer_pays(ctx, specs[j].kind, T, values, true);
+            bool supported = true;  // all matrices of the kind
+            int row_tiles = 0;
+            for (size_t i = 0; i < n_jobs; ++i) {
+                if (specs[i].kind != specs[j].kind) continue;
+                values += K * (size_t)specs[i].F;
+                row_tiles += (specs[i].F + TS_ROWS - 1) / TS_ROWS;
+                supported = supported && integer_jobs_supported(&specs[i], 1, K);
+            }
+            integer[j] = supported && integer_pays(ctx, specs[j].kind, T, K, values, true);
             all_integer = all_integer && integer[j];
             tensor = integer[j] ||
                 ((ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > (size_t)GEMV_MAX_T &&
                  gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) && act_half_fused_smem(jobs[j].kind, (int)K) <= 48 * 1024);
         }
+            if (!integer[j]) continue;
+            // Or matrix by matrix (pairs where they are alike) with the mma.sync kernel for some, behind a prologue kernel of its own (3 us).
+            double parts = pr.op == MCU_PROLOGUE_NONE ? 0.0 : 3.0;
+            for (size_t i = 0; i < n_jobs; i += alike(jobs, n_jobs, i) ? 2 : 1) {
+                if (specs[i].kind != specs[j].kind) continue;
+                const int mats = alike(jobs, n_jobs, i) ? 2 : 1, F = specs[i].F, sms = device_sm_count();
+                parts += i8_takes(ctx, specs[i].kind, specs[i].W, mats == 2 ? specs[i + 1].W : nullptr, T, K, (size_t)F)
+                    ? i8_us(specs[i].kind, (int)T, (int)K, mats * ((F + I8_ROWS - 1) / I8_ROWS), sms)
+                    : ti_us(specs[i].kind, (int)T, (int)K, mats * ((F + TS_ROWS - 1) / TS_ROWS), sms);
+            }
+            by_parts = by_parts || parts < ti_us(specs[j].kind, (int)T, (int)K, row_tiles, device_sm_count());
         tensor = tensor && (all_integer || T > (size_t)GEMV_MAX_T);
-        if (!tensor && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
+        by_parts = by_parts && tensor;
+        tensor = tensor && !by_parts;
+        if (!tensor && !by_parts && (ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMV) && T <= (size_t)GEMV_MAX_T &&
             gemv_stream_jobs_supported(specs, (int)n_jobs, (int)T, (int)K, gp)) {
             MCU_CUDA(launch_gemv_stream_jobs(specs, (int)n_jobs, x_dev, (int)ldx, (int)T, (int)K, gp, ctx->dev_err, ctx->stream));
             count_launches(1);
@@ -947,8 +1003,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
     std::lock_guard<std::mutex> lock(ctx->mu);
     for (size_t j = 0; j < n_jobs;) {
         const mcu_linear_job_t &a = jobs[j];
-        const bool pair = j + 1 < n_jobs && jobs[j + 1].kind == a.kind && jobs[j + 1].F == a.F && jobs[j + 1].ldo == a.ldo &&
-            a.bias_dev == nullptr && jobs[j + 1].bias_dev == nullptr;
+        const bool pair = alike(jobs, n_jobs, j);
         if (int rc = linear_locked(ctx, a.kind, act, ld_act, a.w_dev, pair ? jobs[j + 1].w_dev : nullptr, T, K, a.F, a.bias_dev,
                                    a.out_dev, pair ? jobs[j + 1].out_dev : nullptr, a.ldo))
             return rc;

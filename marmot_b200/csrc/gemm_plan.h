@@ -15,6 +15,7 @@ constexpr int TS_MAX_JOBS = 4;
 constexpr int TS_MAX_GROUPS = 256;
 constexpr int TS_MAX_SPLIT = 8;
 constexpr int TI_COLS = 16;      // tokens of a tile of the integer kernel
+constexpr int I8_MAX_T = 16, I8_ROWS = 64, I8_COLS_PER_STAGE = 4;  // the mma.sync kernel (gemm_i8.cu): a stage is 64 rows x four blocks
 
 MCU_HD int ts_min(int a, int b) { return a < b ? a : b; }
 
@@ -187,9 +188,9 @@ inline TsPlan ts_plan(int kind, int T, int K, const int *F, int n_jobs, int sms)
 inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
     const long U = (long)tiles * KS, n_most = U < sms ? U : sms, upc = (U + n_most - 1) / n_most;
     const double unit = kind == KIND_Q4_K ? 900.0 : 2100.0;
-    TsPlan best{TI_COLS, 0, 1, (int)n_most, 1e30};
+    TsPlan best{TI_COLS, 1, 1, (int)n_most, 1e30};
     auto consider = [&](int split, long n, double cost) {
-        if (cost < best.cost) best = TsPlan{TI_COLS, 0, split, (int)n, cost};
+        if (cost < best.cost) best = TsPlan{TI_COLS, 1, split, (int)n, cost};
     };
     consider(1, tiles, (double)((tiles + sms - 1) / sms) * (KS * unit + 3500.0));
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2)
@@ -197,6 +198,30 @@ inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
     const bool cut = U % n_most != 0 || upc % KS != 0;
     consider(1, n_most, (double)upc * unit + 2000.0 + (cut ? 9000.0 + 700.0 * ((double)KS / upc + 1.0) : 0.0));
     return best;
+}
+
+// Microseconds of a call of 5 to 16 tokens on `row_tiles` tiles of 128 rows with the integer kernel, staging included, and on `groups`
+// groups of 64 rows with the mma.sync one: fitted to both at 5, 8, 9, 12 and 16 tokens, K 1024 to 14336 and 512 to 32000 rows (within
+// 10 % of all but a few).  A stage of the latter takes 2.25 or 2.45 us and its first ones are 8 to 11; the former's cycles are those
+// of its plan, which single waves, with SMs to spare, beat.
+inline double ti_us(int kind, int T, int K, int row_tiles, int sms) {
+    const TsPlan pl = ti_plan(kind, row_tiles, (K + QK_K - 1) / QK_K, sms);
+    const bool wave = pl.split == 1 && pl.n_cta == row_tiles && row_tiles <= sms;
+    return 4.6 + (T <= 8 ? (wave ? 0.47 : 0.57) : (wave ? 0.62 : 0.68)) * 1e-3 * pl.cost;
+}
+inline double i8_us(int kind, int T, int K, int groups, int sms) {
+    if (kind == KIND_Q4_K) return T <= 8 ? 5.0 : 5.6;  // (where i8_pays: a stage to a CTA)
+    const int stages = ((K + QK_K - 1) / QK_K + I8_COLS_PER_STAGE - 1) / I8_COLS_PER_STAGE;  // of a group of rows
+    const double per_cta = (double)groups * stages / sms;
+    if (per_cta <= 1.0) return T <= 8 ? 7.2 + 0.47 * stages : 8.0 + 0.52 * stages;
+    return T <= 8 ? 10.5 + 2.25 * per_cta : 12.3 + 2.45 * per_cta;
+}
+// Does a matrix of F rows (two: `mats`) belong on the mma.sync kernel rather than the tcgen05 one?  Q4_K: rows of up to four blocks, a stage
+// for every CTA (5 us, 7 there whatever the size); larger ones never by more than a few per cent.  Q6_K: by the times above.
+inline bool i8_pays(int kind, int T, int K, int F, int mats, int sms) {
+    const int groups = mats * ((F + I8_ROWS - 1) / I8_ROWS);
+    if (kind == KIND_Q4_K) return K <= QK_K * I8_COLS_PER_STAGE && groups <= sms;
+    return i8_us(kind, T, K, groups, sms) < ti_us(kind, T, K, mats * ((F + TS_ROWS - 1) / TS_ROWS), sms);
 }
 
 }  // namespace mcu

@@ -107,6 +107,16 @@ cudaError_t launch_gemv_stream(int kind, const void *W, const void *W2, const fl
 cudaError_t launch_linear_f16(int kind, const void *W, const __half *x, size_t ldx, int T, int K, int F, const float *bias,
                               float *out32, __half *out16, size_t ldo, cudaStream_t s);
 
+// Few tokens on integer tensor-core instructions of mma.sync (gemm_i8.cu): activations packed to Q8_K by a first launch, exact int32
+// sub-block dots, f32 scaling per block; Q4_K and Q6_K, rows a multiple of 16 bytes.  The caller provides the workspace (sizes from
+// gemm_i8_workspace_bytes); `tickets` must be zero before the first launch and is left zero.
+bool gemm_i8_supported(int kind, const void *W, const void *W2, int T, int K, int F);
+void gemm_i8_workspace_bytes(int T, int K, int F, bool dual, size_t *qs_bytes, size_t *dT_bytes, size_t *partial_bytes,
+                             size_t *ticket_bytes);
+cudaError_t launch_gemm_i8(int kind, const void *W, const void *W2, const float *x, int ldx, int T, int K, int F,
+                           const float *bias, float *out, float *out2, int ldo, int8_t *qs, float *dT, float *partial,
+                           int *tickets, int *err_flag, cudaStream_t s);
+
 // Row-parallel matmul fused with its all-reduce over peer memory (gemm_tma, T <= 64, full 128-row tiles): every CTA
 // that holds a finished output tile stores it into this rank's peer-visible staging buffer, releases one flag per
 // rank and tile, waits (bounded) for the same tile of all ranks, pulls their tiles with plain peer loads and adds

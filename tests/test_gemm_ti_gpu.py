@@ -265,3 +265,22 @@ def test_rows_longer_than_the_static_shared_memory(ctx, oracle, kind, T, K):
     got = ctx.linear(kind, torch.from_numpy(x).cuda(), ctx.upload(W), F).cpu().numpy()
     ctx.synchronize()
     assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= 5e-5
+
+
+@pytest.mark.parametrize("kind,T,K,F", [(KIND_Q4_K, 8, 1024, 2000), (KIND_Q4_K, 9, 256, 70), (KIND_Q4_K, 16, 1000, 129), (KIND_Q6_K, 5, 2048, 4097),
+                                        (KIND_Q6_K, 9, 4096, 2049), (KIND_Q6_K, 16, 14336, 513), (KIND_Q6_K, 8, 2048, 20003)])
+def test_mma_sync_sizes(ctx, oracle, kind, T, K, F):
+    """Sizes that stay with the mma.sync kernel: one stage per CTA, row groups cut between CTAs, ragged rows, one and two token tiles."""
+    import torch
+
+    rng = np.random.default_rng(T + K + F)
+    W, W2 = random_blocks(kind, F, K, rng), random_blocks(kind, F, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    bias = rng.normal(0, 1, F).astype(np.float32)
+    xd = torch.from_numpy(x).cuda()
+    got = ctx.linear(kind, xd, ctx.upload(W), F, bias=torch.from_numpy(bias).cuda()).cpu().numpy()
+    assert max_rel_err(got, oracle.linear(kind, x, W, F) + bias) <= 2e-5
+    a, b = ctx.linear_dual(kind, xd, ctx.upload(W), ctx.upload(W2), F)
+    ctx.synchronize()
+    assert max_rel_err(a.cpu().numpy(), oracle.linear(kind, x, W, F)) <= 2e-5
+    assert max_rel_err(b.cpu().numpy(), oracle.linear(kind, x, W2, F)) <= 2e-5
