@@ -578,9 +578,9 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
 //         5 tokens  1024 x 1024 4.7, 6.8; 2048 x 2048 7.3, 7.3; 4096 x 1024 8.2, 7.4; 4096 x 4096 11.9, 9.0
 //   Q6_K  4 tokens  4096 x 4096 11.0, 11.7; 14336 x 4096 33.3, 23.6; 4096 x 28672 39.7, 44.7
 //         5 tokens  1024 x 1024 4.2, 7.0; 2048 x 2048 7.9, 8.0; 4096 x 1024 8.8, 8.6; 4096 x 4096 13.5, 11.7
-// From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
 // Small matrices of long rows are a chain for the dp4a kernel's warps, short rows leave little to chain: a line of tokens x K, or of
 // tokens x rows, for those (8 tokens: 3072 x 125 Q4_K 9.5, 7.0; 2048 x 256 7.8, 6.9; 1024 x 1024 5.6, 4.9 with gemm_i8; 1024 x 512 5.0, 4.8).
+// From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
 // And from three tokens on where the rows cannot be streamed (Q6_K of ragged sizes), against the plain-load kernel: 3072 x 125 3, 4,
 // 8 tokens 13.5, 16.6, 21.2 us, 7.5, 7.7, 7.8 here; 1280 x 300 7.5, 9.1, 12.5, then 7.6 to 7.7.
 static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, size_t values, bool streams) {
@@ -590,7 +590,6 @@ static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, s
     if (T >= 5) return values >= (size_t)4 << 20 || T * K >= 16384 || (kind == KIND_Q4_K && K <= 1024 && T * values >= 8192 * K);
     return kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20;
 }
-static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K) {
 // The integer matmul by mma.sync, for the sizes where it is the faster one.
 static bool i8_takes(const mcu_context *ctx, int kind, const void *w, const void *w2, size_t T, size_t K, size_t F) {
     return ctx->regime == MCU_REGIME_AUTO && T >= 5 && T <= (size_t)I8_MAX_T && gemm_i8_supported(kind, w, w2, (int)T, (int)K, (int)F) &&
@@ -612,6 +611,7 @@ static int i8_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, con
     count_launches(2);
     return MCU_SUCCESS;
 }
+static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K) {
     for (int j = 0; j < n_jobs; ++j)
         if (!gemm_ti_supported(jobs[j].kind, jobs[j].W, (int)K, jobs[j].F) || act_half_fused_smem(jobs[j].kind, (int)K) > ACT_INT_MAX_SMEM) return false;
     return true;
@@ -840,13 +840,13 @@ int mcu_linear_dual(mcu_context_t *ctx, int kind, const float *x_dev, size_t ldx
     return linear_locked(ctx, kind, x_dev, ldx, w_a_dev, w_b_dev, T, K, F, nullptr, out_a_dev, out_b_dev, ldo);
 }
 
-int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t T, size_t K, const mcu_prologue_t *prologue,
 // Matrices j and j + 1 as one dual matmul?
 static bool alike(const mcu_linear_job_t *jobs, size_t n_jobs, size_t j) {
     return j + 1 < n_jobs && jobs[j + 1].kind == jobs[j].kind && jobs[j + 1].F == jobs[j].F && jobs[j + 1].ldo == jobs[j].ldo &&
         jobs[j].bias_dev == nullptr && jobs[j + 1].bias_dev == nullptr;
 }
 
+int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t T, size_t K, const mcu_prologue_t *prologue,
                      const mcu_linear_job_t *jobs, size_t n_jobs) {
     if (int rc = check_ctx(ctx)) return rc;
     if (jobs == nullptr || n_jobs == 0 || n_jobs > (size_t)MCU_LINEAR_MAX_JOBS)
@@ -915,7 +915,6 @@ static bool alike(const mcu_linear_job_t *jobs, size_t n_jobs, size_t j) {
             tensor = integer[j] ||
                 ((ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > (size_t)GEMV_MAX_T &&
                  gemm_ts_supported(jobs[j].kind, jobs[j].w_dev, (int)T, (int)K, (int)jobs[j].F) && act_half_fused_smem(jobs[j].kind, (int)K) <= 48 * 1024);
-        }
             if (!integer[j]) continue;
             // Or matrix by matrix (pairs where they are alike) with the mma.sync kernel for some, behind a prologue kernel of its own (3 us).
             double parts = pr.op == MCU_PROLOGUE_NONE ? 0.0 : 3.0;
@@ -927,6 +926,7 @@ static bool alike(const mcu_linear_job_t *jobs, size_t n_jobs, size_t j) {
                     : ti_us(specs[i].kind, (int)T, (int)K, mats * ((F + TS_ROWS - 1) / TS_ROWS), sms);
             }
             by_parts = by_parts || parts < ti_us(specs[j].kind, (int)T, (int)K, row_tiles, device_sm_count());
+        }
         tensor = tensor && (all_integer || T > (size_t)GEMV_MAX_T);
         by_parts = by_parts && tensor;
         tensor = tensor && !by_parts;
