@@ -255,8 +255,10 @@ int mcu_topk(
  *      topk_ids [T][k] int32, topk_weights [T][k] f32; out [T][H] f32.
  *      With T * k >= 256 (gate and up of one kind) the call reads nothing back: it is asynchronous, may be recorded by
  *      mcu_graph_capture_begin/end, and an expert id outside [0, E) is reported by the next mcu_synchronize as
- *      MCU_ERROR_INVALID_ARGUMENT.  Smaller batches report a bad id from the call itself, which waits for the routing (a recorded
- *      call reports it as above); those with weights other than Q4_K / Q6_K, or of two kinds, read the group sizes back too. ---- */
+ *      MCU_ERROR_INVALID_ARGUMENT.  Smaller batches report a bad id from the call itself, which waits for the routing and leaves
+ *      `out` as it was (a recorded call reports it as above).  Of those, calls with other weights than Q4_K / Q6_K or of two kinds,
+ *      and calls with many or next to no rows per expert, read the group sizes back too and go expert by expert: more than
+ *      sixteen rows of an expert then are multiplied in fp16, which a recorded call of that size does for all. ---- */
 int mcu_moe_experts(
     mcu_context_t *ctx, int gate_kind, int up_kind, int down_kind, const float *hidden_dev, size_t T, size_t H,
     size_t FF, size_t E, const void *gate_dev, const void *up_dev, const void *down_dev, const int32_t *topk_ids_dev,

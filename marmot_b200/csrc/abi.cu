@@ -1131,12 +1131,40 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     static const bool no_grouped = getenv("MARMOT_CUDA_MOE_NO_GROUPED") != nullptr;  // diagnostic switch
     // Few routes (a decode batch): the integer tensor-core kernel over all local experts, one launch for gate and up, one for
     // down, tiles of sixteen tokens sized from the device-resident counts; exact sub-block dots, as the per-expert launches
-    // below (16 tokens, top 2 of 8 experts of 3 x 14336 x 4096: 480 us with those, which wait for the counts on the host, 244 here).
-    const bool few = !no_grouped && routes < 256 && routed_rows_ext == nullptr && gate_kind == up_kind && e_count <= (size_t)TS_MAX_GROUPS &&
+    // below (16 tokens, top 2 of 8 experts of 3 x 14336 x 4096: 398 us with those, which wait for the counts on the host, 223 here).
+    // It reads the weights again for every sixteen rows of an expert, which large experts and Q6_K notice first; those launches cost 25 us
+    // an expert whatever its size, and take it for large experts only.  Rows per expert, here and there, us at 4 experts of 3 x 14336 x 4096:
+    // Q4_K 16 238, 265; 32 262 to 317, 273; 48 375, 282.  Q6_K down 16 279, 313; 32 348, 314.  Q6_K 12 278, 332; 16 402, 348; 48 756, 373.
+    // At 4 of 3 x 5632 x 2048: Q4_K 48 122, 140; 63 165, 156.  Q6_K down 48 158, 166; 60 195, 174.  Q6_K 32 153 to 174, 174; 48 206, 176.
+    // Next to no routes leave most experts out: 1 token of 8 experts of 3 x 14336 x 4096 107, 92; all Q6_K 199, 110, and 2 rows 428 to 728, 352 to 429.
+    const size_t n6 = (gate_kind == KIND_Q6_K ? 1 : 0) + (down_kind == KIND_Q6_K ? 1 : 0);
+    const bool large = H * FF > (size_t)26 << 20, capturing = stream_is_capturing(s);
+    const size_t most_rows = (large ? 48 : 128) / (2 + n6);
+    const bool fp16_suits = gate_kind == up_kind && gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
+        gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) && gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H) &&
+        act_half_fused_smem(gate_kind, (int)H) <= 48 * 1024 && act_half_fused_smem(down_kind, (int)FF) <= 48 * 1024;
+    const bool few_suits = !no_grouped && routes < 256 && routed_rows_ext == nullptr && gate_kind == up_kind && e_count <= (size_t)TS_MAX_GROUPS &&
         integer_jobs_supported(gate_up, 2, H) && integer_jobs_supported(&down_job, 1, FF) && gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
         gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) && gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H);
+    // A recorded call cannot read the counts: this kernel or the grouped fp16 one.
+    const bool few_recorded = few_suits && (routes <= most_rows * E || !fp16_suits);
+    const bool few = capturing ? few_recorded
+                               : few_suits && routes <= most_rows * E && routes * 4 > E && (!large || n6 < 2 || routes >= 4 * E);
+    auto few_workspace = [&]() -> int {
+        const size_t xq_h = gemm_ti_xq_bytes(gate_kind, (int)routes, (int)H), xq_f = gemm_ti_xq_bytes(down_kind, (int)routes, (int)FF);
+        const size_t nb_max = ((H > FF ? H : FF) + QK_K - 1) / QK_K;
+        if (int rc = ensure(ctx, ctx->act_qs, xq_h > xq_f ? xq_h : xq_f)) return rc;
+        if (int rc = ensure(ctx, ctx->act_d, routes * nb_max * sizeof(float))) return rc;
+        return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes());
+    };
+    const size_t kp_h = (H + block_values(gate_kind) - 1) / block_values(gate_kind) * block_values(gate_kind);
+    const size_t kp_f = (FF + block_values(down_kind) - 1) / block_values(down_kind) * block_values(down_kind);
+    auto fp16_workspace = [&]() -> int {
+        if (int rc = ensure(ctx, ctx->act_half, routes * (kp_h > kp_f ? kp_h : kp_f) * sizeof(__half))) return rc;
+        if (int rc = ensure(ctx, ctx->act_rowscale, routes * sizeof(float))) return rc;
+        return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes());
+    };
     if (few) {
-        const bool capturing = stream_is_capturing(s);
         // A bad expert id is reported by the call itself, as ever for few routes: the flag is fetched behind the routing and
         // waited for once everything is enqueued, so that the device does not wait for the host.
         int *flag_host = ctx->err_host != nullptr ? ctx->err_host + 1 : nullptr;
@@ -1145,11 +1173,7 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
             MCU_CUDA(cudaMemcpyAsync(flag_host, rb.counts + E, sizeof(int), cudaMemcpyDeviceToHost, s));
             MCU_CUDA(cudaEventRecord(ctx->moe_event, s));
         }
-        const size_t xq_h = gemm_ti_xq_bytes(gate_kind, (int)routes, (int)H), xq_f = gemm_ti_xq_bytes(down_kind, (int)routes, (int)FF);
-        const size_t nb_max = ((H > FF ? H : FF) + QK_K - 1) / QK_K;
-        if (int rc = ensure(ctx, ctx->act_qs, xq_h > xq_f ? xq_h : xq_f)) return rc;
-        if (int rc = ensure(ctx, ctx->act_d, routes * nb_max * sizeof(float))) return rc;
-        if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+        if (int rc = few_workspace()) return rc;
         uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
         float *dT = (float *)ctx->act_d.ptr, *part = (float *)ctx->gemm_partial.ptr;
         MCU_CUDA(launch_act_int_fused(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xq, dT, s));
@@ -1179,25 +1203,14 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     // Fewer routes that the integer kernel does not take have per-expert launches sized from counts read back on the host
     // (small groups then get the GEMV kernels); a call that is being recorded into a CUDA graph cannot read anything back, so it
     // takes the grouped launches whatever its size.
-    const bool grouped = !no_grouped && (routes >= 256 || stream_is_capturing(s) || routed_rows_ext != nullptr) &&
-        gate_kind == up_kind &&
-        gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
-        gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) &&
-        gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H) &&
-        act_half_fused_smem(gate_kind, (int)H) <= 48 * 1024 && act_half_fused_smem(down_kind, (int)FF) <= 48 * 1024 &&
-        routes < ((size_t)1 << 24);
+    const bool grouped = !no_grouped && (routes >= 256 || capturing || routed_rows_ext != nullptr) && fp16_suits && routes < ((size_t)1 << 24);
     if (grouped) {
-        const size_t kp_h = (H + block_values(gate_kind) - 1) / block_values(gate_kind) * block_values(gate_kind);
-        const size_t kp_f = (FF + block_values(down_kind) - 1) / block_values(down_kind) * block_values(down_kind);
-        const size_t kp_max = kp_h > kp_f ? kp_h : kp_f;
-        if (int rc = ensure(ctx, ctx->act_half, routes * kp_max * sizeof(__half))) return rc;
-        if (int rc = ensure(ctx, ctx->act_rowscale, routes * sizeof(float))) return rc;
+        if (int rc = fp16_workspace()) return rc;
         __half *xh = (__half *)ctx->act_half.ptr;
         float *rowscale = (float *)ctx->act_rowscale.ptr;
         // The staging kernels fetch their rows themselves: the routed token's hidden row for gate/up, act(gate) * up
         // for down.  Routes of other ranks' experts (outside [offsets[e_begin], offsets[e_end])) are skipped there,
         // never multiplied and never combined.
-        if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
         float *part = (float *)ctx->gemm_partial.ptr;
         int *tick = ctx->gemm_counters;
         MCU_CUDA(launch_act_half_fused_from(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xh, rowscale, s));
@@ -1218,9 +1231,15 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     }
     if (routed_rows_ext != nullptr)
         return fail(MCU_ERROR_NOT_IMPLEMENTED, "this MoE shape does not take the grouped path: no routed rows to exchange");
-    if (stream_is_capturing(s))
+    if (capturing)
         return fail(MCU_ERROR_INVALID_OPERATION,
                     "this MoE shape reads the group sizes back to size the per-expert launches: the call cannot be captured");
+    // The same call, recorded, finds its workspace.
+    if (few_recorded) {
+        if (int rc = few_workspace()) return rc;
+    } else if (fp16_suits && !no_grouped) {
+        if (int rc = fp16_workspace()) return rc;
+    }
     // The per-expert launches need the group sizes on the host.
     ctx->host_counts.resize(2 * (E + 1));
     MCU_CUDA(cudaMemcpyAsync(ctx->host_counts.data(), rb.counts, 2 * (E + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -147,7 +147,8 @@ __global__ void moe_glu_kernel(float *__restrict__ gate, const float *__restrict
 // out[t][c] = sum over the token's routes, in ascending sorted position (= the reference's route
 // order, moe_ops.c:1034-1042), of w * down[pos][c]; products and sums rounded separately.  Positions outside [pos_lo, pos_hi) are
 // another rank's experts or rejected ids.  With offsets the range comes from the device (experts [e_begin, e_end)): no host
-// read-back; block 0 then also reports an out-of-range expert id through the error flag.
+// read-back; block 0 then also reports an out-of-range expert id through the error flag.  Without a flag the caller reports it, and `out`
+// stays as it was.
 // grid (tokens, slices of 1024 columns): loads of several routes and slices are in flight together (one column and route at a time
 // per thread: 21 us for 16 tokens of 4096, 43 for 2048; 4 and 18 so).
 struct CombineRange {
@@ -165,6 +166,7 @@ moe_combine_kernel(const float *__restrict__ route_down, const float *__restrict
     constexpr int N = sizeof(V) / sizeof(float), BATCH = 4;
     __shared__ int pos_s[MOE_MAX_TOPK];
     __shared__ float w_s[MOE_MAX_TOPK];
+    __shared__ bool leave_s;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t = blockIdx.x;
     if (threadIdx.x < (unsigned)k) {
@@ -175,6 +177,7 @@ moe_combine_kernel(const float *__restrict__ route_down, const float *__restrict
             bad = *range.bad_id_count != 0;  // the call is rejected as a whole: zeros out
             if (bad && t == 0 && blockIdx.y == 0 && threadIdx.x == 0 && range.err != nullptr) atomicExch(range.err, 40);
         }
+        if (threadIdx.x == 0) leave_s = bad && range.err == nullptr;
         const int32_t *mine = route_pos + (size_t)t * k;
         const int p = mine[threadIdx.x];
         int rank = 0;
@@ -184,6 +187,7 @@ moe_combine_kernel(const float *__restrict__ route_down, const float *__restrict
         w_s[rank] = use ? sorted_w[p] : 0.0f;
     }
     __syncthreads();
+    if (leave_s) return;
     const int c1 = min(H, ((int)blockIdx.y + 1) * COMBINE_COLS);
     for (int c = (int)blockIdx.y * COMBINE_COLS + N * (int)threadIdx.x; c < c1; c += N * 256) {
         float acc[N];

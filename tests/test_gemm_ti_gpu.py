@@ -267,6 +267,46 @@ def test_rows_longer_than_the_static_shared_memory(ctx, oracle, kind, T, K):
     assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= 5e-5
 
 
+@pytest.mark.parametrize("kind,T,E,k", [(KIND_Q6_K, 40, 4, 4), (KIND_Q4_K, 1, 8, 2), (KIND_Q6_K, 9, 3, 2)])
+def test_recorded_moe_after_an_eager_call(ctx, oracle, kind, T, E, k):
+    """Few-route calls that go expert by expert when the counts can be read (many rows or next to none per expert) can still be recorded
+    after one eager call, and give the same up to a re-quantised intermediate; an id out of range leaves the output alone."""
+    import torch
+    from marmot_b200 import Context, MarmotCudaError
+
+    H, FF = 512, 256
+    rng = np.random.default_rng(T + E)
+    hid = rng.normal(0, 1, (T, H)).astype(np.float32)
+    gate, up, down = (random_blocks(kind, F, K, rng, d_sigma=0.0005) for F, K in ((E * FF, H), (E * FF, H), (E * H, FF)))
+    vals, ids = oracle.topk(rng.random((T, E)).astype(np.float32), k)
+    ref = oracle.moe_experts((kind,) * 3, hid, gate, up, down, ids, vals, FF, E)
+    c = Context(0, use_torch_stream=False)  # (a workspace of its own)
+    stream = torch.cuda.Stream()
+    c.set_stream(stream.cuda_stream)
+    with torch.cuda.stream(stream):
+        hd, vd, idd = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (hid, vals, ids))
+        gd, ud, dd = (c.upload(w) for w in (gate, up, down))
+        out = torch.empty((T, H), device="cuda")
+        call = lambda i: c.moe_experts_local((kind,) * 3, hd, gd, ud, dd, i, vd, FF, E, 0, E, out=out)
+        assert max_rel_err(call(idd).cpu().numpy(), ref) <= TOL_MOE
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            call(idd)
+        out.zero_()
+        g.replay()
+        c.synchronize()
+        assert max_rel_err(out.cpu().numpy(), ref) <= TOL_MOE
+        out.fill_(7.0)
+        bad = idd.clone()
+        bad[0, 0] = E
+        with pytest.raises(MarmotCudaError):
+            call(bad)
+        c.synchronize()
+        assert (out == 7.0).all()
+        del g
+    c.close()
+
+
 @pytest.mark.parametrize("kind,T,K,F", [(KIND_Q4_K, 8, 1024, 2000), (KIND_Q4_K, 9, 256, 70), (KIND_Q4_K, 16, 1000, 129), (KIND_Q6_K, 5, 2048, 4097),
                                         (KIND_Q6_K, 9, 4096, 2049), (KIND_Q6_K, 16, 14336, 513), (KIND_Q6_K, 8, 2048, 20003)])
 def test_mma_sync_sizes(ctx, oracle, kind, T, K, F):
