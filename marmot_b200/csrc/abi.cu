@@ -91,7 +91,7 @@ struct mcu_context {
     std::vector<int> host_counts;
     size_t moe_last_routes = 0, moe_last_experts = 0;  // shape of the last MoE call (mcu_moe_last_buffers)
     int moe_last_grouped = 0;
-    int *dev_err = nullptr;  // set by kernels whose bounded device-side waits ran out
+    int *dev_err = nullptr;  // set by kernels whose bounded device-side waits ran out; the word behind it: PagedParams::odd_v
     int *err_host = nullptr; // page-locked words: the flag's copy on a synchronize, the bad-id count of a small MoE call
     cudaEvent_t moe_event = nullptr;
     // Small host <-> device copies go through page-locked slots owned by the context: an upload is a host memcpy into a
@@ -159,6 +159,7 @@ static int sync_and_check(mcu_context *ctx, cudaStream_t s) {
 namespace mcu {
 int context_device(const mcu_context *ctx) { return ctx->device; }
 int *context_err_flag(mcu_context *ctx) { return ctx->dev_err; }
+int *context_odd_flag(mcu_context *ctx) { return ctx->dev_err + 1; }
 int context_attention_scratch(mcu_context *ctx, size_t bytes, void **out) {
     std::lock_guard<std::mutex> lock(ctx->mu);
     if (int rc = ensure(ctx, ctx->attn_partial, bytes)) return rc;
@@ -241,8 +242,8 @@ int mcu_context_create(int device, mcu_context_t **out) {
         return cuda_fail(e, "cudaStreamCreate");
     }
     ctx->stream = ctx->own_stream;
-    e = cudaMalloc(&ctx->dev_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(ctx->dev_err, 0, sizeof(int));
+    e = cudaMalloc(&ctx->dev_err, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(ctx->dev_err, 0, 2 * sizeof(int));
     if (e == cudaSuccess && cudaHostAlloc((void **)&ctx->err_host, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
         (void)cudaGetLastError();
         ctx->err_host = nullptr;  // the flag is then fetched with a blocking copy

@@ -11,7 +11,8 @@
 // - Decode steps (attention_decode_kernel): persistent, chunk x of the list of all chunks to warp x % warps, every warp with its own
 //   ring of tiles, so the next tiles are on their way under the arithmetic.
 // - Prompts (attention_prompt_kernel): a CTA fetches the chunk once for the tokens of its block that stand at consecutive
-//   positions of a sequence; every warp takes as many of them as fill the eight rows of A.
+//   positions of a sequence; every warp takes as many of them as fill the eight rows of A.  A block of short runs (decode steps among
+//   prompts) is taken token by token, four warps to a token.
 //
 // Measured: 64 sequences of 256 to 4096 positions, 8 KV heads of 128 (570 MB): 143 -> 102 us, 5.6 TB/s; a prompt of 500 tokens of the
 // same model 119 -> 51.  A warp takes 20000 cycles per chunk of the first (four tiles of 1000 for the scores and 800 for P V, the
@@ -31,6 +32,7 @@ constexpr int AT_HALF_BYTES = PM_TILE * 128;  // 64 dimensions of a tile's rows
 constexpr int AT_RING_BYTES = 24 * 1024;      // of a warp (decode steps)
 constexpr int AT_MAX_TOKENS = 256;            // decode steps: the tokens' chunk counts are summed up in shared memory
 constexpr int AT_BLOCK = 32;                  // prompts: most tokens of a CTA
+constexpr int AT_SHORT = 4;                   // prompts: blocks with runs of fewer tokens on average are taken token by token
 
 struct AttnMaps {
     CUtensorMap k, v;  // [pool block, layer and KV head][64 dimensions][position][dimension]
@@ -40,6 +42,7 @@ template <int HD>
 struct At {
     static constexpr int HALVES = HD / 64, TILE = HALVES * AT_HALF_BYTES, KS = HD / 16, NT = HD / 8, SLOTS = AT_RING_BYTES / TILE;
     static constexpr int Q_BYTES = KS * 32 * 16;  // a warp's A fragments: heads and tails
+    static constexpr int PROMPT_TILES = HD == 64 ? 16 : 8;  // of a prompt CTA: K 0..3, V 0..3; token by token two or one per warp
 };
 
 __device__ __forceinline__ void at_tma_4d(uint32_t dst, const CUtensorMap *map, int row, int slab, uint32_t bar) {
@@ -99,20 +102,6 @@ __device__ __forceinline__ void at_zero_rows(const AtRows<HD> &rows, uint32_t ti
         if (!((live >> row) & 1u))
             asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(tile + rows.piece(row, pc)), "r"(0u) : "memory");
     }
-}
-
-// Does a V tile hold an infinity or a NaN?  (Rows without data are zero by now.)
-template <int HD>
-__device__ __forceinline__ bool at_not_finite(uint32_t tile, int lane) {
-    uint32_t bad = 0;
-#pragma unroll 4
-    for (int i = lane; i < At<HD>::TILE / 16; i += 32) {
-        uint32_t w[4];
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(tile + 16u * (uint32_t)i) : "memory");
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bad |= __vcmpeq2(w[j] & 0x7C007C00u, 0x7C007C00u);  // all bits of the exponent
-    }
-    return __any_sync(0xffffffffu, bad != 0);
 }
 
 // A fragments of Q into this lane's part of `qf`: row g of A (of this lane) is `qrow` (null: zeros), rotated when there is a table.
@@ -319,7 +308,7 @@ attention_decode_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, in
     __shared__ __align__(8) uint64_t bars[AT_WARPS][A::SLOTS];
     __shared__ uint32_t slot_live[AT_WARPS][A::SLOTS];
     __shared__ int scan[AT_WARPS], prefix[AT_MAX_TOKENS + 1];  // chunks of the tokens ahead
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), g = lane >> 2, tq = lane & 3;
     const uint32_t raw = tm_smem_u32(at_smem), base = (raw + 1023u) & ~1023u;
     const uint32_t ring = base + (uint32_t)warp * AT_RING_BYTES;
     uint8_t *ring_ptr = at_smem + (ring - raw);
@@ -498,22 +487,117 @@ attention_decode_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, in
     }
 }
 
+struct AtPromptShared {
+    __align__(8) uint64_t bars[AT_WARPS][2];
+    uint32_t tile_live[AT_WARPS], seq[AT_BLOCK], pos[AT_BLOCK];
+    float m[AT_WARPS][8], l[AT_WARPS][8];
+};
+
+// The tokens of a block one by one: group g of four warps takes the tokens g, g + 2 ..; a warp takes a tile of 32 positions of the chunk, and
+// the four states are merged through shared memory (as in paged_attention_mma_kernel).  For blocks of short runs: run by run a token costs its CTA 5.5 us, and
+// seven warps stand by (64 sequences of 2000 positions with a token each, 8 KV heads of 128: 247 us run by run, 120 so).
+template <int HD>
+__device__ __forceinline__ bool at_tokens(const AttnMaps &maps, const PagedParams &p, int t_lo, int n_tok, int h, int c, int n_chunks, float *partial,
+                                          uint32_t base, uint4 *qf_all, AtPromptShared &sh) {
+    using A = At<HD>;
+    constexpr bool BOTH = A::PROMPT_TILES == 2 * AT_WARPS;  // a slot for K and one for V
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3, group = warp >> 2, wl = warp & 3;
+    const int gsize = p.n_q_heads / p.n_kv_heads;
+    const AtRows<HD> rows{min(p.block_shift, 5)};
+    const uint32_t tile_k = base + (uint32_t)(warp * (BOTH ? 2 : 1) * A::TILE), tile_v = BOTH ? tile_k + (uint32_t)A::TILE : tile_k;
+    const uint32_t bar = tm_smem_u32(&sh.bars[warp][0]), p0 = (uint32_t)c * PM_CHUNK;
+    uint4 *qf = qf_all + warp * (A::Q_BYTES / 16);
+    uint32_t phase = 0;  // bit 0: of the warp's first barrier, bit 1: of its second one
+    bool ok = true;
+    auto group_sync = [&] {  // (barrier numbers as constants: a number in a register takes all sixteen)
+        if (group == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+        else asm volatile("bar.sync 2, 128;" ::: "memory");
+    };
+    for (int i = group; i < n_tok; i += 2) {
+        const uint32_t seq = sh.seq[i], len = sh.pos[i] + 1u;
+        if (len <= p0) continue;
+        const size_t head_row = (size_t)(t_lo + i) * p.n_q_heads + (size_t)h * gsize;
+        float m = -INFINITY, l = 0.0f;
+        if (p0 + (uint32_t)(wl * PM_TILE) < len && ok) {
+            const uint32_t blocks = at_blocks(p, seq, len, p0, lane);
+            uint32_t live = at_load_tile<HD>(p, &maps.k, blocks, len, h, p0, wl, tile_k, bar, lane, seq);
+            if (BOTH) at_load_tile<HD>(p, &maps.v, blocks, len, h, p0, wl, tile_v, bar + 8u, lane, seq);
+            at_load_q<HD>(g < gsize ? p.q + (head_row + g) * HD : nullptr, nullptr, 0, p.scale, qf, lane);
+            ok = ts_wait(bar, phase & 1u);
+            ok = __all_sync(0xffffffffu, ok);
+            phase ^= 1u;
+            if (ok) {
+                uint32_t phi[4], plo[4];
+                at_scores<HD>(rows, tile_k, qf, live, lane, phi, plo, m, l);
+                __syncwarp();
+                if (!BOTH) live = at_load_tile<HD>(p, &maps.v, blocks, len, h, p0, wl, tile_v, bar, lane, seq);
+                ok = BOTH ? ts_wait(bar + 8u, (phase >> 1) & 1u) : ts_wait(bar, phase & 1u);
+                ok = __all_sync(0xffffffffu, ok);
+                phase ^= BOTH ? 2u : 1u;
+                if (live != 0xffffffffu) at_zero_rows<HD>(rows, tile_v, live, lane);
+                __syncwarp();
+                float acc[A::NT][2];
+#pragma unroll
+                for (int k = 0; k < A::NT; ++k) acc[k][0] = acc[k][1] = 0.0f;
+                at_pv<HD>(rows, tile_v, phi, plo, 1.0f, lane, acc);
+                if (live != 0xffffffffu) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                // (the query's fragments are done with: their place takes the warp's eight rows)
+                float *to = (float *)qf + g * HD + 2 * tq;
+                if (g < gsize) {
+#pragma unroll
+                    for (int k = 0; k < A::NT; ++k) *(float2 *)(to + 8 * k) = make_float2(acc[k][0], acc[k][1]);
+                }
+            }
+        }
+        if (tq == 0) sh.m[warp][g] = ok ? m : -INFINITY, sh.l[warp][g] = l;
+        group_sync();
+        for (int k = wl * 32 + lane; k < gsize * HD; k += 128) {
+            const int hh = k / HD, d = k % HD;
+            float M = -INFINITY, L = 0.0f, O = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) M = fmaxf(M, sh.m[4 * group + w][hh]);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const float mw = sh.m[4 * group + w][hh];
+                if (M == -INFINITY || mw == -INFINITY) continue;
+                const float e = expf(mw - M);
+                L += sh.l[4 * group + w][hh] * e;
+                O += ((const float *)(qf_all + (4 * group + w) * (A::Q_BYTES / 16)))[k] * e;
+            }
+            if (len <= (uint32_t)PM_CHUNK || n_chunks == 1) {
+                p.out[(head_row + hh) * HD + d] = L > 0.0f ? O / L : 0.0f;
+                continue;
+            }
+            float *pr = partial + ((head_row + hh) * n_chunks + c) * (HD + 2);
+            if (d == 0) *(float2 *)pr = make_float2(M, L);
+            pr[2 + d] = O;
+        }
+        group_sync();
+    }
+    return ok;
+}
+
 // Prompts: the tokens' K and V rows are in the pool, q is rotated.  grid (KV heads, blocks of tokens, chunks).
 template <int HD>
 __global__ void __launch_bounds__(32 * AT_WARPS, 2)
 attention_prompt_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, int block_tokens, int n_chunks, float *partial, int *err) {
     using A = At<HD>;
     extern __shared__ uint8_t at_smem[];
-    __shared__ __align__(8) uint64_t bars[AT_WARPS];
-    __shared__ uint32_t tile_live[AT_WARPS], tile_odd[AT_WARPS], s_seq[AT_BLOCK], s_pos[AT_BLOCK];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
-    const uint32_t raw = tm_smem_u32(at_smem), base = (raw + 1023u) & ~1023u;  // K tiles 0..3, V tiles 0..3
-    uint4 *qf = (uint4 *)(at_smem + (base - raw) + 8 * A::TILE + warp * A::Q_BYTES);
-    const uint32_t bar = tm_smem_u32(&bars[warp]);
-    if (lane == 0) tm_mbar_init(bar, 1);
+    __shared__ AtPromptShared sh;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), g = lane >> 2, tq = lane & 3;
+    const uint32_t raw = tm_smem_u32(at_smem), base = (raw + 1023u) & ~1023u;
+    uint4 *qf_all = (uint4 *)(at_smem + (base - raw) + A::PROMPT_TILES * A::TILE), *qf = qf_all + warp * (A::Q_BYTES / 16);
+    const uint32_t bar = tm_smem_u32(&sh.bars[warp][0]);
+    if (lane == 0) {
+        tm_mbar_init(bar, 1);
+        tm_mbar_init(bar + 8u, 1);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    uint32_t *s_seq = sh.seq, *s_pos = sh.pos, *tile_live = sh.tile_live;
+    const int odd_v = *p.odd_v;
     const int h = blockIdx.x, c = blockIdx.z, t_lo = blockIdx.y * block_tokens, n_tok = min(block_tokens, p.n_tokens - t_lo);
     const int H = p.n_kv_heads, gsize = p.n_q_heads / H, per_pass = 8 / gsize;
     const AtRows<HD> rows{min(p.block_shift, 5)};
@@ -523,9 +607,20 @@ attention_prompt_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, in
         s_pos[threadIdx.x] = p.meta[(t_lo + threadIdx.x) * 4 + 1];
     }
     __syncthreads();
+    // A run: tokens of one sequence at consecutive positions.  Blocks whose runs are short are taken token by token, and so is everything
+    // where a V value of the call is not finite: a run's tokens share the V rows of its longest context, and a token's zero
+    // probability times such a value beyond its own context would be NaN.
     bool ok = true;
     uint32_t phase = 0;
-    // a run: tokens of one sequence at consecutive positions
+    const int n_runs = __popc(__ballot_sync(0xffffffffu, lane < n_tok && (lane == 0 || s_seq[lane] != s_seq[lane - 1] || s_pos[lane] != s_pos[lane - 1] + 1u)));
+    const bool by_token = (n_tok < AT_SHORT * n_runs && (n_runs > 1 || n_tok == 1)) || odd_v != 0;
+    if (by_token) {
+        if (!at_tokens<HD>(maps, p, t_lo, n_tok, h, c, n_chunks, partial, base, qf_all, sh)) {
+            if (lane == 0) atomicExch(err, 61);
+            for (int i = 0; i < 200; ++i) __nanosleep(1000);
+        }
+        return;
+    }
     for (int first = 0, n = 1; first < n_tok; first += n) {
         const uint32_t seq = s_seq[first], pos = s_pos[first];
         for (n = 1; first + n < n_tok && s_seq[first + n] == seq && s_pos[first + n] == pos + (uint32_t)n; ++n) {}
@@ -545,56 +640,38 @@ attention_prompt_kernel(const __grid_constant__ AttnMaps maps, PagedParams p, in
             if (warp >= 4 && live != 0xffffffffu) {
                 at_zero_rows<HD>(rows, tile, live, lane);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
             }
-            const bool odd = warp >= 4 && live != 0u && ok && at_not_finite<HD>(tile, lane);
-            if (lane == 0) tile_odd[warp] = odd;
         }
         if (__syncthreads_or(!ok)) break;
-        // A token's probabilities are zero beyond its own context, but the V rows there, of later tokens, are in the tiles: where one
-        // is not finite, zero times it would be NaN.  Then the tokens are taken one by one, the last first, and a token's V row is
-        // cleared behind it.
-        const bool one_by_one = (tile_odd[4] | tile_odd[5] | tile_odd[6] | tile_odd[7]) && n > 1 && pos < p0 + PM_CHUNK;
-        for (int hi = n, lo; hi > 0; hi = lo) {
-            lo = one_by_one ? hi - 1 : 0;
-            for (int sub = lo + warp * per_pass; sub < hi; sub += AT_WARPS * per_pass) {
-                // row g of A: query head g % gsize of token g / gsize of the pass
-                const int tok = g / gsize, last = min(sub + per_pass, hi);  // of the pass
-                const bool row_ok = tok < per_pass && sub + tok < hi;
-                const int t = t_lo + first + sub + (row_ok ? tok : 0);
-                const uint32_t row_len = s_pos[t - t_lo] + 1u, most = pos + (uint32_t)last;  // context of the row's token; the longest
-                if (most <= p0) continue;
-                const size_t row = (size_t)t * p.n_q_heads + (size_t)h * gsize + (row_ok ? g - tok * gsize : 0);
-                at_load_q<HD>(row_ok ? p.q + row * HD : nullptr, nullptr, 0, p.scale, qf, lane);
-                AtTiles tiles;
-                float M, L;
+        for (int sub = warp * per_pass; sub < n; sub += AT_WARPS * per_pass) {
+            // row g of A: query head g % gsize of token g / gsize of the pass
+            const int tok = g / gsize, last = min(sub + per_pass, n);  // of the pass
+            const bool row_ok = tok < per_pass && sub + tok < n;
+            const int t = t_lo + first + sub + (row_ok ? tok : 0);
+            const uint32_t row_len = s_pos[t - t_lo] + 1u, most = pos + (uint32_t)last;  // context of the row's token; the longest
+            if (most <= p0) continue;
+            // (32 bits, as the warp number is one per warp: what else is kept spills; 9 tokens in each of 64 sequences of 2000 439 us, 409 so)
+            const int row = t * p.n_q_heads + h * gsize + (row_ok ? g - tok * gsize : 0);
+            at_load_q<HD>(row_ok ? p.q + (size_t)row * HD : nullptr, nullptr, 0, p.scale, qf, lane);
+            AtTiles tiles;
+            float M, L;
 #pragma unroll 1
-                for (int w = 0; w < 4; ++w) {
-                    const uint32_t k0 = p0 + (uint32_t)w * PM_TILE;
-                    tiles.push();
-                    if (k0 >= most) continue;
-                    const uint32_t row_live = row_len <= k0 ? 0u : tile_live[w] & (row_len - k0 >= 32u ? 0xffffffffu : (1u << (row_len - k0)) - 1u);
-                    at_scores<HD>(rows, base + (uint32_t)(w * A::TILE), qf, row_live, lane, tiles.phi[0], tiles.plo[0], tiles.m[0], tiles.l[0]);
-                }
-                tiles.weigh(M, L);
-                float acc[A::NT][2];
+            for (int w = 0; w < 4; ++w) {
+                const uint32_t k0 = p0 + (uint32_t)w * PM_TILE;
+                tiles.push();
+                if (k0 >= most) continue;
+                const uint32_t row_live = row_len <= k0 ? 0u : tile_live[w] & (row_len - k0 >= 32u ? 0xffffffffu : (1u << (row_len - k0)) - 1u);
+                at_scores<HD>(rows, base + (uint32_t)(w * A::TILE), qf, row_live, lane, tiles.phi[0], tiles.plo[0], tiles.m[0], tiles.l[0]);
+            }
+            tiles.weigh(M, L);
+            float acc[A::NT][2];
 #pragma unroll
-                for (int k = 0; k < A::NT; ++k) acc[k][0] = acc[k][1] = 0.0f;
+            for (int k = 0; k < A::NT; ++k) acc[k][0] = acc[k][1] = 0.0f;
 #pragma unroll 1
-                for (int w = 0; w < 4 && p0 + (uint32_t)w * PM_TILE < most; ++w, tiles.shift())
-                    at_pv<HD>(rows, base + (uint32_t)((4 + w) * A::TILE), tiles.phi[3], tiles.plo[3], tiles.l[3], lane, acc);
-                if (row_ok && row_len > p0)
-                    at_store<HD>(p, partial, n_chunks, row, c, row_len <= (uint32_t)PM_CHUNK || n_chunks == 1, M, L, tq, acc);
-            }
-            if (one_by_one && lo > 0) {
-                __syncthreads();
-                const uint32_t own = pos + (uint32_t)lo - p0;  // position of token lo, in the chunk
-                if (pos + (uint32_t)lo >= p0 && own < PM_CHUNK && warp == 4 + (int)(own / PM_TILE)) {
-                    at_zero_rows<HD>(rows, base + (uint32_t)(warp * A::TILE), ~(1u << (own % PM_TILE)), lane);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                }
-                __syncthreads();
-            }
+            for (int w = 0; w < 4 && p0 + (uint32_t)w * PM_TILE < most; ++w, tiles.shift())
+                at_pv<HD>(rows, base + (uint32_t)((4 + w) * A::TILE), tiles.phi[3], tiles.plo[3], tiles.l[3], lane, acc);
+            if (row_ok && row_len > p0)
+                at_store<HD>(p, partial, n_chunks, row, c, row_len <= (uint32_t)PM_CHUNK || n_chunks == 1, M, L, tq, acc);
         }
     }
     if (!ok) {
@@ -637,18 +714,18 @@ static cudaError_t at_maps(const PagedParams &p, int head_dim, AttnMaps &maps) {
     return at_encode(&maps.v, p.kv_v, head_dim, p.block_shift);
 }
 
-bool attention_decode_supported(int n_tokens) { return n_tokens <= AT_MAX_TOKENS; }
+// Heads of 64 stay with paged_attention_mma_kernel: its small CTAs keep seven chunks of four warps on an SM, and a tile is too short to
+// pay for a warp's turn here (32 sequences of 1000, 16 heads of 64: 33 us there, 48 here; 32 heads on 8 of 128: 44 and 41).
+bool attention_decode_supported(int n_tokens, int head_dim) { return n_tokens <= AT_MAX_TOKENS && head_dim == 128; }
 
-cudaError_t launch_attention_decode(const PagedParams &p, int head_dim, int n_chunks, float *partial, const FusedDecode &fd, int *err,
+cudaError_t launch_attention_decode(const PagedParams &p, int n_chunks, float *partial, const FusedDecode &fd, int *err,
                                     cudaStream_t s) {
     AttnMaps maps;
-    if (cudaError_t e = at_maps(p, head_dim, maps)) return e;
+    if (cudaError_t e = at_maps(p, 128, maps)) return e;
     const long warps = (long)p.n_tokens * p.n_kv_heads * n_chunks, most = device_sm_count();
     const long ctas = (warps + AT_WARPS - 1) / AT_WARPS;
     const dim3 grid((unsigned)(ctas < most ? ctas : most));
-    const size_t smem = 1024 + AT_WARPS * (AT_RING_BYTES + (head_dim == 64 ? At<64>::Q_BYTES : At<128>::Q_BYTES));
-    return head_dim == 64 ? at_launch(attention_decode_kernel<64>, grid, smem, s, maps, p, n_chunks, partial, fd, err)
-                          : at_launch(attention_decode_kernel<128>, grid, smem, s, maps, p, n_chunks, partial, fd, err);
+    return at_launch(attention_decode_kernel<128>, grid, 1024 + AT_WARPS * (AT_RING_BYTES + At<128>::Q_BYTES), s, maps, p, n_chunks, partial, fd, err);
 }
 
 cudaError_t launch_attention_prompt(const PagedParams &p, int head_dim, int n_chunks, float *partial, int *err, cudaStream_t s) {
@@ -659,7 +736,8 @@ cudaError_t launch_attention_prompt(const PagedParams &p, int head_dim, int n_ch
     int block = AT_BLOCK;
     while (block > 1 && (long)p.n_kv_heads * n_chunks * ((p.n_tokens + block - 1) / block) < 2l * device_sm_count()) block /= 2;
     const dim3 grid((unsigned)p.n_kv_heads, (unsigned)((p.n_tokens + block - 1) / block), (unsigned)n_chunks);
-    const size_t smem = 1024 + 8 * (head_dim == 64 ? At<64>::TILE + At<64>::Q_BYTES : At<128>::TILE + At<128>::Q_BYTES);
+    auto bytes = [](int tiles, int tile, int q) { return (size_t)(1024 + tiles * tile + AT_WARPS * q); };
+    const size_t smem = head_dim == 64 ? bytes(At<64>::PROMPT_TILES, At<64>::TILE, At<64>::Q_BYTES) : bytes(At<128>::PROMPT_TILES, At<128>::TILE, At<128>::Q_BYTES);
     return head_dim == 64 ? at_launch(attention_prompt_kernel<64>, grid, smem, s, maps, p, block, n_chunks, partial, err)
                           : at_launch(attention_prompt_kernel<128>, grid, smem, s, maps, p, block, n_chunks, partial, err);
 }

@@ -312,6 +312,8 @@ __device__ __forceinline__ void kv_store(__half *p, float v) { *p = __float2half
 
 // K/V rows of the new tokens into the pool (f16 pools: round to nearest even, as the reference's NEON / F16C
 // conversions).  grid (T, kv_heads), threads over head_dim.
+__device__ __forceinline__ bool kv_finite(float) { return true; }  // (asked of f16 pools only)
+__device__ __forceinline__ bool kv_finite(__half v) { return (__half_as_ushort(v) & 0x7C00u) != 0x7C00u; }
 template <typename KV>
 __global__ void kv_append_kernel(PagedParams p, int head_dim) {
     MCU_PDL_PROLOGUE();
@@ -324,7 +326,10 @@ __global__ void kv_append_kernel(PagedParams p, int head_dim) {
     const size_t src = ((size_t)t * p.n_kv_heads + h) * head_dim;
     for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
         kv_store((KV *)p.kv_k + base + d, p.k_new[src + d]);
-        kv_store((KV *)p.kv_v + base + d, p.v_new[src + d]);
+        KV v;
+        kv_store(&v, p.v_new[src + d]);
+        ((KV *)p.kv_v)[base + d] = v;
+        if (p.odd_v != nullptr && !kv_finite(v)) *p.odd_v = 1;
     }
 }
 
@@ -491,14 +496,15 @@ __global__ void __launch_bounds__(32 * PA_MAX_GROUP) paged_attention_kernel(Page
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
-// Decode steps (at most one token per sequence in the call) only: the neighbours of the attention are folded into the
-// same launch.  RoPE: the query heads are rotated on their way into the A fragments, and the warp whose tile holds the
+// FUSED (decode steps: at most one token per sequence in the call) folds the neighbours of the attention into the same launch.  RoPE: the query heads are rotated on their way into the A fragments, and the warp whose tile holds the
 // token's own position rotates the new K row, converts K and V to f16 and puts them into its tile AND into the pool
 // (no other CTA of the launch reads that pool row: every other position belongs to an earlier step).  Merge: a CTA
 // that is alone on its token writes the output itself; otherwise each CTA writes its chunk state, takes a ticket, and
 // the CTA that draws the last ticket of a (token, KV head) merges the chunk states in chunk order -- the arithmetic of
 // paged_attention_merge_kernel, so both forms give the same bits.
-template <int HD>
+// Otherwise RoPE and the KV append have run, and every chunk's state is merged by paged_attention_merge_kernel: calls with few CTAs,
+// where four warps to a chunk are ahead of the prompt kernel's one (launch rule at mcu_paged_attention).
+template <int HD, bool FUSED>
 __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(PagedParams p, float *partial, FusedDecode fd) {
     constexpr int ROWB = HD * 2;            // bytes of a K or V row
     constexpr int PIECES = ROWB / 16;       // 16-byte pieces per row
@@ -525,9 +531,9 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
     const uint32_t sV = sK + TILEB;
     const uint32_t k0 = p0 + (uint32_t)(warp * PM_TILE);  // this warp's positions [k0, k0 + 32)
     const bool has_tile = k0 < p1;                        // uniform over the warp
-    // the token's own row (position kv_len - 1) comes from k_new / v_new, not from the pool
+    // FUSED: the token's own row (position kv_len - 1) comes from k_new / v_new, not from the pool
     const uint32_t new_pos = kv_len - 1u;
-    const int new_row = new_pos >= k0 && new_pos < k0 + PM_TILE ? (int)(new_pos - k0) : -1;
+    const int new_row = FUSED && new_pos >= k0 && new_pos < k0 + PM_TILE ? (int)(new_pos - k0) : -1;
     // stage the tile: lane r looks up the pool block of position k0 + r, the warp copies two rows per step
     uint32_t live = 0;
     if (has_tile) {
@@ -551,7 +557,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (new_row >= 0) {
+        if (FUSED && new_row >= 0) {
             // the new K row rotated, the new V row, both as f16: into this warp's tile and into the pool slot
             const int half = HD / 2, r = new_row;
             const float2 *rope = fd.rope + (size_t)t * half;
@@ -581,7 +587,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
     }
 
     // A fragments of Q (row g = query head g of the group): a0 = dims 16s + 2tq, +1; a2 = dims 16s + 8 + 2tq, +1.
-    // The values are rotated on the way (the partner of a dimension is its neighbour, or lies half a head
+    // FUSED: the values are rotated on the way (the partner of a dimension is its neighbour, or lies half a head
     // away with the NeoX pairing; either way this lane reads it itself).
     uint32_t qhi[KS][2], qlo[KS][2];
     {
@@ -595,7 +601,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
 #pragma unroll
             for (int hk = 0; hk < 2; ++hk)
                 qv[s][hk] = head_ok ? *(const float2 *)(qrow + 16 * s + 8 * hk + 2 * tq) : make_float2(0.0f, 0.0f);
-        {
+        if (FUSED) {
             const float2 *rope = fd.rope + (size_t)t * (HD / 2);
             if (!fd.neox) {  // the pair (d, d + 1) is one float2
                 float2 cs[KS][2];
@@ -752,7 +758,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
             L += s_l[w * 8 + hh] * e;
             O += s_o[((size_t)w * 8 + hh) * HD + d] * e;
         }
-        if (fd.tickets != nullptr && (kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1)) {  // the only chunk of its token: this is the result
+        if (FUSED && fd.tickets != nullptr && (kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1)) {  // the only chunk of its token: this is the result
             p.out[((size_t)t * p.n_q_heads + (size_t)h * gsize + hh) * HD + d] = L > 0.0f ? O / L : 0.0f;
             continue;
         }
@@ -766,7 +772,7 @@ __global__ void __launch_bounds__(32 * PM_WARPS) paged_attention_mma_kernel(Page
         }
         pr[2 + d] = O;
     }
-    if (kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1 || fd.tickets == nullptr) return;
+    if (!FUSED || kv_len <= (uint32_t)PM_CHUNK || n_chunks == 1 || fd.tickets == nullptr) return;
     // the last CTA of this (token, KV head) to finish merges the chunk states
     const int live_chunks = min(n_chunks, (int)((kv_len + (uint32_t)PM_CHUNK - 1u) / (uint32_t)PM_CHUNK));
     __threadfence();
@@ -846,6 +852,7 @@ paged_attention_merge_kernel(PagedParams p, int chunk, int n_chunks, int direct,
     const int lane = threadIdx.x & 31;
     const long pair = (long)blockIdx.x * MERGE_WARPS + (threadIdx.x >> 5);
     const int t = (int)(pair / p.n_q_heads);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && p.odd_v != nullptr) *p.odd_v = 0;  // for the next call
     if (t >= p.n_tokens) return;
     const uint32_t kv_len = p.meta[t * 4 + 1] + 1u;
     const int live = min(n_chunks, (int)((kv_len + (uint32_t)chunk - 1u) / (uint32_t)chunk));
@@ -1106,6 +1113,7 @@ int mcu_paged_attention(mcu_context_t *ctx, const uint32_t *token_meta_dev, size
     while (((size_t)1 << p.block_shift) < block_size) ++p.block_shift;
     p.scale = scale;
     p.n_tokens = (int)T;
+    p.odd_v = kv_dtype == MCU_KV_F16 ? context_odd_flag(ctx) : nullptr;
     if (n_q_heads / n_kv_heads > (size_t)PA_MAX_GROUP)
         return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention supports up to 8 query heads per KV head");
     // chunk of positions per CTA: long enough to amortise the set-up, short enough that every SM gets several CTAs
@@ -1123,17 +1131,30 @@ int mcu_paged_attention(mcu_context_t *ctx, const uint32_t *token_meta_dev, size
     if (int rc = context_attention_scratch(ctx, T * n_q_heads * n_chunks * (head_dim + 2) * sizeof(float), &scratch))
         return rc;
     float *partial = (float *)scratch;
-    const dim3 ag((unsigned)T, (unsigned)n_kv_heads);
+    const dim3 ag((unsigned)T, (unsigned)n_kv_heads), qg((unsigned)n_kv_heads, (unsigned)T, (unsigned)n_chunks);
+    // A CTA per token, KV head and chunk where that is a few rounds of the SMs; with long contexts (in which a prompt CTA finds little to
+    // share) some more, and more of the small CTAs of 64 dimensions (32 heads on 8 of 128, 18 tokens at 1000: 21 us, 25 as a prompt;
+    // 128 tokens at 30: 19, 17.8; 16 heads of 64, 18 tokens at 1000: 18, 22).  A single chunk of small groups: a prompt CTA, which takes
+    // two tokens at a time, is the faster one for few tokens too (32 heads on 8 of 128, 32 tokens at 30: 9.7, 8.0; 16 of 64, 16 at 64: 9.7, 7.2).
+    const size_t ctas = T * n_kv_heads * n_chunks, rounds = n_chunks == 1 && n_q_heads / n_kv_heads <= 4 ? 0 : n_chunks < 4 ? 6 : head_dim == 64 ? 18 : 10;
+    const bool by_token = mma_path && ctas <= rounds * (size_t)device_sm_count();
     if (mma_path) {
         DEC_CUDA(launch_pdl(kv_append_kernel<__half>, ag, dim3(128), s, p, (int)head_dim));
-        DEC_CUDA(launch_attention_prompt(p, (int)head_dim, (int)n_chunks, partial, context_err_flag(ctx), s));
+        if (by_token) {
+            const size_t smem = (size_t)PM_WARPS * 2 * PM_TILE * head_dim * 2;  // >= the warps' merge states (8 heads each)
+            auto kernel = head_dim == 64 ? paged_attention_mma_kernel<64, false> : paged_attention_mma_kernel<128, false>;
+            DEC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            DEC_CUDA(launch_pdl_smem(kernel, qg, dim3(32 * PM_WARPS), smem, s, p, partial, FusedDecode{}));
+        } else {
+            DEC_CUDA(launch_attention_prompt(p, (int)head_dim, (int)n_chunks, partial, context_err_flag(ctx), s));
+        }
     } else {
-        const dim3 qg((unsigned)n_kv_heads, (unsigned)T, (unsigned)n_chunks), tb(32u * (unsigned)(n_q_heads / n_kv_heads));
+        const dim3 tb(32u * (unsigned)(n_q_heads / n_kv_heads));
         DEC_CUDA(launch_pdl(kv_append_kernel<float>, ag, dim3(128), s, p, (int)head_dim));
         if (head_dim == 64) DEC_CUDA(launch_pdl(paged_attention_kernel<float, 64>, qg, tb, s, p, (int)chunk, partial));
         else DEC_CUDA(launch_pdl(paged_attention_kernel<float, 128>, qg, tb, s, p, (int)chunk, partial));
     }
-    DEC_CUDA(launch_merge(p, head_dim, chunk, n_chunks, mma_path, partial, s));
+    DEC_CUDA(launch_merge(p, head_dim, chunk, n_chunks, mma_path && !by_token, partial, s));
     count_launches(3);
     return MCU_SUCCESS;
 }
@@ -1205,6 +1226,7 @@ int mcu_paged_attention_decode(mcu_context_t *ctx, const uint32_t *token_meta_de
     while (((size_t)1 << p.block_shift) < block_size) ++p.block_shift;
     p.scale = scale;
     p.n_tokens = (int)T;
+    p.odd_v = nullptr;
     const size_t max_positions = max_blocks_per_seq * block_size;
     const size_t n_chunks = (max_positions + PM_CHUNK - 1) / PM_CHUNK;
     if (n_chunks > 6000) return set_error(MCU_ERROR_NOT_IMPLEMENTED, "paged_attention context bound too long");
@@ -1212,7 +1234,7 @@ int mcu_paged_attention_decode(mcu_context_t *ctx, const uint32_t *token_meta_de
     // CTAs: the fence and the ticket keep every CTA (and its shared memory) alive for a round trip to L2 longer, which
     // at 64 sequences x 8 KV heads x ~17 chunks cost 25 % of the kernel (measured); a merge kernel is cheaper there.
     const bool ticket_merge = n_kv_heads * T * n_chunks <= 4 * (size_t)device_sm_count();
-    const bool by_warp = !ticket_merge && attention_decode_supported((int)T);
+    const bool by_warp = !ticket_merge && attention_decode_supported((int)T, (int)head_dim);
     void *scratch = nullptr, *tickets = nullptr;
     if (int rc = context_attention_scratch(ctx, T * n_q_heads * n_chunks * (head_dim + 2) * sizeof(float), &scratch)) return rc;
     if (ticket_merge)
@@ -1230,13 +1252,13 @@ int mcu_paged_attention_decode(mcu_context_t *ctx, const uint32_t *token_meta_de
     const dim3 qg((unsigned)n_kv_heads, (unsigned)T, (unsigned)n_chunks);
     const size_t smem = (size_t)PM_WARPS * 2 * PM_TILE * head_dim * 2;
     if (by_warp) {
-        DEC_CUDA(launch_attention_decode(p, (int)head_dim, (int)n_chunks, (float *)scratch, fd, context_err_flag(ctx), s));
+        DEC_CUDA(launch_attention_decode(p, (int)n_chunks, (float *)scratch, fd, context_err_flag(ctx), s));
     } else if (head_dim == 64) {
-        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<64>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
+        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<64, true>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
     } else {
-        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<128>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
+        DEC_CUDA(cudaFuncSetAttribute(paged_attention_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        DEC_CUDA(launch_pdl_smem(paged_attention_mma_kernel<128, true>, qg, dim3(32 * PM_WARPS), smem, s, p, (float *)scratch, fd));
     }
     count_launches(1);
     if (!ticket_merge) {

@@ -157,6 +157,7 @@ struct mcu_context;
 namespace mcu {
 int context_device(const mcu_context *ctx);
 int *context_err_flag(mcu_context *ctx);
+int *context_odd_flag(mcu_context *ctx);  // zero between calls of mcu_paged_attention
 // workspace of the context for the split-KV attention partials (grows on demand)
 int context_attention_scratch(mcu_context *ctx, size_t bytes, void **out);
 int context_attention_tickets(mcu_context *ctx, size_t bytes, void **out);  // zero-filled counters

@@ -17,6 +17,7 @@ struct PagedParams {
     int n_q_heads, n_kv_heads, max_blocks, n_layers, layer, block_shift;
     float scale;
     int n_tokens;
+    int *odd_v;  // prompts: set by the append when a V value of the call is not finite, cleared by the merge
 };
 
 constexpr int PM_WARPS = 4;
@@ -59,8 +60,8 @@ struct FusedDecode {
 // One warp per (token, KV head, chunk), tiles by TMA (attention.cu): decode steps, RoPE and KV append included, and tokens whose K and
 // V rows are in the pool already.  Both leave chunk states for paged_attention_merge_kernel, except for tokens with a single
 // chunk, whose results they write.
-bool attention_decode_supported(int n_tokens);
-cudaError_t launch_attention_decode(const PagedParams &p, int head_dim, int n_chunks, float *partial, const FusedDecode &fd, int *err,
+bool attention_decode_supported(int n_tokens, int head_dim);
+cudaError_t launch_attention_decode(const PagedParams &p, int n_chunks, float *partial, const FusedDecode &fd, int *err,
                                     cudaStream_t s);
 cudaError_t launch_attention_prompt(const PagedParams &p, int head_dim, int n_chunks, float *partial, int *err, cudaStream_t s);
 
