@@ -202,10 +202,12 @@ inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
 
 // Microseconds of a call of 5 to 16 tokens on `row_tiles` tiles of 128 rows with the integer kernel, staging included, and on `groups`
 // groups of 64 rows with the mma.sync one: fitted to both at 5, 8, 9, 12 and 16 tokens, K 1024 to 14336 and 512 to 32000 rows (within
-// 10 % of all but a few).  A stage of the latter takes 2.25 or 2.45 us and its first ones are 8 to 11; the former's cycles are those
-// of its plan, which single waves, with SMs to spare, beat.
+// 10 % of all but a few).  A stage of the latter takes 2.35 or 2.45 us and its first ones are 8 to 10; the former's cycles are those
+// of its plan, which clusters on less than half of the SMs beat, and single waves, with SMs to spare.  (Q6_K, 8 tokens: 4096 x 1024 8.5 us
+// on 64 SMs here, 9.0 with the other; 2048 x 4096 9.8 on 128, 8.3; 14336 x 4096 23.7, 25.0, and with 16 tokens 28.8, 27.5.)
 inline double ti_us(int kind, int T, int K, int row_tiles, int sms) {
     const TsPlan pl = ti_plan(kind, row_tiles, (K + QK_K - 1) / QK_K, sms);
+    if (kind == KIND_Q6_K && pl.split > 1 && 2 * pl.n_cta <= sms) return (T <= 8 ? 2.5 : 1.35) + (T <= 8 ? 0.6 : 0.8) * 1e-3 * pl.cost;
     const bool wave = pl.split == 1 && pl.n_cta == row_tiles && row_tiles <= sms;
     return 4.6 + (T <= 8 ? (wave ? 0.47 : 0.57) : (wave ? 0.62 : 0.68)) * 1e-3 * pl.cost;
 }
@@ -214,7 +216,7 @@ inline double i8_us(int kind, int T, int K, int groups, int sms) {
     const int stages = ((K + QK_K - 1) / QK_K + I8_COLS_PER_STAGE - 1) / I8_COLS_PER_STAGE;  // of a group of rows
     const double per_cta = (double)groups * stages / sms;
     if (per_cta <= 1.0) return T <= 8 ? 7.2 + 0.47 * stages : 8.0 + 0.52 * stages;
-    return T <= 8 ? 10.5 + 2.25 * per_cta : 12.3 + 2.45 * per_cta;
+    return T <= 8 ? 10.4 + 2.35 * per_cta : 12.3 + 2.45 * per_cta;
 }
 // Does a matrix of F rows (two: `mats`) belong on the mma.sync kernel rather than the tcgen05 one?  Q4_K: rows of up to four blocks, a stage
 // for every CTA (5 us, 7 there whatever the size); larger ones never by more than a few per cent.  Q6_K: by the times above.
