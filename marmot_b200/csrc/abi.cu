@@ -1178,12 +1178,12 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
         uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
         float *dT = (float *)ctx->act_d.ptr, *part = (float *)ctx->gemm_partial.ptr;
         MCU_CUDA(launch_act_int_fused(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xq, dT, s));
-        MCU_CUDA(launch_gemm_ti_grouped(gate_kind, gate_up, 2, (int)e_count, xq, dT, (int)routes, (int)H, cnt, off, INT_MAX, part,
+        MCU_CUDA(launch_gemm_ti_grouped(gate_kind, gate_up, 2, (int)e_count, xq, dT, (int)routes, (int)H, cnt, off, part,
                                         ctx->gemm_counters, ctx->dev_err, s));
         ActSource down_src = from_glu;
         down_src.x_out = gate_out;  // (gate_out holds act(gate) * up afterwards, as with the per-expert launches)
         MCU_CUDA(launch_act_int_fused(down_kind, gate_out, (int)FF, down_src, (int)routes, (int)FF, xq, dT, s));
-        MCU_CUDA(launch_gemm_ti_grouped(down_kind, &down_job, 1, (int)e_count, xq, dT, (int)routes, (int)FF, cnt, off, INT_MAX, part,
+        MCU_CUDA(launch_gemm_ti_grouped(down_kind, &down_job, 1, (int)e_count, xq, dT, (int)routes, (int)FF, cnt, off, part,
                                         ctx->gemm_counters, ctx->dev_err, s));
         MCU_CUDA(launch_moe_combine_dev(route_down, rb.sorted_w, rb.route_pos, (int)T, (int)k, (int)H, rb.offsets, (int)e_begin,
                                         (int)(e_begin + e_count), rb.counts + E, capturing ? ctx->dev_err : nullptr, out_dev, H, s));
@@ -1217,9 +1217,9 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
         MCU_CUDA(launch_act_half_fused_from(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xh, rowscale, s));
         for (int j = 0; j < 2; ++j)
             MCU_CUDA(launch_gemm_ts_grouped(gate_kind, &gate_up[j], 1, (int)e_count, xh, rowscale, (int)kp_h, (int)routes, (int)H, cnt,
-                                            off, 1, part, tick, ctx->dev_err, s));
+                                            off, part, tick, ctx->dev_err, s));
         MCU_CUDA(launch_act_half_fused_from(down_kind, gate_out, (int)FF, from_glu, (int)routes, (int)FF, xh, rowscale, s));
-        MCU_CUDA(launch_gemm_ts_grouped(down_kind, &down_job, 1, (int)e_count, xh, rowscale, (int)kp_f, (int)routes, (int)FF, cnt, off, 1,
+        MCU_CUDA(launch_gemm_ts_grouped(down_kind, &down_job, 1, (int)e_count, xh, rowscale, (int)kp_f, (int)routes, (int)FF, cnt, off,
                                         part, tick, ctx->dev_err, s));
         if (routed_rows_ext == nullptr) {
             MCU_CUDA(launch_moe_combine_dev(route_down, rb.sorted_w, rb.route_pos, (int)T, (int)k, (int)H, rb.offsets,

@@ -66,13 +66,6 @@ struct GemmI8Params {
     int tx_bytes;                                // bytes the copies of one stage deliver
 };
 
-// first stage unit of CTA c of C
-__host__ __device__ inline int i8_span_begin(int SU, int c, int C) { return (int)(((long long)SU * c) / C); }
-// the CTA whose span holds stage unit x
-__host__ __device__ inline int i8_owner(int SU, int x, int C) {
-    return (int)((((long long)(x + 1) * C + SU - 1) / SU) - 1);
-}
-
 __device__ __forceinline__ void mma_s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                            uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"

@@ -39,7 +39,6 @@ struct TsParams {
     int split;              // > 1: clusters of `split` CTAs (pairs) share a tile along K; otherwise ranges of units
     int tiles, t_tiles;     // output tiles in all; token tiles per row tile
     int groups, row_tiles;  // grouped launches: number of groups, row tiles per group
-    int count_lo, count_hi; // grouped launches: groups with a count in this range
 };
 
 // One output tile: which weights, which tokens, where the result goes.
@@ -218,6 +217,10 @@ inline double i8_us(int kind, int T, int K, int groups, int sms) {
     if (per_cta <= 1.0) return T <= 8 ? 7.2 + 0.47 * stages : 8.0 + 0.52 * stages;
     return T <= 8 ? 10.4 + 2.35 * per_cta : 12.3 + 2.45 * per_cta;
 }
+// The mma.sync kernel's stage units: the first one of CTA c of C, and the CTA whose span holds unit x.
+MCU_HD int i8_span_begin(int SU, int c, int C) { return (int)(((long long)SU * c) / C); }
+MCU_HD int i8_owner(int SU, int x, int C) { return (int)((((long long)(x + 1) * C + SU - 1) / SU) - 1); }
+
 // Does a matrix of F rows (two: `mats`) belong on the mma.sync kernel rather than the tcgen05 one?  Q4_K: rows of up to four blocks, a stage
 // for every CTA (5 us, 7 there whatever the size); larger ones never by more than a few per cent.  Q6_K: by the times above.
 inline bool i8_pays(int kind, int T, int K, int F, int mats, int sms) {

@@ -16,14 +16,15 @@
 //
 // Work is divided as in gemm_ts.cu: one tile per CTA, a tile over a cluster, or equal ranges of slabs.
 //
-// Measured, staging included, against the kernels it took the place of (mma.sync, dp4a): Q4_K 8 x 4096 x 14336 19.5 -> 13.6 us
-// (2.4 TB/s), 16 tokens 22.4 -> 16.0, 8 x 4096 x 4096 12.1 -> 9.1; Q6_K 8 x 4096 x 14336 25.1 -> 22.3.  A slab costs the Q4_K
-// scalers and converters about 500 cycles, the Q6_K ones (eighteen products of 32 columns, 4 KB of sums per row) 900: those
-// bound Q6_K, the kernel's prologue, staging launch and first loads (about 5 us) the small sizes.
+// Measured, staging included, against the kernels that had these calls (mma.sync, dp4a): Q4_K 8 x 4096 x 14336 19.9 -> 13.5 us
+// (2.4 TB/s), 16 tokens 22.4 -> 16.0, 8 x 4096 x 4096 12.3 -> 9.3; Q6_K 8 x 4096 x 14336 25.2 -> 21.8.  The mma.sync kernel keeps the
+// calls of up to 16 tokens for which it is the faster one (gemm_i8.cu; i8_pays in gemm_plan.h).  A slab costs the Q4_K scalers and
+// converters 500 to 700 cycles by their own stamps, the Q6_K ones (eighteen products of 32 columns, 4 KB of sums per row) 900 to 1800; a
+// CTA's time grows by 900 and 2100 with each (ti_plan).  Those bound Q6_K, the kernel's prologue, staging launch and first loads (about
+// 5 us) the small sizes.
 #include "gemm_ts_dev.cuh"
 
 #include <atomic>
-#include <climits>
 #include <cstring>
 #include <type_traits>
 
@@ -622,13 +623,13 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
 }
 
 cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq, const float *dT,
-                                   int total_rows, int K, const int *group_counts, const int *group_offsets, int count_hi, float *partial,
+                                   int total_rows, int K, const int *group_counts, const int *group_offsets, float *partial,
                                    int *counters, int *err_flag, cudaStream_t s) {
     if (n_groups <= 0 || total_rows <= 0) return cudaSuccess;
     if (n_jobs < 1 || n_jobs > TS_MAX_JOBS || n_groups > TS_MAX_GROUPS) return cudaErrorInvalidValue;
     TsParams p;
     TsMaps maps;
-    if (cudaError_t e = ts_grouped_params(kind, jobs, n_jobs, n_groups, total_rows, K, group_counts, group_offsets, 1, count_hi, p, maps))
+    if (cudaError_t e = ts_grouped_params(kind, jobs, n_jobs, n_groups, total_rows, K, group_counts, group_offsets, p, maps))
         return e;
     p.bn = TI_COLS;
     p.rowscale = dT;

@@ -16,11 +16,11 @@
 //                 multiples (Q6_K with K % 2048 != 0) come as eight copies of every eighth row: eight rows always are.
 //
 // Measured (whole mcu_linear call, graph replay, microseconds before -> now): Q4_K 64 x 4096 x 14336 31.0 -> 18.0,
-// 17 x 4096 x 4096 12.8 -> 10.4, 64 x 4096 x 1024 18.5 -> 9.8, 2048 x 4096 x 14336 274 -> 214 (1120 TFLOP/s: 0.82 of the
-// sustained cuBLAS rate, the clock is at the power limit); Q6_K 37 x 14336 x 4096 39.6 -> 29.4, 512 x 5632 x 2048 142 -> 43.
-// Up to 128 tokens the converters bound a slab (about 1500 cycles for 32768 weights, instruction issue); from 256 on the MMAs
-// run at their peak rate (2075 cycles per slab) and what is left is the epilogue (4000 cycles of a tile's 37000).  Beside the
-// kernel a call has its staging launch: of the 17 us at 64 x 4096 x 14336 it and the releases around it take 6.5.
+// 17 x 4096 x 4096 13.2 -> 10.5, 64 x 4096 x 1024 17.2 -> 9.6, 2048 x 4096 x 14336 274 -> 213 (1130 TFLOP/s: 0.82 of the
+// sustained cuBLAS rate, the clock is at the power limit); Q6_K 32 x 14336 x 4096 37.1 -> 29.8, 512 x 5632 x 2048 142 -> 30.3.
+// Up to 128 tokens the converters bound a slab (Q4_K about 1100 cycles for 32768 weights in tiles of up to 64 tokens, 1500 in wider ones;
+// instruction issue); from 256 on the MMAs run at their peak rate (2075 cycles per slab) and what is left is the epilogue (4000 cycles of
+// a tile's 37000).  Beside the kernel a call has its staging launch: of the 18 us at 64 x 4096 x 14336 it and the releases around it take 6.5.
 //
 // A CTA has one output tile, or a cluster shares one along K and adds its shares up through distributed shared memory, or the slabs of
 // all tiles are cut into equal ranges: a tile cut between CTAs is then summed from partial tiles by the one that draws the last
@@ -34,14 +34,12 @@
 #include <cuda.h>
 
 #include <atomic>
-#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
 
 namespace mcu {
 
-constexpr int TS_BK = 128;      // values of K per stage, half a slab: eight MMAs per barrier wait and commit (see the issuer)
 constexpr int TS_STAGES = 4;    // = converter groups: group g owns stage slot g, so every barrier phase is seen in order
 constexpr int TS_CONV = 16;     // converter warps
 constexpr int TS_MMA_WARP = TS_CONV, TS_B_WARP = TS_CONV + 1, TS_W_WARP = TS_CONV + 2;
@@ -225,8 +223,8 @@ __device__ __forceinline__ void ts_store16(float *outp, int ldo, int col0, int c
     }
 }
 
-// LOOSE: the weight rows are not 16-byte multiples.  (Decided in the kernel, it costs aligned rows 5 % in Q6_K: 256 routes to 8 experts of
-// 3 x 14336 x 4096 475 us, 499.)
+// LOOSE: the weight rows are not 16-byte multiples.  (A branch in the kernel costs the aligned rows registers, in Q6_K most: 256
+// routes to 8 experts of 3 x 14336 x 4096 499 us, 461 so.)
 template <int KIND, bool LOOSE>
 __global__ void __launch_bounds__(TS_THREADS, 1)
 gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsParams p) {
@@ -767,7 +765,7 @@ bool gemm_ts_grouped_supported(int kind, const void *W, int K, int F) {
 
 // What grouped launches share: the weights and the tiles (activations and their map are the caller's).
 cudaError_t ts_grouped_params(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, int total_rows, int K,
-                              const int *group_counts, const int *group_offsets, int count_lo, int count_hi, TsParams &p, TsMaps &maps) {
+                              const int *group_counts, const int *group_offsets, TsParams &p, TsMaps &maps) {
     memset(&p, 0, sizeof(p));
     p.nb = (K + block_values(kind) - 1) / block_values(kind);
     p.row_bytes = (long)p.nb * block_bytes(kind);
@@ -776,8 +774,6 @@ cudaError_t ts_grouped_params(int kind, const GemvJobSpec *jobs, int n_jobs, int
     p.split = 1;
     p.T = total_rows;
     p.groups = n_groups;
-    p.count_lo = count_lo;
-    p.count_hi = count_hi;
     p.group_counts = group_counts;
     p.group_offsets = group_offsets;
     for (int j = 0; j < n_jobs; ++j) {
@@ -799,7 +795,7 @@ cudaError_t ts_grouped_params(int kind, const GemvJobSpec *jobs, int n_jobs, int
 // n_groups matmuls over stacked weight matrices (MoE experts): group g multiplies its group_counts[g] rows of xh (from row
 // group_offsets[g], both device data) with the weight rows [g * F, (g + 1) * F) of every job.
 cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const __half *xh, const float *rowscale,
-                                   int ldxh, int total_rows, int K, const int *group_counts, const int *group_offsets, int count_lo,
+                                   int ldxh, int total_rows, int K, const int *group_counts, const int *group_offsets,
                                    float *partial, int *counters, int *err_flag, cudaStream_t s) {
     if (n_groups <= 0 || total_rows <= 0) return cudaSuccess;
     if (n_jobs < 1 || n_jobs > TS_MAX_JOBS) return cudaErrorInvalidValue;
@@ -813,14 +809,14 @@ cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
                     (size_t)g * jobs[j].F * ((K + block_values(kind) - 1) / block_values(kind)) * block_bytes(kind);
             }
             if (cudaError_t e = launch_gemm_ts_grouped(kind, part, n_jobs, n, xh, rowscale, ldxh, total_rows, K, group_counts + g,
-                                                       group_offsets + g, count_lo, partial, counters, err_flag, s))
+                                                       group_offsets + g, partial, counters, err_flag, s))
                 return e;
         }
         return cudaSuccess;
     }
     TsParams p;
     TsMaps maps;
-    if (cudaError_t e = ts_grouped_params(kind, jobs, n_jobs, n_groups, total_rows, K, group_counts, group_offsets, count_lo, INT_MAX, p, maps))
+    if (cudaError_t e = ts_grouped_params(kind, jobs, n_jobs, n_groups, total_rows, K, group_counts, group_offsets, p, maps))
         return e;
     // The counts are not known here: tiles for an even spread, up to 256 tokens.
     const int even = (total_rows + n_groups - 1) / n_groups;

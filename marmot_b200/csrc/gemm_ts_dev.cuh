@@ -72,15 +72,13 @@ __device__ __forceinline__ void ts_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         : "memory");
 }
 
-// The first tile of every group of a grouped launch (one warp).  Groups with a count outside [count_lo, count_hi] are another
-// launch's.  May be called before griddepcontrol.wait: the staging kernel ahead lets this one start only after its own wait, when the
+// The first tile of every group of a grouped launch (one warp).  May be called before griddepcontrol.wait: the staging kernel ahead lets this one start only after its own wait, when the
 // kernels that wrote the counts are complete (stage_begin in act_quant.cu).
 __device__ __forceinline__ void ts_group_table(const TsParams &p, int bn, int *group_tile0, int lane) {
     int base = 0;
     for (int g0 = 0; g0 < p.groups; g0 += 32) {
         const int g = g0 + lane;
-        const int count = g < p.groups ? p.group_counts[g] : 0;
-        int n = count >= p.count_lo && count <= p.count_hi ? (count + bn - 1) / bn * p.row_tiles : 0;
+        int n = g < p.groups ? (p.group_counts[g] + bn - 1) / bn * p.row_tiles : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int up = __shfl_up_sync(0xffffffffu, n, o);

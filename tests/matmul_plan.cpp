@@ -119,3 +119,7 @@ extern "C" int check_groups(int slabs, const int *counts, int groups, const int 
     p.group_offsets = offsets.data();
     return check(p, bn, sms, sms, tile0.data(), want);
 }
+
+// the mma.sync kernel's division
+extern "C" int i8_begin(int SU, int c, int C) { return i8_span_begin(SU, c, C); }
+extern "C" int i8_holder(int SU, int x, int C) { return i8_owner(SU, x, C); }

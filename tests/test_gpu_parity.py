@@ -157,23 +157,6 @@ def test_gemm_tensor_core_vs_oracle(ctx, oracle, name, T, K, F):
     assert cosine(got, ref) >= 0.999
 
 
-def test_register_operand_kernel_on_q4_k():
-    """Q6_K takes the register-operand (mma.sync) kernel for 8 < T <= 64 by default; Q4_K only behind a switch that is
-    read once per process, so its parity cases run in a child process with the switch set."""
-    import os
-    import subprocess
-    import sys
-
-    from pathlib import Path
-
-    REPO_ROOT = Path(__file__).resolve().parents[1]
-    env = {**os.environ, "MARMOT_CUDA_GEMM_WARP_Q4K": "1"}
-    r = subprocess.run([sys.executable, "-m", "pytest", "tests/test_gpu_parity.py", "-x", "-q", "-k",
-                        "(test_gemm_tensor_core_vs_oracle or test_dual_output_equals_two_singles) and q4_k"],
-                       cwd=REPO_ROOT, env=env, capture_output=True, text=True, timeout=600)
-    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
-
-
 def test_config_q8_0_prefill_gemm_full_size(ctx, oracle):
     """Q8_0 prefill GEMM, 512 tokens x K = 4096 x F = 14336, with the benchmark's value distributions."""
     kind, T, K, F = KIND_Q8_0, 512, 4096, 14336
@@ -504,19 +487,17 @@ def test_moe_duplicate_routes_and_unused_experts(ctx, oracle):
     assert e.value.code == -1
 
 
-# ---- few tokens on integer tensor-core instructions (csrc/gemm_i8.cu) ----
+# ---- few tokens on integer tensor-core instructions (csrc/gemm_ti.cu) ----
 @pytest.mark.parametrize("name", ["q4_k", "q6_k"])
 @pytest.mark.parametrize("T,K,F", [(2, 4096, 4096), (5, 2048, 200), (8, 4096, 1024), (9, 2048, 333), (16, 4096, 14336),
                                    (33, 2048, 64), (64, 4096, 4096), (64, 14336, 512), (3, 2048 + 256 * 5, 96)])
 def test_integer_mma_matmul_vs_oracle(ctx, oracle, name, T, K, F):
-    """2..64 tokens take the mma.sync s8 kernel: exact integer sub-block dots, so the result must sit at the
-    fp32-accumulate tolerance whatever the token count; row groups that span several CTAs (and several row groups in
-    one CTA), a ragged last row group, bias, and a strided input are all in the list."""
+    """2..64 tokens on the tcgen05 integer kernel: exact integer sub-block dots, so the result must sit at the
+    fp32-accumulate tolerance whatever the token count; tiles cut between CTAs and shared by clusters, a ragged last row
+    tile, Q6_K rows off 16 bytes, bias, and a strided input are all in the list."""
     import torch
 
     kind = KINDS[name]
-    if kind == KINDS["q6_k"] and (K // 256) % 8:
-        K = (K // 2048 + 1) * 2048  # Q6_K rows must be 16-byte multiples for the tensor map
     rng = np.random.default_rng(T * 131 + F)
     W = random_blocks(kind, F, K, rng)
     ldx = K + 8
