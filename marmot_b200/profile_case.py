@@ -3,6 +3,7 @@ self-ending command that a profiler (ncu) or a quick timing wraps.
 
     python -m marmot_b200.profile_case --kind q4_k -T 1 -K 4096 -F 4096 --copies 16 --iters 3
     python -m marmot_b200.profile_case --op attention --seqs 64 --ctx 2048 --layers 4 --iters 2 --time
+    python -m marmot_b200.profile_case --op attention --seqs 1 --ctx 0 --new 500 --time    (a prompt)
     python -m marmot_b200.profile_case --op attention --decode --seqs 1 --ctx 250 --q-heads 32 --kv-heads 4 --head-dim 64
     python -m marmot_b200.profile_case --op layer --layers 22 --iters 2 --time      (the decode step's five kernels)
     python -m marmot_b200.profile_case --op step --ctx 250 --iters 3 --time         (one-token step: the persistent kernel)
@@ -24,32 +25,33 @@ REGIMES = {"auto": 0, "gemv": 1, "gemm": 2, "gemv_plain": 3, "i8mma": 4}
 
 
 def attention_case(args) -> None:
-    """Decode-step attention: `seqs` sequences of `ctx` cached positions each, one new token per sequence, the layers of
+    """Attention: `seqs` sequences of `ctx` cached positions each, `new` tokens per sequence (one: a decode step), the layers of
     the pool visited in turn (so that consecutive calls read different memory).  Pool bytes read per call:
-    2 (K and V) * seqs * (ctx + 1) * kv_heads * head_dim * element size."""
+    2 (K and V) * seqs * (ctx + new) * kv_heads * head_dim * element size."""
     import torch
 
     dev = torch.device("cuda", 0)
     ctx = Context(0)
     hq, hkv, hd, bs, L = args.q_heads, args.kv_heads, args.head_dim, 16, args.layers
     kv_dtype = torch.float16 if args.kv == "f16" else torch.float32
-    per_seq = (args.ctx + 1 + bs - 1) // bs
+    new, T = args.new, args.seqs * args.new
+    per_seq = (args.ctx + new + bs - 1) // bs
     n_blocks = args.seqs * per_seq
     gen = torch.Generator(device=dev).manual_seed(0)
     kv_k = torch.randn((n_blocks, L, hkv, bs, hd), device=dev, generator=gen).to(kv_dtype)
     kv_v = torch.randn((n_blocks, L, hkv, bs, hd), device=dev, generator=gen).to(kv_dtype)
     table = torch.arange(n_blocks, dtype=torch.int32, device=dev).view(args.seqs, per_seq).contiguous()
-    meta = np.zeros((args.seqs, 4), dtype=np.uint32)
-    meta[:, 0] = np.arange(args.seqs)
-    meta[:, 1] = args.ctx
-    meta[:, 2] = np.arange(args.seqs) * per_seq * bs + args.ctx
+    meta = np.zeros((T, 4), dtype=np.uint32)
+    meta[:, 0] = np.repeat(np.arange(args.seqs), new)
+    meta[:, 1] = args.ctx + np.tile(np.arange(new), args.seqs)
+    meta[:, 2] = meta[:, 0] * per_seq * bs + meta[:, 1]
+    pos = torch.from_numpy(meta[:, 1].astype(np.int32)).to(dev)
     meta = torch.from_numpy(meta.view(np.int32)).to(dev)
-    q = torch.randn((args.seqs, hq * hd), device=dev, generator=gen)
-    k = torch.randn((args.seqs, hkv * hd), device=dev, generator=gen)
-    v = torch.randn((args.seqs, hkv * hd), device=dev, generator=gen)
+    q = torch.randn((T, hq * hd), device=dev, generator=gen)
+    k = torch.randn((T, hkv * hd), device=dev, generator=gen)
+    v = torch.randn((T, hkv * hd), device=dev, generator=gen)
     out = torch.empty_like(q)
 
-    pos = torch.full((args.seqs,), args.ctx, dtype=torch.int32, device=dev)
     rope = ctx.rope_table(pos, hd, 500000.0)
 
     def one_pass():
@@ -66,8 +68,8 @@ def attention_case(args) -> None:
         for _ in range(args.iters):
             one_pass()
     torch.cuda.synchronize()
-    nbytes = 2 * args.seqs * (args.ctx + 1) * hkv * hd * kv_k.element_size()
-    print(f"attention seqs={args.seqs} ctx={args.ctx} heads={hq}/{hkv}x{hd} kv={args.kv}: {L} layers, {args.iters} passes, "
+    nbytes = 2 * args.seqs * (args.ctx + new) * hkv * hd * kv_k.element_size()
+    print(f"attention seqs={args.seqs} ctx={args.ctx} new={new} heads={hq}/{hkv}x{hd} kv={args.kv}: {L} layers, {args.iters} passes, "
           f"{ctx.launch_count()} kernel launches, {nbytes} pool bytes per call, pool {2 * kv_k.numel() * kv_k.element_size() >> 20} MiB")
     if args.time:
         graph = torch.cuda.CUDAGraph()
@@ -293,7 +295,8 @@ def main() -> None:
     ap.add_argument("--decode", action="store_true", help="attention: the one-launch decode form (RoPE + append + merge folded in)")
     ap.add_argument("--experts", type=int, default=8, help="moe: experts")
     ap.add_argument("--top-k", type=int, default=2, help="moe: routes per token")
-    ap.add_argument("--seqs", type=int, default=64, help="attention: sequences (one new token each)")
+    ap.add_argument("--seqs", type=int, default=64, help="attention: sequences")
+    ap.add_argument("--new", type=int, default=1, help="attention: new tokens per sequence")
     ap.add_argument("--ctx", type=int, default=2048, help="attention: cached positions per sequence")
     ap.add_argument("--layers", type=int, default=4, help="attention: layers in the pool, visited in turn")
     ap.add_argument("--q-heads", type=int, default=32)

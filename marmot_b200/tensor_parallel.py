@@ -50,7 +50,7 @@ def shard_rows(blocks: np.ndarray, kind: int, F: int, K: int, world: int, rank: 
 
 def k_granule(kind: int, K: int) -> int:
     """Granule (in values) for splitting K: the smallest run of blocks whose bytes are a multiple of 16, so that
-    every shard's rows stay 16-byte multiples and the TMA-fed matmul applies (Q4_K: 256, Q6_K: 2048, Q8_0: 256);
+    every shard's rows stay 16-byte multiples and the matmul fused with its all-reduce applies (Q4_K: 256, Q6_K: 2048, Q8_0: 256);
     the block size when K is not a multiple of that."""
     bv, bb = BLOCK_VALUES[kind], BLOCK_BYTES[kind]
     blocks = 16 // np.gcd(bb, 16)
