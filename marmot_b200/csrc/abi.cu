@@ -602,6 +602,8 @@ static int i8_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, con
     gemm_i8_workspace_bytes((int)T, (int)K, (int)F, w2 != nullptr, &qs_b, &dT_b, &part_b, &tick_b);
     if (int rc = ensure(ctx, ctx->act_qs, qs_b)) return rc;
     if (int rc = ensure(ctx, ctx->act_d, dT_b)) return rc;
+    // (the shares for any call of the context, and tickets for a million rows: a recorded call keeps their addresses when larger ones follow)
+    tick_b = tick_b > (size_t)256 << 10 ? tick_b : (size_t)256 << 10;
     if (int rc = ensure(ctx, ctx->i8_partial, part_b)) return rc;
     if (tick_b > ctx->i8_tickets.cap) {  // a fresh ticket area starts at zero; the kernel keeps it so
         if (int rc = ensure(ctx, ctx->i8_tickets, tick_b)) return rc;

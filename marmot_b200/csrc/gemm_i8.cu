@@ -473,7 +473,7 @@ void gemm_i8_workspace_bytes(int T, int K, int F, bool dual, size_t *qs_bytes, s
     const int RG = (F + I8_ROWS - 1) / I8_ROWS;
     *qs_bytes = (size_t)Tpad * nb * QK_K;
     *dT_bytes = (size_t)nb * Tpad * (sizeof(float) + 8 * sizeof(int16_t));  // scales, then the sub-block sums
-    *partial_bytes = (size_t)device_sm_count() * 2 * I8_WM * (Tpad / 8) * 4 * 32 * sizeof(float);
+    *partial_bytes = (size_t)device_sm_count() * 2 * I8_WM * (I8_MAX_T / 8) * 4 * 32 * sizeof(float);  // (whatever T is)
     *ticket_bytes = (size_t)RG * (dual ? 2 : 1) * I8_WM * sizeof(int);
 }
 

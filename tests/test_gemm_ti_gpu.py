@@ -324,3 +324,34 @@ def test_mma_sync_sizes(ctx, oracle, kind, T, K, F):
     ctx.synchronize()
     assert max_rel_err(a.cpu().numpy(), oracle.linear(kind, x, W, F)) <= 2e-5
     assert max_rel_err(b.cpu().numpy(), oracle.linear(kind, x, W2, F)) <= 2e-5
+
+
+def test_recorded_mma_sync_call_keeps_its_workspace(ctx, oracle):
+    """A recorded call replays after calls of more rows and of more tokens per tile: shares and tickets stay where they were."""
+    import torch
+    from marmot_b200 import Context
+
+    T, K, F, more = 16, 2048, 20003, 40001
+    rng = np.random.default_rng(F)
+    W, W2 = random_blocks(KIND_Q6_K, F, K, rng), random_blocks(KIND_Q6_K, more, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    c = Context(0, use_torch_stream=False)  # (a workspace of its own)
+    stream = torch.cuda.Stream()
+    c.set_stream(stream.cuda_stream)
+    with torch.cuda.stream(stream):
+        xd, wd, wd2 = torch.from_numpy(x).cuda(), c.upload(W), c.upload(W2)
+        out = torch.empty((8, F), device="cuda")
+        c.linear(KIND_Q6_K, xd, wd, F)  # (the staged activations of sixteen tokens are reserved)
+        c.linear(KIND_Q6_K, xd[:8], wd, F, out=out)
+        first = out.clone()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            c.linear(KIND_Q6_K, xd[:8], wd, F, out=out)
+        c.linear(KIND_Q6_K, xd, wd2, more)
+        out.zero_()
+        g.replay()
+        c.synchronize()
+        assert torch.equal(out, first)
+        del g
+    assert max_rel_err(first.cpu().numpy(), oracle.linear(KIND_Q6_K, x[:8], W, F)) <= 2e-5
+    c.close()
