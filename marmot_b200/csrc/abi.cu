@@ -1139,7 +1139,9 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     // an expert whatever its size, and take it for large experts only.  Rows per expert, here and there, us at 4 experts of 3 x 14336 x 4096:
     // Q4_K 16 238, 265; 32 262 to 317, 273; 48 375, 282.  Q6_K down 16 279, 313; 32 348, 314.  Q6_K 12 278, 332; 16 402, 348; 48 756, 373.
     // At 4 of 3 x 5632 x 2048: Q4_K 48 122, 140; 63 165, 156.  Q6_K down 48 158, 166; 60 195, 174.  Q6_K 32 153 to 174, 174; 48 206, 176.
-    // Next to no routes leave most experts out: 1 token of 8 experts of 3 x 14336 x 4096 107, 92; all Q6_K 199, 110, and 2 rows 428 to 728, 352 to 429.
+    // A single route leaves all other experts out (3 x 5632 x 2048 Q4_K 55, 45; 3 x 14336 x 4096 73, 66; all Q6_K 97, 75), where two cost more
+    // so (93, 102), and so do few routes of large experts in Q6_K, whose launches are the streaming kernels' (8 experts of 3 x 14336 x 4096,
+    // 3, 8, 12, 16 routes: 174, 149; 326, 302; 372, 378; 413, 444.  16 of 3 x 7168 x 4096, 3, 8, 12: 120, 110; 208, 212; 274, 292).
     const size_t n6 = (gate_kind == KIND_Q6_K ? 1 : 0) + (down_kind == KIND_Q6_K ? 1 : 0);
     const bool large = H * FF > (size_t)26 << 20, capturing = stream_is_capturing(s);
     const size_t most_rows = (large ? 48 : 128) / (2 + n6);
@@ -1151,8 +1153,8 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
         gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) && gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H);
     // A recorded call cannot read the counts: this kernel or the grouped fp16 one.
     const bool few_recorded = few_suits && (routes <= most_rows * E || !fp16_suits);
-    const bool few = capturing ? few_recorded
-                               : few_suits && routes <= most_rows * E && routes * 4 > E && (!large || n6 < 2 || routes >= 4 * E);
+    const size_t apart = large && n6 == 2 ? (E < 8 ? E : 8) : 1;  // most routes that go expert by expert for being few
+    const bool few = capturing ? few_recorded : few_suits && routes <= most_rows * E && routes > apart;
     auto few_workspace = [&]() -> int {
         const size_t xq_h = gemm_ti_xq_bytes(gate_kind, (int)routes, (int)H), xq_f = gemm_ti_xq_bytes(down_kind, (int)routes, (int)FF);
         const size_t nb_max = ((H > FF ? H : FF) + QK_K - 1) / QK_K;

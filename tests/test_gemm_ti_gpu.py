@@ -267,7 +267,7 @@ def test_rows_longer_than_the_static_shared_memory(ctx, oracle, kind, T, K):
     assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= 5e-5
 
 
-@pytest.mark.parametrize("kind,T,E,k", [(KIND_Q6_K, 40, 4, 4), (KIND_Q4_K, 1, 8, 2), (KIND_Q6_K, 9, 3, 2)])
+@pytest.mark.parametrize("kind,T,E,k", [(KIND_Q6_K, 40, 4, 4), (KIND_Q4_K, 1, 8, 1), (KIND_Q4_K, 1, 8, 2), (KIND_Q6_K, 9, 3, 2)])
 def test_recorded_moe_after_an_eager_call(ctx, oracle, kind, T, E, k):
     """Few-route calls that go expert by expert when the counts can be read (many rows or next to none per expert) can still be recorded
     after one eager call, and give the same up to a re-quantised intermediate; an id out of range leaves the output alone."""
