@@ -621,18 +621,15 @@ static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K
 }
 static int integer_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, const GemvJobSpec *jobs, int n_jobs,
                           const ActSource *src, int *staged_kind) {
-    const size_t nb = (K + QK_K - 1) / QK_K;
     if (int rc = ensure(ctx, ctx->act_qs, gemm_ti_xq_bytes(kind, (int)T, (int)K))) return rc;
-    if (int rc = ensure(ctx, ctx->act_d, T * nb * sizeof(float))) return rc;
     if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
     uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
-    float *dT = (float *)ctx->act_d.ptr;
     if (staged_kind == nullptr || *staged_kind != kind) {
-        MCU_CUDA(launch_act_int_fused(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K, xq, dT, ctx->stream));
+        MCU_CUDA(launch_act_int_fused(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K, xq, ctx->stream));
         count_launches(1);
         if (staged_kind != nullptr) *staged_kind = kind;
     }
-    MCU_CUDA(launch_gemm_ti(kind, jobs, n_jobs, xq, dT, (int)T, (int)K, (float *)ctx->gemm_partial.ptr, ctx->gemm_counters, ctx->dev_err,
+    MCU_CUDA(launch_gemm_ti(kind, jobs, n_jobs, xq, (int)T, (int)K, (float *)ctx->gemm_partial.ptr, ctx->gemm_counters, ctx->dev_err,
                             ctx->stream));
     count_launches(1);
     return MCU_SUCCESS;
@@ -1157,9 +1154,7 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     const bool few = capturing ? few_recorded : few_suits && routes <= most_rows * E && routes > apart;
     auto few_workspace = [&]() -> int {
         const size_t xq_h = gemm_ti_xq_bytes(gate_kind, (int)routes, (int)H), xq_f = gemm_ti_xq_bytes(down_kind, (int)routes, (int)FF);
-        const size_t nb_max = ((H > FF ? H : FF) + QK_K - 1) / QK_K;
         if (int rc = ensure(ctx, ctx->act_qs, xq_h > xq_f ? xq_h : xq_f)) return rc;
-        if (int rc = ensure(ctx, ctx->act_d, routes * nb_max * sizeof(float))) return rc;
         return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes());
     };
     const size_t kp_h = (H + block_values(gate_kind) - 1) / block_values(gate_kind) * block_values(gate_kind);
@@ -1180,14 +1175,14 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
         }
         if (int rc = few_workspace()) return rc;
         uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
-        float *dT = (float *)ctx->act_d.ptr, *part = (float *)ctx->gemm_partial.ptr;
-        MCU_CUDA(launch_act_int_fused(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xq, dT, s));
-        MCU_CUDA(launch_gemm_ti_grouped(gate_kind, gate_up, 2, (int)e_count, xq, dT, (int)routes, (int)H, cnt, off, part,
+        float *part = (float *)ctx->gemm_partial.ptr;
+        MCU_CUDA(launch_act_int_fused(gate_kind, hidden_dev, (int)H, from_hidden, (int)routes, (int)H, xq, s));
+        MCU_CUDA(launch_gemm_ti_grouped(gate_kind, gate_up, 2, (int)e_count, xq, (int)routes, (int)H, cnt, off, part,
                                         ctx->gemm_counters, ctx->dev_err, s));
         ActSource down_src = from_glu;
         down_src.x_out = gate_out;  // (gate_out holds act(gate) * up afterwards, as with the per-expert launches)
-        MCU_CUDA(launch_act_int_fused(down_kind, gate_out, (int)FF, down_src, (int)routes, (int)FF, xq, dT, s));
-        MCU_CUDA(launch_gemm_ti_grouped(down_kind, &down_job, 1, (int)e_count, xq, dT, (int)routes, (int)FF, cnt, off, part,
+        MCU_CUDA(launch_act_int_fused(down_kind, gate_out, (int)FF, down_src, (int)routes, (int)FF, xq, s));
+        MCU_CUDA(launch_gemm_ti_grouped(down_kind, &down_job, 1, (int)e_count, xq, (int)routes, (int)FF, cnt, off, part,
                                         ctx->gemm_counters, ctx->dev_err, s));
         MCU_CUDA(launch_moe_combine_dev(route_down, rb.sorted_w, rb.route_pos, (int)T, (int)k, (int)H, rb.offsets, (int)e_begin,
                                         (int)(e_begin + e_count), rb.counts + E, capturing ? ctx->dev_err : nullptr, out_dev, H, s));

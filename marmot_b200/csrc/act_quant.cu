@@ -408,11 +408,10 @@ act_half_fused_kernel(const float *x, int ldx, ActSource src, int K, int nb, __h
 // The operands of the integer tensor-core matmul (gemm_ti.cu) for K-quants: per row and 256-value block 384 bytes, the 256
 // quants, then the sums of its sub-blocks split as 64 * hi + lo into 8-bit values (lo from byte 256, hi from byte 288 on).
 // SUB = 32 (Q4_K: eight sums) or 16 (Q6_K: sixteen sums, and two planes of quants, in which the even / the odd sub-blocks are
-// zero: the matmul multiplies 32 values at a time and needs the sums of 16).  dT[block][row]: the block scales.
+// zero: the matmul multiplies 32 values at a time and needs the sums of 16).  The block's scale follows at byte 320.
 template <int SUB, int OP>
 __global__ void __launch_bounds__(1024)
-act_int_fused_kernel(const float *x, int ldx, ActSource src, int K, int nb, uint8_t *__restrict__ xq, size_t plane,
-                     float *__restrict__ dT, int ld_dT) {
+act_int_fused_kernel(const float *x, int ldx, ActSource src, int K, int nb, uint8_t *__restrict__ xq, size_t plane) {
     extern __shared__ __align__(16) uint8_t act_sm[];
     int8_t *q_s = (int8_t *)act_sm;
     float *d_s = (float *)(act_sm + nb * QK_K);
@@ -422,8 +421,8 @@ act_int_fused_kernel(const float *x, int ldx, ActSource src, int K, int nb, uint
     stage_begin(src);
     if (!quantize_row<true, OP>(x, ldx, src, K, nb, t, q_s, d_s, red, inv_s)) return;
     __syncthreads();
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) dT[(size_t)b * ld_dT + t] = d_s[b];
     uint8_t *row = xq + (size_t)t * nb * 384;
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) *(float *)(row + b * 384 + 320) = d_s[b];
     constexpr int PER = SUB / 16;  // a sub-block per thread: one or two 16-byte words
     for (int g = threadIdx.x; g < nb * (QK_K / SUB); g += blockDim.x) {
         const int blk = g / (QK_K / SUB), at = g % (QK_K / SUB);
@@ -494,8 +493,7 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
 #undef MCU_STAGE
 }
 
-cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSource &src, int rows, int K, uint8_t *xq, float *dT,
-                                 cudaStream_t s) {
+cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSource &src, int rows, int K, uint8_t *xq, cudaStream_t s) {
     if (rows <= 0) return cudaSuccess;
     const int nb = (K + QK_K - 1) / QK_K;
     cudaLaunchConfig_t cfg = {};
@@ -512,7 +510,7 @@ cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSou
     auto launch = [&](auto kernel) {
         if (cfg.dynamicSmemBytes > 48 * 1024)  // (rows of more than 48,000 values)
             if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ACT_INT_MAX_SMEM)) return e;
-        return cudaLaunchKernelEx(&cfg, kernel, x, ldx, src, K, nb, xq, plane, dT, rows);
+        return cudaLaunchKernelEx(&cfg, kernel, x, ldx, src, K, nb, xq, plane);
     };
 #define MCU_STAGE(OP) (kind == KIND_Q6_K ? launch(act_int_fused_kernel<16, OP>) : launch(act_int_fused_kernel<32, OP>))
     switch (stage_op(src)) {

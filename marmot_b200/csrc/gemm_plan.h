@@ -28,7 +28,7 @@ struct TsJob {
 };
 struct TsParams {
     TsJob jobs[TS_MAX_JOBS];
-    const float *rowscale;  // fp16: per-token power-of-two factor undone in the epilogue; integers: block scales [block][row]
+    const float *rowscale;  // fp16: per-token power-of-two factor undone in the epilogue
     float *partial;         // two slots of 128 x bn floats per CTA
     int *counters;          // one ticket per CTA, zero between launches
     int *err;

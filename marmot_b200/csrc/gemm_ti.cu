@@ -146,7 +146,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     const uint32_t R = 1u << p.raw_shift;
     const uint32_t a_full = bar_base, b_full = bar_base + 16u, ab_empty = bar_base + 48u, d_full = bar_base + 80u, d_empty = bar_base + 96u,
                    seg_full = bar_base + 112u, seg_free = bar_base + 120u, share_bar = bar_base + 128u, ticket_bar = bar_base + 136u,
-                   raw_full = bar_base + 144u, raw_empty = bar_base + 208u;
+                   raw_full = bar_base + 144u, raw_empty = bar_base + 208u, dx_read = bar_base + 272u;
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
     __shared__ volatile int last_s;
@@ -164,6 +164,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
         for (uint32_t i = 0; i < TI_B_SLOTS; ++i) {
             tm_mbar_init(b_full + 8u * i, 1);
             tm_mbar_init(ab_empty + 8u * i, 1);
+            tm_mbar_init(dx_read + 8u * i, Q4 ? 4 : 8);  // the scalers that read the block scales of a slot
         }
         for (uint32_t i = 0; i < R; ++i) {
             tm_mbar_init(raw_full + 8u * i, 1);
@@ -200,7 +201,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                 const int row = work.tile(p, tile).t_row0;
                 for (int k = k_lo; k < k_hi; ++k, ++j) {
                     const uint32_t st = j & (TI_B_SLOTS - 1), use = j / TI_B_SLOTS;
-                    if (use >= 1 && !ts_wait(ab_empty + 8u * st, (use - 1) & 1u)) {
+                    if (use >= 1 && !(ts_wait(ab_empty + 8u * st, (use - 1) & 1u) && ts_wait(dx_read + 8u * st, (use - 1) & 1u))) {
                         ok = false;
                         break;
                     }
@@ -370,7 +371,12 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     }
                     __syncwarp();
                     if (lane == 0) tm_mbar_arrive(raw_empty + 8u * rs);
-                    const float *dx = p.rowscale + (size_t)(u0 + j - tile * KS) * p.T + t.t_row0;
+                    // The tokens' block scales come with the activation tile: byte 320 of 384, in the last box (128-byte swizzle).  Read from
+                    // memory here they were a trip to L2 in every slab, and what bounded the scalers: 16 x 4096 x 14336 Q4_K 19.5 -> 15.0 us,
+                    // 8 x 4096 x 28672 30.7 -> 27.1, Q6_K 8 x 4096 x 14336 27.4 -> 23.7, MoE of 16 tokens 246 -> 199.
+                    const uint32_t slot = (uint32_t)j & (TI_B_SLOTS - 1);
+                    const uint8_t *dx = smem_raw + (tile_base + slot * B_BYTES + (Q4 ? 4096u : 8192u) - raw_addr);
+                    if (ok) ok = ts_wait(b_full + 8u * slot, ((uint32_t)j >> 2) & 1u);
                     if (ok) ok = ts_wait(d_full + 8u * group, (Q4 ? (uint32_t)j >> 1 : (uint32_t)j) & 1u);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
@@ -379,14 +385,17 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     auto release = [&] {
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
-                        if (lane == 0) tm_mbar_arrive(d_empty + 8u * group);
+                        if (lane == 0) {
+                            tm_mbar_arrive(d_empty + 8u * group);
+                            tm_mbar_arrive(dx_read + 8u * slot);
+                        }
                     };
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {  // eight tokens at a time
                         if (8 * hh >= t.t_count) break;
                         float dxv[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) dxv[i] = __ldg(dx + min(8 * hh + i, t.t_count - 1));
+                        for (int i = 0; i < 8; ++i) dxv[i] = *(const float *)(dx + (8 * hh + i) * 128 + ((4 ^ i) << 4));
                         int sum[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i) sum[i] = 0;
@@ -593,7 +602,7 @@ static cudaError_t ti_encode_x(int kind, CUtensorMap *m, const uint8_t *xq, int 
                      TI_COLS, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const uint8_t *xq, const float *dT, int T, int K, float *partial,
+cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const uint8_t *xq, int T, int K, float *partial,
                            int *counters, int *err_flag, cudaStream_t s) {
     if (n_jobs < 1 || n_jobs > TS_MAX_JOBS || T < 1) return cudaErrorInvalidValue;
     TsParams p;
@@ -601,7 +610,6 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     memset(&p, 0, sizeof(p));
     p.nb = p.slabs = (K + QK_K - 1) / QK_K;
     p.row_bytes = (long)p.nb * block_bytes(kind);
-    p.rowscale = dT;
     p.partial = partial;
     p.counters = counters;
     p.err = err_flag;
@@ -622,7 +630,7 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     return ti_dispatch(kind, maps, p, pl.n_cta, s);
 }
 
-cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq, const float *dT,
+cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq,
                                    int total_rows, int K, const int *group_counts, const int *group_offsets, float *partial,
                                    int *counters, int *err_flag, cudaStream_t s) {
     if (n_groups <= 0 || total_rows <= 0) return cudaSuccess;
@@ -632,7 +640,6 @@ cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
     if (cudaError_t e = ts_grouped_params(kind, jobs, n_jobs, n_groups, total_rows, K, group_counts, group_offsets, p, maps))
         return e;
     p.bn = TI_COLS;
-    p.rowscale = dT;
     p.partial = partial;
     p.counters = counters;
     p.err = err_flag;

@@ -24,13 +24,13 @@ cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
                                    int ldxh, int total_rows, int K, const int *group_counts, const int *group_offsets,
                                    float *partial, int *counters, int *err_flag, cudaStream_t s);
 
-// The same on integers for a handful of tokens (gemm_ti.cu: Q4_K, Q6_K): exact sub-block dots.  xq / dT from
+// The same on integers for a handful of tokens (gemm_ti.cu: Q4_K, Q6_K): exact sub-block dots.  xq from
 // launch_act_int_fused.
 size_t gemm_ti_xq_bytes(int kind, int rows, int K);
 bool gemm_ti_supported(int kind, const void *W, int K, int F);
-cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const uint8_t *xq, const float *dT, int T, int K,
+cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const uint8_t *xq, int T, int K,
                            float *partial, int *counters, int *err_flag, cudaStream_t s);
-cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq, const float *dT,
+cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq,
                                    int total_rows, int K, const int *group_counts, const int *group_offsets,
                                    float *partial, int *counters, int *err_flag, cudaStream_t s);
 

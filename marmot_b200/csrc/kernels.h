@@ -48,10 +48,10 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
                                        __half *xh, float *rowscale, cudaStream_t s);
 
 // The same rows as operands of the integer tensor-core matmul (K-quants; layout at the kernel, act_quant.cu): xq
-// [planes][rows][blocks][384] bytes, dT [blocks][rows].  A row is staged in shared memory, act_half_fused_smem() of it, up to here
+// [planes][rows][blocks][384] bytes.  A row is staged in shared memory, act_half_fused_smem() of it, up to here
 // (rows of 193,000 values).
 constexpr size_t ACT_INT_MAX_SMEM = 192 * 1024;
-cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSource &src, int rows, int K, uint8_t *xq, float *dT,
+cudaError_t launch_act_int_fused(int kind, const float *x, int ldx, const ActSource &src, int rows, int K, uint8_t *xq,
                                  cudaStream_t s);
 
 // blocks -> f32 (bit-exact with the reference dequantizers)
