@@ -96,15 +96,21 @@ __device__ __forceinline__ void ti_conv_q4k(const uint8_t *rowp, Done done, Emit
 }
 // Q6_K: value 128 n + 32 c + l has its low four bits in byte 64 n + 32 (c & 1) + l of ql (high nibble for c >= 2), its high two
 // in bits 2 c of byte 32 n + l of qh.  The quants stay 0..63 here.
-template <class Done, class Emit>
-__device__ __forceinline__ void ti_conv_q6k(const uint8_t *blk, Done done, Emit emit) {
+// EVEN: all rows start at byte `phase` behind a 16-byte boundary.
+template <bool EVEN, class Done, class Emit>
+__device__ __forceinline__ void ti_conv_q6k(const uint8_t *blk, uint32_t phase, Done done, Emit emit) {
     uint32_t sc[4];
     tm_lds_words<4>(blk + 192, sc);
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         uint32_t ql[16], qh[8], o[32];
-        tm_lds_words<16>(blk + 64 * n, ql);
-        tm_lds_words<8>(blk + 128 + 32 * n, qh);
+        if (EVEN) {
+            ts_lds_phase<16>(blk - phase + 64 * n, phase, ql);
+            ts_lds_phase<8>(blk - phase + 128 + 32 * n, phase, qh);
+        } else {
+            tm_lds_words<16>(blk + 64 * n, ql);
+            tm_lds_words<8>(blk + 128 + 32 * n, qh);
+        }
         if (n == 1) done();
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -329,7 +335,8 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     if (lane == 0) tm_mbar_arrive(raw_empty + 8u * rs);
                 };
                 if constexpr (Q4) ti_conv_q4k(row_of(j), done, emit);
-                else ti_conv_q6k(row_of(j), done, emit);
+                else if (loose) ti_conv_q6k<false>(row_of(j), 0u, done, emit);
+                else ti_conv_q6k<true>(row_of(j), (uint32_t)((u0 + j - tile * KS) * SL::BYTES) & 15u, done, emit);
                 if (!ok) break;
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

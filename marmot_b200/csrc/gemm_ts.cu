@@ -110,11 +110,17 @@ __device__ __forceinline__ void ts_conv_q4k(const uint8_t *rowp, int n, Done don
 // Q6_K: value 128 n + 32 c + l has its low four bits in byte 64 n + 32 (c & 1) + l of ql (high nibble for c >= 2), its high two
 // in bits 2 c of byte 32 n + l of qh.  d * sc is rounded to fp16 before the product with the quant; ONCE: that product is formed in 32
 // bits and rounded once (error of the result 2.9e-4 instead of 3.6e-4): rows that are not 16-byte multiples, which always had it.
+// Such rows start anywhere; the others all at byte `phase` behind a 16-byte boundary.
 template <bool ONCE, class Done, class Emit>
-__device__ __forceinline__ void ts_conv_q6k(const uint8_t *blk, int n, Done done, Emit emit) {
+__device__ __forceinline__ void ts_conv_q6k(const uint8_t *blk, uint32_t phase, int n, Done done, Emit emit) {
     uint32_t ql[16], qh[8], sc[2];
-    tm_lds_words<16>(blk + n * 64, ql);
-    tm_lds_words<8>(blk + 128 + n * 32, qh);
+    if (ONCE) {
+        tm_lds_words<16>(blk + n * 64, ql);
+        tm_lds_words<8>(blk + 128 + n * 32, qh);
+    } else {
+        ts_lds_phase<16>(blk - phase + n * 64, phase, ql);
+        ts_lds_phase<8>(blk - phase + 128 + n * 32, phase, qh);
+    }
     tm_lds_words<2>(blk + 192 + n * 8, sc);
     const float d = half_bits_to_float(*(const uint16_t *)(blk + 208));
     done();
@@ -541,8 +547,8 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     ts_conv_q4k(rowp, half, done, emit);
                 } else if constexpr (KIND == KIND_Q6_K) {
                     const int k = u0 + j - tile * KS;
-                    const uint8_t *blk = rowp + ((row_phase + (uint32_t)(k * SL::BYTES)) & row_mask);
-                    ts_conv_q6k<loose>(blk, half, done, emit);
+                    const uint32_t phase = (row_phase + (uint32_t)(k * SL::BYTES)) & row_mask;
+                    ts_conv_q6k<loose>(rowp + phase, phase, half, done, emit);
                 } else {
                     const int n_blk = p.nb - 8 * (u0 + j - tile * KS);
                     if (loose) ts_conv_q8_0_loose(rowp + row_phase, half, n_blk, done, emit);
