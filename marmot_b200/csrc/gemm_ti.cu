@@ -48,14 +48,6 @@ __device__ __forceinline__ void ti_mma(uint32_t d, uint32_t a, uint64_t b_desc, 
 __host__ __device__ constexpr uint32_t ti_idesc(int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TS_ROWS >> 4) << 24);
 }
-__device__ __forceinline__ void ti_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
-}
 __device__ __forceinline__ void ti_ld8(uint32_t taddr, int (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -325,7 +317,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                         if (ok) ts_st32(to + 32u * (uint32_t)h, o);
                     }
                     __device__ __forceinline__ void corrections(const uint32_t (&c)[16]) const {
-                        if (ok) ti_st16(to + 64u, c);
+                        if (ok) ts_st16(to + 64u, c);
                     }
                 };
                 const uint32_t prev = (uint32_t)j - 2u;

@@ -54,7 +54,7 @@ __device__ __forceinline__ void ts_mma(uint32_t d, uint32_t a, uint64_t b_desc, 
 }
 // ---- converters: 128 values of one weight row (half `n` of a 256-value slab) as 64 packed-half columns, K order (0, 2, 1, 3)
 //      inside every group of four.  Everything is read from the slab first and the slab released (`done`),
-//      so that its refill overlaps the arithmetic; `emit` gets the columns in two halves. ----
+//      so that its refill overlaps the arithmetic; `emit` gets the columns in four quarters (registers). ----
 
 // Q4_K: the arithmetic keeps the 6-bit scales and the fp16 block scales in packed halves: d * sc and dmin * m are single
 // fp16 roundings of exact products, and a weight is one HFMA2 of exact operands.
@@ -91,19 +91,22 @@ __device__ __forceinline__ void ts_conv_q4k(const uint8_t *rowp, int n, Done don
         const __half2 m2 = __hmul2(__hsub2(as_half2(__byte_perm(mn4, 0x64646464u, pick)), k1024), nd);
         const __half2 sa = bcast_lo(s2), sb = bcast_hi(s2), ma = bcast_lo(m2), mb = bcast_hi(m2);
         const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        uint32_t o[32];
+        uint32_t o[16];
+        // 0x6400 | v = 1024 + v;  0x5400 | (v << 4) = 64 + v
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const uint32_t ws = w[i] >> 8;
-            // 0x6400 | v = 1024 + v;  0x5400 | (v << 4) = 64 + v
-            const __half2 a0 = as_half2(ts_and_or(w[i], 0x000F000Fu, 0x64006400u)), a1 = as_half2(ts_and_or(ws, 0x000F000Fu, 0x64006400u));
-            const __half2 b0 = as_half2(ts_and_or(w[i], 0x00F000F0u, 0x54005400u)), b1 = as_half2(ts_and_or(ws, 0x00F000F0u, 0x54005400u));
+            const __half2 a0 = as_half2(ts_and_or(w[i], 0x000F000Fu, 0x64006400u)), a1 = as_half2(ts_and_or(w[i] >> 8, 0x000F000Fu, 0x64006400u));
             o[2 * i] = as_u32(__hfma2(__hsub2(a0, k1024), sa, ma));
             o[2 * i + 1] = as_u32(__hfma2(__hsub2(a1, k1024), sa, ma));
-            o[16 + 2 * i] = as_u32(__hfma2(__hsub2(b0, k64), sb, mb));
-            o[16 + 2 * i + 1] = as_u32(__hfma2(__hsub2(b1, k64), sb, mb));
         }
-        emit(h, o);
+        emit(2 * h, o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const __half2 b0 = as_half2(ts_and_or(w[i], 0x00F000F0u, 0x54005400u)), b1 = as_half2(ts_and_or(w[i] >> 8, 0x00F000F0u, 0x54005400u));
+            o[2 * i] = as_u32(__hfma2(__hsub2(b0, k64), sb, mb));
+            o[2 * i + 1] = as_u32(__hfma2(__hsub2(b1, k64), sb, mb));
+        }
+        emit(2 * h + 1, o);
     }
 }
 
@@ -127,9 +130,9 @@ __device__ __forceinline__ void ts_conv_q6k(const uint8_t *blk, uint32_t phase, 
     const __half2 off = as_half2(0x64206420u);  // 1024 + 32
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        uint32_t o[32];
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
+            uint32_t o[16];
             const int c = 2 * t + b;
             const uint32_t sw = sc[t] >> (16 * b);
             const float f0 = __fmul_rn(d, (float)(int8_t)sw), f1 = __fmul_rn(d, (float)(int8_t)(sw >> 8));  // (exact)
@@ -143,21 +146,21 @@ __device__ __forceinline__ void ts_conv_q6k(const uint8_t *blk, uint32_t phase, 
                 if (ONCE) {
                     const float f = j < 4 ? f0 : f1;
                     const float2 w0 = __half22float2(v0), w1 = __half22float2(v1);
-                    o[16 * b + 2 * j] = as_u32(__floats2half2_rn(__fmul_rn(w0.x, f), __fmul_rn(w0.y, f)));
-                    o[16 * b + 2 * j + 1] = as_u32(__floats2half2_rn(__fmul_rn(w1.x, f), __fmul_rn(w1.y, f)));
+                    o[2 * j] = as_u32(__floats2half2_rn(__fmul_rn(w0.x, f), __fmul_rn(w0.y, f)));
+                    o[2 * j + 1] = as_u32(__floats2half2_rn(__fmul_rn(w1.x, f), __fmul_rn(w1.y, f)));
                     continue;
                 }
                 const __half2 ds = j < 4 ? ds0 : ds1;
-                o[16 * b + 2 * j] = as_u32(__hmul2(v0, ds));
-                o[16 * b + 2 * j + 1] = as_u32(__hmul2(v1, ds));
+                o[2 * j] = as_u32(__hmul2(v0, ds));
+                o[2 * j + 1] = as_u32(__hmul2(v1, ds));
             }
+            emit(c, o);
         }
-        emit(t, o);
     }
 }
 
 // Q8_0: blocks 4 n .. 4 n + 3 of the slab; blocks at or beyond `n_blk` (the end of the row) are zero.
-__device__ __forceinline__ void ts_conv_q8_block(const uint32_t (&q)[8], uint32_t d_bits, uint32_t *o) {
+__device__ __forceinline__ void ts_conv_q8_block(const uint32_t (&q)[8], uint32_t d_bits, uint32_t (&o)[16]) {
     const __half2 off = as_half2(0x64806480u);  // 1024 + 128
     const __half2 dh = as_half2(__byte_perm(d_bits, 0u, 0x1010));
 #pragma unroll
@@ -185,33 +188,34 @@ __device__ __forceinline__ void ts_conv_q8_0(const uint8_t *rowp, int n_blk, Don
     for (int t = 0; t < 2; ++t) {
         const uint32_t (&w)[20] = w2[t];
         const int o4 = 2 * N + t;  // word offset of the pair inside its window
-        uint32_t o[32], q[8];
+        uint32_t o[16], q[8];
         const int c = 4 * N + 2 * t;
 #pragma unroll
         for (int j = 0; j < 8; ++j) q[j] = __funnelshift_r(w[o4 + j], w[o4 + j + 1], 16);
         // (quants are finite whatever the bytes, so a zero scale clears a block)
         ts_conv_q8_block(q, c < n_blk ? w[o4] : 0u, o);
+        emit(2 * t, o);
 #pragma unroll
         for (int j = 0; j < 8; ++j) q[j] = w[o4 + 9 + j];
-        ts_conv_q8_block(q, c + 1 < n_blk ? w[o4 + 8] >> 16 : 0u, o + 16);
-        emit(t, o);
+        ts_conv_q8_block(q, c + 1 < n_blk ? w[o4 + 8] >> 16 : 0u, o);
+        emit(2 * t + 1, o);
     }
 }
 template <class Done, class Emit>
 __device__ __forceinline__ void ts_conv_q8_0_loose(const uint8_t *rowp, int n, int n_blk, Done done, Emit emit) {
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        uint32_t o[32];
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
+            uint32_t o[16];
             const int c = 4 * n + 2 * t + b;
             const uint8_t *blk = rowp + c * Q8_0_BYTES;
             uint32_t q[8];
             tm_lds_words<8>(blk + 2, q);
-            ts_conv_q8_block(q, c < n_blk ? *(const uint16_t *)blk : 0u, o + 16 * b);
+            ts_conv_q8_block(q, c < n_blk ? *(const uint16_t *)blk : 0u, o);
+            if (2 * t + b == 3) done();
+            emit(2 * t + b, o);
         }
-        if (t == 1) done();
-        emit(t, o);
     }
 }
 
@@ -290,7 +294,13 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     const uint32_t tmem = tmem_slot;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    const TsWork work = ts_work(p, grouped, group_tile0, bn, cta, n_cta);
+    // (In shared memory, and the converted columns in quarters, for the registers: what a thread spills misses the few KB of L1 that
+    // are left.  48 to 56 bytes a thread before, 24 to 56 so: Q6_K 37 x 14336 x 4096 27.4 -> 25.7 us, Q4_K 64 x 4096 x 14336 18.3 -> 17.8; with
+    // 120 or 200 bytes the large sizes were 10 and 25 % slower.)
+    __shared__ TsWork work_s;
+    if (threadIdx.x == 0) work_s = ts_work(p, grouped, group_tile0, bn, cta, n_cta);
+    __syncthreads();
+    const TsWork &work = work_s;
     const int KS = p.slabs, u0 = work.u0, u1 = work.u1;
     auto tile_of = [&](int tile) { return work.tile(p, tile); };
 
@@ -534,14 +544,14 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     __syncwarp();
                     if (lane == 0) tm_mbar_arrive(raw_empty + 8u * rs);
                 };
-                auto emit = [&](int t, const uint32_t (&o)[32]) {
+                auto emit = [&](int t, const uint32_t (&o)[16]) {
                     if (t == 0) {
                         // The slot's previous MMAs: waited for only now, the conversion has hidden some of it.
                         if (ok && j >= 2) ok = ts_wait(empty + 8u * group, ((uint32_t)(j >> 1) - 1u) & 1u);
                         ok = __all_sync(0xffffffffu, ok);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     }
-                    if (ok) ts_st32(lane_addr + TS_D_COLS + (uint32_t)group * 64u + 32u * (uint32_t)t, o);
+                    if (ok) ts_st16(lane_addr + TS_D_COLS + (uint32_t)group * 64u + 16u * (uint32_t)t, o);
                 };
                 if constexpr (KIND == KIND_Q4_K) {
                     ts_conv_q4k(rowp, half, done, emit);
