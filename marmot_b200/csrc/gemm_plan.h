@@ -37,6 +37,7 @@ struct TsParams {
     int n_jobs, T, bn, nb, slabs, raw_shift;  // raw_shift: log2 of the slab ring's depth
     int loose;              // weight rows that are not 16-byte multiples, or do not start on one
     int split;              // > 1: clusters of `split` CTAs (pairs) share a tile along K; otherwise ranges of units
+    int whole;              // the tiles are dealt to the CTAs whole, in turn
     int tiles, t_tiles;     // output tiles in all; token tiles per row tile
     int groups, row_tiles;  // grouped launches: number of groups, row tiles per group
 };
@@ -97,6 +98,12 @@ MCU_HD TsWork ts_work(const TsParams &p, bool grouped, const int *group_tile0, i
     w.bn = bn;
     w.units = (long long)(grouped ? group_tile0[p.groups] : p.tiles) * KS;
     w.n_use = (int)(w.units < n_cta ? w.units : n_cta);  // (a grouped launch may find fewer units than CTAs)
+    if (p.whole) {  // as many CTAs as tiles, or fewer: the first ones take one more
+        const int each = p.tiles / n_cta, more = p.tiles - each * n_cta;
+        w.u0 = KS * (cta * each + ts_min(cta, more));
+        w.u1 = w.u0 + KS * (each + (cta < more ? 1 : 0));
+        return w;
+    }
     w.u0 = cta < w.n_use ? (int)(w.units * cta / w.n_use) : 0;
     w.u1 = cta < w.n_use ? (int)(w.units * (cta + 1) / w.n_use) : 0;
     if (p.split > 1) {
@@ -122,12 +129,15 @@ MCU_HD int ts_share_slot(const TsWork &w, int tile, int KS, int cta) { return w.
 struct TsPlan {
     int bn, t_tiles, split, n_cta;
     double cost;
+    int whole = 0;
 };
 
 // How to spread `tiles` output tiles of KS slabs over `room` SMs, and what it costs in cycles, by measurements of all the forms at 70 to 512
 // tokens and 2048 x 2048 to 4096 x 28672 weights.  A slab takes the longer of its conversion (less in tiles of up to 64 columns, whose
 // stages hold 128 values of K) and its MMAs; a tile ends with its epilogue.
-// - One tile per CTA, in as many waves as it takes: 2000 for a CTA's start.
+// - Whole tiles, one or several to a CTA: 2000 for a CTA's start, 2500 between two tiles of it.  (As a CTA of its own, a further tile cost its
+//   start as well, and the kernels behind could not start early before the last wave: 20 x 2304 x 35840 Q4_K 25.4 -> 20.5 us, 39 x 1536 x 51200
+//   Q8_0 34.5 -> 27.5, 512 x 4096 x 14336 Q8_0 80.1 -> 77.9.)
 // - A tile over a cluster: the exchange of the shares through the CTAs' shared memories.
 // - Equal ranges of slabs: cut tiles have their shares written to memory, and read again by the CTA that comes last; a tile of 256
 //   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).  The way
@@ -140,10 +150,11 @@ inline TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles, int ro
     const double conv = kind == KIND_Q4_K ? (wide ? 1500 : 1120) : kind == KIND_Q6_K ? (wide ? 2100 : 1700) : (wide ? 1750 : 1500);
     const double mma = 8.5 * bn, unit = mma > conv ? mma : conv, tile_end = 1000.0 + 8.0 * bn;
     TsPlan best{bn, t_tiles, 1, 0, 1e30};
-    auto consider = [&](int split, long n, double cost) {
-        if (cost < best.cost) best = TsPlan{bn, t_tiles, split, (int)n, cost};
+    auto consider = [&](int split, long n, double cost, int whole = 0) {
+        if (cost < best.cost) best = TsPlan{bn, t_tiles, split, (int)n, cost, whole};
     };
-    consider(1, tiles, (double)((tiles + room - 1) / room) * (KS * unit + tile_end + 2000.0));
+    const int waves = (tiles + room - 1) / room;
+    consider(1, tiles < room ? tiles : room, waves * (KS * unit) + (waves - 1) * 2500.0 + tile_end + 2000.0, 1);
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2) {
         // A cluster is placed inside a GPC (16 to 20 SMs): sixteen clusters of eight did not run at once (2048 x 2048: 12.6 us,
         // 64 CTAs in clusters of four 7.5), fourteen do.

@@ -760,6 +760,7 @@ cudaError_t launch_gemm_ts(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     p.bn = pl.bn;
     p.t_tiles = pl.t_tiles;
     p.split = pl.split;
+    p.whole = pl.whole;
     for (int j = 0; j < n_jobs; ++j) p.loose |= ts_loose(kind, jobs[j].W, p.row_bytes);
     int row_tiles = 0;
     for (int j = 0; j < n_jobs; ++j) {

@@ -95,6 +95,39 @@ extern "C" int check_plan(int integer, int kind, int T, int K, const int *F, int
     return check(p, pl.bn, pl.n_cta, sms, nullptr, want);
 }
 
+// the plans that deal the tiles whole: every CTA has tiles, the counts differ by one at most (-1: the plan is another one)
+extern "C" int check_whole(int integer, int kind, int T, int K, const int *F, int n_jobs, int sms) {
+    TsParams p{};
+    p.nb = (K + block_values(kind) - 1) / block_values(kind);
+    p.slabs = (p.nb * block_values(kind) + TS_SLAB_K - 1) / TS_SLAB_K;
+    p.n_jobs = n_jobs;
+    p.T = T;
+    int row_tiles = 0;
+    std::vector<std::pair<int, int>> want;
+    for (int j = 0; j < n_jobs; ++j) {
+        p.jobs[j].F = F[j];
+        p.jobs[j].row_tile0 = row_tiles;
+        row_tiles += (F[j] + TS_ROWS - 1) / TS_ROWS;
+        want.push_back({F[j], T});
+    }
+    p.t_tiles = (T + TI_COLS - 1) / TI_COLS;
+    const TsPlan pl = integer ? ti_plan(kind, row_tiles * p.t_tiles, p.slabs, sms) : ts_plan(kind, T, K, F, n_jobs, sms);
+    if (!pl.whole) return -1;
+    if (!integer) p.t_tiles = pl.t_tiles;
+    p.split = pl.split;
+    p.whole = 1;
+    p.tiles = row_tiles * p.t_tiles;
+    int least = 1 << 30, most = 0;
+    for (int c = 0; c < pl.n_cta; ++c) {
+        const TsWork w = ts_work(p, false, nullptr, pl.bn, c, pl.n_cta);
+        if (w.u0 % p.slabs != 0 || w.u1 % p.slabs != 0) return 20;
+        least = ts_min(least, w.u1 - w.u0);
+        most = most > w.u1 - w.u0 ? most : w.u1 - w.u0;
+    }
+    if (pl.split != 1 || pl.n_cta > sms || least < p.slabs || most - least > p.slabs) return 21;
+    return check(p, pl.bn, pl.n_cta, sms, nullptr, want);
+}
+
 // groups of `counts` tokens over stacked matrices of F rows each, as ts_group_table lays them out
 extern "C" int check_groups(int slabs, const int *counts, int groups, const int *F, int n_jobs, int bn, int sms) {
     TsParams p{};

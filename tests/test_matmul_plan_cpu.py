@@ -52,6 +52,22 @@ def test_integer_plans(lib, kind):
                 assert rc == 0, (rc, kind, T, K, F, sms)
 
 
+@pytest.mark.parametrize("kind,integer", [(KIND_Q4_K, 0), (KIND_Q6_K, 0), (KIND_Q8_0, 0)])
+def test_whole_tiles(lib, kind, integer):
+    """Plans that deal whole tiles: more tiles than CTAs, as many, fewer."""
+    rng = np.random.default_rng(kind)
+    several = 0
+    for T in (1, 9, 16) if integer else (1, 17, 39, 64, 65, 257, 512, 2048):
+        shapes = [(256, [1]), (2304, [17920, 17920]), (1536, [25600, 25600]), (4096, [14336, 14336]), (512, [128 * 148]), (512, [128 * 149])]
+        shapes += [(int(rng.integers(1, 9000)), [int(f) for f in np.exp(rng.uniform(0, np.log(60000), rng.integers(1, 5)))]) for _ in range(40)]
+        for K, F in shapes:
+            for sms in SMS:
+                rc = lib.check_whole(integer, kind, T, K, ints(F), len(F), sms)
+                assert rc <= 0, (rc, kind, T, K, F, sms)
+                several += rc == 0 and sum((f + 127) // 128 for f in F) > sms
+    assert several > 20
+
+
 @pytest.mark.parametrize("bn", [16, 64, 128, 256])
 def test_groups(lib, bn):
     """Groups of any size, empty ones and all empty ones among them."""
