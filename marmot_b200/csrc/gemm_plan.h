@@ -191,18 +191,20 @@ inline TsPlan ts_plan(int kind, int T, int K, const int *F, int n_jobs, int sms)
     return best;
 }
 
-// The same for the integer kernel: one tile per CTA, in waves if need be, a tile over a cluster, or equal ranges, whichever ends
-// first, by a sweep of all three at nine tokens: a slab takes about 900 cycles (Q6_K 2100), the start of a CTA 3500, a cluster's exchange 1500; a tile cut between
+// The same for the integer kernel: whole tiles, one or several to a CTA, a tile over a cluster, or equal ranges, whichever ends
+// first, by a sweep of all three at nine tokens: a slab takes about 900 cycles (Q6_K 2100), the start of a CTA 2700 and each of its tiles 800 (8 x 4096 x 28672
+// Q4_K, 224 tiles: 27.0 us in ranges, 24.6 so), a cluster's exchange 1500; a tile cut between
 // ranges costs 9000 and 700 for every share that the last CTA reads (13056 x 1792 Q4_K: 22 us in ranges of five slabs, 13 in
 // clusters of eight).  Clusters of eight: as in ts_spread.
 inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
     const long U = (long)tiles * KS, n_most = U < sms ? U : sms, upc = (U + n_most - 1) / n_most;
     const double unit = kind == KIND_Q4_K ? 900.0 : 2100.0;
     TsPlan best{TI_COLS, 1, 1, (int)n_most, 1e30};
-    auto consider = [&](int split, long n, double cost) {
-        if (cost < best.cost) best = TsPlan{TI_COLS, 1, split, (int)n, cost};
+    auto consider = [&](int split, long n, double cost, int whole = 0) {
+        if (cost < best.cost) best = TsPlan{TI_COLS, 1, split, (int)n, cost, whole};
     };
-    consider(1, tiles, (double)((tiles + sms - 1) / sms) * (KS * unit + 3500.0));
+    const int waves = (tiles + sms - 1) / sms;
+    consider(1, tiles < sms ? tiles : sms, waves * (KS * unit + 800.0) + 2700.0, 1);
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2)
         if ((long)tiles * sp <= (sp >= 8 ? sms * 7 / 9 : sms)) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + 5000.0);
     const bool cut = U % n_most != 0 || upc % KS != 0;

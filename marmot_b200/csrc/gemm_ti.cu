@@ -626,6 +626,7 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     if (cudaError_t e = ti_encode_x(kind, &maps.x, xq, T, p.nb)) return e;
     const TsPlan pl = ti_plan(kind, p.tiles, p.slabs, device_sm_count());
     p.split = pl.split;
+    p.whole = pl.whole;
     return ti_dispatch(kind, maps, p, pl.n_cta, s);
 }
 

@@ -52,7 +52,7 @@ def test_integer_plans(lib, kind):
                 assert rc == 0, (rc, kind, T, K, F, sms)
 
 
-@pytest.mark.parametrize("kind,integer", [(KIND_Q4_K, 0), (KIND_Q6_K, 0), (KIND_Q8_0, 0)])
+@pytest.mark.parametrize("kind,integer", [(KIND_Q4_K, 0), (KIND_Q6_K, 0), (KIND_Q8_0, 0), (KIND_Q4_K, 1), (KIND_Q6_K, 1)])
 def test_whole_tiles(lib, kind, integer):
     """Plans that deal whole tiles: more tiles than CTAs, as many, fewer."""
     rng = np.random.default_rng(kind)
