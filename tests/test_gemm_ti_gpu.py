@@ -53,6 +53,40 @@ def test_rows_that_cannot_be_streamed(ctx, oracle, T, K, F):
     assert max_rel_err(got, oracle.linear(KIND_Q6_K, x, W, F)) <= TOL_FP32
 
 
+@pytest.mark.parametrize("kind,T,K,F", [(KIND_Q4_K, 2, 1024, 12289), (KIND_Q4_K, 2, 16384, 3100), (KIND_Q4_K, 3, 1536, 8200), (KIND_Q4_K, 3, 14336, 1030),
+                                        (KIND_Q4_K, 4, 768, 8200), (KIND_Q6_K, 3, 2048, 12300), (KIND_Q6_K, 4, 1024, 8200), (KIND_Q6_K, 4, 14336, 1030)])
+def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
+    """Sizes just beyond the lines: the dp4a kernel's results but for the order of the f32 terms, and, recorded in a context without a
+    workspace, the dp4a kernel itself."""
+    import torch
+    from marmot_b200 import Context
+    from marmot_b200.runtime import REGIME_AUTO, REGIME_GEMV
+
+    rng = np.random.default_rng(T + K + F)
+    W = random_blocks(kind, F, K, rng)
+    x = rng.normal(0, 1, (T, K)).astype(np.float32)
+    xd, wd = torch.from_numpy(x).cuda(), ctx.upload(W)
+    got = ctx.linear(kind, xd, wd, F).cpu().numpy()
+    ctx.set_regime(REGIME_GEMV)
+    ref = ctx.linear(kind, xd, wd, F).cpu().numpy()
+    ctx.set_regime(REGIME_AUTO)
+    ctx.synchronize()
+    assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= TOL_FP32
+    assert max_rel_err(got, ref) <= 1e-5
+    fresh = Context(0, use_torch_stream=False)
+    stream = torch.cuda.Stream()
+    fresh.set_stream(stream.cuda_stream)
+    out = torch.zeros((T, F), device="cuda")
+    torch.cuda.synchronize()
+    fresh.graph_capture_begin()
+    fresh.linear(kind, xd, wd, F, out=out)
+    graph = fresh.graph_capture_end()
+    graph.launch()
+    fresh.synchronize()
+    assert np.array_equal(out.cpu().numpy(), ref)
+    fresh.close()
+
+
 @pytest.mark.parametrize("T,K,F", [(3, 4096, 5632), (4, 4096, 4096), (5, 2048, 2056), (8, 4096, 1030), (16, 512, 40)])
 def test_two_matrices_of_each_kind_with_prologues(ctx, oracle, T, K, F):
     """The sizes at which linear_multi leaves the dp4a kernel: every result equals the one of the plain regime, and x' is exact."""
