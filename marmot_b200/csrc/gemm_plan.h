@@ -98,6 +98,12 @@ MCU_HD TsWork ts_work(const TsParams &p, bool grouped, const int *group_tile0, i
     w.bn = bn;
     w.units = (long long)(grouped ? group_tile0[p.groups] : p.tiles) * KS;
     w.n_use = (int)(w.units < n_cta ? w.units : n_cta);  // (a grouped launch may find fewer units than CTAs)
+    if (p.split > 1) {
+        const int t = cta / p.split, part = cta - t * p.split;
+        w.u0 = t * KS + KS * part / p.split;
+        w.u1 = t * KS + KS * (part + 1) / p.split;
+        return w;
+    }
     if (p.whole) {  // as many CTAs as tiles, or fewer: the first ones take one more
         const int each = p.tiles / n_cta, more = p.tiles - each * n_cta;
         w.u0 = KS * (cta * each + ts_min(cta, more));
@@ -106,11 +112,6 @@ MCU_HD TsWork ts_work(const TsParams &p, bool grouped, const int *group_tile0, i
     }
     w.u0 = cta < w.n_use ? (int)(w.units * cta / w.n_use) : 0;
     w.u1 = cta < w.n_use ? (int)(w.units * (cta + 1) / w.n_use) : 0;
-    if (p.split > 1) {
-        const int t = cta / p.split, part = cta - t * p.split;
-        w.u0 = t * KS + KS * part / p.split;
-        w.u1 = t * KS + KS * (part + 1) / p.split;
-    }
     return w;
 }
 
