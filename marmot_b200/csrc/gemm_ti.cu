@@ -14,12 +14,12 @@
 //   warp 16       issues the MMAs: ten (Q4_K) or twelve (Q6_K) per slab of 128 rows x 32 values x 16 or 32 columns
 //   warp 17       activation tiles by TMA;  warp 18  packed weight slabs by TMA (as in gemm_ts.cu)
 //
-// Work is divided as in gemm_ts.cu: one tile per CTA, a tile over a cluster, or equal ranges of slabs.
+// Work is divided as in gemm_ts.cu: whole tiles, a tile over a cluster, or equal ranges of slabs.
 //
-// Measured, staging included, against the kernels that had these calls (mma.sync, dp4a): Q4_K 8 x 4096 x 14336 19.9 -> 13.5 us
-// (2.4 TB/s), 16 tokens 22.4 -> 16.0, 8 x 4096 x 4096 12.3 -> 9.3; Q6_K 8 x 4096 x 14336 25.2 -> 21.8.  The mma.sync kernel keeps the
+// Measured, staging included, against the kernels that had these calls (mma.sync, dp4a): Q4_K 8 x 4096 x 14336 19.9 -> 12.7 us
+// (2.6 TB/s), 8 x 4096 x 28672 22.5 (2.9 TB/s), 16 x 4096 x 14336 22.4 -> 14.2; Q6_K 8 x 4096 x 14336 25.2 -> 21.3.  The mma.sync kernel keeps the
 // calls of up to 16 tokens for which it is the faster one (gemm_i8.cu; i8_pays in gemm_plan.h).  A slab costs the Q4_K scalers and
-// converters 500 to 700 cycles by their own stamps, the Q6_K ones (eighteen products of 32 columns, 4 KB of sums per row) 900 to 1800; a
+// converters 500 to 700 cycles by their own stamps (740 by the time of a CTA with sixteen), the Q6_K ones (eighteen products of 32 columns, 4 KB of sums per row) 900 to 1800; a
 // CTA's time grows by 900 and 2100 with each (ti_plan).  Those bound Q6_K, the kernel's prologue, staging launch and first loads (about
 // 5 us) the small sizes.
 #include "gemm_ts_dev.cuh"

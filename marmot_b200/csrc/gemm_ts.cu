@@ -15,12 +15,12 @@
 //   warp 18       packed weight slabs (128 rows x 256 values) into a shared-memory ring, by TMA.  Rows that are not 16-byte
 //                 multiples (Q6_K with K % 2048 != 0) come as eight copies of every eighth row: eight rows always are.
 //
-// Measured (whole mcu_linear call, graph replay, microseconds before -> now): Q4_K 64 x 4096 x 14336 31.0 -> 18.0,
+// Measured (whole mcu_linear call, graph replay, microseconds before -> now): Q4_K 64 x 4096 x 14336 31.0 -> 17.3,
 // 17 x 4096 x 4096 13.2 -> 10.5, 64 x 4096 x 1024 17.2 -> 9.6, 2048 x 4096 x 14336 274 -> 213 (1130 TFLOP/s: 0.82 of the
-// sustained cuBLAS rate, the clock is at the power limit); Q6_K 32 x 14336 x 4096 37.1 -> 29.8, 512 x 5632 x 2048 142 -> 30.3.
+// sustained cuBLAS rate, the clock is at the power limit); Q6_K 37 x 14336 x 4096 40.0 -> 24.8, 512 x 5632 x 2048 142 -> 29.2.
 // Up to 128 tokens the converters bound a slab (Q4_K about 1100 cycles for 32768 weights in tiles of up to 64 tokens, 1500 in wider ones;
-// instruction issue); from 256 on the MMAs run at their peak rate (2075 cycles per slab) and what is left is the epilogue (4000 cycles of
-// a tile's 37000).  Beside the kernel a call has its staging launch: of the 18 us at 64 x 4096 x 14336 it and the releases around it take 6.5.
+// instruction issue); from 256 on the MMAs run at their peak rate (2050 cycles per slab) and what is left is the epilogue (7500 cycles
+// beside a tile's 33000 of MMAs, about half of them ahead of the next tile's).  Beside the kernel a call has its staging launch: of the 17 us at 64 x 4096 x 14336 it and the releases around it take 6.5.
 //
 // A CTA has one output tile, or a cluster shares one along K and adds its shares up through distributed shared memory, or the slabs of
 // all tiles are cut into equal ranges: a tile cut between CTAs is then summed from partial tiles by the one that draws the last
