@@ -584,9 +584,9 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
 // From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
 // And from three tokens on where the rows cannot be streamed (Q6_K of ragged sizes), against the plain-load kernel: 3072 x 125 3, 4,
 // 8 tokens 13.5, 16.6, 21.2 us, 7.5, 7.7, 7.8 here; 1280 x 300 7.5, 9.1, 12.5, then 7.6 to 7.7.
-// Single calls of two to four tokens have lines of their own, as their dp4a launch does without the staging launch but depends on the shape
-// more: it suffers from short rows and from long ones (twenty-four shapes at 2, 3 and 4 tokens, recorded; times in us, dp4a then here).  Called
-// one by one, two launches cost the host 7.2 us where one costs 4.2, so that what gains less than about 10 % stays there.
+// Single calls of two to four tokens that are not being recorded have lines of their own, as their dp4a launch does without the staging launch but depends on the shape
+// more: it suffers from short rows and from long ones (twenty-four shapes at 2, 3 and 4 tokens; times in us on the device, dp4a then here).
+// Called one by one, two launches cost the host 7 us where one costs 4, so that what gains less than about 10 % stays there.
 //   Q4_K  2 tokens  1024 x 12288 8.6, 6.4; 2048 x 32000 17.9, 14.6; 14336 x 4096 21.2, 16.1; 4096 x 14336 13.3, 13.1; x 28672 20.5, 23.0
 //         3 tokens  1024 x 4096 5.7, 7.4; x 8192 9.1, 7.6; 4096 x 4096 9.0, 9.3; x 6144 11.1, 10.6; 14336 x 1024 13.4, 11.9
 //         4 tokens  1024 x 4096 6.7, 7.4; x 6144 8.9, 7.4; 2048 x 4096 7.3, 7.9; 1536 x 6144 9.3, 7.9; 4096 x 2048 8.1, 8.4
@@ -604,17 +604,12 @@ static bool few_tokens_pay(int kind, size_t T, size_t K, size_t values) {
             (values >= 32 * M && values <= 96 * M);
     return T == 3 && ((K <= 2048 && rows >= 12288 && values >= 12 * M) || (K > 8192 && values >= 48 * M));
 }
-static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, size_t values, bool streams, bool single) {
+static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, size_t values, bool streams) {
     static const bool off = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch
     if (off || ctx->regime != MCU_REGIME_AUTO || T > (size_t)TI_COLS) return false;
     if (T > (size_t)GEMV_MAX_T || (T >= 3 && !streams)) return true;
     if (T >= 5) return values >= (size_t)4 << 20 || T * K >= 16384 || (kind == KIND_Q4_K && K <= 1024 && T * values >= 8192 * K);
-    return (kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20) || (single && kind != KIND_Q8_0 && few_tokens_pay(kind, T, K, values));
-}
-// A call that is being recorded cannot grow the workspace; the dp4a kernel needs none.
-static bool integer_workspace_there(const mcu_context *ctx, int kind, size_t T, size_t K) {
-    return (ctx->act_qs.cap >= gemm_ti_xq_bytes(kind, (int)T, (int)K) && ctx->gemm_partial.cap >= gemm_ts_workspace_bytes()) ||
-        !stream_is_capturing(ctx->stream);
+    return kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20;
 }
 // The integer matmul by mma.sync, for the sizes where it is the faster one.
 static bool i8_takes(const mcu_context *ctx, int kind, const void *w, const void *w2, size_t T, size_t K, size_t F) {
@@ -670,8 +665,11 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     // a handful of tokens: exact integer dots on the tensor core
     const size_t values = K * F * (w2 != nullptr ? 2 : 1);
     const bool streams = T < 3 || T > (size_t)GEMV_MAX_T || gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F);
-    bool integer = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, K, values, streams, true);
-    if (integer && T <= 4 && ctx->regime == MCU_REGIME_AUTO) integer = integer_workspace_there(ctx, kind, T, K);
+    bool integer = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, K, values, streams);
+    // (Not while a call is being recorded: the dp4a kernel has no workspace, and what was recorded with it stays good when a larger call
+    // makes the workspace move.)
+    if (!integer && T <= 4 && ctx->regime == MCU_REGIME_AUTO && kind != MCU_KIND_Q8_0 && few_tokens_pay(kind, T, K, values))
+        integer = !stream_is_capturing(ctx->stream);
     if (integer && (w2 == nullptr || bias == nullptr)) {
         if (i8_takes(ctx, kind, w, w2, T, K, F)) return i8_locked(ctx, kind, x, ldx, w, w2, T, K, F, bias, out, out2, ldo);
         const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};
@@ -936,7 +934,7 @@ int mcu_linear_multi(mcu_context_t *ctx, const float *x_dev, size_t ldx, size_t 
                 row_tiles += (specs[i].F + TS_ROWS - 1) / TS_ROWS;
                 supported = supported && integer_jobs_supported(&specs[i], 1, K);
             }
-            integer[j] = supported && integer_pays(ctx, specs[j].kind, T, K, values, true, false);
+            integer[j] = supported && integer_pays(ctx, specs[j].kind, T, K, values, true);
             all_integer = all_integer && integer[j];
             tensor = integer[j] ||
                 ((ctx->regime == MCU_REGIME_AUTO || ctx->regime == MCU_REGIME_GEMM) && T > (size_t)GEMV_MAX_T &&

@@ -56,8 +56,8 @@ def test_rows_that_cannot_be_streamed(ctx, oracle, T, K, F):
 @pytest.mark.parametrize("kind,T,K,F", [(KIND_Q4_K, 2, 1024, 12289), (KIND_Q4_K, 2, 16384, 3100), (KIND_Q4_K, 3, 1536, 8200), (KIND_Q4_K, 3, 14336, 1030),
                                         (KIND_Q4_K, 4, 768, 8200), (KIND_Q6_K, 3, 2048, 12300), (KIND_Q6_K, 4, 1024, 8200), (KIND_Q6_K, 4, 14336, 1030)])
 def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
-    """Sizes just beyond the lines: the dp4a kernel's results but for the order of the f32 terms, and, recorded in a context without a
-    workspace, the dp4a kernel itself."""
+    """Sizes just beyond the lines: the dp4a kernel's results but for the order of the f32 terms, and, recorded, the dp4a kernel itself, whose
+    graph holds no address of the workspace that a later, larger call moves."""
     import torch
     from marmot_b200 import Context
     from marmot_b200.runtime import REGIME_AUTO, REGIME_GEMV
@@ -77,10 +77,16 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
     stream = torch.cuda.Stream()
     fresh.set_stream(stream.cuda_stream)
     out = torch.zeros((T, F), device="cuda")
+    more = torch.from_numpy(rng.normal(0, 1, (16, K)).astype(np.float32)).cuda()
     torch.cuda.synchronize()
+    fresh.linear(kind, xd, wd, F, out=out)
+    fresh.synchronize()
     fresh.graph_capture_begin()
     fresh.linear(kind, xd, wd, F, out=out)
     graph = fresh.graph_capture_end()
+    fresh.linear(kind, more, wd, F)
+    out.zero_()
+    torch.cuda.synchronize()
     graph.launch()
     fresh.synchronize()
     assert np.array_equal(out.cpu().numpy(), ref)
