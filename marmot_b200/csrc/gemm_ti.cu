@@ -124,14 +124,16 @@ __device__ __forceinline__ void ti_conv_q6k(const uint8_t *blk, uint32_t phase, 
 // EARLY: the scalers give the sums' place back as soon as they have read them, ahead of the last operations on them.  Worth 4 % where tiles
 // hold one to eight tokens (MoE of 16 tokens 231 -> 222 us) and with Q6_K; with Q4_K it costs registers that larger tiles miss (16 x 4096 x
 // 14336 15.6 -> 15.9), so single matrices do without.
-template <int KIND, bool EARLY>
+// LOOSE: Q6_K rows that are not 16-byte multiples (as a branch beside the 16-byte loads of the others it cost them about 1 %: 7 x 4608 x 2176
+// 12.27 us, 12.17 so).
+template <int KIND, bool EARLY, bool LOOSE>
 __global__ void __launch_bounds__(TI_THREADS, 1)
 gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsParams p) {
     extern __shared__ uint8_t smem_raw[];
     using SL = TsSlab<KIND>;
     constexpr bool Q4 = KIND == KIND_Q4_K;
     constexpr uint32_t B_BYTES = ti_b_bytes<KIND>();
-    const bool loose = !Q4 && p.loose;
+    constexpr bool loose = LOOSE;
     const uint32_t SLAB = loose ? ts_slab_bytes<KIND>(true) : ts_slab_bytes<KIND>(false);
     const uint32_t raw_addr = tm_smem_u32(smem_raw);
     const uint32_t bar_base = (raw_addr + 15u) & ~15u;
@@ -328,8 +330,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     if (lane == 0) tm_mbar_arrive(raw_empty + 8u * rs);
                 };
                 if constexpr (Q4) ti_conv_q4k(row_of(j), done, emit);
-                else if (loose) ti_conv_q6k<false>(row_of(j), 0u, done, emit);
-                else ti_conv_q6k<true>(row_of(j), (uint32_t)((u0 + j - tile * KS) * SL::BYTES) & 15u, done, emit);
+                else ti_conv_q6k<!LOOSE>(row_of(j), (uint32_t)((u0 + j - tile * KS) * SL::BYTES) & 15u, done, emit);
                 if (!ok) break;
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -579,10 +580,10 @@ bool gemm_ti_supported(int kind, const void *W, int K, int F) {
     return (kind == KIND_Q4_K || kind == KIND_Q6_K) && gemm_ts_supported(kind, W, 1, K, F);
 }
 
-template <int KIND, bool EARLY>
+template <int KIND, bool EARLY, bool LOOSE>
 static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
     const int fixed = 16 + 512 + 1024 + TI_B_SLOTS * (int)ti_b_bytes<KIND>() + 2 * TI_COLS * TS_ROWS * 4;
-    const int slab = ts_slab_bytes<KIND>(p.loose != 0);
+    const int slab = ts_slab_bytes<KIND>(LOOSE);
     constexpr int MOST = 224 * 1024;
     p.raw_shift = fixed + 8 * slab <= MOST ? 3 : 2;
     const int smem = fixed + (slab << p.raw_shift);
@@ -590,7 +591,7 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     if (dev >= 64 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
-        if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND, EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
+        if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND, EARLY, LOOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
         if (dev < 64) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
@@ -606,11 +607,11 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.split > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND, EARLY>, maps, p);
+    return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND, EARLY, LOOSE>, maps, p);
 }
 static cudaError_t ti_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
-    if (kind == KIND_Q6_K) return ti_launch<KIND_Q6_K, true>(maps, p, n_cta, s);
-    return p.group_counts != nullptr ? ti_launch<KIND_Q4_K, true>(maps, p, n_cta, s) : ti_launch<KIND_Q4_K, false>(maps, p, n_cta, s);
+    if (kind == KIND_Q6_K) return p.loose ? ti_launch<KIND_Q6_K, true, true>(maps, p, n_cta, s) : ti_launch<KIND_Q6_K, true, false>(maps, p, n_cta, s);
+    return p.group_counts != nullptr ? ti_launch<KIND_Q4_K, true, false>(maps, p, n_cta, s) : ti_launch<KIND_Q4_K, false, false>(maps, p, n_cta, s);
 }
 static cudaError_t ti_encode_x(int kind, CUtensorMap *m, const uint8_t *xq, int rows, int nb) {
     return ts_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, xq, (cuuint64_t)nb * 384, (cuuint64_t)rows * ti_planes(kind), (cuuint64_t)nb * 384, 128,
