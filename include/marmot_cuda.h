@@ -98,7 +98,9 @@ int mcu_context_set_regime(mcu_context_t *ctx, int regime);
  *      the whole sequence with one launch (a decode step of a few hundred small kernels is bound by launch latency
  *      otherwise).  Run the sequence once before capturing: workspace cannot grow during a capture, and the entry
  *      points that wait for the device (mcu_linear_host, mcu_vec_dot_host, mcu_moe_experts, mcu_synchronize) refuse
- *      to be captured.  The recorded pointers are the ones passed during capture: update inputs in place. ---- */
+ *      to be captured.  The recorded pointers are the ones passed during capture: update inputs in place.  A graph keeps the
+ *      context's workspace that it was recorded with: a later, larger call gets new memory, and the old one is given back behind
+ *      mcu_graph_destroy, or, where the caller captured the stream by other means, with the context. ---- */
 typedef struct mcu_graph mcu_graph_t;
 int mcu_graph_capture_begin(mcu_context_t *ctx);
 int mcu_graph_capture_end(mcu_context_t *ctx, mcu_graph_t **out_graph); /* out_graph NULL: discard the capture */

@@ -8,13 +8,16 @@
 #include "kernels.h"
 #include "moe.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <climits>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <vector>
 
 namespace mcu {
@@ -60,9 +63,16 @@ int device_sm_count() {
     return v;
 }
 
+// A workspace allocation that a recorded sequence of calls may hold the address of (in kernel arguments and tensor maps) has a
+// GraphHold, shared with the graphs that were recorded with it: it outlives its place in the workspace until they are gone.
+struct GraphHold {
+    bool elsewhere = false;  // recorded by a capture of the caller's own, whose graph this library does not see: until the context goes
+};
 struct Buffer {
     void *ptr = nullptr;
     size_t cap = 0;
+    std::shared_ptr<GraphHold> hold;
+    bool tickets = false;  // zero between launches
 };
 
 }  // namespace mcu
@@ -101,6 +111,9 @@ struct mcu_context {
     cudaEvent_t pin_event[PIN_SLOTS] = {};
     bool pin_used[PIN_SLOTS] = {};
     int pin_next = 0;
+    std::vector<Buffer> retired;                         // allocations that graphs still hold, replaced by larger ones
+    bool recording = false;                              // between mcu_graph_capture_begin and mcu_graph_capture_end
+    std::vector<std::shared_ptr<GraphHold>> holds;       // of the recording at hand
 };
 
 static bool stream_is_capturing(cudaStream_t s) {
@@ -112,23 +125,63 @@ static bool stream_is_capturing(cudaStream_t s) {
     return st != cudaStreamCaptureStatusNone;
 }
 
-static int ensure(mcu_context *ctx, Buffer &b, size_t bytes) {
-    if (bytes <= b.cap) return MCU_SUCCESS;
-    // Growing means a synchronize, a free and an allocation: none of that can be recorded into a CUDA graph, and the
-    // graph would keep the old address anyway.
-    if (stream_is_capturing(ctx->stream))
+// The call at hand is being recorded with the address of `b`.
+static int hold_for_graph(mcu_context *ctx, Buffer &b) {
+    try {
+        if (b.hold == nullptr) b.hold = std::make_shared<GraphHold>();
+        if (!ctx->recording)
+            b.hold->elsewhere = true;
+        else if (std::find(ctx->holds.begin(), ctx->holds.end(), b.hold) == ctx->holds.end())
+            ctx->holds.push_back(b.hold);
+    } catch (const std::bad_alloc &) {
+        return fail(MCU_ERROR_OUT_OF_MEMORY, "host memory exhausted while a call is recorded");
+    }
+    return MCU_SUCCESS;
+}
+
+// A capture that mcu_graph_capture_begin opened was ended by other means: who ended it has the graph.
+static void graph_not_ours(mcu_context *ctx) {
+    for (const std::shared_ptr<GraphHold> &h : ctx->holds) h->elsewhere = true;
+    ctx->holds.clear();
+    ctx->recording = false;
+}
+
+// At least `bytes` in `b`.  `recording`: the call is being captured into a CUDA graph (asking costs the host 40 ns).
+// An allocation that a graph holds is not freed when a larger call replaces it: replays go on staging their rows there.  A recording keeps
+// one allocation per buffer at most, and those whose graphs have been destroyed are given back the next time any buffer grows.
+static int ensure(mcu_context *ctx, Buffer &b, size_t bytes, bool recording) {
+    if (bytes <= b.cap) return recording && bytes > 0 ? hold_for_graph(ctx, b) : MCU_SUCCESS;
+    // Growing means a synchronize and an allocation: none of that can be recorded into a CUDA graph.
+    if (recording)
         return fail(MCU_ERROR_INVALID_OPERATION,
                     "workspace would have to grow during stream capture: run the same call once before capturing");
     // Kernels already enqueued may still read the old allocation.
     MCU_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (b.ptr != nullptr) MCU_CUDA(cudaFree(b.ptr));
-    b.ptr = nullptr;
-    b.cap = 0;
+    for (size_t i = 0; i < ctx->retired.size();) {
+        const Buffer &old = ctx->retired[i];
+        if (old.hold->elsewhere || old.hold.use_count() > 1) {
+            ++i;
+            continue;
+        }
+        MCU_CUDA(cudaFree(old.ptr));  // (waits for the device: a replay of a graph that is gone may still be under way)
+        ctx->retired.erase(ctx->retired.begin() + (ptrdiff_t)i);
+    }
+    if (b.hold != nullptr && (b.hold->elsewhere || b.hold.use_count() > 1)) {
+        try {
+            ctx->retired.push_back(b);
+        } catch (const std::bad_alloc &) {
+            return fail(MCU_ERROR_OUT_OF_MEMORY, "host memory exhausted");
+        }
+    } else if (b.ptr != nullptr) {
+        MCU_CUDA(cudaFree(b.ptr));
+    }
+    b = Buffer{};
     const size_t want = (bytes + 255) & ~(size_t)255;
     MCU_CUDA(cudaMalloc(&b.ptr, want));
     b.cap = want;
     return MCU_SUCCESS;
 }
+static int ensure(mcu_context *ctx, Buffer &b, size_t bytes) { return ensure(ctx, b, bytes, stream_is_capturing(ctx->stream)); }
 
 // A kernel reported `flag` and the stream `s` is idle.  A matmul that gave up on a bounded wait leaves the tickets that it has drawn: the
 // next one would take a share for the last of its tile too early, so they start from zero again.
@@ -136,6 +189,8 @@ static int report_flag(mcu_context *ctx, cudaStream_t s, int flag) {
     MCU_CUDA(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), s));
     MCU_CUDA(cudaMemsetAsync(ctx->gemm_counters, 0, GEMM_TMA_MAX_TILE_COUNTERS * sizeof(int), s));  // (whatever the flag: the last report wins)
     if (ctx->i8_tickets.ptr != nullptr) MCU_CUDA(cudaMemsetAsync(ctx->i8_tickets.ptr, 0, ctx->i8_tickets.cap, s));
+    for (const Buffer &b : ctx->retired)
+        if (b.tickets) MCU_CUDA(cudaMemsetAsync(b.ptr, 0, b.cap, s));
     if (flag == 40) return fail(MCU_ERROR_INVALID_ARGUMENT, "MoE expert id is out of range (found by an earlier call)");
     return fail(MCU_ERROR_INVALID_OPERATION, "a device-side wait timed out (code %d)", flag);
 }
@@ -178,6 +233,8 @@ int context_attention_tickets(mcu_context *ctx, size_t bytes, void **out) {
     if (bytes > ctx->attn_tickets.cap) {
         if (int rc = ensure(ctx, ctx->attn_tickets, bytes)) return rc;
         MCU_CUDA(cudaMemsetAsync(ctx->attn_tickets.ptr, 0, ctx->attn_tickets.cap, ctx->stream));
+    } else if (int rc = ensure(ctx, ctx->attn_tickets, bytes)) {
+        return rc;
     }
     *out = ctx->attn_tickets.ptr;
     return MCU_SUCCESS;
@@ -272,6 +329,7 @@ void mcu_context_destroy(mcu_context_t *ctx) {
                       &ctx->bias_stage, &ctx->moe_meta, &ctx->moe_hidden, &ctx->moe_gate, &ctx->moe_up, &ctx->moe_down, &ctx->gemm_partial, &ctx->attn_partial, &ctx->i8_partial, &ctx->i8_tickets, &ctx->pro_h, &ctx->attn_tickets, &ctx->rope_table};
     for (Buffer *b : bufs)
         if (b->ptr != nullptr) cudaFree(b->ptr);
+    for (Buffer &b : ctx->retired) cudaFree(b.ptr);
     if (ctx->dev_err != nullptr) cudaFree(ctx->dev_err);
     if (ctx->err_host != nullptr) cudaFreeHost(ctx->err_host);
     if (ctx->moe_event != nullptr) cudaEventDestroy(ctx->moe_event);
@@ -311,6 +369,7 @@ void *mcu_context_get_stream(mcu_context_t *ctx) { return ctx != nullptr ? (void
 struct mcu_graph {
     cudaGraphExec_t exec = nullptr;
     mcu_context *ctx = nullptr;
+    std::vector<std::shared_ptr<GraphHold>> holds;  // the workspace that it was recorded with
 };
 
 int mcu_graph_capture_begin(mcu_context_t *ctx) {
@@ -321,6 +380,8 @@ int mcu_graph_capture_begin(mcu_context_t *ctx) {
         return fail(MCU_ERROR_INVALID_OPERATION,
                     "the default stream cannot be captured: give the context a stream of its own (mcu_context_set_stream)");
     MCU_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    graph_not_ours(ctx);
+    ctx->recording = true;
     return MCU_SUCCESS;
 }
 
@@ -328,7 +389,13 @@ int mcu_graph_capture_end(mcu_context_t *ctx, mcu_graph_t **out) {
     if (int rc = check_ctx(ctx)) return rc;
     std::lock_guard<std::mutex> lock(ctx->mu);
     if (out != nullptr) *out = nullptr;
-    if (!stream_is_capturing(ctx->stream)) return fail(MCU_ERROR_INVALID_OPERATION, "no capture in progress");
+    if (!stream_is_capturing(ctx->stream)) {
+        graph_not_ours(ctx);
+        return fail(MCU_ERROR_INVALID_OPERATION, "no capture in progress");
+    }
+    std::vector<std::shared_ptr<GraphHold>> holds = std::move(ctx->holds);
+    ctx->holds.clear();
+    ctx->recording = false;
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     if (e != cudaSuccess || graph == nullptr) {
@@ -351,6 +418,7 @@ int mcu_graph_capture_end(mcu_context_t *ctx, mcu_graph_t **out) {
         return cuda_fail(e, "cudaGraphInstantiate");
     }
     g->ctx = ctx;
+    g->holds = std::move(holds);
     *out = g;
     return MCU_SUCCESS;
 }
@@ -501,13 +569,14 @@ static int pack_activations(mcu_context *ctx, int kind, const float *x, size_t l
                             ActBuffers &ab) {
     const size_t bv = (size_t)block_values(kind);
     const size_t nb = (K + bv - 1) / bv, kp = nb * bv;
-    if (int rc = ensure(ctx, ctx->act_qs, T * kp)) return rc;
-    if (int rc = ensure(ctx, ctx->act_d, T * nb * sizeof(float))) return rc;
+    const bool rec = stream_is_capturing(ctx->stream);
+    if (int rc = ensure(ctx, ctx->act_qs, T * kp, rec)) return rc;
+    if (int rc = ensure(ctx, ctx->act_d, T * nb * sizeof(float), rec)) return rc;
     if (kind != MCU_KIND_Q8_0)
-        if (int rc = ensure(ctx, ctx->act_bsums, T * nb * 16 * sizeof(int16_t))) return rc;
+        if (int rc = ensure(ctx, ctx->act_bsums, T * nb * 16 * sizeof(int16_t), rec)) return rc;
     if (want_half) {
-        if (int rc = ensure(ctx, ctx->act_half, T * kp * sizeof(__half))) return rc;
-        if (int rc = ensure(ctx, ctx->act_rowscale, T * sizeof(float))) return rc;
+        if (int rc = ensure(ctx, ctx->act_half, T * kp * sizeof(__half), rec)) return rc;
+        if (int rc = ensure(ctx, ctx->act_rowscale, T * sizeof(float), rec)) return rc;
     }
     ab.qs = (int8_t *)ctx->act_qs.ptr;
     ab.d = (float *)ctx->act_d.ptr;
@@ -547,11 +616,12 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
     const bool kq = kind != MCU_KIND_Q8_0;
     const size_t bv = (size_t)block_values(kind);
     const size_t kp = (K + bv - 1) / bv * bv;
+    const bool rec = stream_is_capturing(ctx->stream);
     if (st != nullptr && st->valid && st->kq == kq) {
         // staged by an earlier matmul of this call
     } else if (act_half_fused_smem(kind, (int)K) <= 48 * 1024) {
-        if (int rc = ensure(ctx, ctx->act_half, T * kp * sizeof(__half))) return rc;
-        if (int rc = ensure(ctx, ctx->act_rowscale, T * sizeof(float))) return rc;
+        if (int rc = ensure(ctx, ctx->act_half, T * kp * sizeof(__half), rec)) return rc;
+        if (int rc = ensure(ctx, ctx->act_rowscale, T * sizeof(float), rec)) return rc;
         MCU_CUDA(launch_act_half_fused_from(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K,
                                             (__half *)ctx->act_half.ptr, (float *)ctx->act_rowscale.ptr, ctx->stream));
         count_launches(1);
@@ -565,7 +635,7 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
         if (int rc = pack_activations(ctx, kind, x, ldx, T, K, true, ab)) return rc;
         if (st != nullptr) st->valid = false;
     }
-    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes(), rec)) return rc;
     MCU_CUDA(launch_gemm_ts(kind, jobs, n_jobs, (const __half *)ctx->act_half.ptr, (const float *)ctx->act_rowscale.ptr, (int)kp,
                             (int)T, (int)K, (float *)ctx->gemm_partial.ptr, ctx->gemm_counters, ctx->dev_err, ctx->stream));
     count_launches(1);
@@ -618,16 +688,20 @@ static bool i8_takes(const mcu_context *ctx, int kind, const void *w, const void
 }
 static int i8_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, const void *w, const void *w2, size_t T, size_t K, size_t F,
                      const float *bias, float *out, float *out2, size_t ldo) {
+    const bool rec = stream_is_capturing(ctx->stream);
     size_t qs_b, dT_b, part_b, tick_b;
     gemm_i8_workspace_bytes((int)T, (int)K, (int)F, w2 != nullptr, &qs_b, &dT_b, &part_b, &tick_b);
-    if (int rc = ensure(ctx, ctx->act_qs, qs_b)) return rc;
-    if (int rc = ensure(ctx, ctx->act_d, dT_b)) return rc;
+    if (int rc = ensure(ctx, ctx->act_qs, qs_b, rec)) return rc;
+    if (int rc = ensure(ctx, ctx->act_d, dT_b, rec)) return rc;
     // (the shares for any call of the context, and tickets for a million rows: a recorded call keeps their addresses when larger ones follow)
     tick_b = tick_b > (size_t)256 << 10 ? tick_b : (size_t)256 << 10;
-    if (int rc = ensure(ctx, ctx->i8_partial, part_b)) return rc;
+    if (int rc = ensure(ctx, ctx->i8_partial, part_b, rec)) return rc;
     if (tick_b > ctx->i8_tickets.cap) {  // a fresh ticket area starts at zero; the kernel keeps it so
-        if (int rc = ensure(ctx, ctx->i8_tickets, tick_b)) return rc;
+        if (int rc = ensure(ctx, ctx->i8_tickets, tick_b, rec)) return rc;
+        ctx->i8_tickets.tickets = true;
         MCU_CUDA(cudaMemsetAsync(ctx->i8_tickets.ptr, 0, ctx->i8_tickets.cap, ctx->stream));
+    } else if (int rc = ensure(ctx, ctx->i8_tickets, tick_b, rec)) {
+        return rc;
     }
     MCU_CUDA(launch_gemm_i8(kind, w, w2, x, (int)ldx, (int)T, (int)K, (int)F, bias, out, out2, (int)ldo, (int8_t *)ctx->act_qs.ptr,
                             (float *)ctx->act_d.ptr, (float *)ctx->i8_partial.ptr, (int *)ctx->i8_tickets.ptr, ctx->dev_err, ctx->stream));
@@ -641,8 +715,9 @@ static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K
 }
 static int integer_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, const GemvJobSpec *jobs, int n_jobs,
                           const ActSource *src, int *staged_kind) {
-    if (int rc = ensure(ctx, ctx->act_qs, gemm_ti_xq_bytes(kind, (int)T, (int)K))) return rc;
-    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes())) return rc;
+    const bool rec = stream_is_capturing(ctx->stream);
+    if (int rc = ensure(ctx, ctx->act_qs, gemm_ti_xq_bytes(kind, (int)T, (int)K), rec)) return rc;
+    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes(), rec)) return rc;
     uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
     if (staged_kind == nullptr || *staged_kind != kind) {
         MCU_CUDA(launch_act_int_fused(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K, xq, ctx->stream));
@@ -1113,11 +1188,12 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     const size_t routes = T * k;
     // routing metadata: counts[E+1] | offsets[E+1] | sorted_tok | sorted_w | route_pos
     const size_t meta_bytes = (2 * (E + 1) + 3 * routes) * sizeof(int32_t);
-    if (int rc = ensure(ctx, ctx->moe_meta, meta_bytes)) return rc;
-    if (int rc = ensure(ctx, ctx->moe_hidden, routes * H * sizeof(float))) return rc;
-    if (int rc = ensure(ctx, ctx->moe_gate, routes * FF * sizeof(float))) return rc;
-    if (int rc = ensure(ctx, ctx->moe_up, routes * FF * sizeof(float))) return rc;
-    if (int rc = ensure(ctx, ctx->moe_down, routes * H * sizeof(float))) return rc;
+    const bool capturing = stream_is_capturing(ctx->stream);
+    if (int rc = ensure(ctx, ctx->moe_meta, meta_bytes, capturing)) return rc;
+    if (int rc = ensure(ctx, ctx->moe_hidden, routes * H * sizeof(float), capturing)) return rc;
+    if (int rc = ensure(ctx, ctx->moe_gate, routes * FF * sizeof(float), capturing)) return rc;
+    if (int rc = ensure(ctx, ctx->moe_up, routes * FF * sizeof(float), capturing)) return rc;
+    if (int rc = ensure(ctx, ctx->moe_down, routes * H * sizeof(float), capturing)) return rc;
     MoeRouteBuffers rb;
     rb.counts = (int *)ctx->moe_meta.ptr;
     rb.offsets = rb.counts + (E + 1);
@@ -1164,7 +1240,7 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     // so (93, 102), and so do few routes of large experts in Q6_K, whose launches are the streaming kernels' (8 experts of 3 x 14336 x 4096,
     // 3, 8, 12, 16 routes: 174, 149; 326, 302; 372, 378; 413, 444.  16 of 3 x 7168 x 4096, 3, 8, 12: 120, 110; 208, 212; 274, 292).
     const size_t n6 = (gate_kind == KIND_Q6_K ? 1 : 0) + (down_kind == KIND_Q6_K ? 1 : 0);
-    const bool large = H * FF > (size_t)26 << 20, capturing = stream_is_capturing(s);
+    const bool large = H * FF > (size_t)26 << 20;
     const size_t most_rows = (large ? 48 : 128) / (2 + n6);
     const bool fp16_suits = gate_kind == up_kind && gemm_ts_grouped_supported(gate_kind, gate_dev, (int)H, (int)FF) &&
         gemm_ts_grouped_supported(up_kind, up_dev, (int)H, (int)FF) && gemm_ts_grouped_supported(down_kind, down_dev, (int)FF, (int)H) &&
@@ -1178,15 +1254,15 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     const bool few = capturing ? few_recorded : few_suits && routes <= most_rows * E && routes > apart;
     auto few_workspace = [&]() -> int {
         const size_t xq_h = gemm_ti_xq_bytes(gate_kind, (int)routes, (int)H), xq_f = gemm_ti_xq_bytes(down_kind, (int)routes, (int)FF);
-        if (int rc = ensure(ctx, ctx->act_qs, xq_h > xq_f ? xq_h : xq_f)) return rc;
-        return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes());
+        if (int rc = ensure(ctx, ctx->act_qs, xq_h > xq_f ? xq_h : xq_f, capturing)) return rc;
+        return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes(), capturing);
     };
     const size_t kp_h = (H + block_values(gate_kind) - 1) / block_values(gate_kind) * block_values(gate_kind);
     const size_t kp_f = (FF + block_values(down_kind) - 1) / block_values(down_kind) * block_values(down_kind);
     auto fp16_workspace = [&]() -> int {
-        if (int rc = ensure(ctx, ctx->act_half, routes * (kp_h > kp_f ? kp_h : kp_f) * sizeof(__half))) return rc;
-        if (int rc = ensure(ctx, ctx->act_rowscale, routes * sizeof(float))) return rc;
-        return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes());
+        if (int rc = ensure(ctx, ctx->act_half, routes * (kp_h > kp_f ? kp_h : kp_f) * sizeof(__half), capturing)) return rc;
+        if (int rc = ensure(ctx, ctx->act_rowscale, routes * sizeof(float), capturing)) return rc;
+        return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes(), capturing);
     };
     if (few) {
         // A bad expert id is reported by the call itself, as ever for few routes: the flag is fetched behind the routing and
