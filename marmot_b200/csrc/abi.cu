@@ -674,9 +674,12 @@ static bool few_tokens_pay(int kind, size_t T, size_t K, size_t values) {
             (values >= 32 * M && values <= 96 * M);
     return T == 3 && ((K <= 2048 && rows >= 12288 && values >= 12 * M) || (K > 8192 && values >= 48 * M));
 }
-static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, size_t values, bool streams) {
+static bool integer_allowed(const mcu_context *ctx) {
     static const bool off = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch
-    if (off || ctx->regime != MCU_REGIME_AUTO || T > (size_t)TI_COLS) return false;
+    return !off && ctx->regime == MCU_REGIME_AUTO;
+}
+static bool integer_pays(const mcu_context *ctx, int kind, size_t T, size_t K, size_t values, bool streams) {
+    if (!integer_allowed(ctx) || T > (size_t)TI_COLS) return false;
     if (T > (size_t)GEMV_MAX_T || (T >= 3 && !streams)) return true;
     if (T >= 5) return values >= (size_t)4 << 20 || T * K >= 16384 || (kind == KIND_Q4_K && K <= 1024 && T * values >= 8192 * K);
     return kind == KIND_Q4_K && T >= 3 && T * values >= (size_t)64 << 20;
@@ -743,7 +746,7 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     bool integer = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, K, values, streams);
     // (Not while a call is being recorded: the dp4a kernel has no workspace, and what was recorded with it stays good when a larger call
     // makes the workspace move.)
-    if (!integer && T <= 4 && ctx->regime == MCU_REGIME_AUTO && kind != MCU_KIND_Q8_0 && few_tokens_pay(kind, T, K, values))
+    if (!integer && T <= 4 && integer_allowed(ctx) && kind != MCU_KIND_Q8_0 && few_tokens_pay(kind, T, K, values))
         integer = !stream_is_capturing(ctx->stream);
     if (integer && (w2 == nullptr || bias == nullptr)) {
         if (i8_takes(ctx, kind, w, w2, T, K, F)) return i8_locked(ctx, kind, x, ldx, w, w2, T, K, F, bias, out, out2, ldo);

@@ -93,6 +93,33 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
     fresh.close()
 
 
+@pytest.mark.parametrize("T,K,F", [(4, 768, 16384), (8, 4096, 4096)])
+def test_diagnostic_switch(T, K, F):
+    """MARMOT_CUDA_NO_I8MMA leaves a call of few tokens to the dp4a kernel, which is one launch (the integer matmul: two)."""
+    import os
+    import subprocess
+    import sys
+
+    program = f"""
+import torch
+from marmot_b200 import Context
+from marmot_b200.runtime import KIND_Q4_K
+ctx = Context(0)
+x, w = torch.zeros(({T}, {K}), device="cuda"), torch.zeros({F} * {K} // 256 * 144, dtype=torch.uint8, device="cuda")
+before = ctx.launch_count()
+ctx.linear(KIND_Q4_K, x, w, {F})
+ctx.synchronize()
+print("launches", ctx.launch_count() - before)
+"""
+    for switch, launches in ((None, 2), ("1", 1)):
+        env = {k: v for k, v in os.environ.items() if k != "MARMOT_CUDA_NO_I8MMA"}
+        if switch:
+            env["MARMOT_CUDA_NO_I8MMA"] = switch
+        r = subprocess.run([sys.executable, "-c", program], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr
+        assert f"launches {launches}" in r.stdout.splitlines(), (switch, r.stdout)
+
+
 @pytest.mark.parametrize("T,K,F", [(3, 4096, 5632), (4, 4096, 4096), (5, 2048, 2056), (8, 4096, 1030), (16, 512, 40)])
 def test_two_matrices_of_each_kind_with_prologues(ctx, oracle, T, K, F):
     """The sizes at which linear_multi leaves the dp4a kernel: every result equals the one of the plain regime, and x' is exact."""
