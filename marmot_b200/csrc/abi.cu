@@ -744,10 +744,10 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     const size_t values = K * F * (w2 != nullptr ? 2 : 1);
     const bool streams = T < 3 || T > (size_t)GEMV_MAX_T || gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F);
     bool integer = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, K, values, streams);
-    // (Not while a call is being recorded: the dp4a kernel has no workspace, and what was recorded with it stays good when a larger call
-    // makes the workspace move.)
+    // (Only where the dp4a kernel streams the rows, so that it has no workspace, and not while a call is being recorded: such a call could
+    // always be recorded without one made before it.)
     if (!integer && T <= 4 && integer_allowed(ctx) && kind != MCU_KIND_Q8_0 && few_tokens_pay(kind, T, K, values))
-        integer = !stream_is_capturing(ctx->stream);
+        integer = (T > 2 ? streams : gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F)) && !stream_is_capturing(ctx->stream);
     if (integer && (w2 == nullptr || bias == nullptr)) {
         if (i8_takes(ctx, kind, w, w2, T, K, F)) return i8_locked(ctx, kind, x, ldx, w, w2, T, K, F, bias, out, out2, ldo);
         const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};

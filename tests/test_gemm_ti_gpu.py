@@ -93,6 +93,34 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
     fresh.close()
 
 
+def test_two_tokens_on_rows_too_long_to_stream():
+    """The call and its recording are the same kernels: the one finds the workspace that the other has reserved."""
+    import torch
+    from marmot_b200 import Context
+
+    T, K, F = 2, 131072, 400
+    rng = np.random.default_rng(3)
+    ctx = Context(0, use_torch_stream=False)
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    x, w = torch.from_numpy(rng.normal(0, 1, (T, K)).astype(np.float32)).cuda(), ctx.upload(random_blocks(KIND_Q4_K, F, K, rng))
+    out = torch.zeros((T, F), device="cuda")
+    torch.cuda.synchronize()
+    ctx.linear(KIND_Q4_K, x, w, F, out=out)
+    ctx.synchronize()
+    first = out.cpu().numpy()
+    ctx.graph_capture_begin()
+    ctx.linear(KIND_Q4_K, x, w, F, out=out)
+    graph = ctx.graph_capture_end()
+    out.zero_()
+    torch.cuda.synchronize()
+    graph.launch()
+    ctx.synchronize()
+    assert np.array_equal(out.cpu().numpy(), first)
+    graph.close()
+    ctx.close()
+
+
 @pytest.mark.parametrize("T,K,F", [(4, 768, 16384), (8, 4096, 4096)])
 def test_diagnostic_switch(T, K, F):
     """MARMOT_CUDA_NO_I8MMA leaves a call of few tokens to the dp4a kernel, which is one launch (the integer matmul: two)."""
