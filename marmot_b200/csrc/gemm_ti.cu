@@ -121,12 +121,9 @@ __device__ __forceinline__ void ti_conv_q6k(const uint8_t *blk, uint32_t phase, 
     emit.corrections(c);
 }
 
-// EARLY: the scalers give the sums' place back as soon as they have read them, ahead of the last operations on them.  Worth 4 % where tiles
-// hold one to eight tokens (MoE of 16 tokens 231 -> 222 us) and with Q6_K; with Q4_K it costs registers that larger tiles miss (16 x 4096 x
-// 14336 15.6 -> 15.9), so single matrices do without.
 // LOOSE: Q6_K rows that are not 16-byte multiples (as a branch beside the 16-byte loads of the others it cost them about 1 %: 7 x 4608 x 2176
 // 12.27 us, 12.17 so).
-template <int KIND, bool EARLY, bool LOOSE>
+template <int KIND, bool LOOSE>
 __global__ void __launch_bounds__(TI_THREADS, 1)
 gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -383,14 +380,6 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t from = lanes + (uint32_t)group * TI_D_COLS;
-                    auto release = [&] {
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) {
-                            tm_mbar_arrive(d_empty + 8u * group);
-                            tm_mbar_arrive(dx_read + 8u * slot);
-                        }
-                    };
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {  // eight tokens at a time
                         if (8 * hh >= t.t_count) break;
@@ -418,7 +407,6 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                         ti_ld8(from + 128u + 8u * hh, lo);
                         ti_ld8(from + 144u + 8u * hh, hi);
                         ti_wait_ld();
-                        if (EARLY && (hh == 1 || t.t_count <= 8)) release();
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             const int corr = lo[i] + 64 * hi[i];
@@ -428,7 +416,14 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                                 acc[hh][i] = fmaf(dxv[i], __fmul_rn(d, (float)(sum[i] - 32 * corr)), acc[hh][i]);
                         }
                     }
-                    if (!EARLY) release();
+                    // (Behind the last operations: given back ahead of them, as soon as the sums are read, Q6_K of 7 x 4608 x 4096 took 13.0 instead
+                    // of 12.5 us, MoE of 24 tokens with a Q6_K down projection 63.7 instead of 62.5, Q4_K of 12 x 3072 x 1024 7.94 instead of 7.84.)
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        tm_mbar_arrive(d_empty + 8u * group);
+                        tm_mbar_arrive(dx_read + 8u * slot);
+                    }
                 }
                 if (!ok) break;
                 // ---- the tile's part is complete: group 1's sums go to group 0 ----
@@ -580,7 +575,7 @@ bool gemm_ti_supported(int kind, const void *W, int K, int F) {
     return (kind == KIND_Q4_K || kind == KIND_Q6_K) && gemm_ts_supported(kind, W, 1, K, F);
 }
 
-template <int KIND, bool EARLY, bool LOOSE>
+template <int KIND, bool LOOSE>
 static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
     const int fixed = 16 + 512 + 1024 + TI_B_SLOTS * (int)ti_b_bytes<KIND>() + 2 * TI_COLS * TS_ROWS * 4;
     const int slab = ts_slab_bytes<KIND>(LOOSE);
@@ -591,7 +586,7 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev)) return e;
     if (dev >= 64 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
-        if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND, EARLY, LOOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
+        if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND, LOOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
         if (dev < 64) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
@@ -607,11 +602,11 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.split > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND, EARLY, LOOSE>, maps, p);
+    return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND, LOOSE>, maps, p);
 }
 static cudaError_t ti_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
-    if (kind == KIND_Q6_K) return p.loose ? ti_launch<KIND_Q6_K, true, true>(maps, p, n_cta, s) : ti_launch<KIND_Q6_K, true, false>(maps, p, n_cta, s);
-    return p.group_counts != nullptr ? ti_launch<KIND_Q4_K, true, false>(maps, p, n_cta, s) : ti_launch<KIND_Q4_K, false, false>(maps, p, n_cta, s);
+    if (kind == KIND_Q4_K) return ti_launch<KIND_Q4_K, false>(maps, p, n_cta, s);
+    return p.loose ? ti_launch<KIND_Q6_K, true>(maps, p, n_cta, s) : ti_launch<KIND_Q6_K, false>(maps, p, n_cta, s);
 }
 static cudaError_t ti_encode_x(int kind, CUtensorMap *m, const uint8_t *xq, int rows, int nb) {
     return ts_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, xq, (cuuint64_t)nb * 384, (cuuint64_t)rows * ti_planes(kind), (cuuint64_t)nb * 384, 128,
