@@ -147,6 +147,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
     __shared__ int cut_tile[2];  // cut tiles that this CTA has to add up: of its range's start and end
+    __shared__ int cut_first[2], cut_last[2], cut_slot[2];  // who has their shares, and which slot of the first one
     __shared__ int group_tile0[TS_MAX_GROUPS + 1];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -337,6 +338,17 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
             err_code = 49;
         } else {
             // ------------------------------ scalers ------------------------------
+            // (Divisions in 64 bits: here they pass while the kernel ahead is waited for.  Between a share and its ticket, and again for every
+            // share that was read, they were 1 us of a launch with short ranges: MoE of 4 tokens on 8 experts of 512 x 1024 25.3 -> 23.2 us,
+            // 16 tokens on 4 of 3584 x 1024 39.6 -> 36.5.)
+            if (warp == TI_CONV && lane < 2 && split == 1 && !p.whole && n_slabs > 0) {
+                const int cut = (lane == 0 ? u0 : u1 - 1) / KS;
+                const TsOwners own = ts_owners(work, cut, KS);
+                cut_first[lane] = own.first;
+                cut_last[lane] = own.last;
+                cut_slot[lane] = ts_share_slot(work, cut, KS, own.first);
+            }
+            __syncwarp();
             asm volatile("griddepcontrol.wait;" ::: "memory");
             float acc[2][8];
             uint32_t segs = 0;
@@ -473,9 +485,8 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                         ok = ts_wait(share_bar + 8u * which, 0u);
                         ok = __all_sync(0xffffffffu, ok);
                         if (lane == 0 && ok) {
-                            const TsOwners own = ts_owners(work, tile, KS);
-                            int *ctr = p.counters + own.first;
-                            if (atomicAdd(ctr, 1) == own.last - own.first) {
+                            int *ctr = p.counters + cut_first[which];
+                            if (atomicAdd(ctr, 1) == cut_last[which] - cut_first[which]) {
                                 *ctr = 0;  // ready for the next launch
                                 cut_tile[which] = tile;
                             }
@@ -532,14 +543,15 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
         __syncwarp();
         ts_cluster_sync();  // nobody leaves while its share is being read
     }
-    // Shares of cut tiles, in the order of K (the scalers: they have waited for the kernel ahead).
-    for (int s = 0; s < 2; ++s) {
+    // Shares of cut tiles, in the order of K (the scalers: they have waited for the kernel ahead).  (Plans without cut tiles pass by without
+    // looking: 8 x 2048 x 2048 Q4_K 7.5 -> 7.25 us.)
+    for (int s = 0; s < 2 && split == 1 && !p.whole; ++s) {
         const int tile = cut_tile[s];
         if (tile < 0 || threadIdx.x < 256 || threadIdx.x >= 512) continue;
         __threadfence();
         const TsTile t = work.tile(p, tile);
         const TsJob &jb = p.jobs[t.job];
-        const TsOwners own = ts_owners(work, tile, KS);
+        const int first = cut_first[s], last = cut_last[s], slot0 = cut_slot[s];
         const int r = threadIdx.x & (TS_ROWS - 1), fr = loose ? (r >> 4) + 8 * (r & 15) : r, f = t.f0 + fr;
         const int c0 = 8 * (int)((threadIdx.x - 256) >> 7);  // eight of the tokens
         if (fr >= t.rows || c0 >= t.t_count) continue;
@@ -547,8 +559,8 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[c] = 0.0f;
 #pragma unroll 4
-        for (int k = own.first; k <= own.last; ++k) {
-            const float *from = p.partial + (size_t)(k * 2 + ts_share_slot(work, tile, KS, k)) * (TS_ROWS * TI_COLS) + c0 * TS_ROWS + r;
+        for (int k = first; k <= last; ++k) {  // (the ranges behind the first one start inside the tile)
+            const float *from = p.partial + (size_t)(k * 2 + (k == first ? slot0 : 0)) * (TS_ROWS * TI_COLS) + c0 * TS_ROWS + r;
             float v[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) v[c] = __ldcg(from + c * TS_ROWS);
