@@ -196,7 +196,8 @@ inline TsPlan ts_plan(int kind, int T, int K, const int *F, int n_jobs, int sms)
 // first, by a sweep of all three at nine tokens: a slab takes about 900 cycles (Q6_K 2100), the start of a CTA 2700 and each of its tiles 800 (8 x 4096 x 28672
 // Q4_K, 224 tiles: 27.0 us in ranges, 24.6 so), a cluster's exchange 1500; a tile cut between
 // ranges costs 9000 and 700 for every share that the last CTA reads (13056 x 1792 Q4_K: 22 us in ranges of five slabs, 13 in
-// clusters of eight).  Clusters of eight: as in ts_spread.
+// clusters of eight).  Clusters of eight: as in ts_spread.  Of clusters of four 33 run at once (a GPC's SMs are not always a multiple of four);
+// the rest were a second wave: 9 tokens x 2048 on 33, 34 row tiles 8.4, 14.1 us, the latter 8.8 in clusters of two; Q6_K x 14336 24.9, 43.5, 28.3.
 inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
     const long U = (long)tiles * KS, n_most = U < sms ? U : sms, upc = (U + n_most - 1) / n_most;
     const double unit = kind == KIND_Q4_K ? 900.0 : 2100.0;
@@ -207,7 +208,7 @@ inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
     const int waves = (tiles + sms - 1) / sms;
     consider(1, tiles < sms ? tiles : sms, waves * (KS * unit + 800.0) + 2700.0, 1);
     for (int sp = 2; sp <= TS_MAX_SPLIT && sp <= KS; sp *= 2)
-        if ((long)tiles * sp <= (sp >= 8 ? sms * 7 / 9 : sms)) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + 5000.0);
+        if ((long)tiles * sp <= (sp >= 8 ? sms * 7 / 9 : sp >= 4 ? sms * 9 / 10 : sms)) consider(sp, (long)tiles * sp, (KS + sp - 1) / sp * unit + 5000.0);
     const bool cut = U % n_most != 0 || upc % KS != 0;
     consider(1, n_most, (double)upc * unit + 2000.0 + (cut ? 9000.0 + 700.0 * ((double)KS / upc + 1.0) : 0.0));
     return best;

@@ -62,6 +62,8 @@ static int check(const TsParams &p, int bn, int n_cta, int sms, const int *group
     std::set<int> tickets;
     for (const auto &h : holders) {
         const TsOwners own = ts_owners(any, h.first, KS);
+        for (int c : h.second)  // (the kernels ask for the first one's slot only)
+            if (c != own.first && ts_share_slot(any, h.first, KS, c) != 0) return 17;
         if (own.first != h.second.front() || own.last != h.second.back() || own.last - own.first + 1 != (int)h.second.size()) return 14;
         if (!tickets.insert(own.first).second) return 15;
     }
@@ -86,6 +88,7 @@ extern "C" int check_plan(int integer, int kind, int T, int K, const int *F, int
     TsPlan pl;
     if (integer) {
         pl = ti_plan(kind, row_tiles * p.t_tiles, p.slabs, sms);
+        if (sms == 148 && pl.n_cta > (pl.split == 8 ? 15 * 8 : pl.split == 4 ? 33 * 4 : sms)) return 16;  // all clusters at once (cudaOccupancyMaxActiveClusters)
     } else {
         pl = ts_plan(kind, T, K, F, n_jobs, sms);
         p.t_tiles = pl.t_tiles;

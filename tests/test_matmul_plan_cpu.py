@@ -47,6 +47,8 @@ def test_integer_plans(lib, kind):
     for T in (1, 3, 5, 8, 9, 16, 17, 33, 64):
         for _ in range(60):
             K, F = int(rng.integers(1, 16000)), [int(f) for f in np.exp(rng.uniform(0, np.log(30000), rng.integers(1, 5)))]
+            if rng.random() < 0.3:  # about as many tiles as clusters of four or eight find SMs
+                F = [128 * int(rng.choice([14, 15, 16, 18, 32, 33, 34, 37, 38]))]
             for sms in SMS:
                 rc = lib.check_plan(1, kind, T, K, ints(F), len(F), sms)
                 assert rc == 0, (rc, kind, T, K, F, sms)
