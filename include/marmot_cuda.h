@@ -100,7 +100,8 @@ int mcu_context_set_regime(mcu_context_t *ctx, int regime);
  *      points that wait for the device (mcu_linear_host, mcu_vec_dot_host, mcu_moe_experts, mcu_synchronize) refuse
  *      to be captured.  The recorded pointers are the ones passed during capture: update inputs in place.  A graph keeps the
  *      context's workspace that it was recorded with: a later, larger call gets new memory, and the old one is given back behind
- *      mcu_graph_destroy, or, where the caller captured the stream by other means, with the context. ---- */
+ *      mcu_graph_destroy, or, where the caller captured the stream by other means, with the context.  A matmul of two to four
+ *      tokens may be another kernel when it is recorded than when it is called: the order of its 32-bit sums then differs. ---- */
 typedef struct mcu_graph mcu_graph_t;
 int mcu_graph_capture_begin(mcu_context_t *ctx);
 int mcu_graph_capture_end(mcu_context_t *ctx, mcu_graph_t **out_graph); /* out_graph NULL: discard the capture */

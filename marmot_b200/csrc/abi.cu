@@ -654,14 +654,19 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
 // From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
 // And from three tokens on where the rows cannot be streamed (Q6_K of ragged sizes), against the plain-load kernel: 3072 x 125 3, 4,
 // 8 tokens 13.5, 16.6, 21.2 us, 7.5, 7.7, 7.8 here; 1280 x 300 7.5, 9.1, 12.5, then 7.6 to 7.7.
-// Single calls of two to four tokens that are not being recorded have lines of their own, as their dp4a launch does without the staging launch but depends on the shape
-// more: it suffers from short rows and from long ones (twenty-four shapes at 2, 3 and 4 tokens; times in us on the device, dp4a then here).
-// Called one by one, two launches cost the host 7 us where one costs 4, so that what gains less than about 10 % stays there.
+// Calls of two to four tokens that are not being recorded have lines of their own, as their dp4a launch does without the staging launch but
+// depends on the shape more: it suffers from short rows and from long ones.  Drawn from twenty-four shapes at 2, 3 and 4 tokens (times in us on
+// the device, dp4a then here); called one by one, two launches cost the host 7 us where one costs 4, so that what gains less than about
+// 10 % stays there.
 //   Q4_K  2 tokens  1024 x 12288 8.6, 6.4; 2048 x 32000 17.9, 14.6; 14336 x 4096 21.2, 16.1; 4096 x 14336 13.3, 13.1; x 28672 20.5, 23.0
 //         3 tokens  1024 x 4096 5.7, 7.4; x 8192 9.1, 7.6; 4096 x 4096 9.0, 9.3; x 6144 11.1, 10.6; 14336 x 1024 13.4, 11.9
 //         4 tokens  1024 x 4096 6.7, 7.4; x 6144 8.9, 7.4; 2048 x 4096 7.3, 7.9; 1536 x 6144 9.3, 7.9; 4096 x 2048 8.1, 8.4
 //   Q6_K  3 tokens  1024 x 12288 12.9, 8.8; 2048 x 32000 31.2, 25.1; 4096 x 14336 22.2, 22.5; 14336 x 4096 26.3, 24.2
 //         4 tokens  1024 x 6144 8.9, 8.6; 2048 x 8192 12.6, 11.6; 4096 x 6144 14.5, 15.4; x 8192 17.4, 16.6; 8192 x 2048 13.5, 14.6
+// Checked on 170 other sizes inside the lines, 768 to 16384 values a row, one matrix and two at once, called one by one: Q4_K 0.24 to 0.97 of the
+// dp4a kernel's time; Q6_K 0.24 to 1.03 but for four, which drew the last two lines closer: rows off 16 bytes (3 x 8448 x 11072 33.0, 36.2;
+// x 18752 two at once 80.1, 75.3; 4 x 3584 x 5376 two at once 20.1, 21.6; 4 x 5888 x 6656 21.8, 19.5) and, at 4096 values a row, more tiles than
+// clusters of two have room for (4 x 4096 x 9280 18.3, 16.0; x 10176 19.8, 20.6; x 14528 25.2, 19.3).
 static bool few_tokens_pay(int kind, size_t T, size_t K, size_t values) {
     const size_t rows = values / K, M = (size_t)1 << 20;
     if (kind == KIND_Q4_K) {
@@ -671,8 +676,8 @@ static bool few_tokens_pay(int kind, size_t T, size_t K, size_t values) {
     }
     if (T == 4)
         return (K <= 1024 && values >= 8 * M) || (K <= 3072 && values >= 16 * M) || (K > 8192 && values >= 14 * M) ||
-            (values >= 32 * M && values <= 96 * M);
-    return T == 3 && ((K <= 2048 && rows >= 12288 && values >= 12 * M) || (K > 8192 && values >= 48 * M));
+            (values >= 32 * M && values <= 96 * M && (K > 4096 || (K % 2048 == 0 && (rows <= 74 * (size_t)TS_ROWS || values >= 52 * M))));
+    return T == 3 && ((K <= 2048 && rows >= 12288 && values >= 12 * M) || (K > 8192 && values >= (K < 10240 ? 128 : 48) * M));
 }
 static bool integer_allowed(const mcu_context *ctx) {
     static const bool off = getenv("MARMOT_CUDA_NO_I8MMA") != nullptr;  // diagnostic switch

@@ -53,11 +53,18 @@ def test_rows_that_cannot_be_streamed(ctx, oracle, T, K, F):
     assert max_rel_err(got, oracle.linear(KIND_Q6_K, x, W, F)) <= TOL_FP32
 
 
-@pytest.mark.parametrize("kind,T,K,F", [(KIND_Q4_K, 2, 1024, 12289), (KIND_Q4_K, 2, 16384, 3100), (KIND_Q4_K, 3, 1536, 8200), (KIND_Q4_K, 3, 14336, 1030),
-                                        (KIND_Q4_K, 4, 768, 8200), (KIND_Q6_K, 3, 2048, 12300), (KIND_Q6_K, 4, 1024, 8200), (KIND_Q6_K, 4, 14336, 1030)])
-def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
-    """Sizes just beyond the lines: the dp4a kernel's results but for the order of the f32 terms, and, recorded, the dp4a kernel itself, whose
-    graph holds no address of the workspace that a later, larger call moves."""
+# Sizes just beyond the lines, and just short of them
+BEYOND = [(KIND_Q4_K, 2, 1024, 12289), (KIND_Q4_K, 2, 16384, 3100), (KIND_Q4_K, 3, 1536, 8200), (KIND_Q4_K, 3, 14336, 1030), (KIND_Q4_K, 4, 768, 8200),
+          (KIND_Q6_K, 3, 2048, 12300), (KIND_Q6_K, 3, 10240, 4928), (KIND_Q6_K, 4, 1024, 8200), (KIND_Q6_K, 4, 14336, 1030), (KIND_Q6_K, 4, 4096, 8200)]
+SHORT = [(KIND_Q4_K, 2, 1024, 12280), (KIND_Q4_K, 2, 16384, 3070), (KIND_Q4_K, 3, 1536, 8184), (KIND_Q4_K, 3, 14336, 1020), (KIND_Q4_K, 4, 768, 8184),
+         (KIND_Q6_K, 3, 2048, 12280), (KIND_Q6_K, 3, 10240, 4912), (KIND_Q6_K, 3, 8448, 8000), (KIND_Q6_K, 4, 1024, 8184), (KIND_Q6_K, 4, 14336, 1020),
+         (KIND_Q6_K, 4, 4096, 8184), (KIND_Q6_K, 4, 4096, 9600), (KIND_Q6_K, 4, 3584, 10752)]
+
+
+@pytest.mark.parametrize("kind,T,K,F,beyond", [(*s, True) for s in BEYOND] + [(*s, False) for s in SHORT])
+def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F, beyond):
+    """Beyond the lines a call is two launches, short of them one, and one where it is being recorded: the dp4a kernel, whose graph holds no address
+    of the workspace that a later, larger call moves.  The results are the dp4a kernel's but for the order of the f32 terms."""
     import torch
     from marmot_b200 import Context
     from marmot_b200.runtime import REGIME_AUTO, REGIME_GEMV
@@ -66,13 +73,18 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
     W = random_blocks(kind, F, K, rng)
     x = rng.normal(0, 1, (T, K)).astype(np.float32)
     xd, wd = torch.from_numpy(x).cuda(), ctx.upload(W)
+    before = ctx.launch_count()
     got = ctx.linear(kind, xd, wd, F).cpu().numpy()
+    assert ctx.launch_count() - before == (2 if beyond else 1)
     ctx.set_regime(REGIME_GEMV)
     ref = ctx.linear(kind, xd, wd, F).cpu().numpy()
     ctx.set_regime(REGIME_AUTO)
     ctx.synchronize()
-    assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= TOL_FP32
     assert max_rel_err(got, ref) <= 1e-5
+    if not beyond:
+        assert np.array_equal(got, ref)
+        return
+    assert max_rel_err(got, oracle.linear(kind, x, W, F)) <= TOL_FP32
     fresh = Context(0, use_torch_stream=False)
     stream = torch.cuda.Stream()
     fresh.set_stream(stream.cuda_stream)
@@ -82,7 +94,9 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
     fresh.linear(kind, xd, wd, F, out=out)
     fresh.synchronize()
     fresh.graph_capture_begin()
+    before = fresh.launch_count()
     fresh.linear(kind, xd, wd, F, out=out)
+    assert fresh.launch_count() - before == 1
     graph = fresh.graph_capture_end()
     fresh.linear(kind, more, wd, F)
     out.zero_()
@@ -90,6 +104,7 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F):
     graph.launch()
     fresh.synchronize()
     assert np.array_equal(out.cpu().numpy(), ref)
+    graph.close()
     fresh.close()
 
 
