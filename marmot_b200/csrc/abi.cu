@@ -114,6 +114,7 @@ struct mcu_context {
     std::vector<Buffer> retired;                         // allocations that graphs still hold, replaced by larger ones
     bool recording = false;                              // between mcu_graph_capture_begin and mcu_graph_capture_end
     std::vector<std::shared_ptr<GraphHold>> holds;       // of the recording at hand
+    bool test_full = false;                              // mcu_test_device_full
 };
 
 static bool stream_is_capturing(cudaStream_t s) {
@@ -155,6 +156,7 @@ static int ensure(mcu_context *ctx, Buffer &b, size_t bytes, bool recording) {
     if (recording)
         return fail(MCU_ERROR_INVALID_OPERATION,
                     "workspace would have to grow during stream capture: run the same call once before capturing");
+    if (ctx->test_full) return fail(MCU_ERROR_OUT_OF_MEMORY, "no device memory (test)");
     // Kernels already enqueued may still read the old allocation.
     MCU_CUDA(cudaStreamSynchronize(ctx->stream));
     for (size_t i = 0; i < ctx->retired.size();) {
@@ -352,6 +354,14 @@ int mcu_test_matmul_gave_up(mcu_context_t *ctx) {
     MCU_CUDA(cudaMemcpyAsync(ctx->gemm_counters, ones.data(), ones.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     MCU_CUDA(cudaMemcpyAsync(ctx->dev_err, &code, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     MCU_CUDA(cudaStreamSynchronize(ctx->stream));
+    return MCU_SUCCESS;
+}
+
+// Test hook (not in the header): workspace cannot grow, as on a device without free memory.
+int mcu_test_device_full(mcu_context_t *ctx, int full) {
+    if (int rc = check_ctx(ctx)) return rc;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    ctx->test_full = full != 0;
     return MCU_SUCCESS;
 }
 
@@ -721,11 +731,13 @@ static bool integer_jobs_supported(const GemvJobSpec *jobs, int n_jobs, size_t K
         if (!gemm_ti_supported(jobs[j].kind, jobs[j].W, (int)K, jobs[j].F) || act_half_fused_smem(jobs[j].kind, (int)K) > ACT_INT_MAX_SMEM) return false;
     return true;
 }
+static int integer_workspace(mcu_context *ctx, int kind, size_t T, size_t K, bool rec) {
+    if (int rc = ensure(ctx, ctx->act_qs, gemm_ti_xq_bytes(kind, (int)T, (int)K), rec)) return rc;
+    return ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes(), rec);
+}
 static int integer_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, size_t T, size_t K, const GemvJobSpec *jobs, int n_jobs,
                           const ActSource *src, int *staged_kind) {
-    const bool rec = stream_is_capturing(ctx->stream);
-    if (int rc = ensure(ctx, ctx->act_qs, gemm_ti_xq_bytes(kind, (int)T, (int)K), rec)) return rc;
-    if (int rc = ensure(ctx, ctx->gemm_partial, gemm_ts_workspace_bytes(), rec)) return rc;
+    if (int rc = integer_workspace(ctx, kind, T, K, stream_is_capturing(ctx->stream))) return rc;
     uint8_t *xq = (uint8_t *)ctx->act_qs.ptr;
     if (staged_kind == nullptr || *staged_kind != kind) {
         MCU_CUDA(launch_act_int_fused(kind, x, (int)ldx, src != nullptr ? *src : ActSource{}, (int)T, (int)K, xq, ctx->stream));
@@ -751,8 +763,12 @@ static int linear_locked(mcu_context *ctx, int kind, const float *x, size_t ldx,
     bool integer = ctx->regime == MCU_REGIME_I8MMA ? (T >= 2 && T <= 64) : integer_pays(ctx, kind, T, K, values, streams);
     // (Only where the dp4a kernel streams the rows, so that it has no workspace, and not while a call is being recorded: such a call could
     // always be recorded without one made before it.)
-    if (!integer && T <= 4 && integer_allowed(ctx) && kind != MCU_KIND_Q8_0 && few_tokens_pay(kind, T, K, values))
-        integer = (T > 2 ? streams : gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F)) && !stream_is_capturing(ctx->stream);
+    // Where its workspace cannot be had the dp4a kernel, which needs none, has the call as well.
+    if (!integer && T <= 4 && integer_allowed(ctx) && kind != MCU_KIND_Q8_0 && few_tokens_pay(kind, T, K, values) &&
+        (T > 2 ? streams : gemv_stream_supported(kind, w, w2, (int)T, (int)K, (int)F)) && !stream_is_capturing(ctx->stream)) {
+        integer = integer_workspace(ctx, kind, T, K, false) == MCU_SUCCESS;
+        if (!integer) (void)cudaGetLastError();
+    }
     if (integer && (w2 == nullptr || bias == nullptr)) {
         if (i8_takes(ctx, kind, w, w2, T, K, F)) return i8_locked(ctx, kind, x, ldx, w, w2, T, K, F, bias, out, out2, ldo);
         const GemvJobSpec jobs[2] = {{kind, w, (int)F, bias, out, (int)ldo}, {kind, w2, (int)F, bias, out2, (int)ldo}};

@@ -108,6 +108,30 @@ def test_lines_of_two_to_four_tokens(ctx, oracle, kind, T, K, F, beyond):
     fresh.close()
 
 
+def test_few_tokens_without_memory_for_workspace():
+    """A call that the dp4a kernel can have does not fail for want of the integer matmul's workspace; a larger one does, and works again later."""
+    import torch
+    from marmot_b200 import Context, MarmotCudaError
+    from marmot_b200.runtime import REGIME_AUTO, REGIME_GEMV
+
+    T, K, F = 4, 768, 16384
+    rng = np.random.default_rng(4)
+    ctx = Context(0)
+    x, w = torch.from_numpy(rng.normal(0, 1, (16, K)).astype(np.float32)).cuda(), ctx.upload(random_blocks(KIND_Q4_K, F, K, rng))
+    ctx.set_regime(REGIME_GEMV)
+    ref = ctx.linear(KIND_Q4_K, x[:T], w, F).cpu().numpy()
+    ctx.set_regime(REGIME_AUTO)
+    ctx._check(ctx.lib.mcu_test_device_full(ctx.handle, 1))
+    assert np.array_equal(ctx.linear(KIND_Q4_K, x[:T], w, F).cpu().numpy(), ref)
+    with pytest.raises(MarmotCudaError, match="no device memory"):
+        ctx.linear(KIND_Q4_K, x, w, F)
+    ctx._check(ctx.lib.mcu_test_device_full(ctx.handle, 0))
+    before = ctx.launch_count()
+    assert max_rel_err(ctx.linear(KIND_Q4_K, x[:T], w, F).cpu().numpy(), ref) <= 1e-5
+    assert ctx.launch_count() - before == 2
+    ctx.close()
+
+
 def test_two_tokens_on_rows_too_long_to_stream():
     """The call and its recording are the same kernels: the one finds the workspace that the other has reserved."""
     import torch
