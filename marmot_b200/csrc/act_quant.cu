@@ -469,8 +469,9 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
     int warps = 8;
     if (T < 512) {
         const int want = kind != KIND_Q8_0 ? nb : nb / 4;  // a 256-value block, or four 32-value ones in turn, per warp
-        // K-quants, more rows than SMs: registers allow 1024 threads on an SM, so two rows at a time on each, and beyond 296 rows as many as
-        // it takes for one wave (whole calls, 32 warps and so: 180 x 14336 x 4096 Q6_K 35.5, 34.8 us, 300 50.9, 48.1, 400 Q4_K 55.0, 52.4; 500 x 4096 x 4096
+        // K-quants, more rows than SMs: registers allow 1024 threads on an SM, so two rows at a time on each, and beyond 296 rows 32 * SMs / T
+        // warps a row: two rows at a time up to 430, three from there on, which is one wave from 431 to 444 rows and two elsewhere, the second one
+        // short (whole calls, 32 warps and so: 180 x 14336 x 4096 Q6_K 35.5, 34.8 us, 300 50.9, 48.1, 400 Q4_K 55.0, 52.4; 500 x 4096 x 4096
         // 27.0, 26.4.  Rows of Q8_0 keep theirs: 300 x 4096 x 14336 46.9, 48.5).
         const int sms = device_sm_count(), most = kind == KIND_Q8_0 || T <= sms ? 32 : T <= 2 * sms ? 16 : 32 * sms / T;
         warps = want > most ? most : want;

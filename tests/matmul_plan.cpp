@@ -31,7 +31,7 @@ static int check(const TsParams &p, int bn, int n_cta, int sms, const int *group
     const long long U = (long long)tiles * KS;
     if (p.split > 1) {
         if (n_cta != tiles * p.split || n_cta > sms || p.split > KS) return 7;
-    } else if (n_cta > sms && n_cta != tiles) {
+    } else if (n_cta > sms) {
         return 8;
     }
     long long at = 0;
@@ -50,7 +50,7 @@ static int check(const TsParams &p, int bn, int n_cta, int sms, const int *group
         for (int u = w.u0; u < w.u1;) {
             const int tile = u / KS, e = ts_min((tile + 1) * KS, w.u1);
             if (e - u != KS) {
-                if (n_cta > sms) return 11;  // shares have a place for one CTA per SM
+                if (p.whole) return 11;
                 holders[tile].push_back(c);
                 const int slot = ts_share_slot(any, tile, KS, c);
                 if (slot != (u == w.u0 ? 0 : 1) || !slots.insert({c, slot}).second) return 12;
@@ -94,6 +94,7 @@ extern "C" int check_plan(int integer, int kind, int T, int K, const int *F, int
         p.t_tiles = pl.t_tiles;
     }
     p.split = pl.split;
+    p.whole = pl.whole;
     p.tiles = row_tiles * p.t_tiles;
     return check(p, pl.bn, pl.n_cta, sms, nullptr, want);
 }
