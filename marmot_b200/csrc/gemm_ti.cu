@@ -192,6 +192,18 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     int err_code = 0;
     if (warp == TI_B_WARP) {
         // ------------------------------ activation tiles ------------------------------
+        // Who shares the cut tiles at this range's ends, for the scalers (which see it behind the barrier of the first tile).  Divisions in
+        // 64 bits: here they pass while the kernel ahead is waited for.  Between a share and its ticket, and again for every share that was
+        // read, they were 1 us of a launch with short ranges: MoE of 4 tokens on 8 experts of 512 x 1024 25.3 -> 23.2 us, 16 tokens on 4 of
+        // 3584 x 1024 39.6 -> 36.5.  (In the scalers' own warps, whose loops they cost registers, FFN input of 8 95.4 -> 97.7.)
+        if (lane < 2 && split == 1 && !p.whole && n_slabs > 0) {
+            const int cut = (lane == 0 ? u0 : u1 - 1) / KS;
+            const TsOwners own = ts_owners(work, cut, KS);
+            cut_first[lane] = own.first;
+            cut_last[lane] = own.last;
+            cut_slot[lane] = ts_share_slot(work, cut, KS, own.first);
+        }
+        __syncwarp();
         if (lane == 0 && n_slabs > 0) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
             uint32_t j = 0;
@@ -338,17 +350,6 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
             err_code = 49;
         } else {
             // ------------------------------ scalers ------------------------------
-            // (Divisions in 64 bits: here they pass while the kernel ahead is waited for.  Between a share and its ticket, and again for every
-            // share that was read, they were 1 us of a launch with short ranges: MoE of 4 tokens on 8 experts of 512 x 1024 25.3 -> 23.2 us,
-            // 16 tokens on 4 of 3584 x 1024 39.6 -> 36.5.)
-            if (warp == TI_CONV && lane < 2 && split == 1 && !p.whole && n_slabs > 0) {
-                const int cut = (lane == 0 ? u0 : u1 - 1) / KS;
-                const TsOwners own = ts_owners(work, cut, KS);
-                cut_first[lane] = own.first;
-                cut_last[lane] = own.last;
-                cut_slot[lane] = ts_share_slot(work, cut, KS, own.first);
-            }
-            __syncwarp();
             asm volatile("griddepcontrol.wait;" ::: "memory");
             float acc[2][8];
             uint32_t segs = 0;
