@@ -655,24 +655,24 @@ static int gemm_locked(mcu_context *ctx, int kind, const float *x, size_t ldx, s
 // The integer tensor-core matmul for few tokens (Q4_K, Q6_K): the same two steps.
 // Its time hardly depends on the token count, the dp4a kernel's (one launch, no staging) grows with it, so up to eight tokens
 // the line is one of tokens x values; times in us at K x F, dp4a then tensor cores:
-//   Q4_K  3 tokens  4096 x 4096 8.5, 9.0; x 14336 18.8, 13.6     4 tokens  2048 x 2048 4.9, 7.3; 4096 x 4096 10.3, 9.0
-//         5 tokens  1024 x 1024 4.7, 6.8; 2048 x 2048 7.3, 7.3; 4096 x 1024 8.2, 7.4; 4096 x 4096 11.9, 9.0
-//   Q6_K  4 tokens  4096 x 4096 11.5, 12.1; 14336 x 4096 34.8, 24.2; 4096 x 28672 41.5, 44.5
-//         5 tokens  1024 x 1024 4.2, 7.0; 2048 x 2048 7.9, 8.0; 4096 x 1024 8.8, 8.6; 4096 x 4096 13.5, 11.7
+//   Q4_K  3 tokens  4096 x 4096 8.7, 8.9; x 14336 19.6, 13.0     4 tokens  2048 x 2048 5.0, 7.1; 4096 x 4096 10.4, 9.0
+//         5 tokens  1024 x 1024 4.4, 6.5; 2048 x 2048 6.9, 7.1; 4096 x 1024 9.2, 7.4; 4096 x 4096 12.7, 9.0
+//   Q6_K  4 tokens  4096 x 4096 11.4, 10.9; 14336 x 4096 34.4, 21.4; 4096 x 28672 41.3, 37.2
+//         5 tokens  1024 x 1024 4.3, 6.7; 2048 x 2048 6.9, 7.4; 4096 x 1024 9.4, 7.8; 4096 x 4096 13.5, 10.9
 // Small matrices of long rows are a chain for the dp4a kernel's warps, short rows leave little to chain: a line of tokens x K, or of
-// tokens x rows, for those (8 tokens: 3072 x 125 Q4_K 9.5, 7.0; 2048 x 256 7.8, 6.9; 1024 x 1024 5.6, 4.9 with gemm_i8; 1024 x 512 5.0, 4.8).
-// From nine to sixteen tokens it always pays (1024 x 1024 8.5, 7.4); beyond, the fp16 kernel does.
+// tokens x rows, for those (8 tokens: 3072 x 125 Q4_K 9.6, 7.1; 2048 x 256 7.7, 6.8; 1024 x 1024 5.6, 4.8 with gemm_i8; 1024 x 512 5.0, 4.8).
+// From nine to sixteen tokens it always pays (1024 x 1024 8.5, 5.5); beyond, the fp16 kernel does.
 // And from three tokens on where the rows cannot be streamed (Q6_K of ragged sizes), against the plain-load kernel: 3072 x 125 3, 4,
-// 8 tokens 13.5, 16.6, 21.2 us, 7.5, 7.7, 7.8 here; 1280 x 300 7.5, 9.1, 12.5, then 7.6 to 7.7.
+// 8 tokens 12.0, 14.3, 20.1 us, 7.7 to 7.9 here; 1280 x 300 7.9, 8.9, 11.5, then 7.6.
 // Calls of two to four tokens that are not being recorded have lines of their own, as their dp4a launch does without the staging launch but
 // depends on the shape more: it suffers from short rows and from long ones.  Drawn from twenty-four shapes at 2, 3 and 4 tokens (times in us on
 // the device, dp4a then here); called one by one, two launches cost the host 7 us where one costs 4, so that what gains less than about
 // 10 % stays there.
-//   Q4_K  2 tokens  1024 x 12288 8.6, 6.4; 2048 x 32000 17.9, 14.6; 14336 x 4096 21.2, 16.1; 4096 x 14336 13.3, 13.1; x 28672 20.5, 23.0
-//         3 tokens  1024 x 4096 5.7, 7.4; x 8192 9.1, 7.6; 4096 x 4096 9.0, 9.3; x 6144 11.1, 10.6; 14336 x 1024 13.4, 11.9
-//         4 tokens  1024 x 4096 6.7, 7.4; x 6144 8.9, 7.4; 2048 x 4096 7.3, 7.9; 1536 x 6144 9.3, 7.9; 4096 x 2048 8.1, 8.4
-//   Q6_K  3 tokens  1024 x 12288 12.9, 8.8; 2048 x 32000 31.2, 25.1; 4096 x 14336 22.2, 22.5; 14336 x 4096 26.3, 24.2
-//         4 tokens  1024 x 6144 8.9, 8.6; 2048 x 8192 12.6, 11.6; 4096 x 6144 14.5, 15.4; x 8192 17.4, 16.6; 8192 x 2048 13.5, 14.6
+//   Q4_K  2 tokens  1024 x 12288 8.5, 6.3; 2048 x 32000 17.6, 14.2; 14336 x 4096 21.2, 16.4; 4096 x 14336 13.1, 13.0; x 28672 20.1, 22.5
+//         3 tokens  1024 x 4096 5.7, 7.1; x 8192 9.1, 7.2; 4096 x 4096 8.7, 8.9; x 6144 11.1, 10.3; 14336 x 1024 13.2, 11.8
+//         4 tokens  1024 x 4096 6.6, 7.1; x 6144 8.8, 7.2; 2048 x 4096 7.2, 7.6; 1536 x 6144 9.2, 7.7; 4096 x 2048 8.1, 8.3
+//   Q6_K  3 tokens  1024 x 12288 12.8, 8.2; 2048 x 32000 31.1, 22.2; 4096 x 14336 21.8, 19.3; 14336 x 4096 26.4, 21.4
+//         4 tokens  1024 x 6144 8.8, 7.9; 2048 x 8192 12.4, 10.5; 4096 x 6144 14.4, 13.4; x 8192 17.3, 14.5; 8192 x 2048 13.3, 13.2
 // Checked on 170 other sizes inside the lines, 768 to 16384 values a row, one matrix and two at once, called one by one: Q4_K 0.24 to 0.97 of the
 // dp4a kernel's time; Q6_K 0.24 to 1.03 but for four, which drew the last two lines closer: rows off 16 bytes (3 x 8448 x 11072 33.0, 36.2;
 // x 18752 two at once 80.1, 75.3; 4 x 3584 x 5376 two at once 20.1, 21.6; 4 x 5888 x 6656 21.8, 19.5) and, at 4096 values a row, more tiles than
@@ -1255,14 +1255,16 @@ static int moe_experts_impl(mcu_context_t *ctx, int gate_kind, int up_kind, int 
     static const bool no_grouped = getenv("MARMOT_CUDA_MOE_NO_GROUPED") != nullptr;  // diagnostic switch
     // Few routes (a decode batch): the integer tensor-core kernel over all local experts, one launch for gate and up, one for
     // down, tiles of sixteen tokens sized from the device-resident counts; exact sub-block dots, as the per-expert launches
-    // below (16 tokens, top 2 of 8 experts of 3 x 14336 x 4096: 398 us with those, which wait for the counts on the host, 223 here).
+    // below (16 tokens, top 2 of 8 experts of 3 x 14336 x 4096: 383 us with those, which wait for the counts on the host, 207 here).
     // It reads the weights again for every sixteen rows of an expert, which large experts and Q6_K notice first; those launches cost 25 us
     // an expert whatever its size, and take it for large experts only.  Rows per expert, here and there, us at 4 experts of 3 x 14336 x 4096:
-    // Q4_K 16 238, 265; 32 262 to 317, 273; 48 375, 282.  Q6_K down 16 279, 313; 32 348, 314.  Q6_K 12 278, 332; 16 402, 348; 48 756, 373.
-    // At 4 of 3 x 5632 x 2048: Q4_K 48 122, 140; 63 165, 156.  Q6_K down 48 158, 166; 60 195, 174.  Q6_K 32 153 to 174, 174; 48 206, 176.
-    // A single route leaves all other experts out (3 x 5632 x 2048 Q4_K 55, 45; 3 x 14336 x 4096 73, 66; all Q6_K 97, 75), where two cost more
-    // so (93, 102), and so do few routes of large experts in Q6_K, whose launches are the streaming kernels' (8 experts of 3 x 14336 x 4096,
-    // 3, 8, 12, 16 routes: 174, 149; 326, 302; 372, 378; 413, 444.  16 of 3 x 7168 x 4096, 3, 8, 12: 120, 110; 208, 212; 274, 292).
+    // Q4_K 16 151, 234; 24 225, 259; 32 242, 261; 48 343, 271.  Q6_K down 16 176, 291; 24 275, 277; 32 297, 280.  Q6_K 12 224, 342; 16 224, 343;
+    // 24 363, 299.  At 4 of 3 x 5632 x 2048: Q4_K 48 119, 145; 63 142, 151.  Q6_K down 32 119, 161; 48 149, 166; 63 182, 175.  Q6_K 32 141, 169;
+    // 48 187, 173.
+    // A single route leaves all other experts out (3 x 5632 x 2048 Q4_K 50, 46; 3 x 14336 x 4096 71, 67; all Q6_K 89, 78), where two cost more
+    // so (91, 106), and few routes of large experts in Q6_K, whose launches are the streaming kernels', cost about as much (8 experts of
+    // 3 x 14336 x 4096, 3, 8, 12 routes: 156, 166; 314, 384; 314, 419.  16 of 3 x 7168 x 4096: 115, 116; 205, 249; 277, 358).
+    // (The lines were drawn by an earlier form of the kernel, which was up to a quarter slower with Q6_K and in short ranges, and not drawn again.)
     const size_t n6 = (gate_kind == KIND_Q6_K ? 1 : 0) + (down_kind == KIND_Q6_K ? 1 : 0);
     const bool large = H * FF > (size_t)26 << 20;
     const size_t most_rows = (large ? 48 : 128) / (2 + n6);

@@ -141,10 +141,10 @@ struct TsPlan {
 //   Q8_0 34.5 -> 27.5, 512 x 4096 x 14336 Q8_0 80.1 -> 77.9.)
 // - A tile over a cluster: the exchange of the shares through the CTAs' shared memories.
 // - Equal ranges of slabs: cut tiles have their shares written to memory, and read again by the CTA that comes last; a tile of 256
-//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 80 us in ranges, 69 in two waves).  The way
+//   columns costs 47000 so, which only many tiles per CTA are worth (512 x 4096 x 14336 Q8_0: 77 us in ranges, 65.5 in whole tiles).  The way
 //   through memory and the tickets costs 6000 besides, 11000 in narrow tiles, by all forms at 9 to 2048 tokens and thirteen sizes
-//   (9 x 2048 x 5632 Q8_0: 19.1 us in ranges, 10.2 in clusters of two; 17 x 2048 x 32000 Q4_K: 25.1, 20.7 in waves; 2048 x 14336 x 4096
-//   Q4_K: 261, 226 in waves; 512 x 4096 x 28672 Q4_K: 119 in ranges, 137 in waves).
+//   (9 x 2048 x 5632 Q8_0: 17.5 us in ranges, 9.8 in clusters of two; 17 x 2048 x 32000 Q4_K: 24.7, 17.7 in whole tiles; 2048 x 14336 x 4096
+//   Q4_K: 266, 231 in whole tiles; 512 x 4096 x 28672 Q4_K: 115.7, 112 in whole tiles).
 inline TsPlan ts_spread(int kind, int tiles, int KS, int bn, int t_tiles, int room) {
     const long U = (long)tiles * KS;
     const bool wide = bn > 64;
@@ -217,8 +217,10 @@ inline TsPlan ti_plan(int kind, int tiles, int KS, int sms) {
 // Microseconds of a call of 5 to 16 tokens on `row_tiles` tiles of 128 rows with the integer kernel, staging included, and on `groups`
 // groups of 64 rows with the mma.sync one: fitted to both at 5, 8, 9, 12 and 16 tokens, K 1024 to 14336 and 512 to 32000 rows (within
 // 10 % of all but a few).  A stage of the latter takes 2.35 or 2.45 us and its first ones are 8 to 10; the former's cycles are those
-// of its plan, which clusters on less than half of the SMs beat, and single waves, with SMs to spare.  (Q6_K, 8 tokens: 4096 x 1024 8.5 us
-// on 64 SMs here, 9.0 with the other; 2048 x 4096 9.8 on 128, 8.3; 14336 x 4096 23.7, 25.0, and with 16 tokens 28.8, 27.5.)
+// of its plan, which clusters on less than half of the SMs beat, and single waves, with SMs to spare.
+// Both are fits to the kernels as they were then, and the integer one has become the faster for more of Q6_K since (8 tokens, integer and mma.sync:
+// 4096 x 1024 7.9, 9.2 us; 2048 x 4096 8.4, 8.4; 4096 x 28672 37.2, 41.3; 14336 x 4096 21.4, 26.7, with 16 tokens 25.5, 28.7).  Over 290 calls
+// of Q6_K and of short Q4_K rows the choice is 4.4 % slower than the better of the two, at most 33 % (8 x 4096 x 5248 17.6, 13.3).
 inline double ti_us(int kind, int T, int K, int row_tiles, int sms) {
     const TsPlan pl = ti_plan(kind, row_tiles, (K + QK_K - 1) / QK_K, sms);
     if (kind == KIND_Q6_K && pl.split > 1 && 2 * pl.n_cta <= sms) return (T <= 8 ? 2.5 : 1.35) + (T <= 8 ? 0.6 : 0.8) * 1e-3 * pl.cost;

@@ -16,8 +16,8 @@
 //
 // Work is divided as in gemm_ts.cu: whole tiles, a tile over a cluster, or equal ranges of slabs.
 //
-// Measured, staging included, against the kernels that had these calls (mma.sync, dp4a): Q4_K 8 x 4096 x 14336 19.9 -> 12.7 us
-// (2.6 TB/s), 8 x 4096 x 28672 22.5 (2.9 TB/s), 16 x 4096 x 14336 22.4 -> 14.2; Q6_K 8 x 4096 x 14336 25.2 -> 21.3.  The mma.sync kernel keeps the
+// Measured, staging included, against the kernels that had these calls (mma.sync, dp4a): Q4_K 8 x 4096 x 14336 19.9 -> 13.0 us
+// (2.5 TB/s), 8 x 4096 x 28672 22.3 (3.0 TB/s), 16 x 4096 x 14336 22.4 -> 14.5; Q6_K 8 x 4096 x 14336 25.2 -> 18.5.  The mma.sync kernel keeps the
 // calls of up to 16 tokens for which it is the faster one (gemm_i8.cu; i8_pays in gemm_plan.h).  A slab costs the Q4_K scalers and
 // converters 500 to 700 cycles by their own stamps (740 by the time of a CTA with sixteen), the Q6_K ones (eighteen products of 32 columns, 4 KB of sums per row) 900 to 1800; a
 // CTA's time grows by 900 and 2100 with each (ti_plan).  Those bound Q6_K, the kernel's prologue, staging launch and first loads (about
@@ -384,7 +384,7 @@ gemm_ti_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
                     if (lane == 0) tm_mbar_arrive(raw_empty + 8u * rs);
                     // The tokens' block scales come with the activation tile: byte 320 of 384, in the last box (128-byte swizzle).  Read from
                     // memory here they were a trip to L2 in every slab, and what bounded the scalers: 16 x 4096 x 14336 Q4_K 19.5 -> 15.0 us,
-                    // 8 x 4096 x 28672 30.7 -> 27.1, Q6_K 8 x 4096 x 14336 27.4 -> 23.7, MoE of 16 tokens 246 -> 199.
+                    // 8 x 4096 x 28672 30.7 -> 27.1, Q6_K 8 x 4096 x 14336 27.4 -> 23.7, MoE of 16 tokens 238 -> 218.
                     const uint32_t slot = (uint32_t)j & (TI_B_SLOTS - 1);
                     const uint8_t *dx = smem_raw + (tile_base + slot * B_BYTES + (Q4 ? 4096u : 8192u) - raw_addr);
                     if (ok) ok = ts_wait(b_full + 8u * slot, ((uint32_t)j >> 2) & 1u);

@@ -16,13 +16,13 @@
 //                 multiples (Q6_K with K % 2048 != 0) come as eight copies of every eighth row: eight rows always are.
 //
 // Measured (whole mcu_linear call, graph replay, microseconds before -> now): Q4_K 64 x 4096 x 14336 31.0 -> 17.3,
-// 17 x 4096 x 4096 13.2 -> 10.5, 64 x 4096 x 1024 17.2 -> 9.6, 2048 x 4096 x 14336 274 -> 213 (1130 TFLOP/s: 0.82 of the
-// sustained cuBLAS rate, the clock is at the power limit); Q6_K 37 x 14336 x 4096 40.0 -> 24.8, 512 x 5632 x 2048 142 -> 29.2.
+// 17 x 4096 x 4096 13.2 -> 10.1, 64 x 4096 x 1024 17.2 -> 9.5, 2048 x 4096 x 14336 274 -> 213 (1127 TFLOP/s: 0.83 of the
+// sustained cuBLAS rate, the clock is at the power limit); Q6_K 37 x 14336 x 4096 40.0 -> 25.4, 512 x 5632 x 2048 142 -> 29.0.
 // Up to 128 tokens the converters bound a slab (Q4_K about 1100 cycles for 32768 weights in tiles of up to 64 tokens, 1500 in wider ones;
 // instruction issue); from 256 on the MMAs run at their peak rate (2050 cycles per slab) and what is left is the epilogue (7500 cycles
 // beside a tile's 33000 of MMAs, about half of them ahead of the next tile's).  Beside the kernel a call has its staging launch: of the 17 us at 64 x 4096 x 14336 it and the releases around it take 6.5.
 //
-// A CTA has one output tile, or a cluster shares one along K and adds its shares up through distributed shared memory, or the slabs of
+// A CTA has one or several output tiles, or a cluster shares one along K and adds its shares up through distributed shared memory, or the slabs of
 // all tiles are cut into equal ranges: a tile cut between CTAs is then summed from partial tiles by the one that draws the last
 // ticket, in a fixed order; nobody waits for another CTA (kernels on several streams may share the device).  ts_spread chooses.
 // Every mbarrier wait is bounded; no TMA multicast.
@@ -295,8 +295,8 @@ gemm_ts_kernel(const __grid_constant__ TsMaps maps, const __grid_constant__ TsPa
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // (In shared memory, and the converted columns in quarters, for the registers: what a thread spills misses the few KB of L1 that
-    // are left.  48 to 56 bytes a thread before, 24 to 56 so: Q6_K 37 x 14336 x 4096 27.4 -> 25.7 us, Q4_K 64 x 4096 x 14336 18.3 -> 17.8; with
-    // 120 or 200 bytes the large sizes were 10 and 25 % slower.)
+    // are left.  Spilled stores and loads in bytes, before and so: Q4_K 96 + 184, 36 + 56 (64 x 4096 x 14336 18.3 -> 17.8 us); Q6_K 100 + 188,
+    // 36 + 60 (37 x 14336 x 4096 27.4 -> 25.7); Q8_0 104 + 232, 88 + 120.  With twice the former the large sizes were 10 to 25 % slower.)
     __shared__ TsWork work_s;
     if (threadIdx.x == 0) work_s = ts_work(p, grouped, group_tile0, bn, cta, n_cta);
     __syncthreads();
