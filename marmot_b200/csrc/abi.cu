@@ -52,10 +52,12 @@ static int cuda_fail(cudaError_t e, const char *what) {
     } while (0)
 
 // SM count of the calling thread's current device (every launcher runs with its context's device current).
-int device_sm_count() {
+int device_sm_count(int *device) {
     static std::atomic<int> cache[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    if (device != nullptr) *device = dev;
+    if (dev < 0 || dev >= 64) return 148;
     int v = cache[dev].load(std::memory_order_relaxed);
     if (v > 0) return v;
     if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;

@@ -473,9 +473,11 @@ cudaError_t launch_act_half_fused_from(int kind, const float *x, int ldx, const 
         // warps a row: two rows at a time up to 430, three from there on, which is one wave from 431 to 444 rows and two elsewhere, the second one
         // short (whole calls, 32 warps and so: 180 x 14336 x 4096 Q6_K 35.5, 34.8 us, 300 50.9, 48.1, 400 Q4_K 55.0, 52.4; 500 x 4096 x 4096
         // 27.0, 26.4.  Rows of Q8_0 keep theirs: 300 x 4096 x 14336 46.9, 48.5).
-        const int sms = device_sm_count(), most = kind == KIND_Q8_0 || T <= sms ? 32 : T <= 2 * sms ? 16 : 32 * sms / T;
-        warps = want > most ? most : want;
-        if (warps < 8) warps = 8;
+        warps = want < 8 ? 8 : want > 32 ? 32 : want;
+        if (kind != KIND_Q8_0 && T > 64 && warps > 8) {  // (else the count of SMs makes no difference)
+            const int sms = device_sm_count(), most = T <= sms ? 32 : T <= 2 * sms ? 16 : 32 * sms / T;
+            if (warps > most) warps = most < 8 ? 8 : most;
+        }
     }
     cfg.blockDim = dim3((unsigned)(32 * warps), 1, 1);
     cfg.dynamicSmemBytes = act_half_fused_smem(kind, K);

@@ -479,13 +479,12 @@ void gemm_i8_workspace_bytes(int T, int K, int F, bool dual, size_t *qs_bytes, s
 
 template <int KIND, int NT>
 static cudaError_t launch_i8(const CUtensorMap &mw0, const CUtensorMap &mw1, const CUtensorMap &mx, const GemmI8Params &p, int grid,
-                             int smem, cudaStream_t s) {
+                             int smem, int dev, cudaStream_t s) {
     static std::atomic<uint64_t> configured{0};  // devices on which the kernel may use that much shared memory
-    int dev = 0;
-    if (cudaError_t e = cudaGetDevice(&dev)) return e;
-    if (dev >= 64 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
+    const bool known = dev >= 0 && dev < 64;
+    if (!known || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
         if (cudaError_t e = cudaFuncSetAttribute(gemm_i8_kernel<KIND, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_MOST_SMEM)) return e;
-        if (dev < 64) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
+        if (known) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid, 1, 1);
@@ -502,9 +501,9 @@ static cudaError_t launch_i8(const CUtensorMap &mw0, const CUtensorMap &mw1, con
 
 template <int KIND>
 static cudaError_t launch_i8_nt(int NT, const CUtensorMap &mw0, const CUtensorMap &mw1, const CUtensorMap &mx, const GemmI8Params &p,
-                                int grid, int smem, cudaStream_t s) {
-    if (NT == 1) return launch_i8<KIND, 1>(mw0, mw1, mx, p, grid, smem, s);
-    return launch_i8<KIND, 2>(mw0, mw1, mx, p, grid, smem, s);
+                                int grid, int smem, int dev, cudaStream_t s) {
+    if (NT == 1) return launch_i8<KIND, 1>(mw0, mw1, mx, p, grid, smem, dev, s);
+    return launch_i8<KIND, 2>(mw0, mw1, mx, p, grid, smem, dev, s);
 }
 
 // Two launches: the activation packer and the matmul.
@@ -581,10 +580,11 @@ cudaError_t launch_gemm_i8(int kind, const void *W, const void *W2, const float 
     p.stages = budget / p.stage_bytes;
     if (p.stages > I8_MAX_STAGES) p.stages = I8_MAX_STAGES;
     if (p.stages < 2) return cudaErrorInvalidValue;
-    const int grid = device_sm_count() < p.SU ? device_sm_count() : p.SU;
+    int dev;
+    const int sms = device_sm_count(&dev), grid = sms < p.SU ? sms : p.SU;
     const int smem = I8_HEADER + p.stages * p.stage_bytes + red_bytes;
-    if (kind == KIND_Q4_K) return launch_i8_nt<KIND_Q4_K>(NT, mw0, mw1, mx, p, grid, smem, s);
-    return launch_i8_nt<KIND_Q6_K>(NT, mw0, mw1, mx, p, grid, smem, s);
+    if (kind == KIND_Q4_K) return launch_i8_nt<KIND_Q4_K>(NT, mw0, mw1, mx, p, grid, smem, dev, s);
+    return launch_i8_nt<KIND_Q6_K>(NT, mw0, mw1, mx, p, grid, smem, dev, s);
 }
 
 }  // namespace mcu

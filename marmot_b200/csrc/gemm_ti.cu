@@ -589,18 +589,17 @@ bool gemm_ti_supported(int kind, const void *W, int K, int F) {
 }
 
 template <int KIND, bool LOOSE>
-static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
+static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, int dev, cudaStream_t s) {
     const int fixed = 16 + 512 + 1024 + TI_B_SLOTS * (int)ti_b_bytes<KIND>() + 2 * TI_COLS * TS_ROWS * 4;
     const int slab = ts_slab_bytes<KIND>(LOOSE);
     constexpr int MOST = 224 * 1024;
     p.raw_shift = fixed + 8 * slab <= MOST ? 3 : 2;
     const int smem = fixed + (slab << p.raw_shift);
     static std::atomic<uint64_t> configured{0};
-    int dev = 0;
-    if (cudaError_t e = cudaGetDevice(&dev)) return e;
-    if (dev >= 64 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
+    const bool known = dev >= 0 && dev < 64;
+    if (!known || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
         if (cudaError_t e = cudaFuncSetAttribute(gemm_ti_kernel<KIND, LOOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
-        if (dev < 64) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
+        if (known) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_cta, 1, 1);
@@ -617,9 +616,9 @@ static cudaError_t ti_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     cfg.numAttrs = p.split > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gemm_ti_kernel<KIND, LOOSE>, maps, p);
 }
-static cudaError_t ti_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
-    if (kind == KIND_Q4_K) return ti_launch<KIND_Q4_K, false>(maps, p, n_cta, s);
-    return p.loose ? ti_launch<KIND_Q6_K, true>(maps, p, n_cta, s) : ti_launch<KIND_Q6_K, false>(maps, p, n_cta, s);
+static cudaError_t ti_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, int dev, cudaStream_t s) {
+    if (kind == KIND_Q4_K) return ti_launch<KIND_Q4_K, false>(maps, p, n_cta, dev, s);
+    return p.loose ? ti_launch<KIND_Q6_K, true>(maps, p, n_cta, dev, s) : ti_launch<KIND_Q6_K, false>(maps, p, n_cta, dev, s);
 }
 static cudaError_t ti_encode_x(int kind, CUtensorMap *m, const uint8_t *xq, int rows, int nb) {
     return ts_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, xq, (cuuint64_t)nb * 384, (cuuint64_t)rows * ti_planes(kind), (cuuint64_t)nb * 384, 128,
@@ -649,10 +648,11 @@ cudaError_t launch_gemm_ti(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     }
     p.tiles = row_tiles * p.t_tiles;
     if (cudaError_t e = ti_encode_x(kind, &maps.x, xq, T, p.nb)) return e;
-    const TsPlan pl = ti_plan(kind, p.tiles, p.slabs, device_sm_count());
+    int dev;
+    const TsPlan pl = ti_plan(kind, p.tiles, p.slabs, device_sm_count(&dev));
     p.split = pl.split;
     p.whole = pl.whole;
-    return ti_dispatch(kind, maps, p, pl.n_cta, s);
+    return ti_dispatch(kind, maps, p, pl.n_cta, dev, s);
 }
 
 cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs, int n_groups, const uint8_t *xq,
@@ -669,7 +669,9 @@ cudaError_t launch_gemm_ti_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
     p.counters = counters;
     p.err = err_flag;
     if (cudaError_t e = ti_encode_x(kind, &maps.x, xq, total_rows, p.nb)) return e;
-    return ti_dispatch(kind, maps, p, device_sm_count(), s);
+    int dev;
+    const int sms = device_sm_count(&dev);
+    return ti_dispatch(kind, maps, p, sms, dev, s);
 }
 
 }  // namespace mcu

@@ -673,7 +673,7 @@ bool ts_loose(int kind, const void *W, long row_bytes) {
 }
 
 template <int KIND, bool LOOSE>
-static cudaError_t ts_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
+static cudaError_t ts_launch(const TsMaps &maps, TsParams &p, int n_cta, int dev, cudaStream_t s) {
     const int stage_bytes = (p.bn > 64 ? 1 : 2) * p.bn * 128;
     const int fixed = 16 + 512 + 1024 + TS_STAGES * stage_bytes;
     constexpr int slab = ts_slab_bytes<KIND>(LOOSE);
@@ -681,11 +681,10 @@ static cudaError_t ts_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     p.raw_shift = fixed + 4 * slab <= MOST ? 2 : 1;
     const int smem = fixed + (slab << p.raw_shift);
     static std::atomic<uint64_t> configured{0};  // devices on which the kernel may use that much shared memory
-    int dev = 0;
-    if (cudaError_t e = cudaGetDevice(&dev)) return e;
-    if (dev >= 64 || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
+    const bool known = dev >= 0 && dev < 64;
+    if (!known || !(configured.load(std::memory_order_relaxed) >> dev & 1)) {
         if (cudaError_t e = cudaFuncSetAttribute(gemm_ts_kernel<KIND, LOOSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST)) return e;
-        if (dev < 64) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
+        if (known) configured.fetch_or((uint64_t)1 << dev, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_cta, 1, 1);
@@ -703,11 +702,11 @@ static cudaError_t ts_launch(const TsMaps &maps, TsParams &p, int n_cta, cudaStr
     return cudaLaunchKernelEx(&cfg, gemm_ts_kernel<KIND, LOOSE>, maps, p);
 }
 
-static cudaError_t ts_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, cudaStream_t s) {
+static cudaError_t ts_dispatch(int kind, const TsMaps &maps, TsParams &p, int n_cta, int dev, cudaStream_t s) {
     switch (kind) {
-    case KIND_Q4_K: return ts_launch<KIND_Q4_K, false>(maps, p, n_cta, s);
-    case KIND_Q6_K: return p.loose ? ts_launch<KIND_Q6_K, true>(maps, p, n_cta, s) : ts_launch<KIND_Q6_K, false>(maps, p, n_cta, s);
-    default: return p.loose ? ts_launch<KIND_Q8_0, true>(maps, p, n_cta, s) : ts_launch<KIND_Q8_0, false>(maps, p, n_cta, s);
+    case KIND_Q4_K: return ts_launch<KIND_Q4_K, false>(maps, p, n_cta, dev, s);
+    case KIND_Q6_K: return p.loose ? ts_launch<KIND_Q6_K, true>(maps, p, n_cta, dev, s) : ts_launch<KIND_Q6_K, false>(maps, p, n_cta, dev, s);
+    default: return p.loose ? ts_launch<KIND_Q8_0, true>(maps, p, n_cta, dev, s) : ts_launch<KIND_Q8_0, false>(maps, p, n_cta, dev, s);
     }
 }
 
@@ -746,7 +745,8 @@ cudaError_t launch_gemm_ts(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     memset(&p, 0, sizeof(p));
     int F[TS_MAX_JOBS];
     for (int j = 0; j < n_jobs; ++j) F[j] = jobs[j].F;
-    const TsPlan pl = ts_plan(kind, T, K, F, n_jobs, device_sm_count());
+    int dev;
+    const TsPlan pl = ts_plan(kind, T, K, F, n_jobs, device_sm_count(&dev));
     if ((long)(pl.t_tiles - 1) * pl.bn >= T) return cudaErrorInvalidValue;  // a tile without tokens is no MMA
     p.nb = (K + block_values(kind) - 1) / block_values(kind);
     p.row_bytes = (long)p.nb * block_bytes(kind);
@@ -772,7 +772,7 @@ cudaError_t launch_gemm_ts(int kind, const GemvJobSpec *jobs, int n_jobs, const 
     if (cudaError_t e = ts_encode(&maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, ldxh, T, (cuuint64_t)ldxh * 2, 64, pl.bn,
                                   CU_TENSOR_MAP_SWIZZLE_128B))
         return e;
-    return ts_dispatch(kind, maps, p, pl.n_cta, s);
+    return ts_dispatch(kind, maps, p, pl.n_cta, dev, s);
 }
 
 bool gemm_ts_grouped_supported(int kind, const void *W, int K, int F) {
@@ -845,7 +845,9 @@ cudaError_t launch_gemm_ts_grouped(int kind, const GemvJobSpec *jobs, int n_jobs
     if (cudaError_t e = ts_encode(&maps.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, ldxh, total_rows, (cuuint64_t)ldxh * 2, 64,
                                   p.bn, CU_TENSOR_MAP_SWIZZLE_128B))
         return e;
-    return ts_dispatch(kind, maps, p, device_sm_count(), s);
+    int dev;
+    const int sms = device_sm_count(&dev);
+    return ts_dispatch(kind, maps, p, sms, dev, s);
 }
 
 }  // namespace mcu

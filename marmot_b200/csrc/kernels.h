@@ -144,7 +144,8 @@ cudaError_t launch_gemm_tma(int kind, const void *W, const __half *xh, const flo
 // Can launch_gemm_tma fuse the all-reduce for this shape (same answer on every rank: it depends on T and F only)?
 bool gemm_tma_can_fuse(int kind, int T, int F);
 
-int device_sm_count();
+// (device: its index, -1 where it cannot be had.  A launcher asks once: each question costs the host 20 to 40 ns of a call's 5 us.)
+int device_sm_count(int *device = nullptr);
 
 // Record the calling thread's error message (read back by mcu_last_error_message) and return `code`.
 int set_error(int code, const char *message);
